@@ -250,8 +250,6 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
       uint4 wq[2 * T2_SUB];
 #pragma unroll
       for (int c = 0; c < 2 * T2_SUB; c++) wq[c] = *(const uint4*)(rrow + ((c ^ (r & 7)) << 4));
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[T2_RAW_EMPTY + rs]);   // the box is in registers: refill it
 #pragma unroll
       for (int u = 0; u < T2_SUB; u++) {
         const int it = q * T2_SUB + u;
@@ -281,6 +279,11 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[T2_A_READY + s]);
       }
+      // The box goes back only here, behind the stores that used all of it.  Given back right after the
+      // loads above (which need not be complete, or even issued, before their first use) it was refilled under its readers:
+      // 60 of 60 products with M = 32, K = 3584, N = 18944 had wrong rows.
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[T2_RAW_EMPTY + rs]);
     }
   } else if (warp < 14) {
     // ---------------- accumulate (sc * group product) + epilogue ----------------
