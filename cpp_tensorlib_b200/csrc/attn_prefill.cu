@@ -10,8 +10,8 @@
 // row (q fragment, running max / sum / accumulator in registers), the four row
 // groups of a warp share each key row, K/V tiles of 32 keys arrive by bulk copy into
 // a two-stage ring.  f32 throughout (the parity bar is 1e-4 against a double CPU
-// reference).  This CUDA-core form serves bf16 caches; f32 caches take the tensor-core form in
-// attn_prefill_mma.cu.
+// reference).  This CUDA-core form is kept for A/B timing against the tensor-core forms: f32 caches
+// take attn_prefill_mma.cu, bf16 caches attn_prefill_bf16.cu.
 #include <cuda_bf16.h>
 
 #include <cstdlib>
@@ -62,15 +62,14 @@ constexpr int PF_THREADS = 256;
 constexpr int PF_QT = 32;   // queries per CTA (8 warps x 4 row groups)
 constexpr int PF_KT = 32;   // keys per tile
 
-// BF: bf16 cache (widened to f32 on load; q, out stay f32), same lane mapping as the decode kernel.
-template <int D, bool BF>
+// f32 cache, same lane mapping as the decode kernel.
+template <int D>
 __global__ void __launch_bounds__(PF_THREADS, 2)
-    attn_prefill_kernel(const float* __restrict__ q, const void* __restrict__ K,
-                        const void* __restrict__ V, float* __restrict__ out, int T,
+    attn_prefill_kernel(const float* __restrict__ q, const float* __restrict__ K,
+                        const float* __restrict__ V, float* __restrict__ out, int T,
                         long long kv_stride, int group, float scale, int pos0, int* status) {
   constexpr int CH = D / 32;
-  constexpr int ELT = BF ? 2 : 4;
-  constexpr int TILE_BYTES = PF_KT * D * ELT;
+  constexpr int TILE_BYTES = PF_KT * D * 4;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
   float* Kt = (float*)base;
@@ -96,17 +95,17 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
   int cta_last_key = pos0 + qt * PF_QT + PF_QT - 1;
   if (cta_last_key > pos0 + T - 1) cta_last_key = pos0 + T - 1;
   const int n_tiles = cta_last_key / PF_KT + 1;
-  const unsigned char* Kh = (const unsigned char*)K + (size_t)kh * kv_stride * ELT;
-  const unsigned char* Vh = (const unsigned char*)V + (size_t)kh * kv_stride * ELT;
+  const unsigned char* Kh = (const unsigned char*)K + (size_t)kh * kv_stride * 4;
+  const unsigned char* Vh = (const unsigned char*)V + (size_t)kh * kv_stride * 4;
 
   auto issue = [&](int i) {
     const int st = i & 1;
     const int r0 = i * PF_KT;
     const int rows = (cta_last_key + 1 - r0) < PF_KT ? (cta_last_key + 1 - r0) : PF_KT;
-    const uint32_t bytes = (uint32_t)rows * D * ELT;
+    const uint32_t bytes = (uint32_t)rows * D * 4;
     mbar_expect_tx(&bars[st], 2 * bytes);
-    bulk_load_1d((unsigned char*)Kt + (size_t)st * TILE_BYTES, Kh + (size_t)r0 * D * ELT, bytes, &bars[st]);
-    bulk_load_1d((unsigned char*)Vt + (size_t)st * TILE_BYTES, Vh + (size_t)r0 * D * ELT, bytes, &bars[st]);
+    bulk_load_1d((unsigned char*)Kt + (size_t)st * TILE_BYTES, Kh + (size_t)r0 * D * 4, bytes, &bars[st]);
+    bulk_load_1d((unsigned char*)Vt + (size_t)st * TILE_BYTES, Vh + (size_t)r0 * D * 4, bytes, &bars[st]);
   };
   if (tid == 0) {
     issue(0);
@@ -118,7 +117,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
     const float* qp = q + ((size_t)h * T + (row_ok ? row : 0)) * D;
 #pragma unroll
     for (int i = 0; i < CH; i++)
-      qf[i] = row_ok ? *(const float4*)(qp + attn_dim0<8, BF>(sub, i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      qf[i] = row_ok ? *(const float4*)(qp + attn_dim0<8, false>(sub, i)) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   float m = -INFINITY, l = 0.f;
   float4 acc[CH];
@@ -137,7 +136,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
     if (!dead) {
       for (int j = 0; j < jmax; j++) {
         float4 kv[CH];
-        attn_load_row<D, 8, CH, BF>(Ks + (size_t)j * D * ELT, sub, kv);
+        attn_load_row<D, 8, CH, false>(Ks + (size_t)j * D * 4, sub, kv);
         float d = 0.f;
 #pragma unroll
         for (int i = 0; i < CH; i++) {
@@ -150,7 +149,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
         d += __shfl_xor_sync(0xffffffffu, d, 2);
         d += __shfl_xor_sync(0xffffffffu, d, 4);
         const float s = d * scale;
-        attn_load_row<D, 8, CH, BF>(Vs + (size_t)j * D * ELT, sub, kv);
+        attn_load_row<D, 8, CH, false>(Vs + (size_t)j * D * 4, sub, kv);
         if (row_ok && k0 + j <= row_last_key) {
           if (s > m) {
             const float corr = __expf(m - s);
@@ -181,7 +180,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
     const float inv = 1.0f / l;
 #pragma unroll
     for (int i = 0; i < CH; i++)
-      *(float4*)(op + attn_dim0<8, BF>(sub, i)) =
+      *(float4*)(op + attn_dim0<8, false>(sub, i)) =
           make_float4(acc[i].x * inv, acc[i].y * inv, acc[i].z * inv, acc[i].w * inv);
   }
 }
@@ -207,40 +206,43 @@ int launch_kv_fill(void* Kc, void* Vc, const float* K, const float* V, int T, lo
   TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, kv_fill_kernel, Kc, Vc, K, V, T, kv_stride, pos0, D, bf));
   return TLB_OK;
 }
-template <int D, bool BF>
+template <int D>
 static int launch_attn_prefill_t(DeviceCtx* c, const float* q, const void* K, const void* V, float* out,
                                  int n_q, int n_kv, int T, long long kv_max, float scale, int pos0,
                                  cudaStream_t s) {
   const int group = n_q / n_kv;
   long long kv_stride = kv_max * D;
-  const size_t smem = 4 * (size_t)PF_KT * D * (BF ? 2 : 4) + 64 + 128;
+  const size_t smem = 4 * (size_t)PF_KT * D * 4 + 64 + 128;
   LaunchCfg lc(dim3((T + PF_QT - 1) / PF_QT, n_q), dim3(PF_THREADS), smem, s, pdl_enabled());
   static std::atomic<unsigned long long> attr_done{0};
   {
-    const int rc_attr = ensure_dynamic_smem(attn_prefill_kernel<D, BF>, 100 * 1024, attr_done);
+    const int rc_attr = ensure_dynamic_smem(attn_prefill_kernel<D>, 100 * 1024, attr_done);
     if (rc_attr) return rc_attr;
   }
-  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, attn_prefill_kernel<D, BF>, q, K, V, out, T, kv_stride, group, scale,
-                              pos0, c->status));
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, attn_prefill_kernel<D>, q, (const float*)K, (const float*)V, out, T, kv_stride,
+                              group, scale, pos0, c->status));
   return TLB_OK;
 }
-bool attn_prefill_mma_eligible(int D, int n_kv, long long kv_max, int bf);
+bool attn_prefill_mma_eligible(int D, int n_kv, long long kv_max);
 int attn_prefill_mma_launch(DeviceCtx* c, const float* q, const void* K, const void* V, float* out, int n_q,
                             int n_kv, int T, long long kv_max, int D, float scale, int pos0, cudaStream_t s);
+int attn_prefill_bf16_launch(DeviceCtx* c, const float* q, long long q_row, long long q_head, const void* K,
+                             const void* V, float* out, long long o_row, long long o_head, int n_q, int n_kv, int T,
+                             long long kv_max, int D, float scale, int pos0, cudaStream_t s);
 
 int launch_attn_prefill(DeviceCtx* c, const float* q, const void* K, const void* V, float* out,
                         int n_q, int n_kv, int T, long long kv_max, int D, float scale, int pos0,
                         int bf, cudaStream_t s) {
+  if (bf)
+    return attn_prefill_bf16_launch(c, q, D, (long long)T * D, K, V, out, D, (long long)T * D, n_q, n_kv, T, kv_max, D,
+                                    scale, pos0, s);
   // f32 caches: the tensor-core form (attn_prefill_mma.cu); TLB_PREFILL_MMA=0 keeps the CUDA-core
-  // form below (a diagnostic switch for A/B timing), which also serves bf16 caches
+  // form above (a diagnostic switch for A/B timing)
   static const bool mma_on = !(getenv("TLB_PREFILL_MMA") && atoi(getenv("TLB_PREFILL_MMA")) == 0);
-  if (mma_on && attn_prefill_mma_eligible(D, n_kv, kv_max, bf))
+  if (mma_on && attn_prefill_mma_eligible(D, n_kv, kv_max))
     return attn_prefill_mma_launch(c, q, K, V, out, n_q, n_kv, T, kv_max, D, scale, pos0, s);
-  if (D == 128)
-    return bf ? launch_attn_prefill_t<128, true>(c, q, K, V, out, n_q, n_kv, T, kv_max, scale, pos0, s)
-              : launch_attn_prefill_t<128, false>(c, q, K, V, out, n_q, n_kv, T, kv_max, scale, pos0, s);
-  return bf ? launch_attn_prefill_t<64, true>(c, q, K, V, out, n_q, n_kv, T, kv_max, scale, pos0, s)
-            : launch_attn_prefill_t<64, false>(c, q, K, V, out, n_q, n_kv, T, kv_max, scale, pos0, s);
+  return D == 128 ? launch_attn_prefill_t<128>(c, q, K, V, out, n_q, n_kv, T, kv_max, scale, pos0, s)
+                  : launch_attn_prefill_t<64>(c, q, K, V, out, n_q, n_kv, T, kv_max, scale, pos0, s);
 }
 
 }  // namespace tlb

@@ -338,8 +338,8 @@ int pm_launch(const PmParams& p, const void* K, const void* V, int n_q, cudaStre
 
 }  // namespace
 
-bool attn_prefill_mma_eligible(int D, int n_kv, long long kv_max, int bf) {
-  return !bf && (D == 64 || D == 128) && (long long)n_kv * kv_max < (1ll << 31);
+bool attn_prefill_mma_eligible(int D, int n_kv, long long kv_max) {
+  return (D == 64 || D == 128) && (long long)n_kv * kv_max < (1ll << 31);
 }
 
 int attn_prefill_mma_launch(DeviceCtx* c, const float* q, const void* K, const void* V, float* out, int n_q,

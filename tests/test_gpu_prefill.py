@@ -158,3 +158,24 @@ def test_kv_cache_bf16_prefill(tl, port):
     Kh[:, :T], Vh[:, :T] = bf16_round(k), bf16_round(v)
     assert cache.pos == T
     assert relerr(got, causal_reference(port, q, Kh, Vh, 0.125, 0)) < 1e-4
+
+
+@pytest.mark.parametrize("n_q,n_kv,D,T,pos0,kv_max", [
+    (2, 2, 64, 1, 0, 1),          # one key; every other row of the tile lies past the cache
+    (4, 2, 64, 63, 0, 63),        # one short of a tile
+    (14, 2, 64, 65, 63, 128),     # chunk that starts and ends off the tile edges, two query tiles
+    (3, 1, 128, 64, 64, 200),     # whole tiles
+    (28, 4, 128, 130, 77, 300),   # three query tiles, four key tiles
+    (2, 1, 128, 17, 400, 417),    # few queries behind many keys: the ring wraps
+])
+def test_attn_prefill_bf16_vs_oracle(tl, port, n_q, n_kv, D, T, pos0, kv_max):
+    """bf16 caches; rows behind the chunk hold NaN, which no result may see.  f32 sums of at most D and
+    pos0 + T terms: 1e-4 of (1 + |value|) as for f32 caches."""
+    seed = 60 + T
+    Kd, Vd = (dev(synth.normal(seed, i, (n_kv, kv_max, D))).to(torch.bfloat16) for i in (1, 2))
+    K, V = Kd.float().cpu().numpy(), Vd.float().cpu().numpy()
+    Kd[:, pos0 + T:], Vd[:, pos0 + T:] = float("nan"), float("nan")
+    q = synth.normal(seed, 3, (n_q, T, D))
+    scale = 1.0 / np.sqrt(D)
+    got = tl.attn_prefill(dev(q), Kd, Vd, scale, pos0=pos0).cpu().numpy()
+    assert relerr(got, causal_reference(port, q, K, V, scale, pos0)) < 1e-4
