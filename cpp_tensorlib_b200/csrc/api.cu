@@ -8,6 +8,7 @@
 #include "../../include/tlb200.h"
 #include "comm.cuh"
 #include "gemv_q4p.cuh"
+#include "q4_planes.cuh"
 
 namespace tlb {
 
@@ -26,8 +27,6 @@ bool gemm_q4_tc_eligible(const void* qw, const void* scales, int N, int K, int M
 int gemm_q4_tc_launch(DeviceCtx* c, const float* x, long long ldx, int M, const void* qw,
                       const float* scales, float* y, long long ldy, int N, int K, float alpha,
                       float beta, float* xsplit, cudaStream_t stream);
-bool gemm_q4_tc2_eligible(const void* qw, const void* scales, int N, int K, int M);
-size_t gemm_q4_tc2_scratch_bytes(int M, int K);
 int gemm_q4_tc2_launch(DeviceCtx* c, const float* x, long long ldx, int M, const void* qw, const float* scales,
                        float* y, long long ldy, int N, int K, float alpha, float beta, void* scratch,
                        cudaStream_t stream);
@@ -295,8 +294,7 @@ int tlb_gemm_q4(const float* x, int64_t M, int64_t ldx, const void* qw, const fl
   // Many rows: tensor-core path (tcgen05, TMEM accumulators).  Default: integer weights x two
   // fp16 activation planes, group scales applied outside the tensor core (gemm_q4_tc2.cu);
   // TLB_GEMM_TC=1 selects the earlier formulation with scaled tf32 hi/lo operands.
-  static const bool tc_old = getenv("TLB_GEMM_TC") && atoi(getenv("TLB_GEMM_TC")) == 1;
-  if (!tc_old && gemm_q4_tc2_eligible(qw, scales, (int)N, (int)K, (int)M)) {
+  if (gemm_q4_planes_eligible(qw, scales, (int)N, (int)K, (int)M)) {
     const size_t need = gemm_q4_tc2_scratch_bytes((int)M, (int)K);
     if (need > c->xsplit_bytes) {
       TLB_CUDA(cudaDeviceSynchronize());

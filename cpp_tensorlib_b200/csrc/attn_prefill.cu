@@ -224,8 +224,9 @@ static int launch_attn_prefill_t(DeviceCtx* c, const float* q, const void* K, co
   return TLB_OK;
 }
 bool attn_prefill_mma_eligible(int D, int n_kv, long long kv_max);
-int attn_prefill_mma_launch(DeviceCtx* c, const float* q, const void* K, const void* V, float* out, int n_q,
-                            int n_kv, int T, long long kv_max, int D, float scale, int pos0, cudaStream_t s);
+int attn_prefill_mma_launch(DeviceCtx* c, const float* q, long long q_row, long long q_head, const void* K,
+                            const void* V, float* out, long long o_row, long long o_head, int n_q, int n_kv, int T,
+                            long long kv_max, int D, float scale, int pos0, cudaStream_t s);
 int attn_prefill_bf16_launch(DeviceCtx* c, const float* q, long long q_row, long long q_head, const void* K,
                              const void* V, float* out, long long o_row, long long o_head, int n_q, int n_kv, int T,
                              long long kv_max, int D, float scale, int pos0, cudaStream_t s);
@@ -240,9 +241,20 @@ int launch_attn_prefill(DeviceCtx* c, const float* q, const void* K, const void*
   // form above (a diagnostic switch for A/B timing)
   static const bool mma_on = !(getenv("TLB_PREFILL_MMA") && atoi(getenv("TLB_PREFILL_MMA")) == 0);
   if (mma_on && attn_prefill_mma_eligible(D, n_kv, kv_max))
-    return attn_prefill_mma_launch(c, q, K, V, out, n_q, n_kv, T, kv_max, D, scale, pos0, s);
+    return attn_prefill_mma_launch(c, q, D, (long long)T * D, K, V, out, D, (long long)T * D, n_q, n_kv, T, kv_max, D,
+                                   scale, pos0, s);
   return D == 128 ? launch_attn_prefill_t<128>(c, q, K, V, out, n_q, n_kv, T, kv_max, scale, pos0, s)
                   : launch_attn_prefill_t<64>(c, q, K, V, out, n_q, n_kv, T, kv_max, scale, pos0, s);
+}
+
+// The same on token-major rows (the decoder's): q rows of ldq floats, out rows of n_q * D.
+int launch_attn_prefill_rows(DeviceCtx* c, const float* q, long long ldq, const void* K, const void* V, float* out,
+                             int n_q, int n_kv, int T, long long kv_max, int D, float scale, int pos0, int bf,
+                             cudaStream_t s) {
+  if (!bf && !attn_prefill_mma_eligible(D, n_kv, kv_max))
+    return set_error(TLB_ERR_UNSUPPORTED, "attn_prefill: a cache of 2^31 rows or more");
+  return (bf ? attn_prefill_bf16_launch : attn_prefill_mma_launch)(c, q, ldq, D, K, V, out, (long long)n_q * D, D, n_q,
+                                                                   n_kv, T, kv_max, D, scale, pos0, s);
 }
 
 }  // namespace tlb

@@ -1,7 +1,7 @@
 // Causal attention over a prompt chunk on the tensor pipe (f32 cache, D = 64 or 128): the
 // contract of cuda::attn_prefill / tl_attn_prefill_tiled_* of the reference
-// (include/cuda.h:1171-1201, kernels/tensorlib_cuda.cu:1211-1350) -- q, out [n_q, T, D]; K, V a
-// [n_kv, kv_max, D] cache; query p sits at absolute position pos0 + p and attends keys
+// (include/cuda.h:1171-1201, kernels/tensorlib_cuda.cu:1211-1350) -- q, out f32 rows with strides of their own;
+// K, V a [n_kv, kv_max, D] cache; query p sits at absolute position pos0 + p and attends keys
 // 0..pos0+p -- as a dense contraction instead of per-row CUDA-core dot products.
 //
 //  * grid = (query tiles of 64, q heads).  Four compute warps own 16 query rows each; a producer
@@ -73,6 +73,7 @@ __device__ __forceinline__ float pm_ex2(float x) {
 struct PmParams {
   const float* q;
   float* out;
+  long long q_row, q_head, o_row, o_head;   // strides in floats
   int T, n_kv, group, kv_rows, pos0;
   float scale;
   int* status;
@@ -139,8 +140,8 @@ __global__ void __launch_bounds__(32 * (PM_WARPS + 1), 1)
   {
     const float qs = p.scale * 1.4426950408889634f;
     const bool r0ok = qrow + g < p.T, r1ok = qrow + g + 8 < p.T;
-    const float* qa = p.q + ((size_t)h * p.T + (r0ok ? qrow + g : 0)) * D;
-    const float* qb = p.q + ((size_t)h * p.T + (r1ok ? qrow + g + 8 : 0)) * D;
+    const float* qa = p.q + h * p.q_head + (r0ok ? qrow + g : 0) * p.q_row;
+    const float* qb = p.q + h * p.q_head + (r1ok ? qrow + g + 8 : 0) * p.q_row;
     uint4* mine = Qf + (size_t)warp * KSTEPS * 64 + lane * 2;
 #pragma unroll 4
     for (int ks = 0; ks < KSTEPS; ks++) {
@@ -305,8 +306,8 @@ __global__ void __launch_bounds__(32 * (PM_WARPS + 1), 1)
     // accumulator columns 2t, 2t + 1 of tile (seg, c): dimensions d, d + 1 with
     // d = 32 seg + 16 ((2t) >> 2) + 4 c + ((2t) & 3)
     const int d = 32 * (j >> 2) + 16 * ((2 * t) >> 2) + 4 * (j & 3) + ((2 * t) & 3);
-    if (ra < p.T) *(float2*)(p.out + ((size_t)h * p.T + ra) * D + d) = make_float2(acc[j][0] * i0, acc[j][1] * i0);
-    if (rb < p.T) *(float2*)(p.out + ((size_t)h * p.T + rb) * D + d) = make_float2(acc[j][2] * i1, acc[j][3] * i1);
+    if (ra < p.T) *(float2*)(p.out + h * p.o_head + ra * p.o_row + d) = make_float2(acc[j][0] * i0, acc[j][1] * i0);
+    if (rb < p.T) *(float2*)(p.out + h * p.o_head + rb * p.o_row + d) = make_float2(acc[j][2] * i1, acc[j][3] * i1);
   }
 }
 
@@ -342,10 +343,12 @@ bool attn_prefill_mma_eligible(int D, int n_kv, long long kv_max) {
   return (D == 64 || D == 128) && (long long)n_kv * kv_max < (1ll << 31);
 }
 
-int attn_prefill_mma_launch(DeviceCtx* c, const float* q, const void* K, const void* V, float* out, int n_q,
-                            int n_kv, int T, long long kv_max, int D, float scale, int pos0, cudaStream_t s) {
+int attn_prefill_mma_launch(DeviceCtx* c, const float* q, long long q_row, long long q_head, const void* K,
+                            const void* V, float* out, long long o_row, long long o_head, int n_q, int n_kv, int T,
+                            long long kv_max, int D, float scale, int pos0, cudaStream_t s) {
   PmParams p;
-  p.q = q; p.out = out; p.T = T; p.n_kv = n_kv; p.group = n_q / n_kv; p.kv_rows = (int)kv_max; p.pos0 = pos0;
+  p.q = q; p.q_row = q_row; p.q_head = q_head;
+  p.out = out; p.o_row = o_row; p.o_head = o_head; p.T = T; p.n_kv = n_kv; p.group = n_q / n_kv; p.kv_rows = (int)kv_max; p.pos0 = pos0;
   p.scale = scale; p.status = c->status;
   if (D == 128) return pm_launch<128>(p, K, V, n_q, s);
   return pm_launch<64>(p, K, V, n_q, s);

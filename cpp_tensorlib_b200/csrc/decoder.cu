@@ -23,6 +23,7 @@
 #include "comm.cuh"
 #include "decoder_base.cuh"
 #include "gemv_q4p.cuh"
+#include "q4_planes.cuh"
 
 namespace tlb {
 
@@ -46,15 +47,13 @@ int attn_decode_launch(DeviceCtx* c, const float* q, const void* K, const void* 
                        int early_kv, int kv_bf16, const GvStream* prefetch = nullptr);
 int launch_rmsnorm(const float*, const float*, float*, int, float, int, cudaStream_t);
 int launch_embed_rows(const float*, const int*, float*, int, int, cudaStream_t);
-int launch_rope(const float*, const float*, float*, int, int, int, unsigned, const unsigned*, float,
-                cudaStream_t);
-int launch_split_heads(const float*, const float*, float*, int, long long, long long, int, int,
-                       cudaStream_t);
-int launch_merge_heads(const float*, float*, int, int, int, cudaStream_t);
-int launch_kv_fill(void*, void*, const float*, const float*, int, long long, int, int, int, int,
-                   cudaStream_t);
-int launch_attn_prefill(DeviceCtx*, const float*, const void*, const void*, float*, int, int, int,
-                        long long, int, float, int, int, cudaStream_t);
+bool prompt_rows_eligible(int n);
+int launch_norm_split(const float*, const float*, const float*, float*, int, float, int, const Q4Planes&, cudaStream_t);
+int launch_swiglu_planes(const float*, int, int, const Q4Planes&, cudaStream_t);
+int launch_qkv_rows(float*, const float*, const float*, const float*, void*, void*, int, int, int, int, int, long long,
+                    float, int, cudaStream_t);
+int launch_attn_prefill_rows(DeviceCtx*, const float*, long long, const void*, const void*, float*, int, int, int,
+                             long long, int, float, int, int, cudaStream_t);
 int launch_add_rmsnorm(const float*, const float*, const float*, float*, float*, int, float, int,
                        cudaStream_t);
 int launch_add_rmsnorm_ar(const float*, const float*, float*, float*, int, float, const CommDev&,
@@ -112,8 +111,9 @@ struct Decoder : DecoderBase {
   // batched prompt pass: row-batched scratch, carved from one allocation of pf_rows rows
   float* pf = nullptr;
   int pf_rows = 0;
-  float *pf_res[2] = {}, *pf_h = nullptr, *pf_h2 = nullptr, *pf_md = nullptr, *pf_qkv = nullptr, *pf_qkvh = nullptr,
-        *pf_ah = nullptr, *pf_at = nullptr, *pf_gu = nullptr, *pf_mb = nullptr;
+  float *pf_res[2] = {}, *pf_h = nullptr, *pf_h2 = nullptr, *pf_md = nullptr, *pf_qkv = nullptr, *pf_at = nullptr,
+        *pf_gu = nullptr, *pf_mb = nullptr;
+  void* pf_planes = nullptr;   // activations of one product as fp16 planes; shares pf_mb's memory
 
   ~Decoder() override;
   int forward(cudaStream_t s) override;
@@ -431,7 +431,10 @@ int Decoder::prefill_begin(int rows, cudaStream_t s) {
   if (pf && pf_rows >= rows) return TLB_OK;
   const int E = hidden, D = hd, QKV = (n_q + 2 * n_kv) * D;
   const size_t CH = rows, n_emb = CH * E, n_qkv = CH * QKV, n_att = CH * n_q * D, n_gu = CH * 2 * ff, n_mb = CH * ff;
-  const size_t total = 5 * n_emb /* res0 res1 h h2 md */ + 2 * n_qkv + 2 * n_att + n_gu + n_mb;
+  // the planes of a product's rows, or the rows in f32 where the product takes those
+  const int wide = ff > E ? ff : E;
+  const size_t n_pl = (gemm_q4_tc2_scratch_bytes(rows, wide) + 3) / 4, n_act = n_mb > n_pl ? n_mb : n_pl;
+  const size_t total = 5 * n_emb /* res0 res1 h h2 md */ + n_qkv + n_att + n_gu + n_act + 64;
   if (pf) {
     TLB_CUDA(cudaStreamSynchronize(s));
     TLB_CUDA(cudaFree(pf));
@@ -443,9 +446,12 @@ int Decoder::prefill_begin(int rows, cudaStream_t s) {
   auto take = [&](size_t n) { float* r = p; p += n; return r; };
   pf_res[0] = take(n_emb); pf_res[1] = take(n_emb);
   pf_h = take(n_emb); pf_h2 = take(n_emb); pf_md = take(n_emb);
-  pf_qkv = take(n_qkv); pf_qkvh = take(n_qkv);
-  pf_ah = take(n_att); pf_at = take(n_att);
-  pf_gu = take(n_gu); pf_mb = take(n_mb);
+  pf_qkv = take(n_qkv);
+  pf_at = take(n_att);
+  pf_gu = take(n_gu);
+  p = (float*)(((uintptr_t)p + 255) & ~(uintptr_t)255);
+  pf_mb = take(n_act);
+  pf_planes = pf_mb;
   return TLB_OK;
 }
 
@@ -455,40 +461,51 @@ int Decoder::prefill_pass(const int* d_ids, int rows, int pos, cudaStream_t s) {
   if (rc) return rc;
   const int E = hidden, D = hd, NQ = n_q, NKV = n_kv, FF = ff;
   const int QKV = (NQ + 2 * NKV) * D;
-  float *hrow = pf_h, *h2 = pf_h2, *md = pf_md, *qkv = pf_qkv, *qkvh = pf_qkvh, *ah = pf_ah, *at = pf_at, *gu = pf_gu,
-        *mb = pf_mb;
+  float *hrow = pf_h, *h2 = pf_h2, *md = pf_md, *qkv = pf_qkv, *at = pf_at, *gu = pf_gu, *mb = pf_mb;
   auto gemm = [&](const Linear& L, const float* x, float* y, int rows) -> int {
     if (!L.q4) return set_error(TLB_ERR_STATE, "decoder: a linear weight was never set");
     return tlb_gemm_q4(x, rows, L.K, L.q4, L.scales(), y, L.N, L.N, L.K, 1.0f, 0.0f, s);
   };
+  // Whether the row operation in front of this product leaves its rows as the planes the product reads: no
+  // other writing and reading of the rows.  Few rows and odd widths take other products, which read f32.
+  auto planes = [&](const Linear& L) {
+    return L.q4 && prompt_rows_eligible(L.K) && gemm_q4_planes_eligible(L.q4, L.scales(), L.N, L.K, rows);
+  };
+  auto gemm_planes = [&](const Linear& L, float* y) {
+    return gemm_q4_planes_launch(c, q4_planes_at(pf_planes, rows, L.K), rows, L.q4, L.scales(), y, L.N, L.N, L.K, 1.0f,
+                                 0.0f, s);
+  };
 #define PF(expr) do { rc = (expr); if (rc) return rc; } while (0)
+  // y = norm(x + b) * w through L; xsum the residual (b NULL: x itself), h f32 rows for products that read those
+  auto norm_gemm = [&](const float* x, const float* b, const float* w, float* xsum, float* h, const Linear& L,
+                       float* y) -> int {
+    if (planes(L)) {
+      PF(launch_norm_split(x, b, w, xsum, E, eps, rows, q4_planes_at(pf_planes, rows, E), s));
+      return gemm_planes(L, y);
+    }
+    if (b) PF(launch_add_rmsnorm(x, b, w, xsum, h, E, eps, rows, s));
+    else PF(launch_rmsnorm(x, w, h, E, eps, rows, s));
+    return gemm(L, h, y, rows);
+  };
   float* x = pf_res[1];   // the chunk's embeddings; layer l writes its residual into pf_res[l & 1]
   PF(launch_embed_rows(embed, d_ids, x, E, rows, s));
-  PF(launch_rmsnorm(x, layers[0].an, hrow, E, eps, rows, s));
+  PF(norm_gemm(x, nullptr, layers[0].an, nullptr, hrow, layers[0].wqkv, qkv));
   for (int l = 0; l < n_layers; l++) {
     DecLayer& L = layers[l];
     float* ro = pf_res[l & 1];
-    PF(gemm(L.wqkv, hrow, qkv, rows));
-    // token-major [rows, q|k|v] -> head-major [n_q + 2 n_kv, rows, D], biases riding along
-    float* kh = qkvh + (size_t)NQ * rows * D;
-    float* vh = qkvh + (size_t)(NQ + NKV) * rows * D;
-    PF(launch_split_heads(qkv, L.bq, qkvh, rows, QKV, 0, NQ, D, s));
-    PF(launch_split_heads(qkv, L.bk, kh, rows, QKV, (long long)NQ * D, NKV, D, s));
-    PF(launch_split_heads(qkv, L.bv, vh, rows, QKV, (long long)(NQ + NKV) * D, NKV, D, s));
-    // [H, rows, D] flattened: row r = h*rows + t, so rope's position is pos + r % rows
-    PF(launch_rope(qkvh, nullptr, qkvh, NQ * rows, rows, D, (unsigned)pos, nullptr, rope_base, s));
-    PF(launch_rope(kh, nullptr, kh, NKV * rows, rows, D, (unsigned)pos, nullptr, rope_base, s));
-    PF(launch_kv_fill(L.Kc, L.Vc, kh, vh, rows, max_ctx, NKV, D, pos, kv_bf16, s));
-    PF(launch_attn_prefill(c, qkvh, L.Kc, L.Vc, ah, NQ, NKV, rows, max_ctx, D, scale, pos,
-                           kv_bf16, s));
-    PF(launch_merge_heads(ah, at, rows, NQ, D, s));
+    PF(launch_qkv_rows(qkv, L.bq, L.bk, L.bv, L.Kc, L.Vc, rows, NQ, NKV, D, pos, max_ctx, rope_base, kv_bf16, s));
+    PF(launch_attn_prefill_rows(c, qkv, QKV, L.Kc, L.Vc, at, NQ, NKV, rows, max_ctx, D, scale, pos, kv_bf16, s));
     PF(gemm(L.wo, at, md, rows));
-    PF(launch_add_rmsnorm(x, md, L.fn, ro, h2, E, eps, rows, s));
-    PF(gemm(L.wgu, h2, gu, rows));
-    PF(launch_swiglu(gu, mb, FF, rows, s));
-    PF(gemm(L.wd, mb, md, rows));
-    const float* nextw = (l + 1 < n_layers) ? layers[l + 1].an : onorm;
-    PF(launch_add_rmsnorm(ro, md, nextw, ro, hrow, E, eps, rows, s));
+    PF(norm_gemm(x, md, L.fn, ro, h2, L.wgu, gu));
+    if (planes(L.wd)) {
+      PF(launch_swiglu_planes(gu, FF, rows, q4_planes_at(pf_planes, rows, FF), s));
+      PF(gemm_planes(L.wd, md));
+    } else {
+      PF(launch_swiglu(gu, mb, FF, rows, s));
+      PF(gemm(L.wd, mb, md, rows));
+    }
+    if (l + 1 < n_layers) PF(norm_gemm(ro, md, layers[l + 1].an, ro, hrow, layers[l + 1].wqkv, qkv));
+    else PF(launch_add_rmsnorm(ro, md, onorm, ro, hrow, E, eps, rows, s));   // every row's: the head may want any
     x = ro;
   }
 #undef PF

@@ -27,9 +27,9 @@
 // 16 KB per SM in flight and paced the whole kernel at ~1 TB/s of weight bytes.)  All waits
 // are bounded; a timeout sets the status word, the kernel still frees its TMEM and returns.
 // No cluster launch, no multicast.
-#include <cuda_fp16.h>
+#include <cstdlib>
 
-#include "common.cuh"
+#include "q4_planes.cuh"
 
 namespace tlb {
 
@@ -374,13 +374,7 @@ __global__ void split_f16_kernel(const float* __restrict__ x, long long ldx, int
   __syncthreads();
   mx = 0.f;
   for (int w = 0; w < (int)(blockDim.x >> 5); w++) mx = fmaxf(mx, sm[w]);
-  int e = 0;
-  if (mx > 0.f && mx < 3.0e38f) {
-    int ex;
-    frexpf(mx, &ex);            // mx = f * 2^ex, f in [0.5, 1)
-    e = ex - 14;                // the scaled row stays below 2^14
-    e = e < -100 ? -100 : (e > 100 ? 100 : e);
-  }
+  const int e = q4_row_exponent(mx);
   const float s = ldexpf(1.0f, -e);
   if (threadIdx.x == 0) rowscale[m] = ldexpf(1.0f, e);
   if (vec) {
@@ -389,17 +383,10 @@ __global__ void split_f16_kernel(const float* __restrict__ x, long long ldx, int
     uint4* o2 = (uint4*)(x2 + (size_t)m * K);
     for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
       const float4 a = __ldg(row4 + 2 * i), b = __ldg(row4 + 2 * i + 1);
-      const float f[8] = {a.x * s, b.x * s, a.y * s, b.y * s, a.z * s, b.z * s, a.w * s, b.w * s};   // k 0,4,1,5,2,6,3,7
-      unsigned w1[4], w2[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const __half ha = __float2half_rn(f[2 * j]), hb = __float2half_rn(f[2 * j + 1]);
-        const __half la = __float2half_rn(f[2 * j] - __half2float(ha)), lb = __float2half_rn(f[2 * j + 1] - __half2float(hb));
-        w1[j] = (unsigned)__half_as_ushort(ha) | ((unsigned)__half_as_ushort(hb) << 16);
-        w2[j] = (unsigned)__half_as_ushort(la) | ((unsigned)__half_as_ushort(lb) << 16);
-      }
-      o1[i] = make_uint4(w1[0], w1[1], w1[2], w1[3]);
-      o2[i] = make_uint4(w2[0], w2[1], w2[2], w2[3]);
+      uint4 w1, w2;
+      q4_split8(a, b, s, w1, w2);
+      o1[i] = w1;
+      o2[i] = w2;
     }
     return;
   }
@@ -439,28 +426,35 @@ bool gemm_q4_tc2_eligible(const void* qw, const void* scales, int N, int K, int 
   return (((uintptr_t)qw & 15) == 0) && (((uintptr_t)scales & 15) == 0);
 }
 
+bool gemm_q4_planes_eligible(const void* qw, const void* scales, int N, int K, int M) {
+  // TLB_GEMM_TC=1 selects the earlier formulation (gemm_q4_tc.cu)
+  static const bool tc_old = getenv("TLB_GEMM_TC") && atoi(getenv("TLB_GEMM_TC")) == 1;
+  return !tc_old && gemm_q4_tc2_eligible(qw, scales, N, K, M);
+}
+
 int gemm_q4_tc2_launch(DeviceCtx* c, const float* x, long long ldx, int M, const void* qw, const float* scales,
                        float* y, long long ldy, int N, int K, float alpha, float beta, void* scratch,
                        cudaStream_t stream) {
+  const Q4Planes pl = q4_planes_at(scratch, M, K);
+  LaunchCfg lc(dim3((unsigned)M), dim3(256), 0, stream, pdl_enabled());
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, split_f16_kernel, x, ldx, K, pl.hi, pl.lo, pl.rowscale));
+  return gemm_q4_planes_launch(c, pl, M, qw, scales, y, ldy, N, K, alpha, beta, stream);
+}
+
+int gemm_q4_planes_launch(DeviceCtx* c, const Q4Planes& x, int M, const void* qw, const float* scales, float* y,
+                          long long ldy, int N, int K, float alpha, float beta, cudaStream_t stream) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return set_error(TLB_ERR_CUDA, "cuTensorMapEncodeTiled entry point not found");
-  __half* x1 = (__half*)scratch;
-  __half* x2 = x1 + (size_t)M * K;
-  float* rowscale = (float*)(((uintptr_t)(x2 + (size_t)M * K) + 255) & ~(uintptr_t)255);
-  {
-    LaunchCfg lc(dim3((unsigned)M), dim3(256), 0, stream, pdl_enabled());
-    TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, split_f16_kernel, x, ldx, K, x1, x2, rowscale));
-  }
   const int MT = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
   CUtensorMap tm1, tm2;
   cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)M};
   cuuint64_t str[1] = {(cuuint64_t)K * 2};
   cuuint32_t box[2] = {(cuuint32_t)T2_KS, (cuuint32_t)MT};
   cuuint32_t es[2] = {1, 1};
-  if (enc(&tm1, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x1, dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  if (enc(&tm1, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x.hi, dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
           CUDA_SUCCESS ||
-      enc(&tm2, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x2, dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+      enc(&tm2, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x.lo, dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
           CUDA_SUCCESS)
     return set_error(TLB_ERR_CUDA, "gemm_q4_tc2: tensor map (activation planes) encode failed");
@@ -474,7 +468,7 @@ int gemm_q4_tc2_launch(DeviceCtx* c, const float* x, long long ldx, int M, const
           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return set_error(TLB_ERR_CUDA, "gemm_q4_tc2: tensor map (packed weights) encode failed");
   T2Params p;
-  p.qw = (const unsigned*)qw; p.scales = scales; p.rowscale = rowscale; p.y = y; p.ldy = ldy;
+  p.qw = (const unsigned*)qw; p.scales = scales; p.rowscale = x.rowscale; p.y = y; p.ldy = ldy;
   p.M = M; p.N = N; p.K = K; p.alpha = alpha; p.beta = beta; p.status = c->status;
   if (MT == 32) return t2_launch<32>(tm1, tm2, tmw, p, stream);
   if (MT == 64) return t2_launch<64>(tm1, tm2, tmw, p, stream);

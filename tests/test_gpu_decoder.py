@@ -373,3 +373,56 @@ def test_decoder_with_bf16_kv_cache(port, cfg, seed):
     K2, _ = d2.kv(0)
     assert np.allclose(K2[:, :11].float().cpu().numpy(), K[:, :11].float().cpu().numpy(), rtol=1e-2, atol=1e-2)
     d.close(); d2.close(); o.close()
+
+
+@pytest.mark.parametrize("hidden,ff,n_q,n_kv,hd,kv", [
+    (256, 640, 4, 2, 64, "f32"),       # every product takes planes
+    (256, 640, 2, 1, 128, "bf16"),
+    (192, 320, 3, 1, 64, "bf16"),      # widths the planes do not serve: f32 rows between the products
+])
+@pytest.mark.parametrize("T", [9, 33, 130])
+def test_prompt_rows_match_the_ops(hidden, ff, n_q, n_kv, hd, kv, T):
+    """The prompt pass against the same layer built from the single operations, at a position that is not 0.
+    Both compute in f32 with sums in different orders.  Two f32 products of such depths differ by up to 4e-6 of
+    their size (2-norm); five in a row and the attention's 2e-6 make 9e-6, and the largest of 500 such normally
+    distributed differences is about 4.5 of them: 4e-5."""
+    from cpp_tensorlib_b200 import cuda as tl
+    from cpp_tensorlib_b200.decoder import Q4Decoder
+    g = torch.Generator(device="cuda").manual_seed(T + hidden)
+    rnd = lambda *s, std=1.0: torch.randn(s, generator=g, device="cuda") * std
+    V, pos, eps, base = 500, 7, 1e-6, 1e6
+    qkv, nq, nk = (n_q + 2 * n_kv) * hd, n_q * hd, n_kv * hd
+    cfg = dict(hidden=hidden, layers=1, n_q=n_q, n_kv=n_kv, hd=hd, ff=ff, vocab=V, eps=eps, rope_base=base)
+    d = Q4Decoder(cfg, pos + T + 3, kv_dtype=kv)
+    W = dict(wqkv=rnd(hidden, qkv, std=.06), wo=rnd(nq, hidden, std=.06), wgu=rnd(hidden, 2 * ff, std=.06), wd=rnd(ff, hidden, std=.06))
+    vec = dict(an=rnd(hidden), fn=rnd(hidden), bq=rnd(nq), bk=rnd(nk), bv=rnd(nk))
+    embed, onorm, head = rnd(V, hidden), rnd(hidden), rnd(hidden, V, std=.06)
+    d.set_vector_full(0, "embed", embed)
+    d.set_vector_full(0, "onorm", onorm)
+    d.set_linear_full(0, "lm_head", head)
+    for n, w in W.items():
+        d.set_linear_full(0, n, w)
+    for n, v in vec.items():
+        d.set_vector_full(0, n, v)
+    kc, vc = rnd(n_kv, pos, hd), rnd(n_kv, pos, hd)
+    d.fill_kv(0, kc, vc)
+    ids = [(37 * i + 5) % V for i in range(T)]
+    d.set_pos(pos)
+    d.prefill(ids)
+    got = d.logits()
+
+    q4 = {n: tl.to_q4(w) for n, w in W.items()}
+    x = embed[torch.tensor(ids, device="cuda")]
+    y = tl.gemm_q4(tl.rmsnorm(x, vec["an"], eps), q4["wqkv"])
+    q = tl.split_heads(y, vec["bq"], T, qkv, 0, n_q, hd)
+    k = tl.split_heads(y, vec["bk"], T, qkv, nq, n_kv, hd)
+    v = tl.split_heads(y, vec["bv"], T, qkv, nq + nk, n_kv, hd)
+    rope = lambda a: tl.rope(a, pos, base=base)
+    cache = tl.kv_cache(n_kv, pos + T + 3, hd, dtype=torch.bfloat16 if kv == "bf16" else torch.float32)
+    cache.fill(kc, vc)
+    o = tl.merge_heads(cache.prefill(rope(q), rope(k), v, hd ** -0.5))
+    x, h = tl.rmsnorm_res(x, tl.gemm_q4(o, q4["wo"]), vec["fn"], eps)
+    x = x + tl.gemm_q4(tl.swiglu(tl.gemm_q4(h, q4["wgu"]), ff), q4["wd"])
+    want = tl.gemm_q4(tl.rmsnorm(x[-1:].contiguous(), onorm, eps), tl.to_q4(head))[0]
+    got = torch.as_tensor(got).to(want.device).reshape(-1)
+    assert ((got - want).abs().max() / want.std()).item() < 4e-5
