@@ -437,8 +437,8 @@ static int launch_t(const AttnParams& p, int splits, cudaStream_t stream, bool b
   return launch_b<D, HW, LPK, false>(p, splits, stream);
 }
 
-bool attn_decode_mma_eligible(int grp, int D, int n_kv, long long kv_max, int kv_bf16);
-int attn_decode_mma_launch(const AttnParams& p, int D, int splits, cudaStream_t stream);
+bool attn_decode_mma_eligible(int grp, int D, int n_kv, long long kv_max);
+int attn_decode_mma_launch(const AttnParams& p, int D, int bf, int splits, cudaStream_t stream);
 
 // ctx >= 1 and d_pos == nullptr: host-position variant.  d_pos != nullptr: the
 // context is *d_pos + 1 and the grid is sized from kv_max.
@@ -463,11 +463,11 @@ int attn_decode_launch(DeviceCtx* c, const float* q, const void* K, const void* 
   const int splits = d_pos ? attn_splits_wanted(n_kv, basis, p.sm2)
                            : (ctx + attn_chunk(n_kv, ctx, p.sm2) - 1) / attn_chunk(n_kv, ctx, p.sm2);
   p.s_cap = d_pos ? splits : attn_splits_wanted(n_kv, basis, p.sm2);
-  // GQA groups of 3..8 heads on an f32 cache: the tensor-core form (attn_decode_mma.cu).
+  // GQA groups of 3..8 heads: the tensor-core form (attn_decode_mma.cu).
   // TLB_ATTN_MMA=0 keeps the CUDA-core form (a diagnostic switch for A/B timing).
   static const bool mma_on = !(getenv("TLB_ATTN_MMA") && atoi(getenv("TLB_ATTN_MMA")) == 0);
-  if (mma_on && attn_decode_mma_eligible(grp, D, n_kv, kv_max, kv_bf16))
-    return attn_decode_mma_launch(p, D, splits, stream);
+  if (mma_on && attn_decode_mma_eligible(grp, D, n_kv, kv_max))
+    return attn_decode_mma_launch(p, D, kv_bf16, splits, stream);
   // heads per warp: the smallest of {1,2,4} such that ceil(grp/HW) divides 8
   int HW = grp == 1 ? 1 : (grp == 2 ? 2 : 4);
   if (D == 128) {

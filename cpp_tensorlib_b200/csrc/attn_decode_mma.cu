@@ -1,4 +1,4 @@
-// Decode attention for GQA groups on the tensor pipe (f32 cache, 3..8 query heads per KV
+// Decode attention for GQA groups on the tensor pipe (f32 or bf16 cache, 3..8 query heads per KV
 // head, D = 64 or 128): the same contract as attn_decode.cu -- out[h,:] =
 // softmax(scale * q[h] . K[kv(h)]^T) . V[kv(h)] over the cache prefix [0, ctx), cuda::attn_decode
 // / attn_decode_dpos of the reference (include/cuda.h:966-1114, kernels
@@ -20,6 +20,9 @@
 //    accumulator layout (a lane holds heads 2t, 2t+1 of keys g, g+8), exp2 with log2(e)
 //    folded into the query.  P goes through 512 bytes of per-warp shared memory to become the
 //    B operand of out^T[D x 8 heads] += V_blk^T . P, again three tf32 MMAs per step.
+//  * A bf16 cache is an exact operand of mma.sync m16n8k16 (boxes of 32 rows x 64 bf16, ldmatrix):
+//    Q and P enter as three bf16 planes each, 24 bits and nothing dropped, again three MMAs per
+//    step, of twice the depth.
 //  * The warps' (acc, m, l) meet in shared memory, the CTA's partial goes to scratch, an
 //    acq_rel ticket per KV head elects the last CTA, which folds the splits in split order
 //    with every load of the fold in flight at once (one L2 round trip).  One launch,
@@ -29,31 +32,33 @@
 #include <string>
 
 #include "attn_split.cuh"
+#include "rows_mma.cuh"
 
 namespace tlb {
 
 namespace {
 
 constexpr int MM_TK = AT_TK;          // keys per TMA tile
-constexpr int MM_BOX_BYTES = 32 * 128;  // one box: 32 rows x 32 floats
+constexpr int MM_BOX_BYTES = 32 * 128;  // one box: 32 rows x 32 floats or 64 bf16
 
-template <int D>
+template <int D, bool BF>
 struct MmaCfg {
   static constexpr int WARPS = D / 16;              // compute warps; + 1 producer warp
   static constexpr int THREADS = 32 * (WARPS + 1);
-  static constexpr int SEGS = D / 32;               // boxes per K (or V) tile
+  static constexpr int SEGS = D / (BF ? 64 : 32);   // boxes per K (or V) tile
   static constexpr int TILE_BYTES = 2 * SEGS * MM_BOX_BYTES;   // K part then V part
   // Ring slots: a multiple of the number of warp pairs (WARPS / 2), so that slot s is always
   // consumed by the same pair.  A pair then never waits for phase k of a slot before it has
   // itself seen phase k - 1 complete, which is what makes a parity wait unambiguous (with a
   // slot shared between pairs, a pair arriving early would read the previous phase's parity
   // as "done").
-  static constexpr int STAGES = D == 128 ? 4 : 6;
+  static constexpr int STAGES = BF ? 8 : (D == 128 ? 4 : 6);
   static_assert(STAGES % (WARPS / 2) == 0, "a ring slot must belong to one warp pair");
-  static constexpr int KSTEPS = D / 8;
+  static constexpr int KSTEPS = D / (BF ? 16 : 8);
+  static constexpr int NT = D / 16;                 // output tiles of 16 dimensions
   // shared memory: ring | Q fragments | per-warp P | per-warp merge entries | barriers
   static constexpr size_t RING = (size_t)STAGES * TILE_BYTES;
-  static constexpr size_t QF = (size_t)KSTEPS * 32 * 16;
+  static constexpr size_t QF = (size_t)KSTEPS * 32 * (BF ? 24 : 16);
   static constexpr size_t PS = (size_t)WARPS * 16 * 8 * 4;
   static constexpr size_t ENT = (size_t)WARPS * (D * 8 + 16) * 4;
   static constexpr size_t BARS = 2 * STAGES * 8;
@@ -90,12 +95,27 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-template <int D>
-__global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
+// two f32 values as three bf16 planes (the first in the low half)
+__device__ __forceinline__ void split3_bf16(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  hi = *(const uint32_t*)&h;
+  rc_split(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u), mid, lo);
+}
+__device__ __forceinline__ void ldm_x4(uint32_t (&r)[4], uint32_t a) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ldm_x4_trans(uint32_t (&r)[4], uint32_t a) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+
+template <int D, bool BF>
+__global__ void __launch_bounds__(MmaCfg<D, BF>::THREADS, 1)
     attn_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                            AttnParams p) {
-  using C = MmaCfg<D>;
-  constexpr int W = C::WARPS, SEGS = C::SEGS, STAGES = C::STAGES, KSTEPS = C::KSTEPS;
+  using C = MmaCfg<D, BF>;
+  constexpr int W = C::WARPS, SEGS = C::SEGS, STAGES = C::STAGES, KSTEPS = C::KSTEPS, NT = C::NT;
   extern __shared__ unsigned char smem_raw[];
   // the swizzle of a TMA box follows the SHARED-space address: align that one to 1024 bytes
   unsigned char* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -143,7 +163,7 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
   // A long context is read once per token and is far larger than the L2 over the layers of a
   // model: mark it evict-first, so that the small things every launch re-reads (biases, norm
   // weights, activations, scratch) stay.  A short one may survive to the next token: leave it.
-  const uint64_t pol = (size_t)p.n_kv * ctx * D * 8 >= ((size_t)8 << 20) ? l2_evict_first_policy()
+  const uint64_t pol = (size_t)p.n_kv * ctx * D * (BF ? 4 : 8) >= ((size_t)8 << 20) ? l2_evict_first_policy()
                                                                           : l2_evict_normal_policy();
   auto issue = [&](int i) {
     const int st = i % STAGES;
@@ -151,8 +171,9 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
     mbar_expect_tx(&full[st], C::TILE_BYTES);
 #pragma unroll
     for (int sg = 0; sg < SEGS; sg++) {
-      tma_load_2d_hint(dst + sg * MM_BOX_BYTES, &tmK, sg * 32, row0 + i * MM_TK, &full[st], pol);
-      tma_load_2d_hint(dst + (SEGS + sg) * MM_BOX_BYTES, &tmV, sg * 32, row0 + i * MM_TK, &full[st], pol);
+      const int x = sg * (BF ? 64 : 32);
+      tma_load_2d_hint(dst + sg * MM_BOX_BYTES, &tmK, x, row0 + i * MM_TK, &full[st], pol);
+      tma_load_2d_hint(dst + (SEGS + sg) * MM_BOX_BYTES, &tmV, x, row0 + i * MM_TK, &full[st], pol);
     }
   };
   const int first = n_tiles < STAGES ? n_tiles : STAGES;
@@ -169,11 +190,27 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
 
   // ======================= Q fragments =======================
   // B operand of S^T = K . Q^T, step ks: b0 = q[head g][8 ks + t], b1 = q[head g][8 ks + t + 4],
-  // scaled by scale * log2(e), split into tf32 hi / lo: one uint4 per (step, lane).
+  // scaled by scale * log2(e), split into tf32 hi / lo: one uint4 per (step, lane).  bf16: b0 = q[head g]
+  // [16 ks + 2t, + 1], b1 = [.. + 8, + 9], in three planes: a uint4 (two planes) and, behind all, a uint2.
   {
     const float qs = p.scale * 1.4426950408889634f;
     for (int i = tid; i < KSTEPS * 32; i += C::THREADS) {
       const int ks = i >> 5, ln = i & 31, hg = ln >> 2, ht = ln & 3;
+      if constexpr (BF) {
+        float2 a = make_float2(0.f, 0.f), b = a;
+        if (hg < p.grp) {
+          const float* qp = p.q + (size_t)(kh * p.grp + hg) * D + 16 * ks + 2 * ht;
+          a = make_float2(qp[0] * qs, qp[1] * qs);
+          b = make_float2(qp[8] * qs, qp[9] * qs);
+        }
+        uint4 f;
+        uint2 l;
+        split3_bf16(a.x, a.y, f.x, f.z, l.x);
+        split3_bf16(b.x, b.y, f.y, f.w, l.y);
+        Qf[i] = f;
+        ((uint2*)(Qf + KSTEPS * 32))[i] = l;
+        continue;
+      }
       float b0 = 0.f, b1 = 0.f;
       if (hg < p.grp) {
         const float* qp = p.q + (size_t)(kh * p.grp + hg) * D + 8 * ks + ht;
@@ -204,9 +241,9 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
   }
 
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;   // heads 2t, 2t+1
-  float acc[2 * SEGS][4];
+  float acc[NT][4];
 #pragma unroll
-  for (int j = 0; j < 2 * SEGS; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+  for (int j = 0; j < NT; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
 
   if (warp < W) {
     const uint32_t ring32 = smem_u32(ring);
@@ -232,8 +269,9 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
           // ragged end: rows past the context hold whatever the cache holds there; P is zero
           // for them, but 0 * NaN is NaN, so their V rows are cleared (this warp is the only
           // reader of these 16 rows)
-          for (int i = lane; i < (16 - valid) * (D / 4); i += 32) {
-            const int r = 16 * half + valid + i / (D / 4), c4 = i % (D / 4);
+          constexpr int CPR = SEGS * 8;   // 16-byte chunks of a row
+          for (int i = lane; i < (16 - valid) * CPR; i += 32) {
+            const int r = 16 * half + valid + i / CPR, c4 = i % CPR;
             const int sg = c4 >> 3, ch = c4 & 7;
             *(float4*)(ring + (size_t)st * C::TILE_BYTES + (size_t)(SEGS + sg) * MM_BOX_BYTES + r * 128 +
                        ((ch ^ (r & 7)) << 4)) = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -245,6 +283,22 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
         // three accumulators, one per term of the split product: three independent MMA chains
         // of KSTEPS instead of one of 3 KSTEPS (the chain's latency is what a block costs)
         float s[4] = {0.f, 0.f, 0.f, 0.f}, s_hl[4] = {0.f, 0.f, 0.f, 0.f}, s_lh[4] = {0.f, 0.f, 0.f, 0.f};
+        if constexpr (BF) {
+#pragma unroll
+          for (int ks = 0; ks < KSTEPS; ks++) {
+            uint32_t a[4];
+            ldm_x4(a, kt + (uint32_t)(ks >> 2) * MM_BOX_BYTES + (uint32_t)(16 * half + (lane & 15)) * 128u +
+                          ((((uint32_t)(ks & 3) * 2 + (lane >> 4)) ^ (lane & 7)) << 4));
+            const uint4 qf = lds_u128(qf32 + (uint32_t)ks * 512u);
+            const uint2 ql = ((const uint2*)(Qf + KSTEPS * 32))[ks * 32 + lane];
+            float h[4] = {0.f, 0.f, 0.f, 0.f};
+            rc_mma(h, a, qf.x, qf.y);
+#pragma unroll
+            for (int i = 0; i < 4; i++) s[i] += h[i];
+            rc_mma(s_hl, a, qf.z, qf.w);
+            rc_mma(s_lh, a, ql.x, ql.y);
+          }
+        } else {
 #pragma unroll
         for (int ks = 0; ks < KSTEPS; ks++) {
           const uint32_t c0 = (uint32_t)((ks & 3) * 2) << 4;
@@ -260,6 +314,7 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
           mma_tf32(s, h0, h1, h2, h3, qf.x, qf.y);
           mma_tf32(s_hl, h0, h1, h2, h3, qf.z, qf.w);
           mma_tf32(s_lh, e0, e1, e2, e3, qf.x, qf.y);
+        }
         }
 #pragma unroll
         for (int i = 0; i < 4; i++) s[i] += s_hl[i] + s_lh[i];
@@ -278,7 +333,7 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
           l0 *= f0;
           l1 *= f1;
 #pragma unroll
-          for (int j = 0; j < 2 * SEGS; j++) {
+          for (int j = 0; j < NT; j++) {
             acc[j][0] *= f0; acc[j][2] *= f0;
             acc[j][1] *= f1; acc[j][3] *= f1;
           }
@@ -293,6 +348,33 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
         *(float2*)(myP + (g + 8) * 8 + 2 * t) = make_float2(p10, p11);
         __syncwarp();
         // ---- out^T[d][head] += V_blk^T . P ----
+        if constexpr (BF) {
+          // B operand: b0 = P[keys 2t, 2t + 1][head g], b1 = keys + 8
+          uint32_t w[3][2];
+#pragma unroll
+          for (int e = 0; e < 2; e++)
+            split3_bf16(myP[(8 * e + 2 * t) * 8 + g], myP[(8 * e + 2 * t + 1) * 8 + g], w[0][e], w[1][e], w[2][e]);
+          uint32_t a[NT][4];   // V_blk^T: 16 dimensions x 16 keys a tile
+          const uint32_t vrow = vt + (uint32_t)(16 * half + ((lane >> 4) << 3) + (lane & 7)) * 128u;
+#pragma unroll
+          for (int j = 0; j < NT; j++)
+            ldm_x4_trans(a[j], vrow + (uint32_t)(j >> 2) * MM_BOX_BYTES +
+                                   ((((uint32_t)(j & 3) * 2 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
+          // each block's sum from zero, smallest plane first, then added in f32: an MMA cuts its sum to 24
+          // bits without rounding, and a chain of them over the keys drifts (3.5e-7 against 2.3e-7 of the
+          // result at 12345 keys)
+          float b[NT][4];
+#pragma unroll
+          for (int j = 0; j < NT; j++) b[j][0] = b[j][1] = b[j][2] = b[j][3] = 0.f;
+#pragma unroll
+          for (int pl = 2; pl >= 0; pl--)
+#pragma unroll
+            for (int j = 0; j < NT; j++) rc_mma(b[j], a[j], w[pl][0], w[pl][1]);
+#pragma unroll
+          for (int j = 0; j < NT; j++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[j][i] += b[j][i];
+        } else {
 #pragma unroll
         for (int kk = 0; kk < 2; kk++) {
           const float pb0 = lds_f32(myP32 + (uint32_t)((8 * kk + t) * 8 + g) * 4u);
@@ -302,7 +384,7 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
           split_tf32(pb1, ph1, pl1);
           const uint32_t vrow = vt + (uint32_t)(16 * half + 8 * kk) * 128u;
 #pragma unroll
-          for (int j = 0; j < 2 * SEGS; j++) {
+          for (int j = 0; j < NT; j++) {
             const uint32_t a = vrow + (uint32_t)(j >> 1) * MM_BOX_BYTES + (vbase ^ ((uint32_t)(j & 1) << 5));
             const float v0 = lds_f32(a), v1 = lds_f32(a ^ 16u), v2 = lds_f32((a ^ 64u) + 512u),
                         v3 = lds_f32((a ^ 80u) + 512u);
@@ -315,6 +397,7 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
             mma_tf32(acc[j], h0, h1, h2, h3, pl0, pl1);
             mma_tf32(acc[j], e0, e1, e2, e3, ph0, ph1);
           }
+        }
         }
         __syncwarp();   // the warp's P is rewritten by its next block
       }
@@ -331,7 +414,12 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
     }
     float* e = ent + (size_t)warp * (D * 8 + 16);
 #pragma unroll
-    for (int j = 0; j < 2 * SEGS; j++) {
+    for (int j = 0; j < NT; j++) {
+      if constexpr (BF) {   // rows of m-tile j: 16 j + g, + 8
+        *(float2*)(e + (16 * j + g) * 8 + 2 * t) = make_float2(acc[j][0], acc[j][1]);
+        *(float2*)(e + (16 * j + g + 8) * 8 + 2 * t) = make_float2(acc[j][2], acc[j][3]);
+        continue;
+      }
       // rows of m-tile j: d(g, hf) = 32 (j >> 1) + 16 (g >> 2) + 4 (2 (j & 1) + hf) + (g & 3)
       const int d0 = 32 * (j >> 1) + 16 * (g >> 2) + 8 * (j & 1) + (g & 3);
       *(float2*)(e + d0 * 8 + 2 * t) = make_float2(acc[j][0], acc[j][1]);
@@ -466,18 +554,18 @@ __global__ void __launch_bounds__(MmaCfg<D>::THREADS, 1)
   if (tid == 0) p.counters[kh] = 0;   // clean for the next launch
 }
 
-template <int D>
+template <int D, bool BF>
 int launch_mma_t(const AttnParams& p, int splits, cudaStream_t stream) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return set_error(TLB_ERR_CUDA, "cuTensorMapEncodeTiled entry point not found");
   CUtensorMap tmK, tmV;
   const cuuint64_t rows = (cuuint64_t)p.n_kv * (cuuint64_t)p.kv_rows;
   cuuint64_t dims[2] = {(cuuint64_t)D, rows};
-  cuuint64_t strides[1] = {(cuuint64_t)D * 4};
-  cuuint32_t box[2] = {32, (cuuint32_t)MM_TK};
+  cuuint64_t strides[1] = {(cuuint64_t)D * (BF ? 2 : 4)};
+  cuuint32_t box[2] = {BF ? 64 : 32, (cuuint32_t)MM_TK};
   cuuint32_t es[2] = {1, 1};
   for (int which = 0; which < 2; which++) {
-    CUresult r = enc(which ? &tmV : &tmK, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+    CUresult r = enc(which ? &tmV : &tmK, BF ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
                      const_cast<void*>(which ? p.V : p.K), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -485,25 +573,25 @@ int launch_mma_t(const AttnParams& p, int splits, cudaStream_t stream) {
   }
   static std::atomic<unsigned long long> attr_done{0};
   {
-    const int rc_attr = ensure_dynamic_smem(attn_decode_mma_kernel<D>, (int)MmaCfg<D>::TOTAL, attr_done);
+    const int rc_attr = ensure_dynamic_smem(attn_decode_mma_kernel<D, BF>, (int)MmaCfg<D, BF>::TOTAL, attr_done);
     if (rc_attr) return rc_attr;
   }
-  LaunchCfg lc(dim3(splits, p.n_kv), dim3(MmaCfg<D>::THREADS), MmaCfg<D>::TOTAL, stream, pdl_enabled());
-  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, attn_decode_mma_kernel<D>, tmK, tmV, p));
+  LaunchCfg lc(dim3(splits, p.n_kv), dim3(MmaCfg<D, BF>::THREADS), MmaCfg<D, BF>::TOTAL, stream, pdl_enabled());
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, attn_decode_mma_kernel<D, BF>, tmK, tmV, p));
   return TLB_OK;
 }
 
 }  // namespace
 
-// f32 cache, 3..8 query heads per KV head, 16-byte aligned operands (checked by the caller),
-// row count of the [n_kv * kv_max, D] view within the TMA coordinate range
-bool attn_decode_mma_eligible(int grp, int D, int n_kv, long long kv_max, int kv_bf16) {
-  return !kv_bf16 && grp >= 3 && grp <= 8 && (D == 64 || D == 128) && (long long)n_kv * kv_max < (1ll << 31);
+// 3..8 query heads per KV head, 16-byte aligned operands (checked by the caller), row count of the
+// [n_kv * kv_max, D] view within the TMA coordinate range
+bool attn_decode_mma_eligible(int grp, int D, int n_kv, long long kv_max) {
+  return grp >= 3 && grp <= 8 && (D == 64 || D == 128) && (long long)n_kv * kv_max < (1ll << 31);
 }
 
-int attn_decode_mma_launch(const AttnParams& p, int D, int splits, cudaStream_t stream) {
-  if (D == 128) return launch_mma_t<128>(p, splits, stream);
-  return launch_mma_t<64>(p, splits, stream);
+int attn_decode_mma_launch(const AttnParams& p, int D, int bf, int splits, cudaStream_t stream) {
+  if (D == 128) return bf ? launch_mma_t<128, true>(p, splits, stream) : launch_mma_t<128, false>(p, splits, stream);
+  return bf ? launch_mma_t<64, true>(p, splits, stream) : launch_mma_t<64, false>(p, splits, stream);
 }
 
 }  // namespace tlb

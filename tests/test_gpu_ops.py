@@ -434,6 +434,26 @@ def test_attn_bf16_cache_vs_oracle(tl, port, n_q, n_kv, D, kv_max, ctxs):
         assert relerr(got, port.attn_decode(q, Kr, Vr, D ** -0.5, ctx=ctx)) < 1e-4, ctx
 
 
+@pytest.mark.parametrize("n_q,n_kv,D,kv_max,ctxs", [
+    (3, 1, 64, 80, (1, 15, 16, 17, 80)),             # the smallest group; blocks of 16 keys, ragged ends
+    (8, 1, 128, 9000, (33, 4097, 9000)),             # the widest; many splits of one head, the ring wraps
+    (20, 4, 128, 600, (63, 65, 599)),                # five heads a group, two tiles a split
+    (28, 7, 64, 3000, (131, 2999)),
+])
+def test_attn_bf16_groups_vs_oracle(tl, port, n_q, n_kv, D, kv_max, ctxs):
+    """Groups of 3..8 heads on a bf16 cache whose rows behind the context hold NaN.  f32 sums of at most
+    D and ctx terms: 1e-4 of (1 + |value|) as for f32 caches."""
+    K = synth.normal(71, 1, (n_kv, kv_max, D))
+    V = synth.normal(71, 2, (n_kv, kv_max, D))
+    q = synth.normal(71, 3, (n_q, D))
+    Kr, Vr = bf16_round(K), bf16_round(V)
+    for ctx in ctxs:
+        Kd, Vd = dev(Kr).to(torch.bfloat16), dev(Vr).to(torch.bfloat16)
+        Kd[:, ctx:], Vd[:, ctx:] = float("nan"), float("nan")
+        got = tl.attn_decode(dev(q), Kd, Vd, D ** -0.5, ctx=ctx).cpu().numpy()
+        assert relerr(got, port.attn_decode(q, Kr, Vr, D ** -0.5, ctx=ctx)) < 1e-4, ctx
+
+
 def test_kv_cache_bf16_append_fill_and_attend(tl, port):
     """kv_cache with dtype bf16: append / fill narrow with round-to-nearest-even (bit-equal to
     the host converter), attention in both position forms reads them back."""
