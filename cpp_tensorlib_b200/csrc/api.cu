@@ -29,7 +29,7 @@ int gemm_q4_tc_launch(DeviceCtx* c, const float* x, long long ldx, int M, const 
                       float beta, float* xsplit, cudaStream_t stream);
 int gemm_q4_tc2_launch(DeviceCtx* c, const float* x, long long ldx, int M, const void* qw, const float* scales,
                        float* y, long long ldy, int N, int K, float alpha, float beta, void* scratch,
-                       cudaStream_t stream);
+                       void* work, cudaStream_t stream);
 size_t attn_partials_bytes(int n_q, int n_kv, long long kv_max, int D, int sm_count);
 int attn_decode_launch(DeviceCtx* c, const float* q, const void* K, const void* V, float* out,
                        int n_q, int n_kv, int ctx, long long kv_max, int D, float scale,
@@ -304,8 +304,15 @@ int tlb_gemm_q4(const float* x, int64_t M, int64_t ldx, const void* qw, const fl
       TLB_CUDA(cudaMalloc(&c->xsplit, need));
       c->xsplit_bytes = need;
     }
+    if (!c->q4_work) {
+      void* w = nullptr;
+      TLB_CUDA(cudaMalloc(&w, gemm_q4_work_bytes(c->sm_count)));
+      TLB_CUDA(cudaMemset(w, 0, Q4_TICKET_BYTES));
+      TLB_CUDA(cudaDeviceSynchronize());
+      c->q4_work = w;
+    }
     return gemm_q4_tc2_launch(c, x, ldx, (int)M, qw, scales, y, ldy, (int)N, (int)K, alpha, beta, c->xsplit,
-                              S(stream));
+                              c->q4_work, S(stream));
   }
   if (gemm_q4_tc_eligible(qw, scales, (int)N, (int)K, (int)M)) {
     const size_t need = (size_t)2 * M * K * sizeof(float);

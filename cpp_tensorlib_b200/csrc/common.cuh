@@ -59,6 +59,7 @@ struct DeviceCtx {
   // tf32 hi/lo planes of the activations for the tensor-core GEMM (grown on demand)
   float* xsplit = nullptr;
   size_t xsplit_bytes = 0;
+  void* q4_work = nullptr;   // gemm_q4_work_bytes, made by the first product of many rows
   unsigned long long* argmax_cell = nullptr;
   int* status = nullptr;        // device, ST_WORDS ints
   int* status_host = nullptr;   // pinned mirror for reads

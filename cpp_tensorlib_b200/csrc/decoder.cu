@@ -113,6 +113,7 @@ struct Decoder : DecoderBase {
   int pf_rows = 0;
   float *pf_res[2] = {}, *pf_h = nullptr, *pf_h2 = nullptr, *pf_md = nullptr, *pf_qkv = nullptr, *pf_at = nullptr,
         *pf_gu = nullptr, *pf_mb = nullptr;
+  void* pf_work = nullptr;     // scratch of the products on planes
   void* pf_planes = nullptr;   // activations of one product as fp16 planes; shares pf_mb's memory
 
   ~Decoder() override;
@@ -417,6 +418,7 @@ Decoder::~Decoder() {
   for (void* sk : sink) cudaFree(sk);
   cudaFree(rope_cs);
   cudaFree(pf);
+  cudaFree(pf_work);
   cudaFree(attn_partials); cudaFree(flags_local);
 }
 
@@ -432,13 +434,21 @@ int Decoder::prefill_begin(int rows, cudaStream_t s) {
   const int E = hidden, D = hd, QKV = (n_q + 2 * n_kv) * D;
   const size_t CH = rows, n_emb = CH * E, n_qkv = CH * QKV, n_att = CH * n_q * D, n_gu = CH * 2 * ff, n_mb = CH * ff;
   // the planes of a product's rows, or the rows in f32 where the product takes those
-  const int wide = ff > E ? ff : E;
+  const int wide = ff > E ? (ff > n_q * D ? ff : n_q * D) : (E > n_q * D ? E : n_q * D);
   const size_t n_pl = (gemm_q4_tc2_scratch_bytes(rows, wide) + 3) / 4, n_act = n_mb > n_pl ? n_mb : n_pl;
   const size_t total = 5 * n_emb /* res0 res1 h h2 md */ + n_qkv + n_att + n_gu + n_act + 64;
   if (pf) {
     TLB_CUDA(cudaStreamSynchronize(s));
     TLB_CUDA(cudaFree(pf));
     pf = nullptr;
+  }
+  if (!pf_work) {
+    DeviceCtx* c = nullptr;
+    const int rc = get_ctx(&c);
+    if (rc) return rc;
+    TLB_CUDA(cudaMalloc(&pf_work, gemm_q4_work_bytes(c->sm_count)));
+    TLB_CUDA(cudaMemset(pf_work, 0, Q4_TICKET_BYTES));
+    TLB_CUDA(cudaDeviceSynchronize());
   }
   TLB_CUDA(cudaMalloc(&pf, total * sizeof(float)));
   pf_rows = rows;
@@ -473,7 +483,7 @@ int Decoder::prefill_pass(const int* d_ids, int rows, int pos, cudaStream_t s) {
   };
   auto gemm_planes = [&](const Linear& L, float* y) {
     return gemm_q4_planes_launch(c, q4_planes_at(pf_planes, rows, L.K), rows, L.q4, L.scales(), y, L.N, L.N, L.K, 1.0f,
-                                 0.0f, s);
+                                 0.0f, pf_work, s);
   };
 #define PF(expr) do { rc = (expr); if (rc) return rc; } while (0)
   // y = norm(x + b) * w through L; xsum the residual (b NULL: x itself), h f32 rows for products that read those
@@ -495,7 +505,12 @@ int Decoder::prefill_pass(const int* d_ids, int rows, int pos, cudaStream_t s) {
     float* ro = pf_res[l & 1];
     PF(launch_qkv_rows(qkv, L.bq, L.bk, L.bv, L.Kc, L.Vc, rows, NQ, NKV, D, pos, max_ctx, rope_base, kv_bf16, s));
     PF(launch_attn_prefill_rows(c, qkv, QKV, L.Kc, L.Vc, at, NQ, NKV, rows, max_ctx, D, scale, pos, kv_bf16, s));
-    PF(gemm(L.wo, at, md, rows));
+    if (planes(L.wo)) {
+      PF(launch_split_rows(at, NQ * D, rows, NQ * D, q4_planes_at(pf_planes, rows, NQ * D), s));
+      PF(gemm_planes(L.wo, md));
+    } else {
+      PF(gemm(L.wo, at, md, rows));
+    }
     PF(norm_gemm(x, md, L.fn, ro, h2, L.wgu, gu));
     if (planes(L.wd)) {
       PF(launch_swiglu_planes(gu, FF, rows, q4_planes_at(pf_planes, rows, FF), s));

@@ -15,8 +15,13 @@
 // the row's f32 group scale and add into registers -- the same order of operations as the
 // reference's dequantise-then-multiply in f32 (include/array.h:666-684, 1980-1984).
 //
-// One CTA = 128 weight rows (UMMA M) x MT activation rows (UMMA N, 32 / 64 / 128), grid =
-// (N / 128, M / MT).  Warp roles (512 threads): warp 0 TMA producer of the X planes (64-k
+// A tile is 128 weight rows (UMMA M) x MT activation rows (UMMA N, 32 / 64 / 128); its work is a row of units of
+// 256 k (one box of packed weights).  The CTAs, one per SM at most, stay for the whole product and take equal
+// ranges of the units, tile after tile: the pipelines below run on across the tiles, so that a tile's first loads and
+// conversions pass under the stores of the one before, and a product with few tiles still uses the
+// whole chip.  A tile whose units lie in several CTAs' ranges is summed by the last of them to finish, in
+// the order of k, from f32 partials in scratch (T2Work): the same bits on every call, and no CTA waits for
+// another.  Warp roles (512 threads): warp 0 TMA producer of the X planes (64-k
 // stages, 128-byte swizzle), warp 1 TMEM allocator, warps 1 and 15 the MMA issuers (first / second group of a stage), warps 2-5
 // nibble -> fp16 converters (thread r owns weight row r; the k order inside every group of 8
 // is the one the nibble extraction produces -- 0,4,1,5,2,6,3,7 -- and the X planes are stored
@@ -27,6 +32,13 @@
 // 16 KB per SM in flight and paced the whole kernel at ~1 TB/s of weight bytes.)  All waits
 // are bounded; a timeout sets the status word, the kernel still frees its TMEM and returns.
 // No cluster launch, no multicast.
+//
+// What bounds it is the instruction issue of the four schedulers, not the tensor pipe: without any MMA a product takes
+// nine tenths of the time, with half of them as long.  So the accumulate warps' loop is unrolled over a block of four
+// scales, one accumulator each, with nothing left to select at run time.  Measured and dropped: weights in TMEM as
+// the A operand, sixteen accumulate warps, one issuer, one commit a stage, spinning waits, register shares by
+// setmaxnreg with 64-column reads.  1000 x 3584 x 37888: 676 -> 583 us; 1000 x 18944 x 3584, one and a half
+// rounds of tiles: 424 -> 328; 517 x 4864 x 896, 35 tiles: 60 -> 40.
 #include <cstdlib>
 
 #include "q4_planes.cuh"
@@ -51,6 +63,34 @@ struct T2Params {
   int M, N, K;
   float alpha, beta;
   int* status;
+  int n_tiles, box;          // tiles along N (the inner ones), units of a tile
+  unsigned per, longer, grain;   // units a CTA / grain, CTAs with one more, grain = 1 or box (whole tiles)
+  float* parts;              // [2 * CTAs][MT][128]
+  int* tickets;              // [CTAs], zero between launches
+};
+
+// Which units are a CTA's: ranges of `per` or per + 1 units (or whole tiles), the tiles in order.
+__device__ __forceinline__ unsigned t2_first(const T2Params& p, unsigned cta) {
+  return (cta * p.per + (cta < p.longer ? cta : p.longer)) * p.grain;
+}
+// the CTA whose range holds unit u
+__device__ __forceinline__ unsigned t2_owner(const T2Params& p, unsigned u) {
+  const unsigned v = u / p.grain, in_longer = p.longer * (p.per + 1);
+  return v < in_longer ? v / (p.per + 1) : p.longer + (v - in_longer) / p.per;
+}
+// The CTA's segments in order: boxes q0 .. q1 of a tile.
+struct T2Segment {
+  unsigned u, end;
+  int tile = 0, q0 = 0, q1 = 0;
+  __device__ __forceinline__ T2Segment(const T2Params& p) : u(t2_first(p, blockIdx.x)), end(t2_first(p, blockIdx.x + 1)) {}
+  __device__ __forceinline__ bool next(const T2Params& p) {
+    if (u >= end) return false;
+    tile = (int)(u / (unsigned)p.box);
+    q0 = (int)(u - (unsigned)tile * (unsigned)p.box);
+    q1 = (unsigned)(p.box - q0) < end - u ? p.box : q0 + (int)(end - u);
+    u += (unsigned)(q1 - q0);
+    return true;
+  }
 };
 
 template <int MT>
@@ -135,7 +175,7 @@ enum { T2_X_FULL = 0, T2_A_READY = 4, T2_ST_EMPTY = 8, T2_D_FULL = 12, T2_D_EMPT
        T2_RAW_EMPTY = 24 };
 // TMEM accumulators in rotation: the MMA thread runs up to T2_NBUF groups ahead of the
 // accumulate warps, whose tcgen05.ld round trip (not the MMAs) is the latency of a group
-constexpr int T2_NBUF = 4;
+constexpr int T2_NBUF = 4;   // the groups of a block of scales, too
 
 template <int MT>
 __global__ void __launch_bounds__(T2_THREADS, 1)
@@ -149,9 +189,10 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
   unsigned char* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* bars = (uint64_t*)(base + S::BARS);
   uint32_t* tmem_slot = (uint32_t*)(base + S::SLOT);
+  volatile int* last_part = (volatile int*)(base + S::SLOT + 8);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n0 = blockIdx.x * T2_ROWS, m0 = blockIdx.y * MT;
-  const int nst = p.K / T2_KS, ngr = p.K / 32, nraw = (nst + T2_SUB - 1) / T2_SUB;
+  const int nst = p.K / T2_KS;   // 64-k stages of a tile
+  T2Segment sg(p);
 
   if (tid == 0) {
     for (int s = 0; s < T2_STAGES; s++) {
@@ -186,23 +227,35 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
   if (warp == 14) {
     // ---------------- TMA producer: packed weights, 128 rows x 256 k per box ----------------
     if (lane == 0) {
-      for (int q = 0; q < nraw; q++) {
-        const int rs = q % T2_RAW_STAGES;
-        if (!mbar_wait_bounded(&bars[T2_RAW_EMPTY + rs], ((q / T2_RAW_STAGES) & 1) ^ 1, p.status, 640)) break;
-        mbar_expect_tx(&bars[T2_RAW_FULL + rs], (uint32_t)T2_RAW_BYTES);
-        tma_load_2d(base + S::RAW + (size_t)rs * T2_RAW_BYTES, &tmW, q * 128, n0, &bars[T2_RAW_FULL + rs]);
+      int cnt = 0;
+      bool ok = true;
+      while (sg.next(p)) {
+        const int n0 = sg.tile % p.n_tiles * T2_ROWS;
+        for (int q = sg.q0; q < sg.q1 && ok; q++, cnt++) {
+          const int rs = cnt % T2_RAW_STAGES;
+          ok = mbar_wait_bounded(&bars[T2_RAW_EMPTY + rs], ((cnt / T2_RAW_STAGES) & 1) ^ 1, p.status, 640);
+          if (!ok) break;
+          mbar_expect_tx(&bars[T2_RAW_FULL + rs], (uint32_t)T2_RAW_BYTES);
+          tma_load_2d(base + S::RAW + (size_t)rs * T2_RAW_BYTES, &tmW, q * 128, n0, &bars[T2_RAW_FULL + rs]);
+        }
       }
     }
   } else if (warp == 0) {
     // ---------------- TMA producer: the two fp16 planes of X, one 64-k stage at a time ----------------
     if (lane == 0) {
-      for (int it = 0; it < nst; it++) {
-        const int s = it % T2_STAGES;
-        if (!mbar_wait_bounded(&bars[T2_ST_EMPTY + s], ((it / T2_STAGES) & 1) ^ 1, p.status, 600)) break;
-        mbar_expect_tx(&bars[T2_X_FULL + s], 2u * MT * 128u);
-        const int kx = it * T2_KS;
-        tma_load_2d(base + S::B + (size_t)(s * 2 + 0) * MT * 128, &tmX1, kx, m0, &bars[T2_X_FULL + s]);
-        tma_load_2d(base + S::B + (size_t)(s * 2 + 1) * MT * 128, &tmX2, kx, m0, &bars[T2_X_FULL + s]);
+      int cnt = 0;
+      bool ok = true;
+      while (sg.next(p)) {
+        const int m0 = sg.tile / p.n_tiles * MT, it1 = sg.q1 * T2_SUB < nst ? sg.q1 * T2_SUB : nst;
+        for (int it = sg.q0 * T2_SUB; it < it1 && ok; it++, cnt++) {
+          const int s = cnt % T2_STAGES;
+          ok = mbar_wait_bounded(&bars[T2_ST_EMPTY + s], ((cnt / T2_STAGES) & 1) ^ 1, p.status, 600);
+          if (!ok) break;
+          mbar_expect_tx(&bars[T2_X_FULL + s], 2u * MT * 128u);
+          const int kx = it * T2_KS;
+          tma_load_2d(base + S::B + (size_t)(s * 2 + 0) * MT * 128, &tmX1, kx, m0, &bars[T2_X_FULL + s]);
+          tma_load_2d(base + S::B + (size_t)(s * 2 + 1) * MT * 128, &tmX2, kx, m0, &bars[T2_X_FULL + s]);
+        }
       }
     }
   } else if (warp == 1 || warp == 15) {
@@ -213,7 +266,9 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
     const int grp = warp == 1 ? 0 : 1;
     const uint32_t idesc = t2_idesc_f16(MT);
     const bool leader = t2_elect_one();
-    for (int it = 0; it < nst; it++) {
+    int stages = 0;   // of all segments: tiles follow one another without a seam
+    while (sg.next(p)) stages += (sg.q1 * T2_SUB < nst ? sg.q1 * T2_SUB : nst) - sg.q0 * T2_SUB;
+    for (int it = 0; it < stages; it++) {
       const int s = it % T2_STAGES;
       const uint32_t ph = (it / T2_STAGES) & 1;
       const int gi = 2 * it + grp, buf = gi % T2_NBUF;
@@ -242,9 +297,13 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
     const int r = tid - 64;
     const __half2 off = __floats2half2_rn(1032.0f, 1032.0f);
     bool conv_ok = true;
-    for (int q = 0; q < nraw && conv_ok; q++) {
-      const int rs = q % T2_RAW_STAGES;
-      if (!mbar_wait_bounded(&bars[T2_RAW_FULL + rs], (q / T2_RAW_STAGES) & 1, p.status, 621)) break;
+    int cnt = 0, it = -1;   // boxes and stages of all segments
+    while (sg.next(p)) for (int q = sg.q0; q < sg.q1 && conv_ok; q++, cnt++) {
+      const int rs = cnt % T2_RAW_STAGES;
+      if (!mbar_wait_bounded(&bars[T2_RAW_FULL + rs], (cnt / T2_RAW_STAGES) & 1, p.status, 621)) {
+        conv_ok = false;
+        break;
+      }
       // the row's 128 packed bytes of this box: chunk c (16 bytes = 32 k) sits at c ^ (r & 7)
       const unsigned char* rrow = base + S::RAW + (size_t)rs * T2_RAW_BYTES + r * 128;
       uint4 wq[2 * T2_SUB];
@@ -252,8 +311,8 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
       for (int c = 0; c < 2 * T2_SUB; c++) wq[c] = *(const uint4*)(rrow + ((c ^ (r & 7)) << 4));
 #pragma unroll
       for (int u = 0; u < T2_SUB; u++) {
-        const int it = q * T2_SUB + u;
-        if (it >= nst) break;
+        if (q * T2_SUB + u >= nst) break;
+        it++;
         const int s = it % T2_STAGES;
         const uint4 c0 = wq[2 * u], c1 = wq[2 * u + 1];
         if (!mbar_wait_bounded(&bars[T2_ST_EMPTY + s], ((it / T2_STAGES) & 1) ^ 1, p.status, 620)) {
@@ -288,55 +347,91 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
   } else if (warp < 14) {
     // ---------------- accumulate (sc * group product) + epilogue ----------------
     const int quarter = warp & 3, half = (warp - 6) >> 2;
-    const int r = quarter * 32 + lane, n = n0 + r;
+    const int r = quarter * 32 + lane;
     const int c_lo = half * HC;
-    const float* sc_row = p.scales + (size_t)(n < p.N ? n : p.N - 1) * (p.K / 32);
-    float acc[HC];
+    bool ok = true;   // a wait that gave up: no more work, but every barrier and ticket below
+    unsigned blocks = 0;   // of four groups, of all segments
+    while (sg.next(p)) {
+      const int tile = sg.tile, q0 = sg.q0, q1 = sg.q1;
+      const int n = tile % p.n_tiles * T2_ROWS + r, m0 = tile / p.n_tiles * MT;
+      float acc[HC];
 #pragma unroll
-    for (int i = 0; i < HC; i++) acc[i] = 0.f;
-    // the row's group scales, four at a time (K % 128 == 0), fetched two blocks ahead: one L2
-    // round trip is longer than a group takes
-    const float4* sc4 = (const float4*)sc_row;
-    const int nblk = ngr / 4;
-    float4 sc_blk = __ldg(sc4), sc_n1 = nblk > 1 ? __ldg(sc4 + 1) : sc_blk, sc_n2 = sc_blk;
-    bool ok = true;
-    for (int gi = 0; gi < ngr; gi++) {
-      const int buf = gi % T2_NBUF;
-      if ((gi & 3) == 0) {
-        if (gi) { sc_blk = sc_n1; sc_n1 = sc_n2; }
-        if ((gi >> 2) + 2 < nblk) sc_n2 = __ldg(sc4 + (gi >> 2) + 2);
-      }
-      const float sc = (gi & 3) == 0 ? sc_blk.x : ((gi & 3) == 1 ? sc_blk.y : ((gi & 3) == 2 ? sc_blk.z : sc_blk.w));
-      if (!mbar_wait_bounded(&bars[T2_D_FULL + buf], (gi / T2_NBUF) & 1, p.status, 630)) { ok = false; break; }
-      t2_fence_after();
-      const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * MT + c_lo);
-      // 32 columns per read; the accumulator goes back to the issuers as soon as the last
-      // read has landed, before its FMAs.  (Measured and dropped: fma.rn.f32x2 pairs -- the
-      // register pairing costs more than the halved FMA count saves, 200 vs 170 us at M = 512 --
-      // and 16-column reads in flight under the previous 16 columns' FMAs.)
-      constexpr int BATCH = HC < 32 ? HC : 32;
+      for (int i = 0; i < HC; i++) acc[i] = 0.f;
+      // the row's group scales, four at a time (K % 128 == 0), fetched a block ahead: an L2 round trip is
+      // shorter than the four groups take
+      const float4* sc4 = (const float4*)(p.scales + (size_t)(n < p.N ? n : p.N - 1) * (p.K / 32)) + q0 * 2;
+      const int nblk = (q1 * 2 < p.K / 128 ? q1 * 2 : p.K / 128) - q0 * 2;
+      float4 sc_blk = __ldg(sc4);
+      for (int b = 0; b < nblk && ok; b++, blocks++) {
+        const float4 sc_next = b + 1 < nblk ? __ldg(sc4 + b + 1) : sc_blk;
 #pragma unroll
-      for (int c0 = 0; c0 < HC; c0 += BATCH) {
-        uint32_t v[BATCH / 16][16];
+        for (int buf = 0; buf < T2_NBUF; buf++) {   // four groups a block, one accumulator each
+            const float sc = buf == 0 ? sc_blk.x : (buf == 1 ? sc_blk.y : (buf == 2 ? sc_blk.z : sc_blk.w));
+          if (!mbar_wait_bounded(&bars[T2_D_FULL + buf], blocks & 1, p.status, 630)) { ok = false; break; }
+          t2_fence_after();
+          const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * MT + c_lo);
+          // 32 columns per read; the accumulator goes back to the issuers as soon as the last
+          // read has landed, before its FMAs.  (Measured and dropped: fma.rn.f32x2 pairs -- the
+          // register pairing costs more than the halved FMA count saves, 200 vs 170 us at M = 512 --
+          // and 16-column reads in flight under the previous 16 columns' FMAs.)
+          constexpr int BATCH = HC < 32 ? HC : 32;
 #pragma unroll
-        for (int b = 0; b < BATCH / 16; b++) t2_ld16_issue(taddr + (uint32_t)(c0 + 16 * b), v[b]);
-        t2_wait_ld();
-        if (c0 + BATCH >= HC) {
-          t2_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars[T2_D_EMPTY + buf]);
+          for (int c0 = 0; c0 < HC; c0 += BATCH) {
+            uint32_t v[BATCH / 16][16];
+#pragma unroll
+            for (int b = 0; b < BATCH / 16; b++) t2_ld16_issue(taddr + (uint32_t)(c0 + 16 * b), v[b]);
+            t2_wait_ld();
+            if (c0 + BATCH >= HC) {
+              t2_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bars[T2_D_EMPTY + buf]);
+            }
+#pragma unroll
+            for (int b = 0; b < BATCH / 16; b++)
+#pragma unroll
+            for (int i = 0; i < 16; i++) acc[c0 + 16 * b + i] = fmaf(sc, __uint_as_float(v[b][i]), acc[c0 + 16 * b + i]);
+          }
         }
-#pragma unroll
-        for (int b = 0; b < BATCH / 16; b++)
-#pragma unroll
-          for (int i = 0; i < 16; i++) acc[c0 + 16 * b + i] = fmaf(sc, __uint_as_float(v[b][i]), acc[c0 + 16 * b + i]);
+        sc_blk = sc_next;
       }
-    }
-    if (ok && n < p.N) {
+      bool mine = true;   // this CTA writes the tile
+        if (q1 - q0 < p.box) {
+        // a part of the tile: into scratch, and the last of the tile's CTAs sums all parts
+        const unsigned u0 = (unsigned)tile * (unsigned)p.box;
+        const int first = (int)t2_owner(p, u0), last = (int)t2_owner(p, u0 + (unsigned)p.box - 1u), me = blockIdx.x;
+        auto part = [&](int cta) {
+          const int second = t2_first(p, cta) < u0;   // the range began in an earlier tile
+            return p.parts + (size_t)(2 * cta + second) * (MT * T2_ROWS) + (size_t)c_lo * T2_ROWS + r;
+        };
+        float* mp = part(me);
 #pragma unroll
-      for (int i = 0; i < HC; i++) {
-        const int m = m0 + c_lo + i;
-        if (m < p.M) p.y[(long long)m * p.ldy + n] = (acc[i] * __ldg(p.rowscale + m)) * p.alpha + p.beta;
+        for (int i = 0; i < HC; i++) __stcg(mp + i * T2_ROWS, acc[i]);
+        __threadfence();
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (warp == 6 && lane == 0) {
+          int old;
+          asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(p.tickets + first) : "memory");
+          *last_part = old == last - first;
+          if (old == last - first) p.tickets[first] = 0;   // clean for the next launch
+          }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        mine = *last_part != 0;
+        if (mine) {
+#pragma unroll
+          for (int i = 0; i < HC; i++) acc[i] = 0.f;
+          for (int cta = first; cta <= last; cta++) {
+            const float* q = part(cta);
+#pragma unroll
+            for (int i = 0; i < HC; i++) acc[i] += __ldcg(q + i * T2_ROWS);
+          }
+        }
+      }
+      if (mine && ok && n < p.N) {
+#pragma unroll
+        for (int i = 0; i < HC; i++) {
+          const int m = m0 + c_lo + i;
+          if (m < p.M) p.y[(long long)m * p.ldy + n] = (acc[i] * __ldg(p.rowscale + m)) * p.alpha + p.beta;
+        }
       }
     }
   }
@@ -403,19 +498,21 @@ __global__ void split_f16_kernel(const float* __restrict__ x, long long ldx, int
 
 template <int MT>
 int t2_launch(const CUtensorMap& tm1, const CUtensorMap& tm2, const CUtensorMap& tmw, const T2Params& p,
-              cudaStream_t stream) {
+              int ctas, cudaStream_t stream) {
   static std::atomic<unsigned long long> attr_done{0};
   {
     const int rc_attr = ensure_dynamic_smem(gemm_q4_tc2_kernel<MT>, (int)T2Smem<MT>::TOTAL, attr_done);
     if (rc_attr) return rc_attr;
   }
-  LaunchCfg lc(dim3((p.N + T2_ROWS - 1) / T2_ROWS, (p.M + MT - 1) / MT), dim3(T2_THREADS), T2Smem<MT>::TOTAL, stream,
-               pdl_enabled());
+  LaunchCfg lc(dim3(ctas), dim3(T2_THREADS), T2Smem<MT>::TOTAL, stream, pdl_enabled());
   TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, gemm_q4_tc2_kernel<MT>, tm1, tm2, tmw, p));
   return TLB_OK;
 }
 
 }  // namespace
+
+// tickets (zeroed once by the owner) and parts of the tiles that several CTAs share
+size_t gemm_q4_work_bytes(int sm_count) { return Q4_TICKET_BYTES + (size_t)2 * sm_count * 128 * T2_ROWS * sizeof(float); }
 
 // bytes of the activation scratch: two fp16 planes + the row scales
 size_t gemm_q4_tc2_scratch_bytes(int M, int K) { return (size_t)M * K * 4 + (size_t)((M + 3) & ~3) * 4 + 256; }
@@ -434,15 +531,20 @@ bool gemm_q4_planes_eligible(const void* qw, const void* scales, int N, int K, i
 
 int gemm_q4_tc2_launch(DeviceCtx* c, const float* x, long long ldx, int M, const void* qw, const float* scales,
                        float* y, long long ldy, int N, int K, float alpha, float beta, void* scratch,
-                       cudaStream_t stream) {
+                       void* work, cudaStream_t stream) {
   const Q4Planes pl = q4_planes_at(scratch, M, K);
+  const int rc = launch_split_rows(x, ldx, M, K, pl, stream);
+  return rc ? rc : gemm_q4_planes_launch(c, pl, M, qw, scales, y, ldy, N, K, alpha, beta, work, stream);
+}
+
+int launch_split_rows(const float* x, long long ldx, int M, int K, const Q4Planes& pl, cudaStream_t stream) {
   LaunchCfg lc(dim3((unsigned)M), dim3(256), 0, stream, pdl_enabled());
   TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, split_f16_kernel, x, ldx, K, pl.hi, pl.lo, pl.rowscale));
-  return gemm_q4_planes_launch(c, pl, M, qw, scales, y, ldy, N, K, alpha, beta, stream);
+  return TLB_OK;
 }
 
 int gemm_q4_planes_launch(DeviceCtx* c, const Q4Planes& x, int M, const void* qw, const float* scales, float* y,
-                          long long ldy, int N, int K, float alpha, float beta, cudaStream_t stream) {
+                          long long ldy, int N, int K, float alpha, float beta, void* work, cudaStream_t stream) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return set_error(TLB_ERR_CUDA, "cuTensorMapEncodeTiled entry point not found");
   const int MT = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
@@ -470,9 +572,28 @@ int gemm_q4_planes_launch(DeviceCtx* c, const Q4Planes& x, int M, const void* qw
   T2Params p;
   p.qw = (const unsigned*)qw; p.scales = scales; p.rowscale = x.rowscale; p.y = y; p.ldy = ldy;
   p.M = M; p.N = N; p.K = K; p.alpha = alpha; p.beta = beta; p.status = c->status;
-  if (MT == 32) return t2_launch<32>(tm1, tm2, tmw, p, stream);
-  if (MT == 64) return t2_launch<64>(tm1, tm2, tmw, p, stream);
-  return t2_launch<128>(tm1, tm2, tmw, p, stream);
+  p.n_tiles = (N + T2_ROWS - 1) / T2_ROWS;
+  p.box = (K / T2_KS + T2_SUB - 1) / T2_SUB;
+  p.tickets = (int*)work;
+  p.parts = (float*)((char*)work + Q4_TICKET_BYTES);
+  // Whole tiles for each CTA, or equal ranges of units (no tile in more than eight or so) where what the last,
+  // partly empty round of tiles would leave idle is worth more than writing and reading the parts: from four units of
+  // 256 k an SM on.  517 x 896 x 9728 (1.7 units idle) takes 46 us in tiles and 51 in ranges, 64 x 3584 x 3584
+  // (11 idle) 34 in tiles and 24 in ranges, 1000 x 3584 x 3584 (6.8 idle) 93 and 85.
+  const long long tiles = (long long)p.n_tiles * ((M + MT - 1) / MT), sms = c->sm_count, units = tiles * p.box;
+  if (units >= 1ll << 31) return set_error(TLB_ERR_UNSUPPORTED, "gemm_q4: 2^31 units of 256 k or more");
+  const long long rounds = (tiles + sms - 1) / sms, idle = (rounds * sms - tiles) * p.box;   // in units
+  const bool split = idle >= 4 * sms;
+  const long long least = (p.box + 7) / 8;
+  const long long grains = split ? units : tiles;
+  long long ctas = split ? units / least : tiles;
+  if (ctas > sms) ctas = sms;
+  p.grain = split ? 1 : (unsigned)p.box;
+  p.per = (unsigned)(grains / ctas);
+  p.longer = (unsigned)(grains % ctas);
+  if (MT == 32) return t2_launch<32>(tm1, tm2, tmw, p, (int)ctas, stream);
+  if (MT == 64) return t2_launch<64>(tm1, tm2, tmw, p, (int)ctas, stream);
+  return t2_launch<128>(tm1, tm2, tmw, p, (int)ctas, stream);
 }
 
 }  // namespace tlb

@@ -21,3 +21,26 @@ def test_calls_in_a_row_agree(M, K, N):
         assert (a - b).abs().max().item() < 1e-4 * a.std().item()
     for r in rest:
         assert all(torch.equal(a, b) for a, b in zip(first, r))
+
+
+@pytest.mark.parametrize("M,K,N", [
+    (9, 128, 100),        # one tile of half a box: one block
+    (32, 384, 129),       # two tiles, the second of one row; a box and a half
+    (33, 2048, 256),      # few tiles, every box a block of its own
+    (65, 4864, 896),      # tiles of several blocks, ragged on both sides
+    (517, 896, 1152),
+    (300, 18944, 3584),   # ranges that begin and end inside tiles
+    (1000, 3584, 4608),   # whole tiles, two to a block
+])
+def test_tiles_shared_by_blocks(M, K, N):
+    """Parts of a tile are summed in the order of k by whichever block is last: every call gives the same bits.
+    With alpha and beta, as the CUDA-core kernel within f32 sums in another order: about 2^-24 sqrt(K) <= 8e-6 of a
+    result, 25 times that for the largest."""
+    from cpp_tensorlib_b200 import cuda as tl
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    w = tl.to_q4(torch.randn((K, N), generator=g, device="cuda") * 0.02)
+    x = torch.randn((M, K), generator=g, device="cuda")
+    want = tl.gemm_q4(x, w, alpha=1.5, beta=0.25, simt=True)
+    got = [tl.gemm_q4(x, w, alpha=1.5, beta=0.25) for _ in range(6)]
+    assert (want - got[0]).abs().max().item() < 2e-4 * want.std().item()
+    assert all(torch.equal(got[0], a) for a in got[1:])
