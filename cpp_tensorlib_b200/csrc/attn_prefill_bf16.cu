@@ -7,7 +7,7 @@
 //    f32 and enter as three bf16 planes each (8 + 8 + 8 mantissa bits, nothing dropped), so the products are those
 //    of the f32 path: three MMAs a step where the tf32 split of attn_prefill_mma.cu would take two of half the
 //    depth at half the rate, and no conversion of K or V.
-//  * grid = (query tiles of 64, q heads), the tiles with most keys first.  Four warps own 16 query rows each, query
+//  * grid = (q heads, query tiles of 64), the tiles with most keys first over all heads.  Four warps own 16 query rows each, query
 //    planes and output accumulators in registers; K/V tiles of 64 keys arrive by TMA (boxes of 64 keys x 64
 //    dimensions, 128-byte swizzle) in a ring of three, 96 KB, so that two CTAs share an SM and the softmax of one
 //    runs under the MMAs of the other.
@@ -90,8 +90,8 @@ __global__ void __launch_bounds__(PB_THREADS, 2)
   unsigned char* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* full = (uint64_t*)(base + C::BARS);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int h = blockIdx.y, row0 = (h / p.group) * p.kv_rows;
-  const int q0 = (int)(gridDim.x - 1 - blockIdx.x) * PB_QT;
+  const int h = blockIdx.x, row0 = (h / p.group) * p.kv_rows;
+  const int q0 = (int)(gridDim.y - 1 - blockIdx.y) * PB_QT;
   if (tid == 0) {
     for (int s = 0; s < PB_STAGES; s++) mbar_init(&full[s], 1);
     mbar_fence_init();
@@ -268,7 +268,7 @@ int pb_launch(const PbParams& p, const void* K, const void* V, int n_q, int n_kv
   static std::atomic<unsigned long long> attr_done{0};
   const int rc = ensure_dynamic_smem(attn_prefill_bf16_kernel<D>, (int)PbCfg<D>::TOTAL, attr_done);
   if (rc) return rc;
-  LaunchCfg lc(dim3((p.T + PB_QT - 1) / PB_QT, n_q), dim3(PB_THREADS), PbCfg<D>::TOTAL, stream, pdl_enabled());
+  LaunchCfg lc(dim3(n_q, (p.T + PB_QT - 1) / PB_QT), dim3(PB_THREADS), PbCfg<D>::TOTAL, stream, pdl_enabled());
   TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, attn_prefill_bf16_kernel<D>, tm[0], tm[1], p));
   return TLB_OK;
 }

@@ -6,7 +6,8 @@
 // One CTA = 64 query rows of one head (4 warps of 16 rows) walking the keys its rows can see: the kept
 // positions first, then the window of its first row up to its last row, 64 keys a tile, fetched row by
 // row from the cache's kept slots and ring with 16-byte cp.async into a double buffer.  Scores and
-// products are mma.sync m16n8k16 with bf16 operands; a tile that every row of a warp sees whole skips
+// products are mma.sync m16n8k16 with bf16 operands.  The tiles with most keys start first, over all heads, so
+// that the short ones fill the end (head by head a third of the SM time was idle); a tile that every row of a warp sees whole skips
 // the mask.  Query/key widths up to 192, values up to 128 (rounded up to a tile width with zero columns).
 #include "mixers.cuh"
 #include "rows_mma.cuh"
@@ -47,7 +48,7 @@ __global__ void __launch_bounds__(AW_THREADS, 2)
   B* ks = (B*)(smem + S::K);
   B* vs = (B*)(smem + S::V);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int r0 = (gridDim.x - 1 - blockIdx.x) * AW_M, h = blockIdx.y, g = h / p.R;
+  const int r0 = (gridDim.y - 1 - blockIdx.y) * AW_M, h = blockIdx.x, g = h / p.R;
   const int nrow = rows - r0 < AW_M ? rows - r0 : AW_M;
   const int dch = p.kw / 8, qch = dch + p.k2w / 8, ech = p.vw / 8;
   // zero columns behind the widths: never written again
@@ -216,7 +217,7 @@ int aw_launch(const AttnTiles& p, void* out, long long ldo, int rows, int pos0, 
   static std::atomic<unsigned long long> done{0};
   const int rc = ensure_dynamic_smem(attn_window_kernel<DK, DV>, smem, done);
   if (rc) return rc;
-  LaunchCfg lc(dim3((rows + AW_M - 1) / AW_M, p.H), dim3(AW_THREADS), smem, s, pdl_enabled());
+  LaunchCfg lc(dim3(p.H, (rows + AW_M - 1) / AW_M), dim3(AW_THREADS), smem, s, pdl_enabled());
   TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, attn_window_kernel<DK, DV>, p, (__nv_bfloat16*)out, ldo, rows, pos0));
   return TLB_OK;
 }
