@@ -14,7 +14,13 @@
 // accumulators for the whole pass.
 //
 //   delta_solve   (chunk, head): T of every chunk, in two planes
-//   recur_chunk   (32 value columns, head): the chunks in order
+//   recur_chunk   (32 or 16 value columns, head, segment): a segment's chunks in order
+//   ssd_state     the same grid: what a segment adds to the state, without its outputs
+//
+// The delta rule is one segment.  The state of ssd only decays by a scalar between two places, so a long prompt
+// is cut into segments that run at once: ssd_state first leaves each segment's own state and log decay, and
+// recur_chunk starts from what the segments in front add up to.  One walk over the chunks has four warps an SM
+// and waits on its own latencies; two CTAs an SM and the second, shorter walk take less.
 #include "mixers.cuh"
 #include "rows_mma.cuh"
 
@@ -22,6 +28,9 @@ namespace tlb {
 
 namespace {
 
+#ifndef RC_MOST
+#define RC_MOST 8
+#endif
 constexpr int RC_L = 64, RC_E = 32, RC_THREADS = 128;
 constexpr int RC_TLD = RC_L + 8, RC_ELD = RC_E + 8;
 
@@ -141,28 +150,36 @@ __global__ void __launch_bounds__(RC_THREADS) delta_solve_kernel(const __grid_co
   }
 }
 
-// ---- the chunks of one head and 32 value columns -----------------------------------------------
-template <int DP, bool DELTA>
+// ---- the chunks of one head and CE value columns -----------------------------------------------
+template <int DP, bool DELTA, int CE>
 struct RcSmem {
   static constexpr int LD = DP + 8;
   static constexpr size_t K = 0;                                            // [2][64][LD]
   static constexpr size_t Q = K + (size_t)2 * RC_L * LD * 2;
   static constexpr size_t X = Q + (size_t)2 * RC_L * LD * 2;                // [2][64][ELD]
-  static constexpr size_t S = X + (size_t)2 * RC_L * RC_ELD * 2;            // [2 planes][DP][ELD]
-  static constexpr size_t W = S + (size_t)2 * DP * RC_ELD * 2;              // [2 planes][64][ELD]
-  static constexpr size_t U = W + (size_t)2 * RC_L * RC_ELD * 2;            // delta: [2 planes][64][ELD]
-  static constexpr size_t T = U + (DELTA ? (size_t)2 * RC_L * RC_ELD * 2 : 0);   // delta: [2][2 planes][64][TLD]
+  static constexpr size_t S = X + (size_t)2 * RC_L * (CE + 8) * 2;            // [2 planes][DP][ELD]
+  static constexpr size_t W = S + (size_t)2 * DP * (CE + 8) * 2;              // [2 planes][64][ELD]
+  static constexpr size_t U = W + (size_t)2 * RC_L * (CE + 8) * 2;            // delta: [2 planes][64][ELD]
+  static constexpr size_t T = U + (DELTA ? (size_t)2 * RC_L * (CE + 8) * 2 : 0);   // delta: [2][2 planes][64][TLD]
   static constexpr size_t SC = T + (DELTA ? (size_t)4 * RC_L * RC_TLD * 2 : 0);  // [4][64] f32
   static constexpr size_t TOTAL = SC + 4 * RC_L * 4;
 };
 
-template <int DP, bool DELTA>
+// Segments of `chunks` chunks each.  carry [segments][H][D][E]: the state in front of the prompt, then every
+// segment's own but the last; decay [segments][H]: its log decay.  One segment: no carry.
+struct RcSegments {
+  int n, chunks;
+  float *carry, *decay;
+};
+
+template <int DP, bool DELTA, int CE>
 __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
     recur_chunk_kernel(const __grid_constant__ RecurP p, const __nv_bfloat16* __restrict__ conv,
                        const float2* __restrict__ gates, const float2* __restrict__ norms,
-                       const __nv_bfloat16* __restrict__ T, float* __restrict__ o, int rows, int pos0) {
-  using SM = RcSmem<DP, DELTA>;
-  constexpr int LD = SM::LD, MT = DP / 64;      // state row tiles of 16 per warp
+                       const __nv_bfloat16* __restrict__ T, float* __restrict__ o, int rows, int pos0,
+                       const __grid_constant__ RcSegments g) {
+  using SM = RcSmem<DP, DELTA, CE>;
+  constexpr int LD = SM::LD, MT = DP / 64, NT = CE / 8;   // state row tiles of 16 per warp, column tiles
   extern __shared__ __align__(16) unsigned char smem[];
   __nv_bfloat16* ksm = (__nv_bfloat16*)(smem + SM::K);
   __nv_bfloat16* qsm = (__nv_bfloat16*)(smem + SM::Q);
@@ -176,8 +193,9 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
   float* snk = sg + RC_L;                       // 1 / |k_s|
   float* snq = snk + RC_L;                      // D^-1/2 / |q_t|
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wr = warp * 16;
-  const int h = blockIdx.y, c0 = blockIdx.x * RC_E, kg = h / (p.H / p.G), D = p.D, E = p.E;
-  const int nch = (rows + RC_L - 1) / RC_L, dch = D / 8, ech = (E - c0 < RC_E ? E - c0 : RC_E) / 8;
+  const int h = blockIdx.y, c0 = blockIdx.x * CE, kg = h / (p.H / p.G), D = p.D, E = p.E;
+  const int nch = (rows + RC_L - 1) / RC_L, ch0 = (int)blockIdx.z * g.chunks, ch1 = ch0 + g.chunks < nch ? ch0 + g.chunks : nch;
+  const int dch = D / 8, ech = (E - c0 < CE ? E - c0 : CE) / 8;
   for (int i = tid; i < (int)(SM::SC / 16); i += RC_THREADS) ((uint4*)smem)[i] = make_uint4(0, 0, 0, 0);
   pdl_wait();
   pdl_launch_dependents();
@@ -194,7 +212,7 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
     for (int i = tid; i < RC_L * ech; i += RC_THREADS) {
       const int r = i / ech, c = i - r * ech;
       const bool on = r < n;
-      rc_cp16(xsm + (buf * RC_L + r) * RC_ELD + c * 8, conv + (size_t)(on ? t0 + r : t0) * p.cv.C + p.cvv + h * E + c0 + c * 8, on);
+      rc_cp16(xsm + (buf * RC_L + r) * (CE + 8) + c * 8, conv + (size_t)(on ? t0 + r : t0) * p.cv.C + p.cvv + h * E + c0 + c * 8, on);
     }
     if (DELTA) {
       const __nv_bfloat16* src = T + ((size_t)ch * p.H + h) * 2 * RC_L * RC_L;
@@ -214,8 +232,8 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
       n1 = t1 < rows ? norms[(size_t)t1 * p.G + kg] : z;
     }
   };
-  // state: this warp's rows of it, 32 columns, as accumulators
-  float s[MT][4][4];
+  // state: this warp's rows of it, CE columns, as accumulators
+  float s[MT][NT][4];
   float* S = p.S + (size_t)h * D * E;
   auto state_at = [&](int mt, int nt, int e, int& r, int& c) {
     r = (warp * MT + mt) * 16 + (lane >> 2) + (e >> 1) * 8;
@@ -224,30 +242,50 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
 #pragma unroll
   for (int mt = 0; mt < MT; mt++)
 #pragma unroll
-    for (int nt = 0; nt < 4; nt++)
+    for (int nt = 0; nt < NT; nt++)
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         int r, c;
         state_at(mt, nt, e, r, c);
-        s[mt][nt][e] = pos0 > 0 && r < D && c < E ? S[(size_t)r * E + c] : 0.f;
+        s[mt][nt][e] = pos0 > 0 && g.n == 1 && r < D && c < E ? S[(size_t)r * E + c] : 0.f;
       }
-  fetch(0, 0);
+  if (!DELTA && g.n > 1) {
+    const size_t HS = (size_t)p.H * D * E;
+    for (int j = pos0 > 0 ? 0 : 1; j <= (int)blockIdx.z; j++) {
+      const float* C = g.carry + j * HS + (size_t)h * D * E;
+      const float f = j > 0 ? expf(g.decay[(j - 1) * p.H + h]) : 0.f;
+#pragma unroll
+      for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) {
+            int r, c;
+            state_at(mt, nt, e, r, c);
+            if (r >= D || c >= E) continue;   // E is even
+            const float2 v = __ldcg((const float2*)(C + (size_t)r * E + c));
+            s[mt][nt][e] = fmaf(f, s[mt][nt][e], v.x);
+            s[mt][nt][e + 1] = fmaf(f, s[mt][nt][e + 1], v.y);
+          }
+    }
+  }
+  fetch(ch0, 0);
   rc_commit();
-  if (warp == 0) scalars(0);
-  for (int ch = 0; ch < nch; ch++) {
-    const int buf = ch & 1, t0 = ch * RC_L, n = rows - t0 < RC_L ? rows - t0 : RC_L;
+  if (warp == 0) scalars(ch0);
+  for (int ch = ch0; ch < ch1; ch++) {
+    const int buf = (ch - ch0) & 1, t0 = ch * RC_L, n = rows - t0 < RC_L ? rows - t0 : RC_L;
     // the state in front of the chunk, in two planes, for the products below
 #pragma unroll
     for (int mt = 0; mt < MT; mt++)
 #pragma unroll
-      for (int nt = 0; nt < 4; nt++)
+      for (int nt = 0; nt < NT; nt++)
 #pragma unroll
         for (int e = 0; e < 2; e++) {
           uint32_t hi, lo;
           rc_split(s[mt][nt][2 * e], s[mt][nt][2 * e + 1], hi, lo);
-          const int at = ((warp * MT + mt) * 16 + (lane >> 2) + e * 8) * RC_ELD + nt * 8 + (lane & 3) * 2;
+          const int at = ((warp * MT + mt) * 16 + (lane >> 2) + e * 8) * (CE + 8) + nt * 8 + (lane & 3) * 2;
           *(uint32_t*)(ssm + at) = hi;
-          *(uint32_t*)(ssm + DP * RC_ELD + at) = lo;
+          *(uint32_t*)(ssm + DP * (CE + 8) + at) = lo;
         }
     if (warp == 0) {
       float b0, b1;
@@ -255,48 +293,55 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
       sb[lane] = b0; sb[lane + 32] = b1;
       sg[lane] = g0.x; sg[lane + 32] = g1.x;
       if (DELTA) { snk[lane] = n0.y; snk[lane + 32] = n1.y; snq[lane] = n0.x; snq[lane + 32] = n1.x; }
-      if (ch + 1 < nch) scalars(ch + 1);
+      if (ch + 1 < ch1) scalars(ch + 1);
     }
     rc_wait<0>();
     __syncthreads();
-    if (ch + 1 < nch) {
+    if (ch + 1 < ch1) {
       fetch(ch + 1, buf ^ 1);
       rc_commit();
     }
-    const __nv_bfloat16 *K = ksm + buf * RC_L * LD, *Q = qsm + buf * RC_L * LD, *X = xsm + buf * RC_L * RC_ELD;
+    const __nv_bfloat16 *K = ksm + buf * RC_L * LD, *Q = qsm + buf * RC_L * LD, *X = xsm + buf * RC_L * (CE + 8);
     const int ra = wr + (lane >> 2), cb = (lane & 3) * 2;     // the thread's rows are ra and ra + 8
     const float ba = sb[ra], bb = sb[ra + 8], bL = sb[RC_L - 1];
     // q S, k S (both planes of S), q k^T for the rows of this warp
-    float qs[4][4], kS[4][4], m[8][4];
+    float qs[NT][4], kS[NT][4], m[8][4];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int e = 0; e < 4; e++) {
 #pragma unroll
-      for (int e = 0; e < 4; e++) qs[i][e] = kS[i][e] = m[i][e] = m[i + 4][e] = 0.f;
+      for (int i = 0; i < NT; i++) qs[i][e] = kS[i][e] = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; i++) m[i][e] = 0.f;
+    }
 #pragma unroll
     for (int k = 0; k < DP; k += 16) {
       uint32_t aq[4], ak[4];
       rc_ldm(aq, rc_a(Q, LD, wr, k, lane));
       if (DELTA) rc_ldm(ak, rc_a(K, LD, wr, k, lane));
+      uint32_t bs[2][CE / 16][4], bk[4][4];   // all of a step's fragments first: one shared-memory latency a step
 #pragma unroll
       for (int pl = 0; pl < 2; pl++)
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-          uint32_t b[4];
-          rc_ldmt(b, rc_bk(ssm + pl * DP * RC_ELD, RC_ELD, k, j * 16, lane));
-          rc_mma(qs[2 * j], aq, b[0], b[1]);
-          rc_mma(qs[2 * j + 1], aq, b[2], b[3]);
+        for (int j = 0; j < CE / 16; j++) rc_ldmt(bs[pl][j], rc_bk(ssm + pl * DP * (CE + 8), (CE + 8), k, j * 16, lane));
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (j <= warp) rc_ldm(bk[j], rc_bn(K, LD, j * 16, k, lane));
+#pragma unroll
+      for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+        for (int j = 0; j < CE / 16; j++) {
+          rc_mma(qs[2 * j], aq, bs[pl][j][0], bs[pl][j][1]);
+          rc_mma(qs[2 * j + 1], aq, bs[pl][j][2], bs[pl][j][3]);
           if (DELTA) {
-            rc_mma(kS[2 * j], ak, b[0], b[1]);
-            rc_mma(kS[2 * j + 1], ak, b[2], b[3]);
+            rc_mma(kS[2 * j], ak, bs[pl][j][0], bs[pl][j][1]);
+            rc_mma(kS[2 * j + 1], ak, bs[pl][j][2], bs[pl][j][3]);
           }
         }
 #pragma unroll
       for (int j = 0; j < 4; j++)
         if (j <= warp) {
-          uint32_t b[4];
-          rc_ldm(b, rc_bn(K, LD, j * 16, k, lane));
-          rc_mma(m[2 * j], aq, b[0], b[1]);
-          rc_mma(m[2 * j + 1], aq, b[2], b[3]);
+          rc_mma(m[2 * j], aq, bk[j][0], bk[j][1]);
+          rc_mma(m[2 * j + 1], aq, bk[j][2], bk[j][3]);
         }
     }
     // decays (and unit norms, step sizes) of q k^T, then as operand planes
@@ -318,22 +363,22 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
       // R = v - exp(b) |k|^-1 (k S), in planes
       const float fa = expf(ba) * snk[ra], fb = expf(bb) * snk[ra + 8];
 #pragma unroll
-      for (int j = 0; j < 4; j++)
+      for (int j = 0; j < NT; j++)
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-          const int at = (ra + 8 * e) * RC_ELD + j * 8 + cb;
+          const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
           const uint32_t v = *(const uint32_t*)(X + at);
           const float f = e ? fb : fa;
           uint32_t hi, lo;
           rc_split(fmaf(-f, kS[j][2 * e], __uint_as_float(v << 16)),
                    fmaf(-f, kS[j][2 * e + 1], __uint_as_float(v & 0xffff0000u)), hi, lo);
           *(uint32_t*)(usm + at) = hi;
-          *(uint32_t*)(usm + RC_L * RC_ELD + at) = lo;
+          *(uint32_t*)(usm + RC_L * (CE + 8) + at) = lo;
         }
       __syncthreads();
-      float u[4][4];
+      float u[NT][4];
 #pragma unroll
-      for (int i = 0; i < 4; i++) u[i][0] = u[i][1] = u[i][2] = u[i][3] = 0.f;
+      for (int i = 0; i < NT; i++) u[i][0] = u[i][1] = u[i][2] = u[i][3] = 0.f;
       const __nv_bfloat16* Tp = tsm + (size_t)buf * 2 * RC_L * RC_TLD;
 #pragma unroll
       for (int k = 0; k < 4; k++)
@@ -342,10 +387,10 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
           rc_ldm(ah, rc_a(Tp, RC_TLD, wr, k * 16, lane));
           rc_ldm(al, rc_a(Tp + RC_L * RC_TLD, RC_TLD, wr, k * 16, lane));
 #pragma unroll
-          for (int j = 0; j < 2; j++) {
+          for (int j = 0; j < CE / 16; j++) {
             uint32_t bh[4], bl[4];
-            rc_ldmt(bh, rc_bk(usm, RC_ELD, k * 16, j * 16, lane));
-            rc_ldmt(bl, rc_bk(usm + RC_L * RC_ELD, RC_ELD, k * 16, j * 16, lane));
+            rc_ldmt(bh, rc_bk(usm, (CE + 8), k * 16, j * 16, lane));
+            rc_ldmt(bl, rc_bk(usm + RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
             rc_mma(u[2 * j], ah, bh[0], bh[1]); rc_mma(u[2 * j + 1], ah, bh[2], bh[3]);
             rc_mma(u[2 * j], ah, bl[0], bl[1]); rc_mma(u[2 * j + 1], ah, bl[2], bl[3]);
             rc_mma(u[2 * j], al, bh[0], bh[1]); rc_mma(u[2 * j + 1], al, bh[2], bh[3]);
@@ -354,51 +399,51 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
       __syncthreads();   // R is read: its planes become U's
       const float ga = expf(bL - ba) * snk[ra], gb = expf(bL - bb) * snk[ra + 8];
 #pragma unroll
-      for (int j = 0; j < 4; j++)
+      for (int j = 0; j < NT; j++)
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-          const int at = (ra + 8 * e) * RC_ELD + j * 8 + cb;
+          const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
           const float f = e ? gb : ga;
           uint32_t hi, lo;
           rc_split(u[j][2 * e], u[j][2 * e + 1], hi, lo);
           *(uint32_t*)(usm + at) = hi;
-          *(uint32_t*)(usm + RC_L * RC_ELD + at) = lo;
+          *(uint32_t*)(usm + RC_L * (CE + 8) + at) = lo;
           rc_split(u[j][2 * e] * f, u[j][2 * e + 1] * f, hi, lo);
           *(uint32_t*)(wsm + at) = hi;
-          *(uint32_t*)(wsm + RC_L * RC_ELD + at) = lo;
+          *(uint32_t*)(wsm + RC_L * (CE + 8) + at) = lo;
         }
     } else {
       const float ga = expf(bL - ba) * sg[ra], gb = expf(bL - bb) * sg[ra + 8];
 #pragma unroll
-      for (int j = 0; j < 4; j++)
+      for (int j = 0; j < NT; j++)
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-          const int at = (ra + 8 * e) * RC_ELD + j * 8 + cb;
+          const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
           const uint32_t v = *(const uint32_t*)(X + at);
           const float f = e ? gb : ga;
           uint32_t hi, lo;
           rc_split(f * __uint_as_float(v << 16), f * __uint_as_float(v & 0xffff0000u), hi, lo);
           *(uint32_t*)(wsm + at) = hi;
-          *(uint32_t*)(wsm + RC_L * RC_ELD + at) = lo;
+          *(uint32_t*)(wsm + RC_L * (CE + 8) + at) = lo;
         }
     }
     __syncthreads();
     // O = exp(b) (q S) + M U
     const float ea = expf(ba) * qa, eb = expf(bb) * qb;
 #pragma unroll
-    for (int j = 0; j < 4; j++) { qs[j][0] *= ea; qs[j][1] *= ea; qs[j][2] *= eb; qs[j][3] *= eb; }
+    for (int j = 0; j < NT; j++) { qs[j][0] *= ea; qs[j][1] *= ea; qs[j][2] *= eb; qs[j][3] *= eb; }
     const __nv_bfloat16* Up = DELTA ? usm : X;
 #pragma unroll
     for (int k = 0; k < 4; k++)
       if (k <= warp) {
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
+        for (int j = 0; j < CE / 16; j++) {
           uint32_t b[4];
-          rc_ldmt(b, rc_bk(Up, RC_ELD, k * 16, j * 16, lane));
+          rc_ldmt(b, rc_bk(Up, (CE + 8), k * 16, j * 16, lane));
           rc_mma(qs[2 * j], mh[k], b[0], b[1]); rc_mma(qs[2 * j + 1], mh[k], b[2], b[3]);
           rc_mma(qs[2 * j], ml[k], b[0], b[1]); rc_mma(qs[2 * j + 1], ml[k], b[2], b[3]);
           if (DELTA) {
-            rc_ldmt(b, rc_bk(usm + RC_L * RC_ELD, RC_ELD, k * 16, j * 16, lane));
+            rc_ldmt(b, rc_bk(usm + RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
             rc_mma(qs[2 * j], mh[k], b[0], b[1]); rc_mma(qs[2 * j + 1], mh[k], b[2], b[3]);
           }
         }
@@ -409,7 +454,7 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
       if (t < n) {
         float* dst = o + ((size_t)(t0 + t) * p.H + h) * E + c0;
 #pragma unroll
-        for (int j = 0; j < 4; j++)
+        for (int j = 0; j < NT; j++)
           if (j < ech) *(float2*)(dst + j * 8 + cb) = make_float2(qs[j][2 * e], qs[j][2 * e + 1]);
       }
     }
@@ -418,7 +463,7 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
 #pragma unroll
     for (int mt = 0; mt < MT; mt++)
 #pragma unroll
-      for (int nt = 0; nt < 4; nt++)
+      for (int nt = 0; nt < NT; nt++)
 #pragma unroll
         for (int e = 0; e < 4; e++) s[mt][nt][e] *= eL;
 #pragma unroll
@@ -426,31 +471,201 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
       uint32_t a[MT][4];
 #pragma unroll
       for (int mt = 0; mt < MT; mt++) rc_ldmt(a[mt], rc_at(K, LD, (warp * MT + mt) * 16, k * 16, lane));
+      uint32_t b[2][CE / 16][4];
 #pragma unroll
       for (int pl = 0; pl < 2; pl++)
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-          uint32_t b[4];
-          rc_ldmt(b, rc_bk(wsm + pl * RC_L * RC_ELD, RC_ELD, k * 16, j * 16, lane));
+        for (int j = 0; j < CE / 16; j++) rc_ldmt(b[pl][j], rc_bk(wsm + pl * RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
+#pragma unroll
+      for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+        for (int j = 0; j < CE / 16; j++)
 #pragma unroll
           for (int mt = 0; mt < MT; mt++) {
-            rc_mma(s[mt][2 * j], a[mt], b[0], b[1]);
-            rc_mma(s[mt][2 * j + 1], a[mt], b[2], b[3]);
+            rc_mma(s[mt][2 * j], a[mt], b[pl][j][0], b[pl][j][1]);
+            rc_mma(s[mt][2 * j + 1], a[mt], b[pl][j][2], b[pl][j][3]);
           }
-        }
     }
     __syncthreads();   // the chunk's operands and planes are read: the next one may overwrite them
   }
+  if ((int)blockIdx.z != g.n - 1) return;
 #pragma unroll
   for (int mt = 0; mt < MT; mt++)
 #pragma unroll
-    for (int nt = 0; nt < 4; nt++)
+    for (int nt = 0; nt < NT; nt++)
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         int r, c;
         state_at(mt, nt, e, r, c);
         if (r < D && c < E) S[(size_t)r * E + c] = s[mt][nt][e];
       }
+}
+
+// ---- what a segment adds to the state of ssd -------------------------------------------------------
+template <int DP>
+struct SsSmem {
+  static constexpr int LD = DP + 8;
+  static constexpr size_t K = 0;                                            // [2][64][LD]
+  static constexpr size_t X = K + (size_t)2 * RC_L * LD * 2;                // [2][64][ELD]
+  static constexpr size_t W = X + (size_t)2 * RC_L * RC_ELD * 2;            // [2 planes][64][ELD]
+  static constexpr size_t SC = W + (size_t)2 * RC_L * RC_ELD * 2;           // [2][64] f32
+  static constexpr size_t TOTAL = SC + 2 * RC_L * 4;
+};
+
+template <int DP>
+__global__ void __launch_bounds__(RC_THREADS, 3)
+    ssd_state_kernel(const __grid_constant__ RecurP p, const __nv_bfloat16* __restrict__ conv,
+                     const float2* __restrict__ gates, int pos0, const __grid_constant__ RcSegments g) {
+  using SM = SsSmem<DP>;
+  constexpr int LD = SM::LD, MT = DP / 64;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __nv_bfloat16* ksm = (__nv_bfloat16*)(smem + SM::K);
+  __nv_bfloat16* xsm = (__nv_bfloat16*)(smem + SM::X);
+  __nv_bfloat16* wsm = (__nv_bfloat16*)(smem + SM::W);
+  float* sb = (float*)(smem + SM::SC);
+  float* sg = sb + RC_L;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = blockIdx.y, c0 = blockIdx.x * RC_E, kg = h / (p.H / p.G), D = p.D, E = p.E;
+  const int ch0 = (int)blockIdx.z * g.chunks, ch1 = ch0 + g.chunks;   // never the last segment: all chunks whole
+  const int dch = D / 8, ech = (E - c0 < RC_E ? E - c0 : RC_E) / 8;
+  for (int i = tid; i < (int)(SM::SC / 16); i += RC_THREADS) ((uint4*)smem)[i] = make_uint4(0, 0, 0, 0);
+  pdl_wait();
+  pdl_launch_dependents();
+  __syncthreads();
+  auto fetch = [&](int ch, int buf) {
+    const __nv_bfloat16* base = conv + (size_t)ch * RC_L * p.cv.C;
+    for (int i = tid; i < RC_L * dch; i += RC_THREADS) {
+      const int r = i / dch, c = i - r * dch;
+      rc_cp16(ksm + (buf * RC_L + r) * LD + c * 8, base + (size_t)r * p.cv.C + p.ck + kg * D + c * 8, true);
+    }
+    for (int i = tid; i < RC_L * ech; i += RC_THREADS) {
+      const int r = i / ech, c = i - r * ech;
+      rc_cp16(xsm + (buf * RC_L + r) * RC_ELD + c * 8, base + (size_t)r * p.cv.C + p.cvv + h * E + c0 + c * 8, true);
+    }
+  };
+  float2 g0, g1;
+  auto scalars = [&](int ch) {
+    g0 = gates[(size_t)(ch * RC_L + lane) * p.H + h];
+    g1 = gates[(size_t)(ch * RC_L + lane + 32) * p.H + h];
+  };
+  float s[MT][4][4], total = 0.f;
+#pragma unroll
+  for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++) s[mt][nt][0] = s[mt][nt][1] = s[mt][nt][2] = s[mt][nt][3] = 0.f;
+  fetch(ch0, 0);
+  rc_commit();
+  if (warp == 0) scalars(ch0);
+  for (int ch = ch0; ch < ch1; ch++) {
+    const int buf = (ch - ch0) & 1;
+    if (warp == 0) {
+      float b0, b1;
+      rc_scan(g0.y, g1.y, b0, b1);
+      sb[lane] = b0; sb[lane + 32] = b1;
+      sg[lane] = g0.x; sg[lane + 32] = g1.x;
+      if (ch + 1 < ch1) scalars(ch + 1);
+    }
+    rc_wait<0>();
+    __syncthreads();
+    if (ch + 1 < ch1) {
+      fetch(ch + 1, buf ^ 1);
+      rc_commit();
+    }
+    const __nv_bfloat16 *K = ksm + buf * RC_L * LD, *X = xsm + buf * RC_L * RC_ELD;
+    const float bL = sb[RC_L - 1];
+    total += bL;
+    // a thread's token, half of its 32 columns: exp(b_L - b_s) dt_s x_s in two planes
+    {
+      const int t = tid >> 1, at = t * RC_ELD + (tid & 1) * 16;
+      const float f = expf(bL - sb[t]) * sg[t];
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const uint32_t v = *(const uint32_t*)(X + at + 2 * i);
+        uint32_t hi, lo;
+        rc_split(f * __uint_as_float(v << 16), f * __uint_as_float(v & 0xffff0000u), hi, lo);
+        *(uint32_t*)(wsm + at + 2 * i) = hi;
+        *(uint32_t*)(wsm + RC_L * RC_ELD + at + 2 * i) = lo;
+      }
+    }
+    const float eL = expf(bL);
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+      for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) s[mt][nt][e] *= eL;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      uint32_t a[MT][4], b[2][2][4];
+#pragma unroll
+      for (int mt = 0; mt < MT; mt++) rc_ldmt(a[mt], rc_at(K, LD, (warp * MT + mt) * 16, k * 16, lane));
+#pragma unroll
+      for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) rc_ldmt(b[pl][j], rc_bk(wsm + pl * RC_L * RC_ELD, RC_ELD, k * 16, j * 16, lane));
+#pragma unroll
+      for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+          for (int mt = 0; mt < MT; mt++) {
+            rc_mma(s[mt][2 * j], a[mt], b[pl][j][0], b[pl][j][1]);
+            rc_mma(s[mt][2 * j + 1], a[mt], b[pl][j][2], b[pl][j][3]);
+          }
+    }
+    __syncthreads();   // the chunk's operands and scalars are read: the next one may overwrite them
+  }
+  const size_t HS = (size_t)p.H * D * E;
+  const float* S = p.S + (size_t)h * D * E;
+  float* out = g.carry + (blockIdx.z + 1) * HS + (size_t)h * D * E;
+#pragma unroll
+  for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+      for (int e = 0; e < 4; e += 2) {
+        const int r = (warp * MT + mt) * 16 + (lane >> 2) + (e >> 1) * 8, c = c0 + nt * 8 + (lane & 3) * 2;
+        if (r >= D || c >= E) continue;
+        *(float2*)(out + (size_t)r * E + c) = make_float2(s[mt][nt][e], s[mt][nt][e + 1]);
+        // the next kernel's last segment overwrites the state, so that its others read a copy
+        if (blockIdx.z == 0 && pos0 > 0)
+          *(float2*)(g.carry + (size_t)h * D * E + (size_t)r * E + c) = *(const float2*)(S + (size_t)r * E + c);
+      }
+  if (blockIdx.x == 0 && tid == 0) g.decay[blockIdx.z * p.H + h] = total;
+}
+
+// Most segments of a prompt (more rows, no fewer): of four chunks at least, since a segment's start reads the states in
+// front of it, eight at most, and no more than four CTAs for each of the places that 148 SMs have.
+int rc_most_segments(const RecurP& p, int rows) {
+  if (p.kind == MIX_DELTA) return 1;
+  const int nch = (rows + RC_L - 1) / RC_L, ctas = (p.E + RC_E - 1) / RC_E * p.H;
+  int n = nch / 4 < RC_MOST ? nch / 4 : RC_MOST;
+  if (n * ctas > 4 * 2 * 148) n = 4 * 2 * 148 / ctas;
+  return n < 2 ? 1 : n;
+}
+RcSegments rc_segments(const RecurP& p, int rows, void* scratch) {
+  const int nch = (rows + RC_L - 1) / RC_L, n = rc_most_segments(p, rows);
+  RcSegments g{1, nch, nullptr, nullptr};
+  if (n == 1) return g;
+  g.chunks = (nch + n - 1) / n;
+  g.n = (nch + g.chunks - 1) / g.chunks;
+  g.carry = (float*)scratch;
+  g.decay = g.carry + (size_t)g.n * p.H * p.D * p.E;
+  return g;
+}
+
+template <int DP, bool DELTA, int CE>
+int rc_walk(const RecurP& p, const void* conv, const float2* gates, const float2* norms, const void* T, float* o, int rows,
+            int pos0, const RcSegments& g, cudaStream_t s) {
+  constexpr int smem = (int)RcSmem<DP, DELTA, CE>::TOTAL;
+  static std::atomic<unsigned long long> done{0};
+  const int rc = ensure_dynamic_smem(recur_chunk_kernel<DP, DELTA, CE>, smem, done);
+  if (rc) return rc;
+  LaunchCfg lc(dim3((p.E + CE - 1) / CE, p.H, g.n), dim3(RC_THREADS), smem, s, pdl_enabled());
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, recur_chunk_kernel<DP, DELTA, CE>, p, (const __nv_bfloat16*)conv, gates, norms,
+                              (const __nv_bfloat16*)T, o, rows, pos0, g));
+  return TLB_OK;
 }
 
 template <int DP, bool DELTA>
@@ -465,14 +680,19 @@ int rc_launch(const RecurP& p, const void* conv, const float2* gates, const floa
     TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, delta_solve_kernel<DP>, p, (const __nv_bfloat16*)conv, gates, norms,
                                 (__nv_bfloat16*)T, rows));
   }
-  constexpr int smem = (int)RcSmem<DP, DELTA>::TOTAL;
-  static std::atomic<unsigned long long> done{0};
-  const int rc = ensure_dynamic_smem(recur_chunk_kernel<DP, DELTA>, smem, done);
-  if (rc) return rc;
-  LaunchCfg lc(dim3((p.E + RC_E - 1) / RC_E, p.H), dim3(RC_THREADS), smem, s, pdl_enabled());
-  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, recur_chunk_kernel<DP, DELTA>, p, (const __nv_bfloat16*)conv, gates, norms,
-                              (const __nv_bfloat16*)T, o, rows, pos0));
-  return TLB_OK;
+  const RcSegments g = rc_segments(p, rows, T);
+  if (!DELTA && g.n > 1) {
+    constexpr int smem = (int)SsSmem<DP>::TOTAL;
+    static std::atomic<unsigned long long> done{0};
+    const int rc = ensure_dynamic_smem(ssd_state_kernel<DP>, smem, done);
+    if (rc) return rc;
+    LaunchCfg lc(dim3((p.E + RC_E - 1) / RC_E, p.H, g.n - 1), dim3(RC_THREADS), smem, s, pdl_enabled());
+    TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, ssd_state_kernel<DP>, p, (const __nv_bfloat16*)conv, gates, pos0, g));
+  }
+  // few heads: half as many columns a CTA, twice the CTAs (16 heads of 128 on 148 SMs: 64 CTAs or 128)
+  if constexpr (DELTA)
+    if ((p.E + RC_E - 1) / RC_E * p.H <= 74) return rc_walk<DP, DELTA, 16>(p, conv, gates, norms, T, o, rows, pos0, g, s);
+  return rc_walk<DP, DELTA, RC_E>(p, conv, gates, norms, T, o, rows, pos0, g, s);
 }
 
 }  // namespace
@@ -480,7 +700,9 @@ int rc_launch(const RecurP& p, const void* conv, const float2* gates, const floa
 bool recur_chunk_eligible(const RecurP& p) { return p.D <= 128 && p.D % 8 == 0 && p.E % 8 == 0 && p.cv.taps <= 8; }
 
 size_t recur_chunk_scratch_bytes(const RecurP& p, int rows) {
-  return p.kind == MIX_DELTA ? (size_t)((rows + RC_L - 1) / RC_L) * p.H * 2 * RC_L * RC_L * 2 : 0;
+  if (p.kind == MIX_DELTA) return (size_t)((rows + RC_L - 1) / RC_L) * p.H * 2 * RC_L * RC_L * 2;
+  const int n = rc_most_segments(p, rows);
+  return n > 1 ? (size_t)n * p.H * ((size_t)p.D * p.E + 1) * sizeof(float) : 0;
 }
 
 int recur_chunk_launch(const RecurP& p, const void* conv, const float2* gates, const float2* norms, void* scratch,

@@ -387,3 +387,19 @@ def test_qwen2_folder_through_the_registry(tmp_path):
     torch.cuda.synchronize()
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("rows,first", [(512, 0), (575, 0), (1100, 100), (2112, 37)])
+def test_long_prompt_in_segments(rows, first):
+    """A prompt long enough for the ssd state to be cut into segments (two to eight, the last one ragged, with and
+    without a state in front) against the same tokens in portions too short for it.  Both keep the state in f32; its
+    sums differ in order, and what that moves in the bf16 roundings behind it is judged like bf16 elsewhere here."""
+    cfg = zc.config([zc.mam(6, 2, 128, 64, 4, 2), zc.mam(4, 2, 64, 128, 4, 1), zc.mam(2, 1, 48, 40, 3, 2)], width=128,
+                    vocab=160, emb=3.0)
+    w = zc.Weights(cfg, 61)
+    toks = zc.tokens(cfg, first + rows + 3, 9)
+    m = make(cfg, w, "bfloat16", 2400)
+    want = run(m, toks, [448] * 9)
+    got = run(m, toks, [first, rows] if first else [rows])
+    assert ok(err(got, want), "bfloat16")
+    close(m)
