@@ -10,8 +10,8 @@
 // operands (64-k stages, 128-byte swizzle, boxes past M, N or K read as zeros), warp 1 issues
 // tcgen05.mma (the whole warp runs the loop, one elected lane issues), warps 4-7 read the
 // accumulator back with tcgen05.ld and store.  Two TMEM accumulators in rotation, so the epilogue
-// of a tile runs under the products of the next.  BN (32 / 64 / 128 / 256) is picked on the host so
-// that short prompts still occupy the SMs.  All waits are bounded: a timeout sets the status word,
+// of a tile runs under the products of the next.  BN, any multiple of 16 up to 256, is picked on the host
+// so that the tiles fill their last round over the SMs (gt_width).  All waits are bounded: a timeout sets the status word,
 // the kernel frees its TMEM and returns.  No cluster launch, no multicast.
 #include <cuda_bf16.h>
 
@@ -32,19 +32,24 @@ struct GtParams {
   __nv_bfloat16* O;
   long long ldo;
   int M, N, K;
-  int mt, nt;        // tiles along M and N
+  int mt, nt, bn;    // tiles along M and N, their width
   float limit;
   int* status;
 };
 
-template <int BN>
+// shared memory for tiles of width bn: stages of A, stages of B, barriers, TMEM address
+constexpr int GT_STAGES = 8;   // most
 struct GtSmem {
-  static constexpr int STAGES = BN == 256 ? 4 : (BN == 128 ? 6 : 8);
-  static constexpr size_t A = 0;
-  static constexpr size_t B = A + (size_t)STAGES * GT_M * 128;
-  static constexpr size_t BARS = B + (size_t)STAGES * BN * 128;
-  static constexpr size_t SLOT = BARS + (2 * STAGES + 4) * 8;
-  static constexpr size_t TOTAL = SLOT + 16 + 1024;
+  int stages;
+  uint32_t B, BARS, SLOT, TOTAL;
+  __host__ __device__ explicit GtSmem(int bn) {
+    const int n = (220 * 1024) / ((GT_M + bn) * 128);
+    stages = n < GT_STAGES ? n : GT_STAGES;
+    B = (uint32_t)(stages * GT_M * 128);
+    BARS = B + (uint32_t)(stages * bn * 128);
+    SLOT = BARS + (2 * GT_STAGES + 4) * 8;
+    TOTAL = SLOT + 16 + 1024;
+  }
 };
 
 __device__ __forceinline__ void gt_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
@@ -83,19 +88,20 @@ __device__ __forceinline__ bool gt_wait_warp(uint64_t* bar, uint32_t parity, int
   return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, status, where));
 }
 
-template <int BN, int EPI>
+template <int EPI>
 __global__ void __launch_bounds__(GT_THREADS, 1)
     gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GtParams p) {
-  using S = GtSmem<BN>;
-  constexpr int ST = S::STAGES;
-  constexpr uint32_t NCOLS = 2 * BN < 32 ? 32 : 2 * BN;
+  const int BN = p.bn;
+  const GtSmem S(BN);
+  const int ST = S.stages;
+  constexpr uint32_t NCOLS = 512;   // two accumulators of up to 256 columns
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  uint64_t* full = (uint64_t*)(base + S::BARS);
-  uint64_t* empty = full + ST;
-  uint64_t* dfull = empty + ST;
+  uint64_t* full = (uint64_t*)(base + S.BARS);
+  uint64_t* empty = full + GT_STAGES;
+  uint64_t* dfull = empty + GT_STAGES;
   uint64_t* dempty = dfull + 2;
-  uint32_t* slot = (uint32_t*)(base + S::SLOT);
+  uint32_t* slot = (uint32_t*)(base + S.SLOT);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nk = (p.K + GT_KS - 1) / GT_KS, tiles = p.mt * p.nt;
 
@@ -118,16 +124,17 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
 
   if (warp == 0) {
     if (lane == 0) {
-      int it = 0;
+      int s = 0;
+      uint32_t ph = 0;   // of the ring
       bool ok = true;
       for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
         const int m0 = (t % p.mt) * GT_M, n0 = (t / p.mt) * BN;
-        for (int k = 0; k < nk; k++, it++) {
-          const int s = it % ST;
-          if (!mbar_wait_bounded(&empty[s], ((it / ST) & 1) ^ 1, p.status, 700)) { ok = false; break; }
+        for (int k = 0; k < nk; k++) {
+          if (!mbar_wait_bounded(&empty[s], ph ^ 1, p.status, 700)) { ok = false; break; }
           mbar_expect_tx(&full[s], (uint32_t)(GT_M + BN) * 128u);
-          tma_load_2d(base + S::A + (size_t)s * GT_M * 128, &tmA, k * GT_KS, m0, &full[s]);
-          tma_load_2d(base + S::B + (size_t)s * BN * 128, &tmB, k * GT_KS, n0, &full[s]);
+          tma_load_2d(base + (size_t)s * GT_M * 128, &tmA, k * GT_KS, m0, &full[s]);
+          tma_load_2d(base + S.B + (size_t)s * BN * 128, &tmB, k * GT_KS, n0, &full[s]);
+          if (++s == ST) { s = 0; ph ^= 1; }
         }
       }
     }
@@ -136,18 +143,18 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
     uint32_t pred;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
     const bool leader = pred != 0;
-    int it = 0, n = 0;
+    int s = 0, n = 0;
+    uint32_t ph = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, n++) {
       const int buf = n & 1;
       if (!gt_wait_warp(&dempty[buf], ((n >> 1) & 1) ^ 1, p.status, 711)) break;
       const uint32_t d = tmem + (uint32_t)(buf * BN);
-      for (int k = 0; k < nk; k++, it++) {
-        const int s = it % ST;
-        if (!gt_wait_warp(&full[s], (it / ST) & 1, p.status, 710)) { ok = false; break; }
+      for (int k = 0; k < nk; k++) {
+        if (!gt_wait_warp(&full[s], ph, p.status, 710)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t a = gt_desc(smem_u32(base + S::A + (size_t)s * GT_M * 128));
-        const uint64_t b = gt_desc(smem_u32(base + S::B + (size_t)s * BN * 128));
+        const uint64_t a = gt_desc(smem_u32(base + (size_t)s * GT_M * 128));
+        const uint64_t b = gt_desc(smem_u32(base + S.B + (size_t)s * BN * 128));
         if (leader) {
 #pragma unroll
           for (int ks = 0; ks < GT_KS / 16; ks++)
@@ -156,6 +163,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
           if (k + 1 == nk) gt_commit(&dfull[buf]);
         }
         __syncwarp();
+        if (++s == ST) { s = 0; ph ^= 1; }
       }
     }
   } else if (warp >= 4) {
@@ -177,23 +185,24 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
           if (lane == 0) mbar_arrive(&dempty[buf]);
         }
         if (m >= p.M) continue;
+        const int w = BN - c0 < 32 ? 16 : 32, lim = p.N - n0 - c0;   // columns of this read, columns there are
         if (EPI == 2) {
           __nv_bfloat16* o = p.O + (long long)m * p.ldo + (n0 + c0) / 2;
-          if (n0 + c0 + 32 <= p.N && (p.ldo & 7) == 0) {
-            uint32_t w[8];
+          if (w <= lim && (p.ldo & 7) == 0) {
+            uint32_t g[8];
 #pragma unroll
             for (int j = 0; j < 8; j++) {
               const __nv_bfloat162 h = __floats2bfloat162_rn(
                   glu_clipped(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), p.limit),
                   glu_clipped(__uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]), p.limit));
-              w[j] = *(const uint32_t*)&h;
+              g[j] = *(const uint32_t*)&h;
             }
-            ((uint4*)o)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-            ((uint4*)o)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+            ((uint4*)o)[0] = make_uint4(g[0], g[1], g[2], g[3]);
+            if (w == 32) ((uint4*)o)[1] = make_uint4(g[4], g[5], g[6], g[7]);
           } else {
 #pragma unroll
             for (int j = 0; j < 16; j++)
-              if (n0 + c0 + 2 * j + 1 < p.N)
+              if (2 * j < w && 2 * j + 1 < lim)
                 o[j] = __float2bfloat16_rn(
                     glu_clipped(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), p.limit));
           }
@@ -203,27 +212,29 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
 #pragma unroll
             for (int j = 0; j < 32; j++) v[j] = __float_as_uint(relu2(__uint_as_float(v[j])));
           }
-          if (n0 + c0 + 32 <= p.N && (p.ldo & 7) == 0) {
+          if (w <= lim && (p.ldo & 7) == 0) {
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-              uint32_t w[4];
+              if (8 * j >= w) break;
+              uint32_t h4[4];
 #pragma unroll
               for (int k = 0; k < 4; k++) {
                 const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[8 * j + 2 * k]), __uint_as_float(v[8 * j + 2 * k + 1]));
-                w[k] = *(const uint32_t*)&h;
+                h4[k] = *(const uint32_t*)&h;
               }
-              ((uint4*)o)[j] = make_uint4(w[0], w[1], w[2], w[3]);
+              ((uint4*)o)[j] = make_uint4(h4[0], h4[1], h4[2], h4[3]);
             }
           } else {
 #pragma unroll
             for (int j = 0; j < 32; j++)
-              if (n0 + c0 + j < p.N) o[j] = __float2bfloat16_rn(__uint_as_float(v[j]));
+              if (j < w && j < lim) o[j] = __float2bfloat16_rn(__uint_as_float(v[j]));
           }
         } else {
           float* o = p.C + (long long)m * p.ldc + n0 + c0;
-          if (n0 + c0 + 32 <= p.N && (p.ldc & 3) == 0) {
+          if (w <= lim && (p.ldc & 3) == 0) {
 #pragma unroll
             for (int j = 0; j < 8; j++) {
+              if (4 * j >= w) break;
               float4 f = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
                                      __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
               if (EPI == 1) {
@@ -235,7 +246,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
           } else {
 #pragma unroll
             for (int j = 0; j < 32; j++)
-              if (n0 + c0 + j < p.N) o[j] = __uint_as_float(v[j]) + (EPI == 1 ? o[j] : 0.f);
+              if (j < w && j < lim) o[j] = __uint_as_float(v[j]) + (EPI == 1 ? o[j] : 0.f);
           }
         }
       }
@@ -261,17 +272,32 @@ int encode_operand(EncodeTiledFn enc, CUtensorMap* tm, const void* p, int rows, 
   return TLB_OK;
 }
 
-template <int BN, int EPI>
+template <int EPI>
 int gt_launch(DeviceCtx* c, const CUtensorMap& ta, const CUtensorMap& tb, const GtParams& p, cudaStream_t s) {
   static std::atomic<unsigned long long> attr_done{0};
   {
-    const int rc = ensure_dynamic_smem(gemm_bf16_tc_kernel<BN, EPI>, (int)GtSmem<BN>::TOTAL, attr_done);
+    const int rc = ensure_dynamic_smem(gemm_bf16_tc_kernel<EPI>, 224 * 1024, attr_done);
     if (rc) return rc;
   }
   const int tiles = p.mt * p.nt;
-  LaunchCfg lc(dim3(tiles < c->sm_count ? tiles : c->sm_count), dim3(GT_THREADS), GtSmem<BN>::TOTAL, s, pdl_enabled());
-  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, gemm_bf16_tc_kernel<BN, EPI>, ta, tb, p));
+  LaunchCfg lc(dim3(tiles < c->sm_count ? tiles : c->sm_count), dim3(GT_THREADS), GtSmem(p.bn).TOTAL, s, pdl_enabled());
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, gemm_bf16_tc_kernel<EPI>, ta, tb, p));
   return TLB_OK;
+}
+
+// The width that finishes first: rounds of tiles over the SMs times what a round takes.  A stage costs an SM the
+// fetching of (128 + BN) rows from the L2, which at 64 bytes a clock takes longer than the stage's MMAs; the last
+// epilogue of a CTA, about 8 clocks a column, runs under nothing.  3001 x 2048 in tiles of 256 is 192 tiles, one
+// round and a third; in tiles of 176 it is 288, two of 296 places.
+int gt_width(int mt, int N, int K, int sms) {
+  long long best = 0;
+  int width = 0;
+  for (int bn = 256; bn >= 32; bn -= 16) {
+    const long long tiles = (long long)mt * ((N + bn - 1) / bn), rounds = (tiles + sms - 1) / sms;
+    const long long cost = rounds * ((K + GT_KS - 1) / GT_KS) * 2 * (GT_M + bn) + 8 * bn;
+    if (!width || cost < best) { best = cost; width = bn; }
+  }
+  return width;
 }
 
 }  // namespace
@@ -288,25 +314,19 @@ int gemm_bf16_tc_launch(DeviceCtx* c, const void* a, long long lda, const void* 
   if (!gemm_bf16_tc_eligible(a, lda, w, ldw) || M <= 0 || N <= 0 || K <= 0)
     return set_error(TLB_ERR_ARG, "gemm_bf16_tc: operands must be 16-byte aligned with row strides of 8 elements");
   const int mt = (M + GT_M - 1) / GT_M;
-  // widest tile that still gives every SM work
-  int BN = 256;
-  while (BN > 32 && mt * ((N + BN - 1) / BN) < c->sm_count) BN >>= 1;
+  const int BN = gt_width(mt, N, K, c->sm_count);
   CUtensorMap ta, tb;
   int rc = encode_operand(enc, &ta, a, M, K, lda, GT_M);
   if (!rc) rc = encode_operand(enc, &tb, w, N, K, ldw, BN);
   if (rc) return rc;
-  GtParams p{C, ldc, (__nv_bfloat16*)O, ldo, M, N, K, mt, (N + BN - 1) / BN, limit, c->status};
-#define GT_CASE(bn)                                                            \
-  if (BN == bn) switch (epi) {                                                 \
-      case 0: return gt_launch<bn, 0>(c, ta, tb, p, s);                        \
-      case 1: return gt_launch<bn, 1>(c, ta, tb, p, s);                        \
-      case 2: return gt_launch<bn, 2>(c, ta, tb, p, s);                        \
-      case 3: return gt_launch<bn, 3>(c, ta, tb, p, s);                        \
-      default: return gt_launch<bn, 4>(c, ta, tb, p, s);                       \
-    }
-  GT_CASE(256) GT_CASE(128) GT_CASE(64) GT_CASE(32)
-#undef GT_CASE
-  return set_error(TLB_ERR_STATE, "gemm_bf16_tc: no tile width");
+  GtParams p{C, ldc, (__nv_bfloat16*)O, ldo, M, N, K, mt, (N + BN - 1) / BN, BN, limit, c->status};
+  switch (epi) {
+    case 0: return gt_launch<0>(c, ta, tb, p, s);
+    case 1: return gt_launch<1>(c, ta, tb, p, s);
+    case 2: return gt_launch<2>(c, ta, tb, p, s);
+    case 3: return gt_launch<3>(c, ta, tb, p, s);
+    default: return gt_launch<4>(c, ta, tb, p, s);
+  }
 }
 
 }  // namespace tlb

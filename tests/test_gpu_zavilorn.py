@@ -403,3 +403,21 @@ def test_long_prompt_in_segments(rows, first):
     got = run(m, toks, [first, rows] if first else [rows])
     assert ok(err(got, want), "bfloat16")
     close(m)
+
+
+@pytest.mark.parametrize("width,ff,rows", [
+    (1024, 1550, 1000),    # products 64, 144, 176 and 208 columns a tile: a last read of 16 columns
+    (776, 1100, 390),      # tiles of 32 and 48 columns, ragged on the right
+])
+def test_wide_products_of_a_long_prompt(width, ff, rows):
+    """A prompt in one pass against the same tokens in short passes, whose products take narrow tiles: a
+    product's sums are the same in any tile, the rest is judged like bf16 elsewhere here."""
+    cfg = zc.config([zc.par((8, 2, 128, 128), (4, 2, 128, 128), window=300, keep=4, rot=64, ff=ff),
+                     zc.mam(16, 2, 64, 64, 4, 2, ff=ff)], width=width, vocab=200, emb=1.0)
+    w = zc.Weights(cfg, 71)
+    toks = zc.tokens(cfg, rows, 12)
+    m = make(cfg, w, "bfloat16", rows + 8)
+    want = run(m, toks, [100] * (rows // 100 + 1))
+    got = run(m, toks, [rows])
+    assert ok(err(got, want), "bfloat16")
+    close(m)
