@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
         const float4 sc_next = b + 1 < nblk ? __ldg(sc4 + b + 1) : sc_blk;
 #pragma unroll
         for (int buf = 0; buf < T2_NBUF; buf++) {   // four groups a block, one accumulator each
-            const float sc = buf == 0 ? sc_blk.x : (buf == 1 ? sc_blk.y : (buf == 2 ? sc_blk.z : sc_blk.w));
+          const float sc = buf == 0 ? sc_blk.x : (buf == 1 ? sc_blk.y : (buf == 2 ? sc_blk.z : sc_blk.w));
           if (!mbar_wait_bounded(&bars[T2_D_FULL + buf], blocks & 1, p.status, 630)) { ok = false; break; }
           t2_fence_after();
           const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * MT + c_lo);
@@ -389,19 +389,19 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
 #pragma unroll
             for (int b = 0; b < BATCH / 16; b++)
 #pragma unroll
-            for (int i = 0; i < 16; i++) acc[c0 + 16 * b + i] = fmaf(sc, __uint_as_float(v[b][i]), acc[c0 + 16 * b + i]);
+              for (int i = 0; i < 16; i++) acc[c0 + 16 * b + i] = fmaf(sc, __uint_as_float(v[b][i]), acc[c0 + 16 * b + i]);
           }
         }
         sc_blk = sc_next;
       }
       bool mine = true;   // this CTA writes the tile
-        if (q1 - q0 < p.box) {
+      if (q1 - q0 < p.box) {
         // a part of the tile: into scratch, and the last of the tile's CTAs sums all parts
         const unsigned u0 = (unsigned)tile * (unsigned)p.box;
         const int first = (int)t2_owner(p, u0), last = (int)t2_owner(p, u0 + (unsigned)p.box - 1u), me = blockIdx.x;
         auto part = [&](int cta) {
           const int second = t2_first(p, cta) < u0;   // the range began in an earlier tile
-            return p.parts + (size_t)(2 * cta + second) * (MT * T2_ROWS) + (size_t)c_lo * T2_ROWS + r;
+          return p.parts + (size_t)(2 * cta + second) * (MT * T2_ROWS) + (size_t)c_lo * T2_ROWS + r;
         };
         float* mp = part(me);
 #pragma unroll
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
           asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(p.tickets + first) : "memory");
           *last_part = old == last - first;
           if (old == last - first) p.tickets[first] = 0;   // clean for the next launch
-          }
+        }
         asm volatile("bar.sync 1, 256;" ::: "memory");
         mine = *last_part != 0;
         if (mine) {
