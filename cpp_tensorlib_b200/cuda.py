@@ -16,12 +16,17 @@ from ._lib import TlbError, check, lib
 kQ4Group = 32  # include/types.h:28
 
 
+# The current stream and an operand's address as plain numbers, which ctypes takes for void pointers: a Stream
+# object and c_void_p objects made for each call were a third of what a short call costs the host.
+_raw_stream = torch._C._cuda_getCurrentRawStream
+
+
 def _s():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _p(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _f32c(t, name):
@@ -98,7 +103,8 @@ def gemv_q4(a, wq, y=None):
         raise ValueError("gemv_q4: a must hold K elements")
     if y is None:
         y = torch.empty(wq.N, dtype=torch.float32, device=a.device)
-    check(lib().tlb_gemv_q4(_p(a), wq.qw_ptr, wq.scales_ptr, _p(y), wq.N, wq.K, kQ4Group, _s()))
+    w = wq.buf.data_ptr()
+    check(lib().tlb_gemv_q4(a.data_ptr(), w, w + wq.N * wq.K // 2, y.data_ptr(), wq.N, wq.K, kQ4Group, _s()))
     return y
 
 
@@ -152,7 +158,8 @@ def gemm_q4(x, wq, alpha=1.0, beta=0.0, y=None, simt=False):
     if y is None:
         y = torch.empty((M, wq.N), dtype=torch.float32, device=x.device)
     fn = lib().tlb_gemm_q4_simt if simt else lib().tlb_gemm_q4
-    check(fn(_p(x2), M, K, wq.qw_ptr, wq.scales_ptr, _p(y), wq.N, wq.N, K, alpha, beta, _s()))
+    w = wq.buf.data_ptr()
+    check(fn(x2.data_ptr(), M, K, w, w + wq.N * K // 2, y.data_ptr(), wq.N, wq.N, K, alpha, beta, _s()))
     return y
 
 
