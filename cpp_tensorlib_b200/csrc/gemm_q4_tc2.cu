@@ -37,7 +37,8 @@
 // nine tenths of the time, with half of them as long.  So the accumulate warps' loop is unrolled over a block of four
 // scales, one accumulator each, with nothing left to select at run time.  Measured and dropped: weights in TMEM as
 // the A operand, sixteen accumulate warps, one issuer, one commit a stage, spinning waits, register shares by
-// setmaxnreg with 64-column reads.  1000 x 3584 x 37888: 676 -> 583 us; 1000 x 18944 x 3584, one and a half
+// setmaxnreg with 64-column reads, leaving out the reads of columns behind the last row (the branch keeps the compiler from
+// running one group's reads under another's FMAs: 570 -> 670 us).  1000 x 3584 x 37888: 676 -> 583 us; 1000 x 18944 x 3584, one and a half
 // rounds of tiles: 424 -> 328; 517 x 4864 x 896, 35 tiles: 60 -> 40.
 #include <cstdlib>
 

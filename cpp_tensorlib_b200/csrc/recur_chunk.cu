@@ -690,7 +690,8 @@ int rc_launch(const RecurP& p, const void* conv, const float2* gates, const floa
     LaunchCfg lc(dim3((p.E + RC_E - 1) / RC_E, p.H, g.n - 1), dim3(RC_THREADS), smem, s, pdl_enabled());
     TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, ssd_state_kernel<DP>, p, (const __nv_bfloat16*)conv, gates, pos0, g));
   }
-  // few heads: half as many columns a CTA, twice the CTAs (16 heads of 128 on 148 SMs: 64 CTAs or 128)
+  // few heads: half as many columns a CTA, twice the CTAs, where those still find an SM each (4096 tokens, 16 heads of
+  // 128: 392 us on 64 SMs, 318 on 128)
   if constexpr (DELTA)
     if ((p.E + RC_E - 1) / RC_E * p.H <= 74) return rc_walk<DP, DELTA, 16>(p, conv, gates, norms, T, o, rows, pos0, g, s);
   return rc_walk<DP, DELTA, RC_E>(p, conv, gates, norms, T, o, rows, pos0, g, s);
