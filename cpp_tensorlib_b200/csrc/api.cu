@@ -283,6 +283,25 @@ int tlb_gemm_q4_simt(const float* x, int64_t M, int64_t ldx, const void* qw, con
                              S(stream));
 }
 
+// rows of `most` that one launch of the skinny kernel takes: their activations have to fit shared memory
+static int skinny_rows(const void* qw, const void* scales, int N, int K, int most) {
+  int mb = most;
+  while (mb > 1 && !gemv_q4_tma_eligible(qw, scales, N, K, mb)) mb = (mb + 1) / 2;
+  return mb;
+}
+// Up to 8 rows that would take three or more launches of the skinny kernel, each streaming all weights, are one
+// product on planes instead: 8 x 18944 x 3584 144 -> 38 us, 3 x 18944 x 3584 54 -> 38, 5 x 11008 x 4096 48 -> 30.  Two
+// launches cost about what the planes do (8 x 3584 x 18944: 34 us, 31 for up to 32 rows on planes).  A stream
+// under capture may not allocate: there the planes need scratch that an earlier product has left.
+static bool few_rows_on_planes(DeviceCtx* c, const void* qw, const void* scales, int N, int K, int M, cudaStream_t s) {
+  if (M < 3 || !gemm_q4_planes_possible(qw, scales, N, K, M)) return false;
+  const int mb = skinny_rows(qw, scales, N, K, M);
+  if ((M + mb - 1) / mb < 3) return false;
+  if (c->q4_work && c->xsplit_bytes >= gemm_q4_tc2_scratch_bytes(M, K)) return true;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+}
+
 int tlb_gemm_q4(const float* x, int64_t M, int64_t ldx, const void* qw, const float* scales,
                 float* y, int64_t ldy, int64_t N, int64_t K, float alpha, float beta,
                 void* stream) {
@@ -294,7 +313,8 @@ int tlb_gemm_q4(const float* x, int64_t M, int64_t ldx, const void* qw, const fl
   // Many rows: tensor-core path (tcgen05, TMEM accumulators).  Default: integer weights x two
   // fp16 activation planes, group scales applied outside the tensor core (gemm_q4_tc2.cu);
   // TLB_GEMM_TC=1 selects the earlier formulation with scaled tf32 hi/lo operands.
-  if (gemm_q4_planes_eligible(qw, scales, (int)N, (int)K, (int)M)) {
+  if (gemm_q4_planes_eligible(qw, scales, (int)N, (int)K, (int)M) ||
+      (M <= 8 && few_rows_on_planes(c, qw, scales, (int)N, (int)K, (int)M, S(stream)))) {
     const size_t need = gemm_q4_tc2_scratch_bytes((int)M, (int)K);
     if (need > c->xsplit_bytes) {
       TLB_CUDA(cudaDeviceSynchronize());
@@ -335,8 +355,7 @@ int tlb_gemm_q4(const float* x, int64_t M, int64_t ldx, const void* qw, const fl
     if (rc) return rc;
     int64_t m0 = 0;
     while (m0 < M) {
-      int mb = (int)((M - m0) < 8 ? (M - m0) : 8);
-      while (mb > 1 && !gemv_q4_tma_eligible(qw, scales, (int)N, (int)K, mb)) mb = (mb + 1) / 2;
+      const int mb = skinny_rows(qw, scales, (int)N, (int)K, (int)((M - m0) < 8 ? (M - m0) : 8));
       rc = gemv_q4_launch(c, tmW, tmS, x + m0 * ldx, ldx, mb, y + m0 * ldy, ldy, (int)N, (int)K,
                           alpha, beta, S(stream), 0, nullptr, 0, nullptr, nullptr, nullptr, 0.f);
       if (rc) return rc;

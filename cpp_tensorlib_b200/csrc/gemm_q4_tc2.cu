@@ -519,12 +519,16 @@ size_t gemm_q4_work_bytes(int sm_count) { return Q4_TICKET_BYTES + (size_t)2 * s
 size_t gemm_q4_tc2_scratch_bytes(int M, int K) { return (size_t)M * K * 4 + (size_t)((M + 3) & ~3) * 4 + 256; }
 
 bool gemm_q4_tc2_eligible(const void* qw, const void* scales, int N, int K, int M) {
-  if (M <= 8 || N <= 0 || M > 65535 * 32) return false;
+  if (M <= 0 || N <= 0 || M > 65535 * 32) return false;
   if (K % 128 != 0) return false;
   return (((uintptr_t)qw & 15) == 0) && (((uintptr_t)scales & 15) == 0);
 }
 
 bool gemm_q4_planes_eligible(const void* qw, const void* scales, int N, int K, int M) {
+  return M > 8 && gemm_q4_planes_possible(qw, scales, N, K, M);
+}
+
+bool gemm_q4_planes_possible(const void* qw, const void* scales, int N, int K, int M) {
   // TLB_GEMM_TC=1 selects the earlier formulation (gemm_q4_tc.cu)
   static const bool tc_old = getenv("TLB_GEMM_TC") && atoi(getenv("TLB_GEMM_TC")) == 1;
   return !tc_old && gemm_q4_tc2_eligible(qw, scales, N, K, M);

@@ -26,8 +26,9 @@ size_t gemm_q4_tc2_scratch_bytes(int M, int K);
 // first; the products leave them zero.
 constexpr int Q4_TICKET_BYTES = 4096;   // room for 1024 SMs
 size_t gemm_q4_work_bytes(int sm_count);
-// whether a product of M rows takes the planes (and not another kernel)
+// whether a product of M rows takes the planes (and not another kernel), whether it could
 bool gemm_q4_planes_eligible(const void* qw, const void* scales, int N, int K, int M);
+bool gemm_q4_planes_possible(const void* qw, const void* scales, int N, int K, int M);
 int gemm_q4_planes_launch(DeviceCtx* c, const Q4Planes& x, int M, const void* qw, const float* scales, float* y,
                           long long ldy, int N, int K, float alpha, float beta, void* work, cudaStream_t stream);
 // x f32 rows -> planes

@@ -44,3 +44,22 @@ def test_tiles_shared_by_blocks(M, K, N):
     got = [tl.gemm_q4(x, w, alpha=1.5, beta=0.25) for _ in range(6)]
     assert (want - got[0]).abs().max().item() < 2e-4 * want.std().item()
     assert all(torch.equal(got[0], a) for a in got[1:])
+
+
+@pytest.mark.parametrize("M,K,N", [(3, 18944, 3584), (8, 18944, 129), (5, 11008, 500), (8, 3584, 1000)])
+def test_few_rows_of_deep_products(M, K, N):
+    """Rows whose activations do not fit the skinny kernel's shared memory at once (the last case needs two launches and
+    stays there): the CUDA-core kernel's values within f32 sums in another order, about 2^-24 sqrt(K) <= 8e-6 of a result, 25
+    times that for the largest; the same bits on every call and in a captured graph."""
+    from cpp_tensorlib_b200 import cuda as tl
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    w = tl.to_q4(torch.randn((K, N), generator=g, device="cuda") * 0.02)
+    x = torch.randn((M, K), generator=g, device="cuda")
+    want = tl.gemm_q4(x, w, simt=True)
+    got = tl.gemm_q4(x, w)
+    assert (want - got).abs().max().item() < 2e-4 * want.std().item()
+    y, graph = torch.zeros_like(got), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        tl.gemm_q4(x, w, y=y)
+    graph.replay()
+    assert torch.equal(got, y) and torch.equal(got, tl.gemm_q4(x, w))
