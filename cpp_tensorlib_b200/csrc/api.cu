@@ -90,6 +90,28 @@ EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
+int scratch_reserve(GrownScratch& g, size_t need, cudaStream_t s) {
+  if (need > g.bytes) {
+    TLB_CUDA(cudaDeviceSynchronize());
+    if (g.captured) g.kept.push_back(g.p);
+    else if (g.p) TLB_CUDA(cudaFree(g.p));
+    g.p = nullptr;
+    g.bytes = 0;
+    g.captured = false;
+    TLB_CUDA(cudaMalloc(&g.p, need));
+    g.bytes = need;
+  }
+  if (!g.captured) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {   // the legacy stream beside a capture
+      cudaGetLastError();
+      g.captured = true;
+    }
+    g.captured = g.captured || st != cudaStreamCaptureStatusNone;
+  }
+  return TLB_OK;
+}
+
 static int create_ctx(int dev, DeviceCtx** out) {
   auto* c = new DeviceCtx();
   c->device = dev;
@@ -111,6 +133,9 @@ static int create_ctx(int dev, DeviceCtx** out) {
   c->attn_max_counters = 1024;
   TLB_CUDA(cudaMalloc(&c->attn_counters, c->attn_max_counters * sizeof(int)));
   TLB_CUDA(cudaMemset(c->attn_counters, 0, c->attn_max_counters * sizeof(int)));
+  TLB_CUDA(cudaMalloc(&c->q4_few, Q4_FEW_BYTES));
+  TLB_CUDA(cudaMalloc(&c->q4_work, gemm_q4_work_bytes(c->sm_count)));
+  TLB_CUDA(cudaMemset(c->q4_work, 0, Q4_TICKET_BYTES));
   TLB_CUDA(cudaMalloc(&c->argmax_cell, 4 * sizeof(unsigned long long)));
   TLB_CUDA(cudaMemset(c->argmax_cell, 0, 4 * sizeof(unsigned long long)));
   TLB_CUDA(cudaMalloc(&c->status, ST_WORDS * sizeof(int)));
@@ -291,15 +316,14 @@ static int skinny_rows(const void* qw, const void* scales, int N, int K, int mos
 }
 // Up to 8 rows that would take three or more launches of the skinny kernel, each streaming all weights, are one
 // product on planes instead: 8 x 18944 x 3584 144 -> 38 us, 3 x 18944 x 3584 54 -> 38, 5 x 11008 x 4096 48 -> 30.  Two
-// launches cost about what the planes do (8 x 3584 x 18944: 34 us, 31 for up to 32 rows on planes).  A stream
-// under capture may not allocate: there the planes need scratch that an earlier product has left.
-static bool few_rows_on_planes(DeviceCtx* c, const void* qw, const void* scales, int N, int K, int M, cudaStream_t s) {
-  if (M < 3 || !gemm_q4_planes_possible(qw, scales, N, K, M)) return false;
+// launches cost about what the planes do (8 x 3584 x 18944: 34 us, 31 for up to 32 rows on planes).  By the shape
+// alone, with scratch that is made with the context and never moves: such a call allocates nothing, gives the same bits
+// under capture, and a graph of it stays valid.  (Rows deeper than that scratch holds, 131000 at 8 rows, stay skinny.)
+static bool few_rows_on_planes(const void* qw, const void* scales, int N, int K, int M) {
+  if (M < 3 || M > 8 || !gemm_q4_planes_possible(qw, scales, N, K, M) || gemm_q4_tc2_scratch_bytes(M, K) > Q4_FEW_BYTES)
+    return false;
   const int mb = skinny_rows(qw, scales, N, K, M);
-  if ((M + mb - 1) / mb < 3) return false;
-  if (c->q4_work && c->xsplit_bytes >= gemm_q4_tc2_scratch_bytes(M, K)) return true;
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+  return (M + mb - 1) / mb >= 3;
 }
 
 int tlb_gemm_q4(const float* x, int64_t M, int64_t ldx, const void* qw, const float* scales,
@@ -313,40 +337,18 @@ int tlb_gemm_q4(const float* x, int64_t M, int64_t ldx, const void* qw, const fl
   // Many rows: tensor-core path (tcgen05, TMEM accumulators).  Default: integer weights x two
   // fp16 activation planes, group scales applied outside the tensor core (gemm_q4_tc2.cu);
   // TLB_GEMM_TC=1 selects the earlier formulation with scaled tf32 hi/lo operands.
-  if (gemm_q4_planes_eligible(qw, scales, (int)N, (int)K, (int)M) ||
-      (M <= 8 && few_rows_on_planes(c, qw, scales, (int)N, (int)K, (int)M, S(stream)))) {
-    const size_t need = gemm_q4_tc2_scratch_bytes((int)M, (int)K);
-    if (need > c->xsplit_bytes) {
-      TLB_CUDA(cudaDeviceSynchronize());
-      if (c->xsplit) TLB_CUDA(cudaFree(c->xsplit));
-      c->xsplit = nullptr;
-      c->xsplit_bytes = 0;
-      TLB_CUDA(cudaMalloc(&c->xsplit, need));
-      c->xsplit_bytes = need;
-    }
-    if (!c->q4_work) {
-      void* w = nullptr;
-      TLB_CUDA(cudaMalloc(&w, gemm_q4_work_bytes(c->sm_count)));
-      TLB_CUDA(cudaMemset(w, 0, Q4_TICKET_BYTES));
-      TLB_CUDA(cudaDeviceSynchronize());
-      c->q4_work = w;
-    }
-    return gemm_q4_tc2_launch(c, x, ldx, (int)M, qw, scales, y, ldy, (int)N, (int)K, alpha, beta, c->xsplit,
-                              c->q4_work, S(stream));
+  if (few_rows_on_planes(qw, scales, (int)N, (int)K, (int)M))
+    return gemm_q4_tc2_launch(c, x, ldx, (int)M, qw, scales, y, ldy, (int)N, (int)K, alpha, beta, c->q4_few, c->q4_work,
+                              S(stream));
+  if (gemm_q4_planes_eligible(qw, scales, (int)N, (int)K, (int)M)) {
+    const int rc = scratch_reserve(c->xsplit, gemm_q4_tc2_scratch_bytes((int)M, (int)K), S(stream));
+    return rc ? rc : gemm_q4_tc2_launch(c, x, ldx, (int)M, qw, scales, y, ldy, (int)N, (int)K, alpha, beta, c->xsplit.p,
+                                        c->q4_work, S(stream));
   }
   if (gemm_q4_tc_eligible(qw, scales, (int)N, (int)K, (int)M)) {
-    const size_t need = (size_t)2 * M * K * sizeof(float);
-    if (need > c->xsplit_bytes) {
-      // grown between launches only; not capturable at a size never seen before
-      TLB_CUDA(cudaDeviceSynchronize());
-      if (c->xsplit) TLB_CUDA(cudaFree(c->xsplit));
-      c->xsplit = nullptr;
-      c->xsplit_bytes = 0;
-      TLB_CUDA(cudaMalloc(&c->xsplit, need));
-      c->xsplit_bytes = need;
-    }
-    return gemm_q4_tc_launch(c, x, ldx, (int)M, qw, scales, y, ldy, (int)N, (int)K, alpha, beta,
-                             c->xsplit, S(stream));
+    const int rc = scratch_reserve(c->xsplit, (size_t)2 * M * K * sizeof(float), S(stream));
+    return rc ? rc : gemm_q4_tc_launch(c, x, ldx, (int)M, qw, scales, y, ldy, (int)N, (int)K, alpha, beta,
+                                       (float*)c->xsplit.p, S(stream));
   }
   // Skinny activations: stream the weights once per block of up to 8 rows.
   if (gemv_q4_tma_eligible(qw, scales, (int)N, (int)K, 1)) {

@@ -9,6 +9,7 @@
 
 #include <atomic>
 #include <string>
+#include <vector>
 
 #include "../../include/tlb200.h"
 
@@ -41,6 +42,18 @@ int cuda_fail(cudaError_t e, const char* what);
 // driver entry points resolved through the runtime (nothing is linked against
 // libcuda).
 // ---------------------------------------------------------------------------
+// Scratch that one op family grows on demand.  A captured graph holds the block's address, so a block that a
+// capture has used stays when the family outgrows it, as long as the context does; other blocks are freed.
+struct GrownScratch {
+  void* p = nullptr;
+  size_t bytes = 0;
+  bool captured = false;       // p is in a graph
+  std::vector<void*> kept;     // outgrown blocks that are
+};
+// p of at least `need` bytes for work on stream s.  Growth waits for the device, so that no work in flight loses its
+// block, and is an error under capture.
+int scratch_reserve(GrownScratch& g, size_t need, cudaStream_t s);
+
 struct DeviceCtx {
   int device = -1;
   int sm_count = 0;
@@ -55,11 +68,11 @@ struct DeviceCtx {
   size_t attn_scratch_bytes = 0;
   int* attn_counters = nullptr;  // [max kv-head*... ] zero between launches
   int attn_max_counters = 0;
+  // planes of the activations for the tensor-core products of more than 8 rows
+  GrownScratch xsplit;
+  // the same for up to 8 rows (Q4_FEW_BYTES) and the products' own scratch (gemm_q4_work_bytes)
+  void *q4_few = nullptr, *q4_work = nullptr;
   // argmax result cell (packed key) + small status block
-  // tf32 hi/lo planes of the activations for the tensor-core GEMM (grown on demand)
-  float* xsplit = nullptr;
-  size_t xsplit_bytes = 0;
-  void* q4_work = nullptr;   // gemm_q4_work_bytes, made by the first product of many rows
   unsigned long long* argmax_cell = nullptr;
   int* status = nullptr;        // device, ST_WORDS ints
   int* status_host = nullptr;   // pinned mirror for reads

@@ -1,5 +1,9 @@
 """The int4 product of many rows, calls one behind the other: every call gives the same bits, and the values of
 the general-shape CUDA-core kernel."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -63,3 +67,50 @@ def test_few_rows_of_deep_products(M, K, N):
         tl.gemm_q4(x, w, y=y)
     graph.replay()
     assert torch.equal(got, y) and torch.equal(got, tl.gemm_q4(x, w))
+
+
+@pytest.mark.parametrize("M,K,N,rows", [(8, 18944, 512, 3000), (32, 3584, 512, 4500), (300, 896, 1152, 6000)])
+def test_captured_products_outlive_larger_ones(M, K, N, rows):
+    """A product that needs more scratch than any before it, run between two replays of a captured product: the graph
+    gives the same bits and leaves memory that was allocated meanwhile alone."""
+    from cpp_tensorlib_b200 import cuda as tl
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    w = tl.to_q4(torch.randn((K, N), generator=g, device="cuda") * 0.02)
+    x = torch.randn((M, K), generator=g, device="cuda")
+    want = tl.gemm_q4(x, w)
+    y, graph = torch.zeros_like(want), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        tl.gemm_q4(x, w, y=y)
+    graph.replay()
+    assert torch.equal(want, y)
+    wide = tl.to_q4(torch.zeros((18944, 128), device="cuda"))
+    tl.gemm_q4(torch.zeros((rows, 18944), device="cuda"), wide)
+    torch.cuda.empty_cache()
+    others = [torch.full((1 << n,), 7, dtype=torch.uint8, device="cuda") for n in range(20, 30) for _ in range(2)]
+    y.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(want, y)
+    assert all(bool((t == 7).all()) for t in others)
+
+
+FRESH = """
+import torch
+from cpp_tensorlib_b200 import check, lib, cuda as tl
+check(lib().tlb_init(0))
+w = tl.to_q4(torch.randn((18944, 512), device="cuda") * 0.02)
+x = torch.randn((8, 18944), device="cuda")
+y, graph = torch.zeros((8, 512), device="cuda"), torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    tl.gemm_q4(x, w, y=y)
+graph.replay()
+tl.gemm_q4(torch.randn((64, 18944), device="cuda"), w)
+assert torch.equal(y, tl.gemm_q4(x, w))
+"""
+
+
+def test_few_rows_captured_before_any_other_product():
+    """Which kernel a product takes follows from its shape: captured as the first product of a process it gives the
+    bits of a later call."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", FRESH], cwd=root, check=True, timeout=300)
