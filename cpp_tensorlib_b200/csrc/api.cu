@@ -101,13 +101,11 @@ int scratch_reserve(GrownScratch& g, size_t need, cudaStream_t s) {
     TLB_CUDA(cudaMalloc(&g.p, need));
     g.bytes = need;
   }
-  if (!g.captured) {
+  if (s && !g.captured) {   // the default stream cannot be captured
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {   // the legacy stream beside a capture
-      cudaGetLastError();
-      g.captured = true;
-    }
-    g.captured = g.captured || st != cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(s, &st);
+    if (e != cudaSuccess) cudaGetLastError();   // it does not say: keep the block
+    g.captured = e != cudaSuccess || st != cudaStreamCaptureStatusNone;
   }
   return TLB_OK;
 }
@@ -417,18 +415,10 @@ static int attn_decode_any(const float* q, const void* K, const void* V, float* 
               "tlb_attn_decode: need 0 < n_q <= 2^24 and n_q % n_kv == 0");
   TLB_REQUIRE(kv_max <= (1ll << 30) && (D == 64 || D == 128), "tlb_attn_decode: kv_max / D out of range");
   CTX(c);
-  size_t need = attn_partials_bytes((int)n_q, (int)n_kv, ctx, (int)D, c->sm_count);
-  if (need > c->attn_scratch_bytes) {
-    // grown between launches only; the old buffer may still be in use by queued work
-    TLB_CUDA(cudaDeviceSynchronize());
-    if (c->attn_scratch) TLB_CUDA(cudaFree(c->attn_scratch));
-    c->attn_scratch = nullptr;
-    c->attn_scratch_bytes = 0;
-    TLB_CUDA(cudaMalloc(&c->attn_scratch, need));
-    c->attn_scratch_bytes = need;
-  }
-  return attn_decode_launch(c, q, K, V, out, (int)n_q, (int)n_kv, (int)ctx, kv_max, (int)D, scale,
-                            nullptr, c->attn_scratch, c->attn_counters, S(stream), 0, kv_bf16);
+  const size_t need = attn_partials_bytes((int)n_q, (int)n_kv, ctx, (int)D, c->sm_count);
+  const int rc = scratch_reserve(c->attn_scratch, need, S(stream));
+  return rc ? rc : attn_decode_launch(c, q, K, V, out, (int)n_q, (int)n_kv, (int)ctx, kv_max, (int)D, scale, nullptr,
+                                      (float*)c->attn_scratch.p, c->attn_counters, S(stream), 0, kv_bf16);
 }
 int tlb_attn_decode(const float* q, const float* K, const float* V, float* out, int64_t n_q,
                     int64_t n_kv, int64_t ctx, int64_t kv_max, int64_t D, float scale,

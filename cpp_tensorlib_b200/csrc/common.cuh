@@ -63,9 +63,7 @@ struct DeviceCtx {
   int* gemv_counters = nullptr;    // [max_row_tiles], zero between launches
   int gemv_max_workers = 0, gemv_max_tiles = 0;
   unsigned long long* chain_cell = nullptr;   // arrival counter of the GEMV chains' phase barrier
-  // attention split-KV partials for the host-ctx entry point (grown on demand)
-  float* attn_scratch = nullptr;
-  size_t attn_scratch_bytes = 0;
+  GrownScratch attn_scratch;   // attention split-KV partials for the host-ctx entry point
   int* attn_counters = nullptr;  // [max kv-head*... ] zero between launches
   int attn_max_counters = 0;
   // planes of the activations for the tensor-core products of more than 8 rows

@@ -454,6 +454,29 @@ def test_attn_bf16_groups_vs_oracle(tl, port, n_q, n_kv, D, kv_max, ctxs):
         assert relerr(got, port.attn_decode(q, Kr, Vr, D ** -0.5, ctx=ctx)) < 1e-4, ctx
 
 
+@pytest.mark.parametrize("n_q,ctx,wide", [(28, 300, 64), (3, 90, 128)])
+def test_captured_attention_outlives_wider_ones(tl, n_q, ctx, wide):
+    """Attention with more partial sums than any before it, between two replays of a captured call: the graph
+    gives the same bits and leaves memory that was allocated meanwhile alone."""
+    g = torch.Generator(device="cuda").manual_seed(ctx)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    q, K, V = rnd(n_q, 64), rnd(n_q, ctx, 64), rnd(n_q, ctx, 64)
+    want = tl.attn_decode(q, K, V, 0.125)
+    out, graph = torch.zeros_like(want), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        tl.attn_decode(q, K, V, 0.125, out=out)
+    graph.replay()
+    assert torch.equal(want, out)
+    tl.attn_decode(rnd(32 * 1024, wide), rnd(1024, 64, wide), rnd(1024, 64, wide), 0.125)
+    torch.cuda.empty_cache()
+    others = [torch.full((1 << n,), 7, dtype=torch.uint8, device="cuda") for n in range(16, 28) for _ in range(4)]
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(want, out)
+    assert all(bool((t == 7).all()) for t in others)
+
+
 def test_kv_cache_bf16_append_fill_and_attend(tl, port):
     """kv_cache with dtype bf16: append / fill narrow with round-to-nearest-even (bit-equal to
     the host converter), attention in both position forms reads them back."""
