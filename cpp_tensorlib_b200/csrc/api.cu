@@ -222,6 +222,10 @@ int tlb_device_status(int* out2, int clear) {
     // the wait limit (words 2..3) survives a clear
     TLB_CUDA(cudaMemset(c->status, 0, 2 * sizeof(int)));
     TLB_CUDA(cudaMemset(&c->status[ST_KV_OVERFLOW], 0, sizeof(int)));
+    // The int4 products' tickets leave a product as they were only if it ran alone: two that overlapped may leave a
+    // count that no later product of that tile can end on.  Nothing may be in flight here.
+    TLB_CUDA(cudaDeviceSynchronize());
+    TLB_CUDA(cudaMemset(c->q4_work, 0, Q4_TICKET_BYTES));
     if (timed_out) {
       // a kernel that gave up may have left its fix-up tickets half counted
       TLB_CUDA(cudaMemset(c->gemv_counters, 0, (size_t)c->gemv_max_tiles * sizeof(int)));
@@ -248,6 +252,12 @@ int tlb_set_wait_limit_cycles(int64_t cycles) {
 // with %globaltimer stamps of its phases (NULL switches it off).
 int tlb_debug_attn_timing(void* dbuf) {
   g_attn_dbg = (unsigned long long*)dbuf;
+  return TLB_OK;
+}
+// Sets every ticket of the tensor-core int4 products, as overlapping ones might leave them.
+int tlb_debug_gemm_tickets(int value) {
+  CTX(c);
+  TLB_CUDA(cudaMemset(c->q4_work, value, Q4_TICKET_BYTES));
   return TLB_OK;
 }
 int tlb_debug_gemv_timing(void* dbuf) {

@@ -23,8 +23,8 @@ inline Q4Planes q4_planes_at(void* scratch, int M, int K) {
 
 size_t gemm_q4_tc2_scratch_bytes(int M, int K);
 constexpr size_t Q4_FEW_BYTES = (size_t)4 << 20;   // a context's planes for products of up to 8 rows
-// The product's own scratch (`work`): one per stream of products, its first bytes (Q4_TICKET_BYTES) zero before the
-// first; the products leave them zero.
+// The product's own scratch (`work`): the context's or a decoder's, for one product at a time.  Its first bytes
+// (Q4_TICKET_BYTES) are zero before a product, and the product leaves them zero.
 constexpr int Q4_TICKET_BYTES = 4096;   // room for 1024 SMs
 size_t gemm_q4_work_bytes(int sm_count);
 // whether a product of M rows takes the planes (and not another kernel), whether it could

@@ -50,6 +50,24 @@ def test_tiles_shared_by_blocks(M, K, N):
     assert all(torch.equal(got[0], a) for a in got[1:])
 
 
+@pytest.mark.parametrize("M,K,N", [(8, 18944, 256), (33, 2048, 256), (300, 18944, 3584)])
+def test_tickets_are_cleared_with_the_status(M, K, N):
+    """Whatever count overlapping products left, the products behind a cleared status are right."""
+    from cpp_tensorlib_b200 import check, cuda as tl, lib
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    w = tl.to_q4(torch.randn((K, N), generator=g, device="cuda") * 0.02)
+    x = torch.randn((M, K), generator=g, device="cuda")
+    want = tl.gemm_q4(x, w)
+    torch.cuda.synchronize()
+    for value in (1, 255):
+        check(lib().tlb_debug_gemm_tickets(value))
+        check(lib().tlb_device_status(None, 1))
+        for _ in range(2):
+            y = torch.zeros_like(want)
+            tl.gemm_q4(x, w, y=y)
+            assert torch.equal(want, y)
+
+
 @pytest.mark.parametrize("M,K,N", [(3, 18944, 3584), (8, 18944, 129), (5, 11008, 500), (8, 3584, 1000)])
 def test_few_rows_of_deep_products(M, K, N):
     """Rows whose activations do not fit the skinny kernel's shared memory at once (the last case needs two launches and
