@@ -113,7 +113,7 @@ struct Decoder : DecoderBase {
   int pf_rows = 0;
   float *pf_res[2] = {}, *pf_h = nullptr, *pf_h2 = nullptr, *pf_md = nullptr, *pf_qkv = nullptr, *pf_at = nullptr,
         *pf_gu = nullptr, *pf_mb = nullptr;
-  void* pf_work = nullptr;     // scratch of the products on planes
+  void* pf_work = nullptr;     // scratch of the products on planes, zero tickets at the start of a prompt
   void* pf_planes = nullptr;   // activations of one product as fp16 planes; shares pf_mb's memory
 
   ~Decoder() override;
@@ -418,7 +418,6 @@ Decoder::~Decoder() {
   for (void* sk : sink) cudaFree(sk);
   cudaFree(rope_cs);
   cudaFree(pf);
-  cudaFree(pf_work);
   cudaFree(attn_partials); cudaFree(flags_local);
 }
 
@@ -430,25 +429,24 @@ Decoder::~Decoder() {
 int Decoder::prefill_begin(int rows, cudaStream_t s) {
   if (tp_size != 1) return set_error(TLB_ERR_UNSUPPORTED, "tlb_decoder_prefill: single GPU only");
   if (!embed || !onorm) return set_error(TLB_ERR_STATE, "decoder: embed / final norm not set");
-  if (pf && pf_rows >= rows) return TLB_OK;
+  if (pf && pf_rows >= rows) {
+    TLB_CUDA(cudaMemsetAsync(pf_work, 0, Q4_TICKET_BYTES, s));
+    return TLB_OK;
+  }
+  DeviceCtx* c = nullptr;
+  const int rc = get_ctx(&c);
+  if (rc) return rc;
   const int E = hidden, D = hd, QKV = (n_q + 2 * n_kv) * D;
   const size_t CH = rows, n_emb = CH * E, n_qkv = CH * QKV, n_att = CH * n_q * D, n_gu = CH * 2 * ff, n_mb = CH * ff;
   // the planes of a product's rows, or the rows in f32 where the product takes those
   const int wide = ff > E ? (ff > n_q * D ? ff : n_q * D) : (E > n_q * D ? E : n_q * D);
   const size_t n_pl = (gemm_q4_tc2_scratch_bytes(rows, wide) + 3) / 4, n_act = n_mb > n_pl ? n_mb : n_pl;
-  const size_t total = 5 * n_emb /* res0 res1 h h2 md */ + n_qkv + n_att + n_gu + n_act + 64;
+  const size_t n_work = gemm_q4_work_bytes(c->sm_count) / 4;
+  const size_t total = 5 * n_emb /* res0 res1 h h2 md */ + n_qkv + n_att + n_gu + n_act + n_work + 64;
   if (pf) {
     TLB_CUDA(cudaStreamSynchronize(s));
     TLB_CUDA(cudaFree(pf));
     pf = nullptr;
-  }
-  if (!pf_work) {
-    DeviceCtx* c = nullptr;
-    const int rc = get_ctx(&c);
-    if (rc) return rc;
-    TLB_CUDA(cudaMalloc(&pf_work, gemm_q4_work_bytes(c->sm_count)));
-    TLB_CUDA(cudaMemset(pf_work, 0, Q4_TICKET_BYTES));
-    TLB_CUDA(cudaDeviceSynchronize());
   }
   TLB_CUDA(cudaMalloc(&pf, total * sizeof(float)));
   pf_rows = rows;
@@ -460,8 +458,10 @@ int Decoder::prefill_begin(int rows, cudaStream_t s) {
   pf_at = take(n_att);
   pf_gu = take(n_gu);
   p = (float*)(((uintptr_t)p + 255) & ~(uintptr_t)255);
+  pf_work = take(n_work);
   pf_mb = take(n_act);
   pf_planes = pf_mb;
+  TLB_CUDA(cudaMemsetAsync(pf_work, 0, Q4_TICKET_BYTES, s));
   return TLB_OK;
 }
 
