@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(PB_THREADS, 2)
   bool dead = false;   // a bounded wait gave up: stop computing, but keep every rendezvous
   for (int it = 0; it < n_tiles; it++) {
     const int s_ = it % PB_STAGES, k0 = it * PB_TK;
-    if (!dead && !mbar_wait_bounded(&full[s_], (it / PB_STAGES) & 1, p.status, 720 + s_)) dead = true;
+    if (!dead && !mbar_wait_warp(&full[s_], (it / PB_STAGES) & 1, p.status, 720 + s_)) dead = true;
     unsigned char* tile = base + (size_t)s_ * C::TILE;
     if (n_keys - k0 < PB_TK) {   // the last tile only: values of rows past the chunk
       const int r0 = n_keys - k0, n = (PB_TK - r0) * 8;

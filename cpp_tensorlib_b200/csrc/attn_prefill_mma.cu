@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(32 * (PM_WARPS + 1), 1)
   for (int it = 0; it < n_tiles; it++) {
     const int st = it % PM_STAGES;
     const int k0 = it * PM_TK;
-    if (!dead && !mbar_wait_bounded(&full[st], (it / PM_STAGES) & 1, p.status, 700 + st)) dead = true;
+    if (!dead && !mbar_wait_warp(&full[st], (it / PM_STAGES) & 1, p.status, 700 + st)) dead = true;
     const uint32_t kt = ring32 + (uint32_t)st * C::TILE_BYTES;
     const uint32_t vt = kt + SEGS * PM_BOX;
     if (it == n_tiles - 1 && n_keys - k0 < PM_TK) {

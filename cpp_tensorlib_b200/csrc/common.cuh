@@ -152,6 +152,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
+// The whole warp waits and agrees on the outcome, so that a wait that gave up cannot split it: some lanes at the next
+// barrier, the others in front of a warp-wide instruction, would wait for each other without a limit.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status, int where) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, status, where));
+}
+
 // 2-D tiled TMA load (no multicast): box lands at dst, completion on bar.
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, int x, int y,
                                             uint64_t* bar) {

@@ -84,9 +84,6 @@ __device__ __forceinline__ uint64_t gt_desc(uint32_t addr) {
 __device__ __forceinline__ uint32_t gt_idesc(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(GT_M >> 4) << 24);
 }
-__device__ __forceinline__ bool gt_wait_warp(uint64_t* bar, uint32_t parity, int* status, int where) {
-  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, status, where));
-}
 
 template <int EPI>
 __global__ void __launch_bounds__(GT_THREADS, 1)
@@ -148,10 +145,10 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
     bool ok = true;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, n++) {
       const int buf = n & 1;
-      if (!gt_wait_warp(&dempty[buf], ((n >> 1) & 1) ^ 1, p.status, 711)) break;
+      if (!mbar_wait_warp(&dempty[buf], ((n >> 1) & 1) ^ 1, p.status, 711)) break;
       const uint32_t d = tmem + (uint32_t)(buf * BN);
       for (int k = 0; k < nk; k++) {
-        if (!gt_wait_warp(&full[s], ph, p.status, 710)) { ok = false; break; }
+        if (!mbar_wait_warp(&full[s], ph, p.status, 710)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t a = gt_desc(smem_u32(base + (size_t)s * GT_M * 128));
         const uint64_t b = gt_desc(smem_u32(base + S.B + (size_t)s * BN * 128));
@@ -172,12 +169,13 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, n++) {
       const int buf = n & 1;
       const int m = (t % p.mt) * GT_M + quarter * 32 + lane, n0 = (t / p.mt) * BN;
-      if (!gt_wait_warp(&dfull[buf], (n >> 1) & 1, p.status, 720)) break;
+      if (!mbar_wait_warp(&dfull[buf], (n >> 1) & 1, p.status, 720)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
         uint32_t v[32];
+        __syncwarp();   // lanes of rows behind the last skip the stores
         gt_ld32(taddr + (uint32_t)c0, v);
         if (c0 + 32 >= BN) {
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

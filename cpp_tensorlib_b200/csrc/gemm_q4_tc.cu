@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     for (int kb = 0; kb < nkb && !failed; kb++) {
       const int ri = kb / TC_RAW_KB, rs = ri % TC_STAGES, c = kb % TC_RAW_KB;
       const int s = kb % TC_STAGES;
-      if (c == 0 && !mbar_wait_bounded(&bars[B_RAW_FULL + rs], (ri / TC_STAGES) & 1, p.status, 520)) { failed = true; break; }
-      if (!mbar_wait_bounded(&bars[B_AB_EMPTY + s], ((kb / TC_STAGES) & 1) ^ 1, p.status, 521)) { failed = true; break; }
+      if (c == 0 && !mbar_wait_warp(&bars[B_RAW_FULL + rs], (ri / TC_STAGES) & 1, p.status, 520)) { failed = true; break; }
+      if (!mbar_wait_warp(&bars[B_AB_EMPTY + s], ((kb / TC_STAGES) & 1) ^ 1, p.status, 521)) { failed = true; break; }
       // raw tile: 64-byte rows, 64-byte swizzle (chunk ^ ((row >> 1) & 3))
       const unsigned char* rw = base + L.raw_w + (size_t)rs * TC_ROWS * 64;
       const uint4 q = *(const uint4*)(rw + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
@@ -254,13 +254,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       }
     }
     // ---------------- epilogue: TMEM -> registers -> Y ----------------
-    if (!failed && mbar_wait_bounded(&bars[B_ACC], 0, p.status, 530)) {
+    if (!failed && mbar_wait_warp(&bars[B_ACC], 0, p.status, 530)) {
       tc_fence_after();
       const int quarter = warp & 3;                 // TMEM lanes this warp may read
       const int n = n0 + quarter * 32 + lane;
       const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16);
       for (int c0 = 0; c0 < p.Mt; c0 += 16) {
         float v[16];
+        __syncwarp();   // lanes of weight rows behind the last skip the stores
         tc_ld16(tbase + (uint32_t)c0, v);
         if (n < p.N) {
 #pragma unroll

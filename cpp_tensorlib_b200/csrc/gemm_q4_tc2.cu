@@ -145,10 +145,6 @@ __device__ __forceinline__ bool t2_elect_one() {
       "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
   return pred != 0;
 }
-// the whole warp waits and agrees on the outcome, so a timeout cannot split it
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status, int where) {
-  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, status, where));
-}
 __device__ __forceinline__ void t2_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // K-major, 128-byte swizzle shared-memory matrix descriptor: rows of 128 bytes, 8-row groups

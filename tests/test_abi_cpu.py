@@ -34,3 +34,25 @@ def test_no_compute_without_gpu_fails_loudly():
     with pytest.raises(TlbError):
         check(lib().tlb_init(0))
     assert lib().tlb_q4_bytes(4864, 896) == 2179072 + 544768  # include/types.h:29-31
+
+
+@pytest.mark.parametrize("name", ["gemm_q4_tc.cu", "gemm_bf16_tc.cu", "attn_decode_mma.cu",
+                                  "attn_prefill_mma.cu", "attn_prefill_bf16.cu"])
+def test_whole_warps_agree_on_a_wait(name):
+    """A wait that gives up for some lanes of a warp and not for others leaves them at different barriers.  Where whole
+    warps wait, in front of warp-wide instructions, they vote (mbar_wait_warp) or go on whatever the outcome; a branch on
+    a plain wait is for a single lane."""
+    text = open(os.path.join(ROOT, "cpp_tensorlib_b200", "csrc", name)).read()
+    text = re.sub(r"//[^\n]*", "", text)
+    heads, start, single = [], 0, 0
+    for i, ch in enumerate(text):
+        if ch in "{};":
+            if "mbar_wait_bounded(" in text[start:i] and not re.search(r"if \((\w+)\) \1 = mbar_wait_bounded\(", text[start:i]):
+                assert any("lane == 0" in h or "producer" in h for h in heads), text[start:i].strip()
+                single += 1
+            if ch == "{":
+                heads.append(text[start:i])
+            elif ch == "}":
+                heads.pop()
+            start = i + 1
+    assert single or name == "attn_prefill_bf16.cu"
