@@ -29,9 +29,7 @@ namespace tlb {
 
 namespace {
 
-#ifndef RC_MOST
-#define RC_MOST 8
-#endif
+constexpr int RC_MOST = 8;   // segments
 constexpr int RC_L = 64, RC_E = 32, RC_THREADS = 128;
 constexpr int RC_TLD = RC_L + 8, RC_ELD = RC_E + 8;
 
@@ -637,16 +635,16 @@ __global__ void __launch_bounds__(RC_THREADS, 3)
 }
 
 // Most segments of a prompt (more rows, no fewer): of four chunks at least, since a segment's start reads the states in
-// front of it, eight at most, and no more than four CTAs for each of the places that 148 SMs have.
-int rc_most_segments(const RecurP& p, int rows) {
+// front of it, eight at most, and no more than four CTAs for each of the SMs' places, two an SM.
+int rc_most_segments(const RecurP& p, int rows, int sms) {
   if (p.kind == MIX_DELTA) return 1;
   const int nch = (rows + RC_L - 1) / RC_L, ctas = (p.E + RC_E - 1) / RC_E * p.H;
   int n = nch / 4 < RC_MOST ? nch / 4 : RC_MOST;
-  if (n * ctas > 4 * 2 * 148) n = 4 * 2 * 148 / ctas;
+  if (n * ctas > 4 * 2 * sms) n = 4 * 2 * sms / ctas;
   return n < 2 ? 1 : n;
 }
-RcSegments rc_segments(const RecurP& p, int rows, void* scratch) {
-  const int nch = (rows + RC_L - 1) / RC_L, n = rc_most_segments(p, rows);
+RcSegments rc_segments(const RecurP& p, int rows, int sms, void* scratch) {
+  const int nch = (rows + RC_L - 1) / RC_L, n = rc_most_segments(p, rows, sms);
   RcSegments g{1, nch, nullptr, nullptr};
   if (n == 1) return g;
   g.chunks = (nch + n - 1) / n;
@@ -672,6 +670,11 @@ int rc_walk(const RecurP& p, const void* conv, const float2* gates, const float2
 template <int DP, bool DELTA>
 int rc_launch(const RecurP& p, const void* conv, const float2* gates, const float2* norms, void* T, float* o, int rows,
               int pos0, cudaStream_t s) {
+  DeviceCtx* c = nullptr;
+  {
+    const int rc = get_ctx(&c);
+    if (rc) return rc;
+  }
   if (DELTA) {
     constexpr int smem = RC_L * (DP + 8) * 2 + (2 * RC_L * (RC_L + 1) + 3 * 16 * 17) * 4;
     static std::atomic<unsigned long long> done{0};
@@ -681,7 +684,7 @@ int rc_launch(const RecurP& p, const void* conv, const float2* gates, const floa
     TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, delta_solve_kernel<DP>, p, (const __nv_bfloat16*)conv, gates, norms,
                                 (__nv_bfloat16*)T, rows));
   }
-  const RcSegments g = rc_segments(p, rows, T);
+  const RcSegments g = rc_segments(p, rows, c->sm_count, T);
   if (!DELTA && g.n > 1) {
     constexpr int smem = (int)SsSmem<DP>::TOTAL;
     static std::atomic<unsigned long long> done{0};
@@ -693,7 +696,8 @@ int rc_launch(const RecurP& p, const void* conv, const float2* gates, const floa
   // few heads: half as many columns a CTA, twice the CTAs, where those still find an SM each (4096 tokens, 16 heads of
   // 128: 392 us on 64 SMs, 318 on 128)
   if constexpr (DELTA)
-    if ((p.E + RC_E - 1) / RC_E * p.H <= 74) return rc_walk<DP, DELTA, 16>(p, conv, gates, norms, T, o, rows, pos0, g, s);
+    if (2 * ((p.E + RC_E - 1) / RC_E * p.H) <= c->sm_count)
+      return rc_walk<DP, DELTA, 16>(p, conv, gates, norms, T, o, rows, pos0, g, s);
   return rc_walk<DP, DELTA, RC_E>(p, conv, gates, norms, T, o, rows, pos0, g, s);
 }
 
@@ -703,7 +707,9 @@ bool recur_chunk_eligible(const RecurP& p) { return p.D <= 128 && p.D % 8 == 0 &
 
 size_t recur_chunk_scratch_bytes(const RecurP& p, int rows) {
   if (p.kind == MIX_DELTA) return (size_t)((rows + RC_L - 1) / RC_L) * p.H * 2 * RC_L * RC_L * 2;
-  const int n = rc_most_segments(p, rows);
+  DeviceCtx* c = nullptr;
+  if (get_ctx(&c)) return 0;   // and the launch fails
+  const int n = rc_most_segments(p, rows, c->sm_count);
   return n > 1 ? (size_t)n * p.H * ((size_t)p.D * p.E + 1) * sizeof(float) : 0;
 }
 

@@ -421,3 +421,31 @@ def test_wide_products_of_a_long_prompt(width, ff, rows):
     got = run(m, toks, [rows])
     assert ok(err(got, want), "bfloat16")
     close(m)
+
+
+@pytest.mark.parametrize("right", [(20, 10, 128, 128),    # 80 blocks of 32 columns: more than half the SMs
+                                   (80, 40, 64, 24),      # the same with narrow heads, columns behind the last
+                                   (18, 9, 128, 128),     # 72: blocks of 16 columns
+                                   (74, 37, 48, 16)])
+def test_delta_rule_blocks_of_both_widths(right):
+    """A prompt in portions of ragged last chunks, the second behind a state, against the oracle."""
+    cfg = zc.config([zc.par((4, 2, 64, 64), right, window=60, rot=32, ff=64)], width=128, vocab=160, emb=3.0)
+    w = zc.Weights(cfg, 81)
+    toks = zc.tokens(cfg, 203, 5)
+    m = make(cfg, w, "bfloat16")
+    assert ok(err(run(m, toks, [70, 131]), orc.forward(cfg, w.f64(), toks)), "bfloat16")
+    close(m)
+
+
+@pytest.mark.parametrize("mix,first", [((80, 4, 64, 64), 0),      # 160 blocks a segment: seven segments, not eight
+                                       ((150, 2, 32, 128), 100)])  # 600 of them: one
+def test_segments_of_wide_mixers(mix, first):
+    """More heads than places for eight segments of their blocks, against the same tokens in short portions."""
+    cfg = zc.config([zc.mam(*mix, 4, 2)], width=128, vocab=160, emb=3.0)
+    w = zc.Weights(cfg, 91)
+    rows = 2049 + 64
+    toks = zc.tokens(cfg, first + rows, 9)
+    m = make(cfg, w, "bfloat16", first + rows + 8)
+    want = run(m, toks, [448] * 6)
+    assert ok(err(run(m, toks, [first, rows] if first else [rows]), want), "bfloat16")
+    close(m)
