@@ -1,4 +1,4 @@
-// int4 dequant-matmul for many activation rows (prefill / batched rows, M > 8), second
+// int4 dequant-matmul for many activation rows (prefill / batched rows, M > 8; fewer with deep weights), second
 // formulation: Y[M,N] = alpha * X[M,K] . dequant(Wq) + beta on the 5th-generation tensor cores
 // with the GROUP SCALES KEPT OUT of the tensor-core operands.
 //
@@ -30,7 +30,7 @@
 // 128 rows x 128 bytes (256 k) per box into a ring of four, 64 KB in flight per SM.  (Register
 // loads by the converters, 32 bytes per row and stage with four stages in flight, kept only
 // 16 KB per SM in flight and paced the whole kernel at ~1 TB/s of weight bytes.)  All waits
-// are bounded; a timeout sets the status word, the kernel still frees its TMEM and returns.
+// are bounded; a timeout sets the status word, the kernel still frees its TMEM and returns, and no warp is split by it.
 // No cluster launch, no multicast.
 //
 // What bounds it is the instruction issue of the four schedulers, not the tensor pipe: without any MMA a product takes
@@ -145,6 +145,32 @@ __device__ __forceinline__ bool t2_elect_one() {
       "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
   return pred != 0;
 }
+// The accumulate warps' wait: mbar_wait_warp with the vote on the first poll.  Per lane, lanes that gave up would leave
+// for the named barrier while others went on to the warp-wide TMEM read, and each would wait for the other.
+__device__ __forceinline__ bool t2_wait_vote(uint64_t* bar, uint32_t parity, int* status, int where) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return mbar_wait_warp(bar, parity, status, where);
+}
+// The converters' wait: no outcome to branch on.  A wait that gives up marks the CTA, the converters then wait no more
+// but stay together to the end, and the epilogue writes nothing.
+__device__ __forceinline__ void t2_wait_or_mark(uint64_t* bar, uint32_t parity, int* status, int where,
+                                                volatile int* gave_up) {
+  if (mbar_try_wait(bar, parity)) return;
+  const long long t0 = clock64();
+  while (clock64() - t0 < 8192)   // see mbar_wait_bounded
+    if (mbar_try_wait(bar, parity)) return;
+  const long long limit = wait_limit(status);
+  while (!*gave_up) {
+    if (mbar_try_wait(bar, parity)) return;
+    if (clock64() - t0 > limit) {
+      *gave_up = 1;
+      if (status) {
+        atomicExch(&status[ST_WAIT_TIMEOUT], 1);
+        atomicExch(&status[ST_WAIT_WHERE], where);
+      }
+    }
+  }
+}
 __device__ __forceinline__ void t2_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // K-major, 128-byte swizzle shared-memory matrix descriptor: rows of 128 bytes, 8-row groups
@@ -186,12 +212,13 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
   unsigned char* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* bars = (uint64_t*)(base + S::BARS);
   uint32_t* tmem_slot = (uint32_t*)(base + S::SLOT);
-  volatile int* last_part = (volatile int*)(base + S::SLOT + 8);
+  volatile int *last_part = (volatile int*)(base + S::SLOT + 8), *gave_up = last_part + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nst = p.K / T2_KS;   // 64-k stages of a tile
   T2Segment sg(p);
 
   if (tid == 0) {
+    *gave_up = 0;
     for (int s = 0; s < T2_STAGES; s++) {
       mbar_init(&bars[T2_X_FULL + s], 1);
       mbar_init(&bars[T2_A_READY + s], 4);
@@ -293,14 +320,10 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
     // ---------------- nibble -> fp16 converters (thread r = weight row r) ----------------
     const int r = tid - 64;
     const __half2 off = __floats2half2_rn(1032.0f, 1032.0f);
-    bool conv_ok = true;
     int cnt = 0, it = -1;   // boxes and stages of all segments
-    while (sg.next(p)) for (int q = sg.q0; q < sg.q1 && conv_ok; q++, cnt++) {
+    while (sg.next(p)) for (int q = sg.q0; q < sg.q1; q++, cnt++) {
       const int rs = cnt % T2_RAW_STAGES;
-      if (!mbar_wait_bounded(&bars[T2_RAW_FULL + rs], (cnt / T2_RAW_STAGES) & 1, p.status, 621)) {
-        conv_ok = false;
-        break;
-      }
+      t2_wait_or_mark(&bars[T2_RAW_FULL + rs], (cnt / T2_RAW_STAGES) & 1, p.status, 621, gave_up);
       // the row's 128 packed bytes of this box: chunk c (16 bytes = 32 k) sits at c ^ (r & 7)
       const unsigned char* rrow = base + S::RAW + (size_t)rs * T2_RAW_BYTES + r * 128;
       uint4 wq[2 * T2_SUB];
@@ -312,10 +335,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
         it++;
         const int s = it % T2_STAGES;
         const uint4 c0 = wq[2 * u], c1 = wq[2 * u + 1];
-        if (!mbar_wait_bounded(&bars[T2_ST_EMPTY + s], ((it / T2_STAGES) & 1) ^ 1, p.status, 620)) {
-          conv_ok = false;
-          break;
-        }
+        t2_wait_or_mark(&bars[T2_ST_EMPTY + s], ((it / T2_STAGES) & 1) ^ 1, p.status, 620, gave_up);
         unsigned char* arow = base + S::A + (size_t)s * T2_ROWS * 128 + r * 128;
         const unsigned words[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
 #pragma unroll
@@ -346,7 +366,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
     const int quarter = warp & 3, half = (warp - 6) >> 2;
     const int r = quarter * 32 + lane;
     const int c_lo = half * HC;
-    bool ok = true;   // a wait that gave up: no more work, but every barrier and ticket below
+    bool ok = true;   // of the warp.  A wait that gave up: no more work, but every barrier and ticket below
     unsigned blocks = 0;   // of four groups, of all segments
     while (sg.next(p)) {
       const int tile = sg.tile, q0 = sg.q0, q1 = sg.q1;
@@ -364,7 +384,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
 #pragma unroll
         for (int buf = 0; buf < T2_NBUF; buf++) {   // four groups a block, one accumulator each
           const float sc = buf == 0 ? sc_blk.x : (buf == 1 ? sc_blk.y : (buf == 2 ? sc_blk.z : sc_blk.w));
-          if (!mbar_wait_bounded(&bars[T2_D_FULL + buf], blocks & 1, p.status, 630)) { ok = false; break; }
+          if (!t2_wait_vote(&bars[T2_D_FULL + buf], blocks & 1, p.status, 630)) { ok = false; break; }
           t2_fence_after();
           const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * MT + c_lo);
           // 32 columns per read; the accumulator goes back to the issuers as soon as the last
@@ -423,13 +443,14 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
           }
         }
       }
-      if (mine && ok && n < p.N) {
+      if (mine && ok && !*gave_up && n < p.N) {
 #pragma unroll
         for (int i = 0; i < HC; i++) {
           const int m = m0 + c_lo + i;
           if (m < p.M) p.y[(long long)m * p.ldy + n] = (acc[i] * __ldg(p.rowscale + m)) * p.alpha + p.beta;
         }
       }
+      __syncwarp();   // lanes of rows behind the last: whole warps again for the next segment's reads
     }
   }
   t2_fence_before();

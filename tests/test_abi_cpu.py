@@ -36,7 +36,7 @@ def test_no_compute_without_gpu_fails_loudly():
     assert lib().tlb_q4_bytes(4864, 896) == 2179072 + 544768  # include/types.h:29-31
 
 
-@pytest.mark.parametrize("name", ["gemm_q4_tc.cu", "gemm_bf16_tc.cu", "attn_decode_mma.cu",
+@pytest.mark.parametrize("name", ["gemm_q4_tc.cu", "gemm_q4_tc2.cu", "gemm_bf16_tc.cu", "attn_decode_mma.cu",
                                   "attn_prefill_mma.cu", "attn_prefill_bf16.cu"])
 def test_whole_warps_agree_on_a_wait(name):
     """A wait that gives up for some lanes of a warp and not for others leaves them at different barriers.  Where whole
