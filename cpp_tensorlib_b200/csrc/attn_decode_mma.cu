@@ -22,8 +22,10 @@
 //    B operand of out^T[D x 8 heads] += V_blk^T . P, again three tf32 MMAs per step.
 //  * A bf16 cache is an exact operand of mma.sync m16n8k16 (boxes of 32 rows x 64 bf16, ldmatrix):
 //    Q and P enter as three bf16 planes each, 24 bits and nothing dropped, again three MMAs per
-//    step, of twice the depth.  28 heads on 4, 12345 keys, 25 MB: 20.7 us a call on the CUDA cores,
-//    bound by their instruction issue, 11.9 here, most of it the host's side of the call.
+//    step, of twice the depth.  Infinite queries, keys and values give NaN: a plane of theirs or of their factor is
+//    zero, or infinity less infinity.  (The prompt form computes such rows again in plain f32; here the check alone, by
+//    warp or by CTA, inlined or not, costs 0.1 to 0.2 of 9.9 us a launch and 1 to 3 % of the 0.5B decoder's tokens.)  28 heads on 4, 12345 keys, 25 MB: 20.7 us a call on the CUDA cores,
+//    bound by their instruction issue, 11.4 here, 9.9 of them the launch.
 //  * The warps' (acc, m, l) meet in shared memory, the CTA's partial goes to scratch, an
 //    acq_rel ticket per KV head elects the last CTA, which folds the splits in split order
 //    with every load of the fold in flight at once (one L2 round trip).  One launch,

@@ -13,9 +13,11 @@
 //    runs under the MMAs of the other.
 //  * What bounds it is mma.sync: 6 D MACs a (query, key) pair, the tensor pipe busy for 61 % of an SM's active time;
 //    the other side is the softmax and the latency between the two.  1000 queries x 28 heads of 128 took 551 us
-//    on the CUDA cores, one f32 FMA a MAC; 114 us here head by head, 87 with the longest tiles first.
+//    on the CUDA cores, one f32 FMA a MAC; 114 us here head by head, 84 with the longest tiles first, 83 with the parameters
+//    read in place.  At D = 128 a thread has 255 registers and spills 200 bytes.
 //  * The last tile's rows past the chunk are cleared in shared memory (their weight is zero, but 0 * NaN is NaN).
-//    A key or value that is infinite gives NaN, as in attn_prefill_mma.cu: its product with a zero plane.
+//    Rows that come out NaN are computed again in plain f32 (attn_row_again), where infinite keys and values give what they
+//    give on the CUDA cores.
 #include "attn_common.cuh"
 #include "rows_mma.cuh"
 
@@ -36,6 +38,7 @@ struct PbCfg {
 
 struct PbParams {
   const float* q;
+  const __nv_bfloat16 *K, *V;
   float* out;
   long long q_row, q_head, o_row, o_head;   // strides in floats
   int T, group, kv_rows, pos0;
@@ -82,10 +85,26 @@ __device__ __forceinline__ float pb_ex2(float x) {
   return y;
 }
 
+// rows of the warp that came out NaN, again
+template <int D>
+__device__ __noinline__ void pb_again(const PbParams& p, unsigned a, unsigned b) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.x;
+  const size_t kv = (size_t)(h / p.group) * p.kv_rows * D;
+  for (int r = 0; r < 16; r++) {
+    if (!(((r < 8 ? a : b) >> (4 * (r & 7))) & 15u)) continue;
+    const int row = (int)(gridDim.y - 1 - blockIdx.y) * PB_QT + 16 * warp + r;
+    const AttnRow<D> x = attn_row_again<D>(p.q + h * p.q_head + row * p.q_row, p.K + kv, p.V + kv,
+                                           p.scale * 1.4426950408889634f, 0, p.pos0 + row + 1, 1);
+    float* out = p.out + h * p.o_head + row * p.o_row + lane * (D / 32);
+#pragma unroll
+    for (int i = 0; i < D / 32; i++) out[i] = x.acc[i] / x.l;
+  }
+}
+
 template <int D>
 __global__ void __launch_bounds__(PB_THREADS, 2)
     attn_prefill_bf16_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                             PbParams p) {
+                             const __grid_constant__ PbParams p) {
   using C = PbCfg<D>;
   constexpr int SEGS = C::SEGS, KS = D / 16, NT = D / 8;
   extern __shared__ unsigned char smem_raw[];
@@ -245,11 +264,17 @@ __global__ void __launch_bounds__(PB_THREADS, 2)
   }
   const float i0 = 1.0f / l0, i1 = 1.0f / l1;
   float* oa = p.out + h * p.o_head + ra * p.o_row + 2 * t;
+  bool nan_a = false, nan_b = false;
 #pragma unroll
   for (int j = 0; j < NT; j++) {
-    if (ra < p.T) *(float2*)(oa + 8 * j) = make_float2(o[j][0] * i0, o[j][1] * i0);
-    if (rb < p.T) *(float2*)(oa + 8 * p.o_row + 8 * j) = make_float2(o[j][2] * i1, o[j][3] * i1);
+    const float2 a = make_float2(o[j][0] * i0, o[j][1] * i0), b = make_float2(o[j][2] * i1, o[j][3] * i1);
+    nan_a |= a.x != a.x || a.y != a.y;
+    nan_b |= b.x != b.x || b.y != b.y;
+    if (ra < p.T) *(float2*)(oa + 8 * j) = a;
+    if (rb < p.T) *(float2*)(oa + 8 * p.o_row + 8 * j) = b;
   }
+  const unsigned again_a = __ballot_sync(0xffffffffu, nan_a && ra < p.T), again_b = __ballot_sync(0xffffffffu, nan_b && rb < p.T);
+  if (again_a | again_b) pb_again<D>(p, again_a, again_b);
 }
 
 template <int D>
@@ -285,6 +310,7 @@ int attn_prefill_bf16_launch(DeviceCtx* c, const float* q, long long q_row, long
     return set_error(TLB_ERR_UNSUPPORTED, "attn_prefill: a bf16 cache of 2^31 rows or more");
   PbParams p;
   p.q = q; p.q_row = q_row; p.q_head = q_head;
+  p.K = (const __nv_bfloat16*)K; p.V = (const __nv_bfloat16*)V;
   p.out = out; p.o_row = o_row; p.o_head = o_head;
   p.T = T; p.group = n_q / n_kv; p.kv_rows = (int)kv_max; p.pos0 = pos0;
   p.scale = scale; p.status = c->status;

@@ -179,3 +179,59 @@ def test_attn_prefill_bf16_vs_oracle(tl, port, n_q, n_kv, D, T, pos0, kv_max):
     scale = 1.0 / np.sqrt(D)
     got = tl.attn_prefill(dev(q), Kd, Vd, scale, pos0=pos0).cpu().numpy()
     assert relerr(got, causal_reference(port, q, K, V, scale, pos0)) < 1e-4
+
+
+def attend_f64(q, K, V, scale):
+    """q [D], K, V [n, D] in 64 bits; a key whose score is -infinity has no weight, whatever its value."""
+    s = (q * K).sum(1) * scale
+    on = s != -np.inf
+    w = np.exp(s[on] - s[on].max())
+    return (w[:, None] * V[on]).sum(0) / w.sum()
+
+
+def same_with_infinities(got, want):
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    fin = np.isfinite(want)
+    inf = ~fin & ~np.isnan(want)
+    assert np.array_equal(got[inf], want[inf])
+    return np.abs(got[fin] - want[fin]).max() < 1e-4 * (1 + np.abs(want[fin]).max())
+
+
+@pytest.mark.parametrize("n_q,n_kv,D,T,pos0", [(14, 2, 64, 70, 3), (4, 1, 128, 130, 0), (2, 2, 128, 17, 150)])
+def test_infinities_in_a_bf16_cache(tl, n_q, n_kv, D, T, pos0):
+    """Infinite keys whose scores are -infinity, infinite values, a NaN: what plain f32 attention makes of them, in rows
+    of a prompt that see them, and nothing in rows that do not.  f32 sums: 1e-4 as elsewhere."""
+    n, g = pos0 + T, n_q // n_kv
+    K, V, q = synth.normal(90, 1, (n_kv, n, D)), synth.normal(90, 2, (n_kv, n, D)), synth.normal(90, 3, (n_q, T, D))
+    q[:, :, 5] = -np.abs(q[:, :, 5]) - 0.1
+    K[:, pos0 + 2, 5] = np.inf
+    V[:, pos0 + 5, 7] = np.inf
+    V[:, pos0 + 9, 8] = -np.inf
+    V[:, pos0 + T - 2, 9] = np.nan
+    K, V = bf16_round(K), bf16_round(V)
+    K[:, pos0 + 2, 5], V[:, pos0 + T - 2, 9] = np.inf, np.nan
+    want = np.zeros((n_q, T, D))
+    for h in range(n_q):
+        for t in range(T):
+            e = pos0 + t + 1
+            want[h, t] = attend_f64(q[h, t].astype(np.float64), K[h // g, :e].astype(np.float64),
+                                    V[h // g, :e].astype(np.float64), 0.125)
+    Kd, Vd = dev(K).to(torch.bfloat16), dev(V).to(torch.bfloat16)
+    assert same_with_infinities(tl.attn_prefill(dev(q), Kd, Vd, 0.125, pos0=pos0).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n_q,n_kv,D", [(14, 2, 64), (4, 1, 128), (2, 2, 128)])
+def test_infinite_values_in_single_token_attention(tl, n_q, n_kv, D):
+    """A bf16 cache with infinite values: the dimensions that hold them are not finite (three planes of the weights make
+    NaN of what is an infinity in one), all others are right."""
+    n, g = 300, n_q // n_kv
+    K, V, q = synth.normal(91, 1, (n_kv, n, D)), synth.normal(91, 2, (n_kv, n, D)), synth.normal(91, 3, (n_q, D))
+    K, V = bf16_round(K), bf16_round(V)
+    V[:, 40, 7], V[:, 250, 9] = np.inf, -np.inf
+    for ctx in (40, 41, 250, 300):
+        want = np.stack([attend_f64(q[h].astype(np.float64), K[h // g, :ctx].astype(np.float64),
+                                    V[h // g, :ctx].astype(np.float64), 0.125) for h in range(n_q)])
+        got = tl.attn_decode(dev(q), dev(K).to(torch.bfloat16), dev(V).to(torch.bfloat16), 0.125, ctx=ctx).cpu().numpy()
+        fin = np.isfinite(want)
+        assert np.array_equal(np.isfinite(got), fin)
+        assert np.abs(got[fin] - want[fin]).max() < 1e-4 * (1 + np.abs(want[fin]).max())
