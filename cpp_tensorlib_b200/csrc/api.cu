@@ -327,6 +327,10 @@ static int skinny_rows(const void* qw, const void* scales, int N, int K, int mos
 // launches cost about what the planes do (8 x 3584 x 18944: 34 us, 31 for up to 32 rows on planes).  By the shape
 // alone, with scratch that is made with the context and never moves: such a call allocates nothing, gives the same bits
 // under capture, and a graph of it stays valid.  (Rows deeper than that scratch holds, 131000 at 8 rows, stay skinny.)
+// The planes have one power of two a row where the skinny kernel has one for every 256 k: an element 2^15 or more
+// below its row's largest keeps fewer than 24 bits, of what is then 2^-39 of that largest.  Against 64 bits the planes
+// are closer: 8 rows of 18944, normally distributed, 2.2e-7 of a result (skinny kernel 1.2e-6); each element times
+// exp(3 z), 2.5e-7 (1.3e-5).
 static bool few_rows_on_planes(const void* qw, const void* scales, int N, int K, int M) {
   if (M < 3 || M > 8 || !gemm_q4_planes_possible(qw, scales, N, K, M) || gemm_q4_tc2_scratch_bytes(M, K) > Q4_FEW_BYTES)
     return false;

@@ -10,8 +10,8 @@
 // row (q fragment, running max / sum / accumulator in registers), the four row
 // groups of a warp share each key row, K/V tiles of 32 keys arrive by bulk copy into
 // a two-stage ring.  f32 throughout (the parity bar is 1e-4 against a double CPU
-// reference).  This CUDA-core form is kept for A/B timing against the tensor-core forms: f32 caches
-// take attn_prefill_mma.cu, bf16 caches attn_prefill_bf16.cu.
+// reference).  This CUDA-core form is kept for A/B timing against the tensor-core form of f32 caches
+// (attn_prefill_mma.cu), in head-major rows only; bf16 caches take attn_prefill_bf16.cu.
 #include <cuda_bf16.h>
 
 #include <cstdlib>

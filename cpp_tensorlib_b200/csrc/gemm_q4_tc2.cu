@@ -38,8 +38,10 @@
 // scales, one accumulator each, with nothing left to select at run time.  Measured and dropped: weights in TMEM as
 // the A operand, sixteen accumulate warps, one issuer, one commit a stage, spinning waits, register shares by
 // setmaxnreg with 64-column reads, leaving out the reads of columns behind the last row (the branch keeps the compiler from
-// running one group's reads under another's FMAs: 570 -> 670 us).  1000 x 3584 x 37888: 676 -> 583 us; 1000 x 18944 x 3584, one and a half
-// rounds of tiles: 424 -> 328; 517 x 4864 x 896, 35 tiles: 60 -> 40.
+// running one group's reads under another's FMAs: 570 -> 670 us).  1000 x 3584 x 37888: 676 -> 575 us; 1000 x 18944 x 3584, one and a half
+// rounds of tiles: 424 -> 322; 517 x 4864 x 896, 35 tiles: 60 -> 34.  At 128 columns a thread has 128 registers and spills 48
+// bytes.  The votes of the accumulate warps' waits matter: behind the first poll 573 us, behind the whole wait 588, an outcome
+// carried along instead of a branch 603 to 647.
 #include <cstdlib>
 
 #include "q4_planes.cuh"
