@@ -260,12 +260,10 @@ __global__ void __launch_bounds__(MmaCfg<D, BF>::THREADS, 1)
     // chunk ((g >> 2) * 4 + 2 p (+1)) XOR (row & 7)
     const uint32_t vbase = (uint32_t)(t * 128 + (g & 3) * 4) | ((uint32_t)((((g >> 2) * 4) ^ t) & 7) << 4);
 
-    bool ok = true;
     for (int it = warp >> 1; it < n_tiles; it += W / 2) {
       const int st = it % STAGES;
       const int blk0 = k_begin + it * MM_TK + 16 * half;     // first key of this warp's block
-      // a wait that gave up: what follows is void, but the warp stays together through it
-      if (ok) ok = mbar_wait_bounded(&full[st], (it / STAGES) & 1, p.status, 200 + st);
+      if (!mbar_poll_warp(&full[st], (it / STAGES) & 1, p.status, 200 + st)) break;
       const int valid = k_end - blk0;                         // keys of the block inside the range
       if (valid > 0) {
         const uint32_t kt = ring32 + (uint32_t)st * C::TILE_BYTES;

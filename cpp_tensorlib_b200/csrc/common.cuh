@@ -157,6 +157,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status, int where) {
   return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, status, where));
 }
+// The same with the vote on the first poll, for waits that mostly find their barrier complete.
+__device__ __forceinline__ bool mbar_poll_warp(uint64_t* bar, uint32_t parity, int* status, int where) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return mbar_wait_warp(bar, parity, status, where);
+}
 
 // 2-D tiled TMA load (no multicast): box lands at dst, completion on bar.
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, int x, int y,

@@ -147,12 +147,6 @@ __device__ __forceinline__ bool t2_elect_one() {
       "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
   return pred != 0;
 }
-// The accumulate warps' wait: mbar_wait_warp with the vote on the first poll.  Per lane, lanes that gave up would leave
-// for the named barrier while others went on to the warp-wide TMEM read, and each would wait for the other.
-__device__ __forceinline__ bool t2_wait_vote(uint64_t* bar, uint32_t parity, int* status, int where) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-  return mbar_wait_warp(bar, parity, status, where);
-}
 // The converters' wait: no outcome to branch on.  A wait that gives up marks the CTA, the converters then wait no more
 // but stay together to the end, and the epilogue writes nothing.
 __device__ __forceinline__ void t2_wait_or_mark(uint64_t* bar, uint32_t parity, int* status, int where,
@@ -386,7 +380,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
 #pragma unroll
         for (int buf = 0; buf < T2_NBUF; buf++) {   // four groups a block, one accumulator each
           const float sc = buf == 0 ? sc_blk.x : (buf == 1 ? sc_blk.y : (buf == 2 ? sc_blk.z : sc_blk.w));
-          if (!t2_wait_vote(&bars[T2_D_FULL + buf], blocks & 1, p.status, 630)) { ok = false; break; }
+          if (!mbar_poll_warp(&bars[T2_D_FULL + buf], blocks & 1, p.status, 630)) { ok = false; break; }
           t2_fence_after();
           const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * MT + c_lo);
           // 32 columns per read; the accumulator goes back to the issuers as soon as the last
