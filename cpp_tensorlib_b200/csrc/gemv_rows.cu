@@ -3,230 +3,380 @@
 // an RMS norm (whole row, or a segment in equal parts) and a silu gate; a residual add, the clipped
 // gated unit or the square of relu behind.  W is bf16 or f32 row-major, everything else f32.
 //
-// HBM bound.  A stream of ks adjacent warps owns one row, or two adjacent rows (gate and up
-// interleaved), each warp its own part of K; ks is picked on the host so that the streams of all SMs
-// come out even.  Every warp keeps eight 16-byte loads in flight plus the next eight; the first eight
-// are issued BEFORE the wait for the preceding kernel, so a launch's weight stream starts under its
-// predecessor's tail.  Weights are marked evict-first in the L2: a token streams gigabytes of them
-// once, and what every launch needs again -- instructions, states, activations -- should stay.
+// HBM bound in the long run, but a token's launch streams 17 - 46 MB (2.6 - 7 us) and used to take 4 us beyond that: what
+// it costs is the chain from the end of the launch in front to the first weight used.  So
+//   - a block takes at most half an SM (112 KB, 96 registers x 288 threads): the next launch's block fits beside it and has
+//     its ring of weights full when this launch ends.  One block an SM, a contiguous range of rows each, so that a stage
+//     of the ring (8 rows of 2048, 4 of 4096, ...) is one bulk copy;
+//   - a thread owns the same 16-byte chunks of every row: its activations go from memory to its registers, without shared
+//     memory or a barrier, all loads in flight at once;
+//   - the factor of a norm over the whole row multiplies the sums instead of the activations; the norms' weights are
+//     fetched in front of the wait; the sums of several rows go through the warp together.
+// Launches of one shape behind each other, cold weights, us (before: two rows a warp in registers, two blocks an SM):
+//   2048 -> 10304 with norm 11.1 -> 10.1, 2048 -> 11264 11.7 -> 10.8, 4096 -> 2048 6.9 -> 4.9, 5632 -> 2048 7.3 -> 7.0;
+//   the first with the weights in the L2 already: 11.0 -> 7.1.
+// What is left is the HBM idling from a launch's last bulk copy to the next one's first free stage, about 3 us.  Tried
+// without gain: the weights behind the ring brought to the L2 early by prefetches (they fetch into the far half of the
+// L2: a read behind them runs at 31 bytes a clock and SM, behind a load at 70) or by loads of a word a line (they delay
+// the activations of the launch that still runs); stages of half the size (305 -> 330 us a token of the 8-layer stack).
+// Weights are marked evict-first in the L2: a token streams gigabytes of them once, and what every launch needs again --
+// instructions, states, activations -- should stay.
 #include "mixers.cuh"
 
 namespace tlb {
 
 namespace {
 
-constexpr int RG_WARPS = 8;
+constexpr int RG_WARPS = 8, RG_THREADS = RG_WARPS * 32;   // and a warp that only requests weights
+// Shared memory of a block: at most half an SM's, so that the next launch's blocks fit beside this one's.
+constexpr size_t RG_SMEM_SHARED = 112 * 1024, RG_SMEM_MAX = 226 * 1024;
 
-__device__ __forceinline__ uint4 rg_ld(const void* p, uint64_t pol) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(pol));
-  return v;
+struct RowPlan {
+  int stages, stage_rows, rows_max;   // ring; rows of a stage; most rows of a block
+  int wpr;                            // warps on a row
+  int* status;
+};
+
+// base[i .. i + N) where it lies in [0, n), else 0: N and n multiples of N, 16-byte aligned
+template <int N>
+__device__ __forceinline__ void rg_ld(const float* base, int i, int n, float (&o)[N]) {
+  const bool on = i >= 0 && i < n;
+  const float4* at = (const float4*)(base + (on ? i : 0));
+#pragma unroll
+  for (int k = 0; k < N; k += 4) {
+    const float4 v = __ldcg(at + k / 4);
+    o[k] = on ? v.x : 0.f; o[k + 1] = on ? v.y : 0.f; o[k + 2] = on ? v.z : 0.f; o[k + 3] = on ? v.w : 0.f;
+  }
+}
+// the same for any n and alignment
+template <int N>
+__device__ __forceinline__ void rg_ld_any(const float* base, int i, int n, float (&o)[N]) {
+#pragma unroll
+  for (int k = 0; k < N; k++) o[k] = i + k >= 0 && i + k < n ? __ldcg(base + i + k) : 0.f;
 }
 
-// x into xs [ldw], zero behind K; returns this thread's share of its sum of squares.  Kept short: a
-// launch runs this code once, from a cold instruction cache.
-__device__ __forceinline__ float rg_stage(const RowGemv& p, float* xs) {
-  float sq = 0.f;
-  const int k4 = ((uintptr_t)p.x & 15) ? 0 : p.K / 4;   // rows of an odd width go one by one
-  for (int i0 = threadIdx.x; i0 < k4; i0 += 4 * RG_WARPS * 32) {
-    float4 v[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-      if (i0 + u * RG_WARPS * 32 < k4) v[u] = ((const float4*)p.x)[i0 + u * RG_WARPS * 32];
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-      if (i0 + u * RG_WARPS * 32 < k4) {
-        ((float4*)xs)[i0 + u * RG_WARPS * 32] = v[u];
-        sq = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, fmaf(v[u].w, v[u].w, sq))));
-      }
-  }
+// What the elements of the row are multiplied with needs sums over it: of the whole row the factor is taken out of
+// the product (rg_scale), of a segment in parts a warp sums each part here.  gs [n_groups], ends with a barrier.
+__device__ __forceinline__ bool rg_whole(const RowGemv& p) { return p.nw && p.n_groups == 1 && p.n_len == p.K; }
+__device__ __forceinline__ void rg_parts(const RowGemv& p, float* gs) {
+  const int m = p.n_len / p.n_groups, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll 1
-  for (int i = 4 * k4 + threadIdx.x; i < p.ldw; i += RG_WARPS * 32) {
-    const float x = i < p.K ? p.x[i] : 0.f;
-    xs[i] = x;
-    sq = fmaf(x, x, sq);
+  for (int g = warp; g < p.n_groups; g += RG_WARPS) {
+    float q = 0.f;
+#pragma unroll 1
+    for (int i0 = 0; i0 < m; i0 += 512) {
+      float v[16];
+#pragma unroll
+      for (int k = 0; k < 16; k++) v[k] = i0 + lane + 32 * k < m ? __ldcg(p.x + p.n_off + g * m + i0 + lane + 32 * k) : 0.f;
+#pragma unroll
+      for (int k = 0; k < 16; k++) q = fmaf(v[k], v[k], q);
+    }
+    q = warp_sum(q);
+    if (lane == 0) gs[g] = rsqrtf(q / m + p.eps) * p.nscale;
   }
-  return sq;
 }
-
-// the preceding sublayer's output, normed, added to the residual: every block computes the row, block 0
-// leaves it for the launches behind.  Returns the thread's share of the new row's sum of squares.
-__device__ __forceinline__ float rg_residual(const RowGemv& p, float* xs, float sq, float* red) {
-  const float s = rsqrtf(block_sum(sq, red) / p.K + p.eps);
-  sq = 0.f;
-#pragma unroll 8
-  for (int i = threadIdx.x; i < p.K; i += RG_WARPS * 32) {
-    const float v = fmaf(xs[i] * s, p.rn[i], p.res[i]);
-    xs[i] = v;
-    if (p.xout && blockIdx.x == 0) p.xout[i] = v;
-    sq = fmaf(v, v, sq);
+// N elements of the staged row from e0 on: v holds them as they are in x, w the norm's weights, r and rn the residual and
+// its weights, g the gate; s is the residual's scale
+template <int N>
+__device__ __forceinline__ void rg_prepare(const RowGemv& p, int e0, float (&v)[N], const float (&w)[N], const float (&r)[N],
+                                           const float (&rn)[N], const float (&g)[N], float s, const float* gs, float& sq) {
+  if (p.res) {
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+      v[k] = fmaf(v[k] * s, rn[k], r[k]);
+      if (p.xout && blockIdx.x == 0 && e0 + k < p.K) p.xout[e0 + k] = v[k];
+    }
   }
-  return sq;
-}
-
-// the norm in place: the whole row by the block, a segment in parts a warp each
-__device__ __forceinline__ void rg_norm(const RowGemv& p, float* xs, float sq, float* red) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  if (p.n_groups == 1 && p.n_len == p.K) {
-    const float s = rsqrtf(block_sum(sq, red) / p.K + p.eps) * p.nscale;
-#pragma unroll 4
-    for (int i = tid; i < p.K; i += RG_WARPS * 32) xs[i] *= p.gate ? s * p.nw[i] * silu_f(p.gate[i]) : s * p.nw[i];
+#pragma unroll
+  for (int k = 0; k < N; k++) sq = fmaf(v[k], v[k], sq);
+  if (!p.nw) return;
+  if (rg_whole(p)) {
+#pragma unroll
+    for (int k = 0; k < N; k++) v[k] *= p.gate ? w[k] * silu_f(g[k]) : w[k];
     return;
+  }
+  if (e0 + N <= p.n_off || e0 >= p.n_off + p.n_len) return;
+  const int m = p.n_len / p.n_groups;
+  int part = e0 <= p.n_off ? 0 : (e0 - p.n_off) / m;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const int e = e0 + k - p.n_off;
+    if (e < 0 || e >= p.n_len) continue;
+    if (e >= (part + 1) * m) part++;
+    v[k] *= p.gate ? gs[part] * w[k] * silu_f(g[k]) : gs[part] * w[k];
+  }
+}
+// R sums over a warp: afterwards lane l holds the sum of v[rg_sum_of<R>(l)] in v[0]
+template <int R>
+__device__ __forceinline__ int rg_sum_of(int lane) { return R == 1 ? 0 : (lane >> 4) + (R >= 4 ? ((lane >> 3) & 1) * 2 : 0) + (R >= 8 ? ((lane >> 2) & 1) * 4 : 0); }
+template <int R>
+__device__ __forceinline__ void rg_warp_sums(float (&v)[R], int lane) {
+  int o = 16;
+#pragma unroll
+  for (int n = R; n > 1; n >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n / 2; i++) {
+      const float send = up ? v[2 * i] : v[2 * i + 1], keep = up ? v[2 * i + 1] : v[2 * i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+    o >>= 1;
+  }
+#pragma unroll
+  for (int k = 0; k < 5; k++)
+    if ((16 >> k) <= o) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16 >> k);
+}
+// sums of the eight warps, the same in every thread behind a barrier
+__device__ __forceinline__ float rg_total(const float* red) {
+  float t = 0.f;
+#pragma unroll
+  for (int w = 0; w < RG_WARPS; w++) t += red[w];
+  return t;
+}
+__device__ __forceinline__ void rg_sync() { asm volatile("bar.sync 1, %0;" ::"n"(RG_THREADS) : "memory"); }
+__device__ __forceinline__ void rg_emit(const RowGemv& p, int n, float a, float b, float y0) {
+  if (p.epi == 2) p.y[n >> 1] = glu_clipped(a, b, p.limit);
+  else p.y[n] = p.epi == 1 ? y0 + a : (p.epi == 3 ? relu2(a) : a);
+}
+__host__ __device__ constexpr int rg_rows_of(int jn) { return jn == 1 ? 8 : (jn == 2 ? 4 : (jn <= 4 ? 2 : 1)); }
+
+// JN: 16-byte chunks of a row that a thread owns
+template <typename WT, int JN>
+__global__ void __launch_bounds__(RG_THREADS + 32, JN < 8 ? 2 : 1) row_gemv_kernel(const __grid_constant__ RowGemv p,
+                                                                      const __grid_constant__ RowPlan pl) {
+  constexpr int CE = Vec16<WT>::N, RB = rg_rows_of(JN);
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ float red[2][RG_WARPS];
+  __shared__ __align__(8) uint64_t full[16], empty[16];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, S = pl.stages;
+  const int u = p.epi == 2 ? 2 : 1, units = (p.N + u - 1) / u, b = blockIdx.x;
+  const int ub = units / (int)gridDim.x, ur = units - ub * (int)gridDim.x;
+  const int r0 = (b * ub + (b < ur ? b : ur)) * u;
+  int rows = (ub + (b < ur)) * u;
+  if (rows > p.N - r0) rows = p.N - r0;
+  const int RS = pl.stage_rows, nst = (rows + RS - 1) / RS, chunks = (int)(p.ldw / CE);
+  const size_t row_bytes = (size_t)p.ldw * sizeof(WT), stage_bytes = RS * row_bytes;
+  float* part = (float*)(smem + S * stage_bytes);   // [wpr][rows_max]
+  auto request = [&](int i, int st, uint64_t pol) {
+    const int n = rows - i * RS < RS ? rows - i * RS : RS;
+    mbar_expect_tx(&full[st], (uint32_t)(n * row_bytes));
+    bulk_load_1d_hint(smem + st * stage_bytes, (const unsigned char*)p.W + (size_t)r0 * row_bytes + i * stage_bytes,
+                      (uint32_t)(n * row_bytes), &full[st], pol);
+  };
+  if (tid == RG_THREADS) {
+    for (int i = 0; i < S; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], RG_WARPS); }
+    mbar_fence_init();
+    const uint64_t pol = l2_evict_first_policy();
+    for (int i = 0; i < S && i < nst; i++) request(i, i, pol);
   }
   __syncthreads();
-  const int m = p.n_len / p.n_groups;
-#pragma unroll 1
-  for (int g = tid >> 5; g < p.n_groups; g += RG_WARPS) {
-    float* seg = xs + p.n_off + g * m;
-    float q = 0.f;
-#pragma unroll 4
-    for (int i = lane; i < m; i += 32) q = fmaf(seg[i], seg[i], q);
-    const float s = rsqrtf(warp_sum(q) / m + p.eps) * p.nscale;
-#pragma unroll 4
-    for (int i = lane; i < m; i += 32)
-      seg[i] *= p.gate ? s * p.nw[g * m + i] * silu_f(p.gate[g * m + i]) : s * p.nw[g * m + i];
-  }
-}
-
-template <int R>
-__device__ __forceinline__ void rg_emit(const RowGemv& p, int rg, const float (&a)[R]) {
-  if (p.epi == 2) {
-    if (R == 2) p.y[rg] = glu_clipped(a[0], a[R - 1], p.limit);
+  if (warp == RG_WARPS) {
+    if (lane) return;
+    const uint64_t pol = l2_evict_first_policy();
+    int st = 0;
+    unsigned parity = 0;
+    for (int i = S; i < nst; i++) {
+      if (!mbar_wait_bounded(&empty[st], parity, pl.status, 801)) break;
+      request(i, st, pol);
+      if (++st == S) { st = 0; parity ^= 1u; }
+    }
     return;
   }
+  if (p.nw)   // the norms' weights into the L2
+    for (int i = tid * 32; i < p.n_len; i += RG_THREADS * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.nw + i));
+  if (p.rn)
+    for (int i = tid * 32; i < p.K; i += RG_THREADS * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.rn + i));
+  const int wpr = pl.wpr, G = RG_WARPS / wpr, grp = warp / wpr, wsub = warp - grp * wpr;
+  const int c0 = JN == 1 ? wsub * 32 + lane : tid;   // this thread's chunks: c0, c0 + 256, ...
+  // what fits the registers beside the row is fetched with it, the norms' weights in front of the wait
+  constexpr bool FEW = JN <= 2, ONE = JN == 1;
+  float x[JN][CE], nw[FEW ? JN : 1][CE], gate[FEW ? JN : 1][CE], rn[CE], res[CE];
+  auto ld_nw = [&](int j, float (&o)[CE]) { if (p.nw) rg_ld<CE>(p.nw, (c0 + j * RG_THREADS) * CE - p.n_off, p.n_len, o); };
+  auto ld_gate = [&](int j, float (&o)[CE]) { if (p.gate) rg_ld<CE>(p.gate, (c0 + j * RG_THREADS) * CE - p.n_off, p.n_len, o); };
+  auto ld_rn = [&](int j) { if (p.rn) rg_ld<CE>(p.rn, (c0 + j * RG_THREADS) * CE, p.K, rn); };
+  auto ld_res = [&](int j) { if (p.res) rg_ld<CE>(p.res, (c0 + j * RG_THREADS) * CE, p.K, res); };
+  if (FEW)
 #pragma unroll
-  for (int r = 0; r < R; r++) {
-    const int n = rg * R + r;
-    if (n < p.N) p.y[n] = p.epi == 1 ? p.y[n] + a[r] : (p.epi == 3 ? relu2(a[r]) : a[r]);
+    for (int j = 0; j < JN; j++) ld_nw(j, nw[FEW ? j : 0]);
+  if (ONE) ld_rn(0);
+  pdl_wait();
+#pragma unroll
+  for (int j = 0; j < JN; j++) rg_ld<CE>(p.x, (c0 + j * RG_THREADS) * CE, p.K, x[j]);
+  if (ONE) ld_res(0);
+  if (FEW)
+#pragma unroll
+    for (int j = 0; j < JN; j++) ld_gate(j, gate[FEW ? j : 0]);
+  const float y0 = p.epi == 1 && tid < rows ? __ldcg(p.y + r0 + tid) : 0.f;   // what the row is added to
+  pdl_launch_dependents();
+  float s = 0.f, sq = 0.f;
+  if (p.res) {   // 1 / rms of the preceding sublayer's output
+#pragma unroll
+    for (int i = 0; i < JN * CE; i++) sq = fmaf(x[i / CE][i % CE], x[i / CE][i % CE], sq);
+    sq = warp_sum(grp == 0 ? sq : 0.f);
+    if (lane == 0) red[0][warp] = sq;
+    rg_sync();
+    s = rsqrtf(rg_total(red[0]) / p.K + p.eps);
+    sq = 0.f;
   }
-}
-
-template <typename WT, int R>
-__global__ void __launch_bounds__(RG_WARPS * 32, 2) row_gemv_kernel(const __grid_constant__ RowGemv p, int ks) {
-  constexpr int CE = Vec16<WT>::N, U = 8 / R;
-  extern __shared__ __align__(16) float xs[];   // [ldw], then the streams' partial sums
-  __shared__ float red[33];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int groups = (p.N + R - 1) / R, ns = RG_WARPS / ks, stream = warp / ks, sub = warp - stream * ks;
-  const int stride = gridDim.x * ns, chunks = (int)(p.ldw / CE), per = (chunks + ks - 1) / ks;
-  const int c_lo = sub * per, c_hi = c_lo + per < chunks ? c_lo + per : chunks;
-  float* part = xs + p.ldw;                     // [local group][stream][R][ks]
-  const WT* W = (const WT*)p.W;
-  const uint64_t pol = l2_evict_first_policy();
-  int rg = blockIdx.x * ns + stream, cb = c_lo, loc = 0;
-  uint4 cur[R][U], nxt[R][U];
-  auto fetch = [&](uint4 (&w)[R][U], int g, int b) {
+  float* gs = part + pl.wpr * pl.rows_max;
+  if (p.nw && !rg_whole(p)) {
+    rg_parts(p, gs);
+    rg_sync();
+  }
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      const WT* row = W + (size_t)(g * R + r < p.N ? g * R + r : p.N - 1) * p.ldw;
+  for (int j = 0; j < JN; j++) {
+    if (!ONE) { ld_rn(j); ld_res(j); }
+    if (!FEW) { ld_nw(j, nw[0]); ld_gate(j, gate[0]); }
+    rg_prepare<CE>(p, (c0 + j * RG_THREADS) * CE, x[j], nw[FEW ? j : 0], res, rn, gate[FEW ? j : 0], s, gs, sq);
+  }
+  if (rg_whole(p)) {
+    sq = warp_sum(grp == 0 ? sq : 0.f);
+    if (lane == 0) red[1][warp] = sq;
+  }
+  bool ok = true;
+  int st = 0;
+  unsigned parity = 0;
+  // chunks that the row does not have: its first is read and dropped
+  constexpr int SURE = JN < 8 ? JN - 1 : 4;
+  auto has = [&](int j) { return j < SURE || c0 + j * RG_THREADS < chunks; };
+  const uint32_t at = smem_u32(smem) + (uint32_t)(grp * row_bytes) + (uint32_t)c0 * 16u, rstep = (uint32_t)(G * row_bytes);
+  const int row_of = rg_sum_of<RB>(lane) * G + grp;
+  float* dst = part + wsub * pl.rows_max;
+  for (int i = 0; i < nst; i++) {
+    ok = ok && mbar_poll_warp(&full[st], parity, pl.status, 800);
+    const uint32_t base = at + (uint32_t)(st * stage_bytes);
+    float acc[RB];
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int c = b + lane + 32 * u;
-        w[r][u] = c < c_hi ? rg_ld(row + (size_t)c * CE, pol) : make_uint4(0, 0, 0, 0);
+    for (int r = 0; r < RB; r++) {   // (rows behind the last one: whatever the slot held, and not kept)
+      acc[r] = 0.f;
+#pragma unroll
+      for (int j = 0; j < JN; j++) {
+        uint4 w;
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
+                     : "r"(base + r * rstep + (has(j) ? (uint32_t)j * (RG_THREADS * 16u) : 0u - (uint32_t)c0 * 16u)));
+        if (!has(j)) w = make_uint4(0, 0, 0, 0);
+        float f[CE];
+        widen16(w, f, (const WT*)nullptr);
+#pragma unroll
+        for (int e = 0; e < CE; e++) acc[r] = fmaf(f[e], x[j][e], acc[r]);
       }
     }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[st]);
+    if (++st == S) { st = 0; parity ^= 1u; }
+    rg_warp_sums<RB>(acc, lane);
+    const int row = i * RS + row_of;
+    if ((lane & (32 / RB - 1)) == 0 && row < rows) dst[row] = acc[0];
+  }
+  rg_sync();
+  const float f = rg_whole(p) ? rsqrtf(rg_total(red[1]) / p.K + p.eps) * p.nscale : 1.f;
+  auto row_sum = [&](int r) {
+    float a = 0.f;
+    for (int k = 0; k < wpr; k++) a += part[k * pl.rows_max + r];
+    return a * f;
   };
-  if (rg < groups) fetch(cur, rg, cb);
-  if (p.nw)   // the norm's weights into the L2
-    for (int i = tid * 32; i < p.n_len; i += RG_WARPS * 32 * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.nw + i));
-  if (p.rn)
-    for (int i = tid * 32; i < p.K; i += RG_WARPS * 32 * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.rn + i));
+  for (int r = tid * u; r < rows; r += RG_THREADS * u)
+    rg_emit(p, r0 + r, row_sum(r), u == 2 ? row_sum(r + 1) : 0.f, p.epi != 1 || r == tid ? y0 : p.y[r0 + r]);
+}
+
+// Rows too long for the registers of a block, and rows of odd widths or places: the staged row in shared memory, weights straight from memory, a block
+// for a row (or pair) at a time.
+template <typename WT>
+__global__ void __launch_bounds__(RG_THREADS) row_gemv_long_kernel(const __grid_constant__ RowGemv p) {
+  constexpr int CE = Vec16<WT>::N;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ float red[33];
+  float* xs = (float*)smem;
+  float* gs = xs + p.ldw;
+  const int tid = threadIdx.x, chunks = (int)(p.ldw / CE), u = p.epi == 2 ? 2 : 1, units = (p.N + u - 1) / u;
   pdl_wait();
   pdl_launch_dependents();
-  float sq = rg_stage(p, xs);
-  if (p.res) sq = rg_residual(p, xs, sq, red);
-  if (p.nw) rg_norm(p, xs, sq, red);
-  __syncthreads();
-  float acc[R][2];
-#pragma unroll
-  for (int r = 0; r < R; r++) acc[r][0] = acc[r][1] = 0.f;
-  while (rg < groups) {
-    int ng = rg, nb = cb + 32 * U;
-    if (nb >= c_hi) { ng += stride; nb = c_lo; }
-    if (ng < groups) fetch(nxt, ng, nb);
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int c = cb + lane + 32 * u;
-      if (c < c_hi) {
-        float x[CE];
-#pragma unroll
-        for (int e = 0; e < CE; e += 4) {
-          const float4 v = *(const float4*)(xs + (size_t)c * CE + e);
-          x[e] = v.x; x[e + 1] = v.y; x[e + 2] = v.z; x[e + 3] = v.w;
-        }
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          float w[CE];
-          widen16(cur[r][u], w, (const WT*)nullptr);
-#pragma unroll
-          for (int e = 0; e < CE; e++) acc[r][e & 1] = fmaf(w[e], x[e], acc[r][e & 1]);
-        }
-      }
-    }
-    if (ng != rg) {
-      float a[R];
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        a[r] = warp_sum(acc[r][0] + acc[r][1]);
-        acc[r][0] = acc[r][1] = 0.f;
-      }
-      if (lane == 0) {
-        if (ks == 1) {
-          rg_emit<R>(p, rg, a);
-        } else {
-#pragma unroll
-          for (int r = 0; r < R; r++) part[((loc * ns + stream) * R + r) * ks + sub] = a[r];
-        }
-      }
-      loc++;
-    }
-    rg = ng;
-    cb = nb;
-#pragma unroll
-    for (int r = 0; r < R; r++)
-#pragma unroll
-      for (int u = 0; u < U; u++) cur[r][u] = nxt[r][u];
+  float s = 0.f, sq = 0.f;
+  if (p.res) {
+    for (int i = tid; i < p.K; i += RG_THREADS) { const float v = p.x[i]; sq = fmaf(v, v, sq); }
+    s = rsqrtf(block_sum(sq, red) / p.K + p.eps);
+    sq = 0.f;
   }
-  if (ks == 1) return;
+  if (p.nw && !rg_whole(p)) rg_parts(p, gs);
   __syncthreads();
-  for (int i = tid;; i += RG_WARPS * 32) {
-    const int l = i / ns, g = (blockIdx.x * ns + i - l * ns) + l * stride;
-    if (l * stride + (int)blockIdx.x * ns >= groups) break;
-    if (g >= groups) continue;
-    float a[R];
+  for (int c = tid; c < chunks; c += RG_THREADS) {
+    float v[CE];
+    float w[CE], r[CE], rn[CE], g[CE];
+    rg_ld_any<CE>(p.x, c * CE, p.K, v);
+    if (p.nw) rg_ld_any<CE>(p.nw, c * CE - p.n_off, p.n_len, w);
+    if (p.rn) rg_ld_any<CE>(p.rn, c * CE, p.K, rn);
+    if (p.res) rg_ld_any<CE>(p.res, c * CE, p.K, r);
+    if (p.gate) rg_ld_any<CE>(p.gate, c * CE - p.n_off, p.n_len, g);
+    rg_prepare<CE>(p, c * CE, v, w, r, rn, g, s, gs, sq);
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      a[r] = 0.f;
-      for (int k = 0; k < ks; k++) a[r] += part[(i * R + r) * ks + k];
+    for (int e = 0; e < CE; e++) xs[c * CE + e] = v[e];
+  }
+  sq = block_sum(sq, red);
+  const float f = rg_whole(p) ? rsqrtf(sq / p.K + p.eps) * p.nscale : 1.f;
+  for (int b = blockIdx.x; b < units; b += gridDim.x) {
+    float a[2] = {0.f, 0.f};
+    for (int r = 0; r < u; r++) {
+      const uint4* w = (const uint4*)((const WT*)p.W + (size_t)(b * u + r) * p.ldw);
+      float acc = 0.f;
+#pragma unroll 4
+      for (int c = tid; c < chunks; c += RG_THREADS) {
+        float wv[CE];
+        widen16(__ldcs(w + c), wv, (const WT*)nullptr);
+#pragma unroll
+        for (int e = 0; e < CE; e++) acc = fmaf(wv[e], xs[c * CE + e], acc);
+      }
+      a[r] = block_sum(acc, red) * f;
     }
-    rg_emit<R>(p, g, a);
+    if (tid == 0) rg_emit(p, b * u, a[0], a[1], p.epi == 1 ? p.y[b] : 0.f);
   }
 }
 
-template <typename WT, int R>
-int rg_launch(DeviceCtx* c, const RowGemv& p, cudaStream_t s) {
+template <typename WT, int JN>
+int rg_launch(const RowGemv& p, const RowPlan& pl, int ctas, size_t smem, cudaStream_t s) {
   static std::atomic<unsigned long long> done{0};
-  const int rc = ensure_dynamic_smem(row_gemv_kernel<WT, R>, 220 * 1024, done);
+  const int rc = ensure_dynamic_smem(row_gemv_kernel<WT, JN>, RG_SMEM_MAX, done);
   if (rc) return rc;
-  const int groups = (p.N + R - 1) / R, chunks = (int)(p.ldw / Vec16<WT>::N), full = 2 * c->sm_count;
-  // warps a stream (single rows): the fewest that come within 3 % of the most even division
-  int ks = 1;
-  double best = 1e30;
-  for (int k = 1; k <= RG_WARPS; k *= 2) {
-    if (k > 1 && chunks / k < 32 * 4) break;
-    const int ns = RG_WARPS / k;
-    const double cost = (double)((groups + full * ns - 1) / (full * ns)) / k;
-    if (cost < best * 0.97) { best = cost; ks = k; }
-    if (R == 2) break;   // two rows a warp: the extra sums cost more than the unevenness
-  }
-  const int ns = RG_WARPS / ks, need = (groups + ns - 1) / ns, ctas = need < full ? need : full;
-  const int local = (groups + ctas * ns - 1) / (ctas * ns);
-  const size_t smem = ((size_t)p.ldw + (ks > 1 ? (size_t)local * ns * R * ks : 0)) * sizeof(float);
-  if (smem > 220 * 1024) return set_error(TLB_ERR_UNSUPPORTED, "row_gemv: the activation row does not fit the shared-memory stage");
-  LaunchCfg lc(dim3(ctas), dim3(RG_WARPS * 32), smem, s, pdl_enabled());
-  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, row_gemv_kernel<WT, R>, p, ks));
+  LaunchCfg lc(dim3(ctas), dim3(RG_THREADS + 32), smem, s, pdl_enabled());
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, row_gemv_kernel<WT, JN>, p, pl));
   return TLB_OK;
+}
+template <typename WT>
+int rg_plan_launch(DeviceCtx* c, const RowGemv& p, cudaStream_t s) {
+  constexpr int CE = Vec16<WT>::N;
+  const int chunks = (int)(p.ldw / CE), u = p.epi == 2 ? 2 : 1, units = (p.N + u - 1) / u;
+  auto aligned = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
+  const bool vec = aligned(p.x) && aligned(p.res) && aligned(p.rn) && aligned(p.nw) && aligned(p.gate) && p.K % CE == 0 &&
+                   (!p.nw || (p.n_off % CE == 0 && p.n_len % CE == 0));
+  const int groups = p.nw ? p.n_groups : 0;
+  const int need = (chunks + RG_THREADS - 1) / RG_THREADS, jn = need <= 4 ? need : (need <= 8 ? 8 : 0);
+  const int ctas = units < c->sm_count ? units : c->sm_count;
+  RowPlan pl{};
+  pl.status = c->status;
+  pl.rows_max = (units + ctas - 1) / ctas * u;
+  pl.wpr = RG_WARPS;
+  while (pl.wpr > 1 && chunks <= pl.wpr / 2 * 32) pl.wpr /= 2;
+  const size_t row = (size_t)p.ldw * sizeof(WT), tail = ((size_t)pl.wpr * pl.rows_max + groups) * sizeof(float) + 16;
+  pl.stage_rows = jn ? rg_rows_of(jn) * (RG_WARPS / pl.wpr) : 1;
+  const size_t stage = row * pl.stage_rows;
+  const int nst = (pl.rows_max + pl.stage_rows - 1) / pl.stage_rows;
+  pl.stages = nst < 16 ? nst : 16;
+  while (pl.stages > 2 && pl.stages * stage + tail > RG_SMEM_SHARED) pl.stages--;
+  const size_t smem = pl.stages * stage + tail;
+  if (!jn || !vec || smem > RG_SMEM_MAX) {
+    const size_t bytes = ((size_t)p.ldw + groups) * sizeof(float);
+    if (bytes > 225 * 1024) return set_error(TLB_ERR_UNSUPPORTED, "row_gemv: the activation row does not fit the shared-memory stage");
+    static std::atomic<unsigned long long> done{0};
+    const int rc = ensure_dynamic_smem(row_gemv_long_kernel<WT>, 225 * 1024, done);
+    if (rc) return rc;
+    LaunchCfg lc(dim3(ctas), dim3(RG_THREADS), bytes, s, pdl_enabled());
+    TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, row_gemv_long_kernel<WT>, p));
+    return TLB_OK;
+  }
+  if (jn == 1) return rg_launch<WT, 1>(p, pl, ctas, smem, s);
+  if (jn == 2) return rg_launch<WT, 2>(p, pl, ctas, smem, s);
+  if (jn == 3) return rg_launch<WT, 3>(p, pl, ctas, smem, s);
+  if (jn == 4) return rg_launch<WT, 4>(p, pl, ctas, smem, s);
+  return rg_launch<WT, 8>(p, pl, ctas, smem, s);
 }
 
 // ---- row ops of the prompt pass --------------------------------------------------------------
@@ -329,10 +479,7 @@ __global__ void relu2_rows_kernel(const float* __restrict__ u, float* __restrict
 }  // namespace
 
 int row_gemv_launch(DeviceCtx* c, const RowGemv& p, bool bf16, cudaStream_t s) {
-  // two rows a stream where the rows come in pairs, or where there are enough of them to fill the SMs
-  const bool two = p.epi == 2 || p.N >= 2 * 2 * c->sm_count * RG_WARPS;
-  if (bf16) return two ? rg_launch<__nv_bfloat16, 2>(c, p, s) : rg_launch<__nv_bfloat16, 1>(c, p, s);
-  return two ? rg_launch<float, 2>(c, p, s) : rg_launch<float, 1>(c, p, s);
+  return bf16 ? rg_plan_launch<__nv_bfloat16>(c, p, s) : rg_plan_launch<float>(c, p, s);
 }
 
 int rms_rows_launch(const float* x, long long ldx, const float* w, void* out, long long ldo, int n, float eps,
