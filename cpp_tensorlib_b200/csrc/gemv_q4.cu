@@ -50,6 +50,7 @@ struct GemvParams {
   int* status;
   int RT, SL;       // row tiles (16 rows), k slabs (256 k)
   unsigned U;       // RT * SL
+  int own;          // 0: warps own unit ranges; else the most row tiles of a block, whose units its warps share
   int x_vec_ok;     // x rows are 16-byte aligned
   int act;          // 0: x as given; 1: x row = [gate(K) | up(K)], activation silu(gate)*up;
                     // 2: x = rmsnorm(x + delta) * nw (M == 1), the sum also written to xout
@@ -64,9 +65,9 @@ struct GemvParams {
 
 // Shared-memory carve-up (host and device agree through this one function).
 struct GemvSmem {
-  size_t w_ring, s_ring, bars, red, pslab, q, bfrag, total;
+  size_t w_ring, s_ring, bars, red, pslab, q, bfrag, ures, total;
 };
-__host__ __device__ inline GemvSmem gemv_smem_layout(int warps, int stages, int M, int K) {
+__host__ __device__ inline GemvSmem gemv_smem_layout(int warps, int stages, int M, int K, int own = 0) {
   const int SL = (K + 255) / 256, G = SL * 8;
   GemvSmem L;
   size_t o = 0;
@@ -80,14 +81,16 @@ __host__ __device__ inline GemvSmem gemv_smem_layout(int warps, int stages, int 
   L.q = o;      o += (size_t)GV_MAXM * G * sizeof(float);
   o = (o + 15) & ~(size_t)15;
   L.bfrag = o;  o += (size_t)G * (2 * M) * 4 * sizeof(uint4);
+  L.ures = o;   o += (size_t)own * SL * M * 16 * sizeof(float);
   L.total = o + 1024;  // slack for the 1 KB alignment of the dynamic base
   return L;
 }
 
-// WARPS x STAGES: 8 x 4 (two CTAs per SM, for K up to ~6K) or 16 x 3 (one CTA per
-// SM, large K whose activation fragments need more shared memory).  Either way
+// WARPS x STAGES: 8 x 4 (two CTAs per SM, for K up to ~6K), 16 x 3 (one CTA per
+// SM, large K whose activation fragments need more shared memory) or, for five to eight
+// rows that only so fit one pass over the weights, 16 x 2.  Either way
 // 16 warps per SM hide the fixed latencies of the LDS -> LOP -> MMA -> FMA chain.
-template <int NT, int WARPS, int STAGES, bool M1>
+template <int NT, int WARPS, int STAGES, bool M1, bool OWN>
 __global__ void __launch_bounds__(WARPS * 32, (WARPS == 8 ? 2 : 1))
     gemv_q4_mma_kernel(const __grid_constant__ CUtensorMap tmW,
                        const __grid_constant__ CUtensorMap tmS, GemvParams p) {
@@ -124,9 +127,18 @@ __global__ void __launch_bounds__(WARPS * 32, (WARPS == 8 ? 2 : 1))
   const unsigned wid = blockIdx.x * WARPS + warp;
   const bool idle = wid >= Wtot;
   const GvSplit sp = {p.U / Wtot, p.U % Wtot};
-  const unsigned u0 = idle ? 0u : gv_start(wid, sp);
+  unsigned u0 = idle ? 0u : gv_start(wid, sp);
   const unsigned u1 = idle ? 0u : gv_start(wid + 1, sp);
-  const int n_units = (int)(u1 - u0);
+  int n_units = (int)(u1 - u0);
+  // Small matrices: the block owns whole row tiles [tile_b, tile_b + tiles), its units go round the warps and meet in
+  // shared memory -- no partials in global memory, no ticket, no last arriver.
+  float* ures = (float*)(base + L.ures);     // [unit][m][16]
+  const int tile_b = OWN ? (int)(((long long)p.RT * blockIdx.x) / gridDim.x) : 0;
+  const int tiles = OWN ? (int)(((long long)p.RT * (blockIdx.x + 1)) / gridDim.x) - tile_b : 0;
+  if (OWN) {
+    u0 = (unsigned)(tile_b * SL + warp);
+    n_units = warp < tiles * SL ? (tiles * SL - warp + WARPS - 1) / WARPS : 0;
+  }
 
   if (lane == 0) {
     for (int s = 0; s < STAGES; s++) mbar_init(&mybar[s], 1);
@@ -142,7 +154,10 @@ __global__ void __launch_bounds__(WARPS * 32, (WARPS == 8 ? 2 : 1))
       tma_load_2d(myW + istage * GV_W_BYTES, &tmW, is * 32, irt * 16, &mybar[istage]);
       tma_load_2d(myS + istage * GV_S_BYTES, &tmS, is * 8, irt * 16, &mybar[istage]);
     }
-    if (++is == SL) { is = 0; irt++; }
+    if (OWN) {
+      is += WARPS;
+      while (is >= SL) { is -= SL; irt++; }
+    } else if (++is == SL) { is = 0; irt++; }
     if (++istage == STAGES) istage = 0;
   };
   // Weights do not depend on the previous kernel: the first stage streams before the
@@ -387,8 +402,9 @@ __global__ void __launch_bounds__(WARPS * 32, (WARPS == 8 ? 2 : 1))
   int rt = (int)(u0 / (unsigned)SL), s = (int)(u0 - (unsigned)rt * SL);
   int st = 0;
   unsigned phase = 0;
+  bool dead = false;
   for (int i = 0; i < n_units; i++) {
-    if (!mbar_wait_bounded(&mybar[st], phase, p.status, 100 + st)) return;
+    if (!mbar_wait_bounded(&mybar[st], phase, p.status, 100 + st)) { dead = true; break; }
     if (i == 0) stamp(3);
     const unsigned* Wst = (const unsigned*)(myW + st * GV_W_BYTES);
     const float* Sst = (const float*)(myS + st * GV_S_BYTES);
@@ -445,6 +461,26 @@ __global__ void __launch_bounds__(WARPS * 32, (WARPS == 8 ? 2 : 1))
     __syncwarp();
     if (i + STAGES < n_units) issue_next();
     if (++st == STAGES) { st = 0; phase ^= 1u; }
+    if (OWN) {
+      float* dst = ures + (size_t)(warp + i * WARPS) * p.M * 16;
+#pragma unroll
+      for (int nt = 0; nt < NT; nt++) {
+        const int m = 4 * nt + t;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          float cr = corr[nt][r];
+          if (M1) {
+            cr += __shfl_xor_sync(0xffffffffu, cr, 1);
+            cr += __shfl_xor_sync(0xffffffffu, cr, 2);
+          }
+          if (m < p.M) dst[m * 16 + g + 8 * r] = acc[nt][r] - cr;
+        }
+        acc[nt][0] = acc[nt][1] = corr[nt][0] = corr[nt][1] = 0.f;
+      }
+      s += WARPS;
+      while (s >= SL) { s -= SL; rt++; }
+      continue;
+    }
     if (++s == SL) {
       flush(rt);
 #pragma unroll
@@ -454,7 +490,16 @@ __global__ void __launch_bounds__(WARPS * 32, (WARPS == 8 ? 2 : 1))
     }
   }
   stamp(4);
-  if (n_units > 0 && s != 0) flush(rt);
+  if (OWN) {
+    __syncthreads();
+    // a thread per output, the tile's units in the order of k
+    for (int i = tid; i < tiles * p.M * 16; i += WARPS * 32) {
+      const int tl = i / (p.M * 16), rest = i - tl * (p.M * 16), n = (tile_b + tl) * 16 + (rest & 15);
+      float v = 0.f;
+      for (int k = 0; k < SL; k++) v += ures[(size_t)(tl * SL + k) * p.M * 16 + rest];
+      if (n < p.N) emit(rest >> 4, n, v);
+    }
+  } else if (!dead && n_units > 0 && s != 0) flush(rt);
   stamp(5);
 
 }
@@ -526,7 +571,7 @@ static void gemv_pick(int M, int K, int* warps, int* stages) {
   }
   const size_t small = gemv_smem_layout(8, 4, M, K).total;
   if (small <= 113 * 1024) { *warps = 8; *stages = 4; }
-  else { *warps = 16; *stages = 3; }
+  else { *warps = 16; *stages = M > 4 && gemv_smem_layout(16, 3, M, K).total > 227 * 1024 ? 2 : 3; }
 }
 
 bool gemv_q4_tma_eligible(const void* qw, const void* scales, int N, int K, int M) {
@@ -538,17 +583,24 @@ bool gemv_q4_tma_eligible(const void* qw, const void* scales, int N, int K, int 
   return N > 0;
 }
 
-template <int NT, int WARPS, int STAGES, bool M1>
-static int gemv_launch_t(const CUtensorMap& tmW, const CUtensorMap& tmS, const GemvParams& p,
+template <int NT, int WARPS, int STAGES, bool M1, bool OWN>
+static int gemv_launch_o(const CUtensorMap& tmW, const CUtensorMap& tmS, const GemvParams& p,
                          int ctas, size_t smem, cudaStream_t stream) {
   static std::atomic<unsigned long long> attr_done{0};
   {
-    const int rc_attr = ensure_dynamic_smem(gemv_q4_mma_kernel<NT, WARPS, STAGES, M1>, 227 * 1024, attr_done);
+    const int rc_attr = ensure_dynamic_smem(gemv_q4_mma_kernel<NT, WARPS, STAGES, M1, OWN>, 227 * 1024, attr_done);
     if (rc_attr) return rc_attr;
   }
   LaunchCfg lc(dim3(ctas), dim3(WARPS * 32), smem, stream, pdl_enabled());
-  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, gemv_q4_mma_kernel<NT, WARPS, STAGES, M1>, tmW, tmS, p));
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, gemv_q4_mma_kernel<NT, WARPS, STAGES, M1, OWN>, tmW, tmS, p));
   return TLB_OK;
+}
+
+template <int NT, int WARPS, int STAGES, bool M1>
+static int gemv_launch_t(const CUtensorMap& tmW, const CUtensorMap& tmS, const GemvParams& p,
+                         int ctas, size_t smem, cudaStream_t stream) {
+  if (p.own) return gemv_launch_o<NT, WARPS, STAGES, M1, true>(tmW, tmS, p, ctas, smem, stream);
+  return gemv_launch_o<NT, WARPS, STAGES, M1, false>(tmW, tmS, p, ctas, smem, stream);
 }
 
 // Diagnostics: when set, every launch records per-CTA phase timestamps there.
@@ -586,7 +638,19 @@ int gemv_q4_launch(DeviceCtx* c, const CUtensorMap& tmW, const CUtensorMap& tmS,
   const int need = (int)((p.U + warps - 1) / warps);
   if (ctas > need) ctas = need;
   if (ctas * warps > c->gemv_max_workers) ctas = c->gemv_max_workers / warps;
-  const size_t smem = gemv_smem_layout(warps, stages, M, K).total;
+  // Block-owned row tiles where that leaves a warp at most two units and a tile has several to add: the partials and the
+  // ticket in global memory cost about a microsecond (in a graph, 1 x 896 x 4864: 5.66 -> 4.67 us, 1 x 896 x 896: 4.79 ->
+  // 3.69, 1 x 3584 x 4608: 8.36 -> 6.84, 8 x 896 x 4864: 8.20 -> 6.69; a tile of one unit, 1 x 128 x 16, would lose:
+  // 3.04 -> 3.78, there is nothing to add).
+  p.own = 0;
+  if (max_ctas <= 0 && !p.push && p.SL > 1) {
+    const int slots = c->sm_count * (warps == 8 ? 2 : 1), most = (p.RT + slots - 1) / slots;
+    if (most * p.SL <= 2 * warps && gemv_smem_layout(warps, stages, M, K, most).total <= (warps == 8 ? 113 : 227) * 1024) {
+      p.own = most;
+      ctas = (p.RT + most - 1) / most;
+    }
+  }
+  const size_t smem = gemv_smem_layout(warps, stages, M, K, p.own).total;
   if (warps == 8) {
     if (M == 1) return gemv_launch_t<1, 8, 4, true>(tmW, tmS, p, ctas, smem, stream);
     if (M <= 4) return gemv_launch_t<1, 8, 4, false>(tmW, tmS, p, ctas, smem, stream);
@@ -595,6 +659,7 @@ int gemv_q4_launch(DeviceCtx* c, const CUtensorMap& tmW, const CUtensorMap& tmS,
   if (M == 1 && stages == 4) return gemv_launch_t<1, 16, 4, true>(tmW, tmS, p, ctas, smem, stream);
   if (M == 1) return gemv_launch_t<1, 16, 3, true>(tmW, tmS, p, ctas, smem, stream);
   if (M <= 4) return gemv_launch_t<1, 16, 3, false>(tmW, tmS, p, ctas, smem, stream);
+  if (stages == 2) return gemv_launch_t<2, 16, 2, false>(tmW, tmS, p, ctas, smem, stream);
   return gemv_launch_t<2, 16, 3, false>(tmW, tmS, p, ctas, smem, stream);
 }
 
