@@ -350,47 +350,8 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
   float* ures = (float*)(base + L.ures);
 
   auto top_up = [&](int limit) { gv_top_up<STAGES>(ring, cur, table, nph, myR, mybar, lane, limit); };
-  // Weights do not depend on the previous kernel: the first stage streams before the
-  // wait.  The other stages are issued right after the activation loads below, so
-  // those small loads are not queued behind the weight traffic.  (Later phases of a chain
-  // find their ring filled by the phase before.)
-  if (phi == 0) {
-    top_up(1);
-    // While the kernel in front still runs: touch what the prep will read, so that the
-    // address translations (and for the norm weights, which nobody writes, the data) are
-    // there when the wait returns.  A prefetch of a line the previous kernel is still
-    // writing is harmless: the L2 is where its stores land.
-    {
-      const int k0 = (s_b + warp) * 256 + lane * 8;
-      if (warp < ks && k0 < p.K) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.x + k0));
-        if (p.act == 1) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.x + p.K + k0));
-        if (p.act == 2) {
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(p.delta + k0));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(p.nw + k0));
-        }
-      }
-    }
-    if (EPI == 2 && own && warp == 0 && ks > 0 && lane < n_loc / ks) {
-      // ... and what the epilogue of this CTA's row tiles will read: the biases of the tile's
-      // eight pairs (two runs of 32 bytes), the rotary table entries
-      const int half = p.epi.D >> 1;
-      const int pi = (tile_b + lane) * 8;
-      const int h = pi / half, j = pi - h * half;
-      const float* bias = h < p.epi.n_q ? p.epi.bq : (h < p.epi.n_q + p.epi.n_kv ? p.epi.bk : p.epi.bv);
-      const int hh = h < p.epi.n_q ? h : (h < p.epi.n_q + p.epi.n_kv ? h - p.epi.n_q : h - p.epi.n_q - p.epi.n_kv);
-      if (bias) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(bias + hh * p.epi.D + j));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(bias + hh * p.epi.D + j + half));
-      }
-      if (p.epi.rope_cs) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.epi.rope_cs + j));
-    }
-    pdl_wait();  // activations and the fix-up scratch are valid from here
-  }
-
   // ---- activation prep.  One warp per slab of 256 k, four slabs in flight per warp.
   // Lane l covers x[256*slab + 8*l .. +8) = group jj = l/4, quad slot tt = l%4.
-  float nrm_inv = 1.f;
   const bool normed = p.act == 2 || (PULL && p.act == 3);
   unsigned pull_seq = 0;
   if (PULL && p.act == 3) pull_seq = comm_seq(p.comm);
@@ -431,86 +392,103 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
   // its LENGTH (measured: 3 us of a 5 us projection with two unrolled slab batches per warp),
   // so there is one copy of the load and one of the conversion, in loops that are not unrolled.
   float xv[8], xu[8], xw[8];   // the slab's activation, its second operand (up / delta), its norm weights
-  auto load_slab = [&](int sl, bool with_w) {
+  auto load_slab = [&](int sl) {
     const int k0 = (s_b + sl) * 256 + lane * 8;
     const bool on = sl < ks && k0 < p.K;   // K % 32 == 0: a lane's 8 values are all in or all out
-    auto load8 = [&](const float* s8, float (&o)[8]) {
-      if (on) {
-        if (p.x_vec_ok) {
-          // .cg in a chain: the vector was written by other SMs earlier in this launch.  A
-          // launch of its own reads through the L1 (measured 1 % of a decode step faster).
-          float4 q0, q1;
-          if (nph > 1) {
-            q0 = __ldcg((const float4*)s8);
-            q1 = __ldcg((const float4*)(s8 + 4));
-          } else {
-            q0 = *(const float4*)s8;
-            q1 = *(const float4*)(s8 + 4);
-          }
-          o[0] = q0.x; o[1] = q0.y; o[2] = q0.z; o[3] = q0.w;
-          o[4] = q1.x; o[5] = q1.y; o[6] = q1.z; o[7] = q1.w;
-        } else {
+    auto load8 = [&](const float* base, float (&o)[8]) {
 #pragma unroll
-          for (int i = 0; i < 8; i++) o[i] = nph > 1 ? __ldcg(s8 + i) : s8[i];
+      for (int i = 0; i < 8; i++) o[i] = 0.f;
+      if (!on) return;   // (no load at all: every SM reads these few lines at the same time)
+      if (p.x_vec_ok) {
+        // .cg in a chain: the vector was written by other SMs earlier in this launch.  A
+        // launch of its own reads through the L1 (measured 1 % of a decode step faster).
+        const float4* at = (const float4*)(base + k0);
+        float4 q0, q1;
+        if (nph > 1) {
+          q0 = __ldcg(at);
+          q1 = __ldcg(at + 1);
+        } else {
+          q0 = at[0];
+          q1 = at[1];
         }
+        o[0] = q0.x; o[1] = q0.y; o[2] = q0.z; o[3] = q0.w;
+        o[4] = q1.x; o[5] = q1.y; o[6] = q1.z; o[7] = q1.w;
       } else {
 #pragma unroll
-        for (int i = 0; i < 8; i++) o[i] = 0.f;
+        for (int i = 0; i < 8; i++) o[i] = nph > 1 ? __ldcg(base + k0 + i) : base[k0 + i];
       }
     };
-    load8(p.x + k0, xv);
-    if (p.act == 1) load8(p.x + p.K + k0, xu);
-    if (p.act == 2) load8(p.delta + k0, xu);
-    // the norm weights travel with the activation: no load left behind the block barrier
-    if (normed && with_w) load8(p.nw + k0, xw);
+    load8(p.x, xv);
+    if (p.act == 1) load8(p.x + p.K, xu);
+    if (p.act == 2) load8(p.delta, xu);
     if constexpr (PULL) {
       if (p.act == 3) pull8(k0, xu, on);
     }
   };
-  load_slab(warp, true);
+  auto load_w = [&](int sl) {
+    const int k0 = (s_b + sl) * 256 + lane * 8;
+    const bool on = sl < ks && k0 < p.K;
+#pragma unroll
+    for (int i = 0; i < 8; i++) xw[i] = 0.f;
+    if (!on) return;
+    if (p.x_vec_ok) {
+      const float4* at = (const float4*)(p.nw + k0);
+      const float4 q0 = __ldg(at), q1 = __ldg(at + 1);
+      xw[0] = q0.x; xw[1] = q0.y; xw[2] = q0.z; xw[3] = q0.w;
+      xw[4] = q1.x; xw[5] = q1.y; xw[6] = q1.z; xw[7] = q1.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; i++) xw[i] = p.nw[k0 + i];
+    }
+  };
+  // Weights do not depend on the previous kernel: the first stage streams before the
+  // wait.  The other stages are issued right after the activation loads below, so
+  // those small loads are not queued behind the weight traffic.  (Later phases of a chain
+  // find their ring filled by the phase before.)
+  if (phi == 0) {
+    // (a short range of its own altogether: it has landed when the activations are asked for)
+    top_up(n_units <= 2 ? 2 : 1);
+    // the first slab's norm weights, which nobody writes
+    if (normed) load_w(warp);
+    pdl_wait();  // activations and the fix-up scratch are valid from here
+  } else if (normed) {
+    load_w(warp);
+  }
+  load_slab(warp);
+  // what the rotary epilogue of this thread's pair needs beside the sums, in flight with the activations
+  float ep_ba = 0.f, ep_bb = 0.f;
+  float2 ep_cs = make_float2(1.f, 0.f);
+  unsigned ep_pos = 0;
+  const bool ep_here = EPI == 2 && own && p.epi.rope_cs && (p.epi.D & (p.epi.D - 1)) == 0;
+  if (ep_here && ks > 0 && tid < n_loc / ks * 8) {
+    const int pi = tile_b * 8 + tid, half = p.epi.D >> 1;
+    const int h = pi >> (31 - __clz(half)), j = pi - h * half;
+    const float* bias = h < p.epi.n_q ? p.epi.bq : (h < p.epi.n_q + p.epi.n_kv ? p.epi.bk : p.epi.bv);
+    const int hh = h < p.epi.n_q ? h : (h < p.epi.n_q + p.epi.n_kv ? h - p.epi.n_q : h - p.epi.n_q - p.epi.n_kv);
+    ep_pos = __ldcg(p.epi.d_pos);
+    ep_cs = __ldcg(p.epi.rope_cs + j);
+    if (bias) {
+      ep_ba = __ldg(bias + hh * p.epi.D + j);
+      ep_bb = __ldg(bias + hh * p.epi.D + j + half);
+    }
+  }
+
   // The rest of the weight ring is queued only when this warp's activation values have
   // ARRIVED (first use below): a small load issued behind 160 KB of bulk copies per SM waits
   // until they have drained -- measured, the prep of a projection took 2 - 4 us that way, the
   // time the ring fill needs from HBM.  (An L2 prefetch of the units behind the ring was tried
   // too and lost 4 us on the 85 MB gate|up matrix for the same reason.)
-  if (normed) {
-    // fused residual add + RMSNorm (tl_add_rmsnorm, kernels/tensorlib_cuda.cu:155-179):
-    // every CTA reduces sum((x+delta)^2) itself, slabs in the same order everywhere, so all
-    // CTAs agree on the scale
-    float sq = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const float sv = xv[i] + xu[i];
-      sq = fmaf(sv, sv, sq);
-    }
-    if (ks > PK_WARPS) {
-      // rows longer than 16 slabs: this warp's further slabs, read once more below
-      float kv[8], ku[8], kw[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) { kv[i] = xv[i]; ku[i] = xu[i]; kw[i] = xw[i]; }
-#pragma unroll 1
-      for (int sl = warp + PK_WARPS; sl < ks; sl += PK_WARPS) {
-        load_slab(sl, false);
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const float sv = xv[i] + xu[i];
-          sq = fmaf(sv, sv, sq);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 8; i++) { xv[i] = kv[i]; xu[i] = ku[i]; xw[i] = kw[i]; }
-    }
-    sq = warp_sum(sq);
-    top_up(STAGES);
-    // The scale 1 / rms is a scalar factor of every activation, so it need not be known before
-    // the digits are made: the digits are those of (x + delta) * w, and the factor multiplies
-    // the outputs (with alpha, below).  That takes a block barrier and the serial sum out of
-    // the prep; the warp sums meet at the barrier that ends it.
-    if (lane == 0) red[warp] = sq;
-  }
+  // Fused residual add + RMSNorm (tl_add_rmsnorm, kernels/tensorlib_cuda.cu:155-179): every CTA reduces sum((x+delta)^2)
+  // itself, slabs in the same order everywhere, so all CTAs agree on the scale.  The scale 1 / rms is a scalar factor of
+  // every activation, so it need not be known before the digits are made: the digits are those of (x + delta) * w, and
+  // the factor multiplies the outputs (with alpha, below).  The warp sums meet at the barrier that ends the prep.
+  float sq = 0.f;
 #pragma unroll 1
   for (int sl = warp; sl < ks; sl += PK_WARPS) {
-    if (sl != warp) load_slab(sl, true);
+    if (sl != warp) {
+      load_slab(sl);
+      if (normed) load_w(sl);
+    }
     float v[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = xv[i];
@@ -524,11 +502,15 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
       const int k0 = sl * 256 + lane * 8;   // (the fused norm is never combined with slab blocks)
 #pragma unroll
       for (int i = 0; i < 8; i++) {
-        const float sv = v[i] + xu[i];
-        const bool in = k0 + i < p.K;
-        if (in && blockIdx.x == 0) p.xout[k0 + i] = sv;
-        v[i] = in ? sv * xw[i] : 0.f;
+        v[i] += xu[i];                      // zero behind K
+        sq = fmaf(v[i], v[i], sq);
       }
+      if (blockIdx.x == 0 && k0 < p.K) {    // K % 32 == 0: a lane's 8 values are all in or all out
+#pragma unroll
+        for (int i = 0; i < 8; i++) p.xout[k0 + i] = v[i];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; i++) v[i] *= xw[i];
     }
     float mx = 0.f;
 #pragma unroll
@@ -581,17 +563,13 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
     if (lane == 0)
       Pslab[sl] = (mx < 3.0e38f) ? __uint_as_float((unsigned)(127 + 13 + e) << 23) : __uint_as_float(0x7fc00000u);
   }
+  if (warp >= ks) top_up(STAGES);
+  if (normed) {
+    sq = warp_sum(sq);
+    if (lane == 0) red[warp] = sq;
+  }
   __syncthreads();
   if (phi == 0) pdl_launch_dependents();
-  if (normed) {
-    // sum of the warp sums in warp order: every warp of every CTA computes the same bits
-    float tot = 0.f;
-#pragma unroll
-    for (int w = 0; w < PK_WARPS; w++) tot += red[w];
-    nrm_inv = 1.0f / sqrtf(tot / (float)p.K + p.eps);
-  }
-  const float alpha_n = p.alpha * nrm_inv;
-
   // ---- streaming loop ------------------------------------------------------
   float acc0 = 0.f, acc1 = 0.f, corr0 = 0.f, corr1 = 0.f;
   uint4 bq[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
@@ -606,7 +584,19 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
   if (PUSH) ar_seq = comm_seq(p.comm);
   const size_t ar_off =
       ((size_t)(ar_seq & 1u) * p.comm.size + p.comm.rank) * (size_t)p.comm.slot_floats;
-  auto emit = [&](int n, float v) {
+  // 1 / rms, from the warp sums in warp order: every warp of every CTA computes the same bits.  Worked out where a sum
+  // is complete, not in front of the stream.
+  auto scale_of = [&]() {
+    if (!normed) return p.alpha;
+    float tot = 0.f;
+#pragma unroll
+    for (int w = 0; w < PK_WARPS; w += 4) {
+      const float4 q = *(const float4*)(red + w);
+      tot += q.x; tot += q.y; tot += q.z; tot += q.w;
+    }
+    return p.alpha * (1.0f / sqrtf(tot / (float)p.K + p.eps));
+  };
+  auto emit = [&](int n, float v, float alpha_n) {
     v = v * alpha_n + p.beta;
     if (PUSH) {
       for (int r = 0; r < p.comm.size; r++) st_packet_sys(&p.comm.stage[r][ar_off + n], v, ar_seq + 1u);
@@ -615,7 +605,7 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
     }
   };
   // pair index pi of a pair-packed matrix, a = its first row's sum, b = its second's
-  auto emit_pair = [&](int pi, float a, float b) {
+  auto emit_pair = [&](int pi, float a, float b, float alpha_n, bool here) {
     a = a * alpha_n + p.beta;
     b = b * alpha_n + p.beta;
     if (EPI == 1) {
@@ -630,7 +620,7 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
     // (head sizes are powers of two in practice: a shift instead of two dozen instructions)
     const int h = (half & (half - 1)) == 0 ? pi >> (31 - __clz(half)) : pi / half;
     const int j = pi - h * half;
-    const unsigned pos = *p.epi.d_pos;
+    const unsigned pos = here ? ep_pos : *p.epi.d_pos;
     if (pos >= (unsigned)p.epi.kv_rows) {
       // the cache is full: write nothing (the attention that follows refuses the position
       // too) and tell the host through the status block
@@ -639,7 +629,8 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
     }
     if (h >= p.epi.n_q + p.epi.n_kv) {
       const int kh = h - p.epi.n_q - p.epi.n_kv;
-      if (p.epi.bv) { a += p.epi.bv[kh * D + j]; b += p.epi.bv[kh * D + j + half]; }
+      if (here) { a += ep_ba; b += ep_bb; }
+      else if (p.epi.bv) { a += p.epi.bv[kh * D + j]; b += p.epi.bv[kh * D + j + half]; }
       const size_t row = (size_t)kh * p.epi.kv_stride + (size_t)pos * D;
       if (p.epi.kv_bf16) {
         __nv_bfloat16* dst = (__nv_bfloat16*)p.epi.Vc + row;
@@ -653,7 +644,10 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
       return;
     }
     float c, sn;
-    if (p.epi.rope_cs) {
+    if (here) {
+      c = ep_cs.x;
+      sn = ep_cs.y;
+    } else if (p.epi.rope_cs) {
       // (cos, sin) of this position, computed once per token by the same expression
       const float2 cs = p.epi.rope_cs[j];
       c = cs.x;
@@ -666,13 +660,15 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
       sn = (float)sd;
     }
     if (h < p.epi.n_q) {
-      if (p.epi.bq) { a += p.epi.bq[h * D + j]; b += p.epi.bq[h * D + j + half]; }
+      if (here) { a += ep_ba; b += ep_bb; }
+      else if (p.epi.bq) { a += p.epi.bq[h * D + j]; b += p.epi.bq[h * D + j + half]; }
       float* dst = p.epi.out + (size_t)h * D;
       dst[j] = a * c - b * sn;
       dst[j + half] = a * sn + b * c;
     } else {
       const int kh = h - p.epi.n_q;
-      if (p.epi.bk) { a += p.epi.bk[kh * D + j]; b += p.epi.bk[kh * D + j + half]; }
+      if (here) { a += ep_ba; b += ep_bb; }
+      else if (p.epi.bk) { a += p.epi.bk[kh * D + j]; b += p.epi.bk[kh * D + j + half]; }
       const size_t row = (size_t)kh * p.epi.kv_stride + (size_t)pos * D;
       if (p.epi.kv_bf16) {
         __nv_bfloat16* dst = (__nv_bfloat16*)p.epi.Kc + row;
@@ -695,13 +691,14 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
     const unsigned t0 = (unsigned)rt * SL, t1 = t0 + SL;
     const bool complete = (u0 <= t0) && (u1 >= t1);
     const int r0 = rt * 16;
+    const float alpha_n = scale_of();
     if (complete) {
       if (t == 0) {
         if (EPI) {
-          emit_pair(rt * 8 + g, v0, v1);
+          emit_pair(rt * 8 + g, v0, v1, alpha_n, false);
         } else {
-          if (r0 + g < p.N) emit(r0 + g, v0);
-          if (r0 + g + 8 < p.N) emit(r0 + g + 8, v1);
+          if (r0 + g < p.N) emit(r0 + g, v0, alpha_n);
+          if (r0 + g + 8 < p.N) emit(r0 + g + 8, v1, alpha_n);
         }
       }
       return;
@@ -736,11 +733,11 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
 #pragma unroll
         for (int k = 0; k < 16; k++) s += pv[k];
       }
-      if (!EPI && r0 + lane < p.N) emit(r0 + lane, s);
+      if (!EPI && r0 + lane < p.N) emit(r0 + lane, s, alpha_n);
     }
     if (EPI) {
       const float s2 = __shfl_down_sync(0xffffffffu, s, 8);   // row lane + 8 of the tile
-      if (lane < 8) emit_pair(rt * 8 + lane, s, s2);
+      if (lane < 8) emit_pair(rt * 8 + lane, s, s2, alpha_n, false);
     }
     if (lane == 0) p.counters[rt] = 0;  // leave the counter clean for the next launch
   };
@@ -828,6 +825,7 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
   if (own) {
     __syncthreads();
     const int ntl = n_loc / ks;   // row tiles of this block
+    const float alpha_n = scale_of();
     // one thread per output row: fold the row's unit results in slab order
     if (EPI) {
       // one thread per pair: rows (lr, lr + 8) of a tile (whole rows only: KB == 1)
@@ -835,8 +833,18 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
         const int tl = idx >> 3, lr = idx & 7;
         const float* srcp = ures + (size_t)tl * ks * 16 + lr;
         float sa = 0.f, sb = 0.f;
-        for (int k = 0; k < ks; k++) { sa += srcp[k * 16]; sb += srcp[k * 16 + 8]; }
-        emit_pair((tile_b + tl) * 8 + lr, sa, sb);
+        for (int k0 = 0; k0 < ks; k0 += 4) {   // four loads in flight, added in slab order
+          float qa[4], qb[4];
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            const bool on = k0 + k < ks;
+            qa[k] = on ? srcp[(k0 + k) * 16] : 0.f;
+            qb[k] = on ? srcp[(k0 + k) * 16 + 8] : 0.f;
+          }
+#pragma unroll
+          for (int k = 0; k < 4; k++) { sa += qa[k]; sb += qb[k]; }
+        }
+        emit_pair((tile_b + tl) * 8 + lr, sa, sb, alpha_n, ep_here && idx == tid);
       }
       return;
     }
@@ -845,10 +853,16 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
       const int tl = idx >> 4, row = idx & 15;
       const float* srcp = ures + (size_t)tl * ks * 16 + row;
       float sum = 0.f;
-      for (int k = 0; k < ks; k++) sum += srcp[k * 16];
+      for (int k0 = 0; k0 < ks; k0 += 8) {
+        float q[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) q[k] = k0 + k < ks ? srcp[(k0 + k) * 16] : 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; k++) sum += q[k];
+      }
       const int n = (tile_b + tl) * 16 + row;
       if (KB == 1) {
-        if (n < p.N) emit(n, sum);
+        if (n < p.N) emit(n, sum, alpha_n);
       } else {
         __stcg(p.partials + ((size_t)kb * p.RT + tile_b + tl) * 16 + row, sum);
       }
@@ -874,7 +888,7 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
 #pragma unroll
         for (int k = 0; k < 8; k++) sum += pv[k];
       }
-      if ((int)off < p.N) emit((int)off, sum);
+      if ((int)off < p.N) emit((int)off, sum, alpha_n);
     }
     if (tid == 0) p.counters[rb] = 0;  // clean for the next launch
     return;
