@@ -21,27 +21,27 @@
 // conversions pass under the stores of the one before, and a product with few tiles still uses the
 // whole chip.  A tile whose units lie in several CTAs' ranges is summed by the last of them to finish, in
 // the order of k, from f32 partials in scratch (T2Work): the same bits on every call, and no CTA waits for
-// another.  Warp roles (512 threads): warp 0 TMA producer of the X planes (64-k
-// stages, 128-byte swizzle), warp 1 TMEM allocator, warps 1 and 15 the MMA issuers (first / second group of a stage), warps 2-5
-// nibble -> fp16 converters (thread r owns weight row r; the k order inside every group of 8
-// is the one the nibble extraction produces -- 0,4,1,5,2,6,3,7 -- and the X planes are stored
-// in the same order, so no byte permute is needed), warps 6-13 accumulate + epilogue (two per
-// TMEM lane quarter, each half of the MT columns), warp 14 TMA producer of the PACKED weights:
-// 128 rows x 128 bytes (256 k) per box into a ring of four, 64 KB in flight per SM.  (Register
-// loads by the converters, 32 bytes per row and stage with four stages in flight, kept only
-// 16 KB per SM in flight and paced the whole kernel at ~1 TB/s of weight bytes.)  All waits
-// are bounded; a timeout sets the status word, the kernel still frees its TMEM and returns, and no warp is split by it.
-// No cluster launch, no multicast.
+// another.  Warp roles (512 threads): warp 0 TMA producer of the X planes (64-k stages, 128-byte swizzle), warp 1 TMEM
+// allocator, warps 1 and 2 the MMA issuers (first / second group of a stage), warp 3 TMA producer of the PACKED weights
+// (128 rows x 128 bytes = 256 k a box, a ring of four: 64 KB in flight an SM), warps 4-7 nibble -> fp16 converters (thread r
+// owns weight row r; the k order inside every group of 8 is the one the nibble extraction produces -- 0,4,1,5,2,6,3,7 -- and
+// the X planes are stored in the same order, so no byte permute is needed), warps 8-15 accumulate + epilogue (two per TMEM
+// lane quarter, each half of the MT columns).  The converters leave the weights in TMEM, a lane a row: the A operand of the
+// MMAs comes from there.  The feeding warpgroups give registers to the accumulating ones.  All waits are bounded; a timeout
+// sets the status word, the kernel still frees its TMEM and returns, and no warp is split by it.  No cluster launch, no
+// multicast.
 //
-// What bounds it is the instruction issue of the four schedulers, not the tensor pipe: without any MMA a product takes
-// nine tenths of the time, with half of them as long.  So the accumulate warps' loop is unrolled over a block of four
-// scales, one accumulator each, with nothing left to select at run time.  Measured and dropped: weights in TMEM as
-// the A operand, sixteen accumulate warps, one issuer, one commit a stage, spinning waits, register shares by
-// setmaxnreg with 64-column reads, leaving out the reads of columns behind the last row (the branch keeps the compiler from
-// running one group's reads under another's FMAs: 570 -> 670 us).  1000 x 3584 x 37888: 676 -> 575 us; 1000 x 18944 x 3584, one and a half
-// rounds of tiles: 424 -> 322; 517 x 4864 x 896, 35 tiles: 60 -> 34.  At 128 columns a thread has 128 registers and spills 48
-// bytes.  The votes of the accumulate warps' waits matter: behind the first poll 573 us, behind the whole wait 588, an outcome
-// carried along instead of a branch 603 to 647.
+// What bounds it: at large sizes the power limit (1620 MHz of 1965 at 1000 x 3584 x 37888), and at all sizes the way of an
+// accumulator from its MMAs to the accumulate warps and back.  Per group of 32 k and 128 columns the tensor pipe works 256
+// cycles; an issuer takes about 600 (61 an MMA to issue, 130 the look at its barriers, 70 the commits), so there are two; an
+// accumulate warp 90 to read 64 columns and about 270 for the FMAs that it shares a scheduler with.  What was done about it,
+// 1000 x 3584 x 37888 / 517 x 896 x 9728 in one loop of products, us: 656 / 38.4 before; all of a warp's columns in one read
+// into registers that setmaxnreg gives it, the accumulator back before the FMAs; one barrier for a stage's two operands and
+// one vote an issuer's group; the look at the next group's barrier under the FMAs; weights in TMEM, which takes 32 of 120 KB
+// a stage off the shared memory; the odd nibbles of a byte converted in place by one FMA: 611 / 34.9.  Measured beside it: two
+// sets of accumulate warps that take the groups in turn (588 against 579 of that time), four stages of operands (no change),
+// one issuer (551 against 517) or three (615 against 611), the next read under a group's FMAs (634), pairs of columns by
+// fma.rn.f32x2 at 128 columns (632), sixteen accumulate warps, leaving out the reads of columns behind the last row.
 #include <cstdlib>
 
 #include "q4_planes.cuh"
@@ -53,9 +53,11 @@ namespace {
 constexpr int T2_THREADS = 512;
 constexpr int T2_ROWS = 128;     // weight rows per CTA (UMMA M)
 constexpr int T2_KS = 64;        // k per stage = two groups = one 128-byte swizzle row of fp16
-constexpr int T2_RAW_STAGES = 4;              // ring of packed-weight boxes
 constexpr int T2_RAW_BYTES = T2_ROWS * 128;   // one box: 128 rows x 128 bytes = 256 k per row
 constexpr int T2_SUB = 4;                     // 64-k stages per packed box
+// registers a thread of the two warpgroups that feed the tensor pipe, and of the two that accumulate: 256 (72 + 184) =
+// what 512 threads of 128 are launched with
+constexpr int T2_REGS_FEED = 72, T2_REGS_ACC = 184;
 
 struct T2Params {
   const unsigned* qw;        // packed nibbles, u32 [N][K/8]
@@ -98,11 +100,10 @@ struct T2Segment {
 
 template <int MT>
 struct T2Smem {
-  static constexpr int STAGES = MT == 128 ? 3 : 4;                            // what fits beside the weight ring
-  static constexpr size_t A = 0;                                              // [stages][128][128 B]
-  static constexpr size_t B = A + (size_t)STAGES * T2_ROWS * 128;             // [stages][2 planes][MT][128 B]
+  static constexpr int STAGES = 4, RAW_STAGES = 4;                            // rings of operands, of weight boxes
+  static constexpr size_t B = 0;                                              // [stages][2 planes][MT][128 B]
   static constexpr size_t RAW = B + (size_t)STAGES * 2 * MT * 128;            // [raw stages][128][128 B]
-  static constexpr size_t BARS = RAW + (size_t)T2_RAW_STAGES * T2_RAW_BYTES;
+  static constexpr size_t BARS = RAW + (size_t)RAW_STAGES * T2_RAW_BYTES;
   static constexpr size_t SLOT = BARS + 32 * 8;
   static constexpr size_t TOTAL = SLOT + 16 + 1024;
 };
@@ -124,12 +125,13 @@ __device__ __forceinline__ void t2_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ void t2_mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+// A from TMEM (a lane a row, two k a column), B from shared memory
+__device__ __forceinline__ void t2_mma_f16(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
                                            uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // 32 lanes x 16 consecutive columns of this warp's TMEM lane quarter (issue only; see t2_wait_ld)
@@ -140,6 +142,22 @@ __device__ __forceinline__ void t2_ld16_issue(uint32_t taddr, uint32_t (&r)[16])
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
+}
+// 32 lanes x 32 consecutive columns of this warp's TMEM lane quarter, written and there when it returns
+__device__ __forceinline__ void t2_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,"
+      "%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+      "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+      "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// two f32 FMAs an instruction: c + (s, s) * (a, b)
+__device__ __forceinline__ void t2_fma2(unsigned long long& c, unsigned long long s2, uint32_t a, uint32_t b) {
+  asm("{\n\t.reg .b64 v;\n\tmov.b64 v, {%2, %3};\n\tfma.rn.f32x2 %0, %1, v, %0;\n\t}" : "+l"(c) : "l"(s2), "r"(a), "r"(b));
 }
 __device__ __forceinline__ bool t2_elect_one() {
   uint32_t pred;
@@ -167,6 +185,18 @@ __device__ __forceinline__ void t2_wait_or_mark(uint64_t* bar, uint32_t parity, 
     }
   }
 }
+// a look at a barrier that never suspends the warp
+__device__ __forceinline__ bool t2_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ void t2_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // K-major, 128-byte swizzle shared-memory matrix descriptor: rows of 128 bytes, 8-row groups
@@ -190,19 +220,23 @@ __device__ __forceinline__ uint32_t t2_idesc_f16(int n) {
 }
 
 // barrier indices
-enum { T2_X_FULL = 0, T2_A_READY = 4, T2_ST_EMPTY = 8, T2_D_FULL = 12, T2_D_EMPTY = 16, T2_RAW_FULL = 20,
+enum { T2_ST_FULL = 0, T2_ST_EMPTY = 8, T2_D_FULL = 12, T2_D_EMPTY = 16, T2_RAW_FULL = 20,
        T2_RAW_EMPTY = 24 };
-// TMEM accumulators in rotation: the MMA thread runs up to T2_NBUF groups ahead of the
-// accumulate warps, whose tcgen05.ld round trip (not the MMAs) is the latency of a group
-constexpr int T2_NBUF = 4;   // the groups of a block of scales, too
+// TMEM accumulators in rotation: the issuers run up to that many groups ahead of the accumulate warps.  The rest of
+// TMEM holds the stages' weights.
+constexpr int t2_nbuf(int mt) { return mt == 128 ? 3 : 4; }
+constexpr int T2_A_COLS = T2_KS / 2;   // TMEM columns of a stage's weights
 
 template <int MT>
 __global__ void __launch_bounds__(T2_THREADS, 1)
     gemm_q4_tc2_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
                        const __grid_constant__ CUtensorMap tmW, T2Params p) {
   using S = T2Smem<MT>;
-  constexpr int T2_STAGES = S::STAGES;
-  constexpr uint32_t NCOLS = T2_NBUF * MT;   // accumulators of MT columns each: 128 / 256 / 512
+  constexpr int T2_STAGES = S::STAGES, T2_RAW_STAGES = S::RAW_STAGES;
+  constexpr int T2_NBUF = t2_nbuf(MT);
+  constexpr uint32_t A_AT = T2_NBUF * MT;    // TMEM: accumulators of MT columns each, then the weights
+  constexpr uint32_t NCOLS = MT == 32 ? 256 : 512;
+  static_assert(A_AT + T2_STAGES * T2_A_COLS <= NCOLS, "TMEM");
   constexpr int HC = MT / 2;              // columns per accumulate warp
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -216,8 +250,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
   if (tid == 0) {
     *gave_up = 0;
     for (int s = 0; s < T2_STAGES; s++) {
-      mbar_init(&bars[T2_X_FULL + s], 1);
-      mbar_init(&bars[T2_A_READY + s], 4);
+      mbar_init(&bars[T2_ST_FULL + s], 5);    // the X planes' copy, four converter warps
       mbar_init(&bars[T2_ST_EMPTY + s], 2);   // one commit per issuer warp
     }
     for (int b = 0; b < T2_NBUF; b++) {
@@ -241,10 +274,12 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
 
   // the packed weights are not written by the kernel before this one: their producer starts
   // at once; every other role touches activations, the status block or y and waits
-  if (warp != 14) pdl_wait();
+  if (warp != 3) pdl_wait();
   pdl_launch_dependents();
 
-  if (warp == 14) {
+  if (warp < 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(T2_REGS_FEED));
+  if (warp == 3) {
     // ---------------- TMA producer: packed weights, 128 rows x 256 k per box ----------------
     if (lane == 0) {
       int cnt = 0;
@@ -271,15 +306,15 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
           const int s = cnt % T2_STAGES;
           ok = mbar_wait_bounded(&bars[T2_ST_EMPTY + s], ((cnt / T2_STAGES) & 1) ^ 1, p.status, 600);
           if (!ok) break;
-          mbar_expect_tx(&bars[T2_X_FULL + s], 2u * MT * 128u);
+          mbar_expect_tx(&bars[T2_ST_FULL + s], 2u * MT * 128u);
           const int kx = it * T2_KS;
-          tma_load_2d(base + S::B + (size_t)(s * 2 + 0) * MT * 128, &tmX1, kx, m0, &bars[T2_X_FULL + s]);
-          tma_load_2d(base + S::B + (size_t)(s * 2 + 1) * MT * 128, &tmX2, kx, m0, &bars[T2_X_FULL + s]);
+          tma_load_2d(base + S::B + (size_t)(s * 2 + 0) * MT * 128, &tmX1, kx, m0, &bars[T2_ST_FULL + s]);
+          tma_load_2d(base + S::B + (size_t)(s * 2 + 1) * MT * 128, &tmX2, kx, m0, &bars[T2_ST_FULL + s]);
         }
       }
     }
-  } else if (warp == 1 || warp == 15) {
-    // ---------------- MMA issuers: warp 1 the first group of every stage, warp 15 the second ----------------
+  } else if (warp == 1 || warp == 2) {
+    // ---------------- MMA issuers: warp 1 the first group of every stage, warp 2 the second ----------------
     // The whole warp runs the loop (waits included) so that descriptors and addresses stay
     // warp-uniform values, and one elected lane issues; two issuers because the issue cost of
     // a tcgen05.mma (not its execution) bounds a single thread at this instruction size.
@@ -292,11 +327,15 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
       const int s = it % T2_STAGES;
       const uint32_t ph = (it / T2_STAGES) & 1;
       const int gi = 2 * it + grp, buf = gi % T2_NBUF;
-      if (!mbar_wait_warp(&bars[T2_D_EMPTY + buf], ((gi / T2_NBUF) & 1) ^ 1, p.status, 612)) break;
-      if (!mbar_wait_warp(&bars[T2_X_FULL + s], ph, p.status, 610)) break;
-      if (!mbar_wait_warp(&bars[T2_A_READY + s], ph, p.status, 611)) break;
+      // one vote for both barriers where they are complete on the first look
+      const uint32_t dph = ((gi / T2_NBUF) & 1) ^ 1;
+      const bool there = mbar_try_wait(&bars[T2_ST_FULL + s], ph) & mbar_try_wait(&bars[T2_D_EMPTY + buf], dph);
+      if (!__all_sync(0xffffffffu, there)) {
+        if (!mbar_wait_warp(&bars[T2_D_EMPTY + buf], dph, p.status, 612)) break;
+        if (!mbar_wait_warp(&bars[T2_ST_FULL + s], ph, p.status, 610)) break;
+      }
       t2_fence_after();
-      const uint64_t a = t2_desc_sw128(smem_u32(base + S::A + (size_t)s * T2_ROWS * 128));
+      const uint32_t a = tmem + A_AT + (uint32_t)(s * T2_A_COLS);
       const uint64_t b1 = t2_desc_sw128(smem_u32(base + S::B + (size_t)(s * 2 + 0) * MT * 128));
       const uint64_t b2 = t2_desc_sw128(smem_u32(base + S::B + (size_t)(s * 2 + 1) * MT * 128));
       const uint32_t d = tmem + (uint32_t)(buf * MT);
@@ -304,52 +343,55 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
 #pragma unroll
         for (int ks = 0; ks < 2; ks++) {
           const uint64_t adv = (uint64_t)(((2 * grp + ks) * 32) >> 4);   // 16 fp16 = 32 bytes along K
-          t2_mma_f16(d, a + adv, b1 + adv, idesc, ks ? 1u : 0u);
-          t2_mma_f16(d, a + adv, b2 + adv, idesc, 1u);
+          const uint32_t ak = a + (uint32_t)((2 * grp + ks) * 8);        // or 8 columns
+          t2_mma_f16(d, ak, b1 + adv, idesc, ks ? 1u : 0u);
+          t2_mma_f16(d, ak, b2 + adv, idesc, 1u);
         }
         t2_commit(&bars[T2_D_FULL + buf]);     // the group's product is complete when these retire
         t2_commit(&bars[T2_ST_EMPTY + s]);     // ... and (with the other issuer's) the stage can be overwritten
       }
       __syncwarp();
     }
-  } else if (warp < 6) {
+  } else if (warp >= 4) {
     // ---------------- nibble -> fp16 converters (thread r = weight row r) ----------------
-    const int r = tid - 64;
-    const __half2 off = __floats2half2_rn(1032.0f, 1032.0f);
+    const int r = tid - 128;
+    const __half2 off = __floats2half2_rn(1032.0f, 1032.0f), odd = __floats2half2_rn(0.0625f, 0.0625f),
+                  odd_off = __floats2half2_rn(-72.0f, -72.0f);
     int cnt = 0, it = -1;   // boxes and stages of all segments
     while (sg.next(p)) for (int q = sg.q0; q < sg.q1; q++, cnt++) {
       const int rs = cnt % T2_RAW_STAGES;
       t2_wait_or_mark(&bars[T2_RAW_FULL + rs], (cnt / T2_RAW_STAGES) & 1, p.status, 621, gave_up);
       // the row's 128 packed bytes of this box: chunk c (16 bytes = 32 k) sits at c ^ (r & 7)
       const unsigned char* rrow = base + S::RAW + (size_t)rs * T2_RAW_BYTES + r * 128;
-      uint4 wq[2 * T2_SUB];
-#pragma unroll
-      for (int c = 0; c < 2 * T2_SUB; c++) wq[c] = *(const uint4*)(rrow + ((c ^ (r & 7)) << 4));
-#pragma unroll
+#pragma unroll 1
       for (int u = 0; u < T2_SUB; u++) {
         if (q * T2_SUB + u >= nst) break;
         it++;
         const int s = it % T2_STAGES;
-        const uint4 c0 = wq[2 * u], c1 = wq[2 * u + 1];
+        const uint4 c0 = *(const uint4*)(rrow + (((2 * u) ^ (r & 7)) << 4));
+        const uint4 c1 = *(const uint4*)(rrow + (((2 * u + 1) ^ (r & 7)) << 4));
         t2_wait_or_mark(&bars[T2_ST_EMPTY + s], ((it / T2_STAGES) & 1) ^ 1, p.status, 620, gave_up);
-        unsigned char* arow = base + S::A + (size_t)s * T2_ROWS * 128 + r * 128;
+        uint32_t qv[32];
         const unsigned words[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
 #pragma unroll
         for (int j = 0; j < 8; j++) {
           // slot e of the chunk holds (k = e, k = e + 4) of this word: fp16(1024 + nib) has the
           // bit pattern 0x6400 | nib, and 1024 + nib - 1032 = nib - 8 exactly
-          unsigned qv[4];
+          // (and the odd nibbles of a byte in place: (1024 + 16 nib) / 16 - 72)
 #pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const unsigned t = ((words[j] >> (4 * e)) & 0x000F000Fu) | 0x64006400u;
+          for (int e = 0; e < 2; e++) {
+            const unsigned w = words[j] >> (8 * e), t = (w & 0x000F000Fu) | 0x64006400u, o = (w & 0x00F000F0u) | 0x64006400u;
             const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&t), off);
-            qv[e] = *reinterpret_cast<const unsigned*>(&v);
+            const __half2 z = __hfma2(*reinterpret_cast<const __half2*>(&o), odd, odd_off);
+            qv[4 * j + 2 * e] = *reinterpret_cast<const unsigned*>(&v);
+            qv[4 * j + 2 * e + 1] = *reinterpret_cast<const unsigned*>(&z);
           }
-          *(uint4*)(arow + ((j ^ (r & 7)) << 4)) = make_uint4(qv[0], qv[1], qv[2], qv[3]);
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> tensor core reads
+        t2_fence_after();
+        t2_st32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + A_AT + (uint32_t)(s * T2_A_COLS), qv);
+        t2_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[T2_A_READY + s]);
+        if (lane == 0) mbar_arrive(&bars[T2_ST_FULL + s]);
       }
       // The box goes back only here, behind the stores that used all of it.  Given back right after the
       // loads above (which need not be complete, or even issued, before their first use) it was refilled under its readers:
@@ -357,56 +399,72 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars[T2_RAW_EMPTY + rs]);
     }
-  } else if (warp < 14) {
+  }
+  } else {
     // ---------------- accumulate (sc * group product) + epilogue ----------------
-    const int quarter = warp & 3, half = (warp - 6) >> 2;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(T2_REGS_ACC));
+    const int quarter = warp & 3, half = (warp - 8) >> 2;
     const int r = quarter * 32 + lane;
     const int c_lo = half * HC;
     bool ok = true;   // of the warp.  A wait that gave up: no more work, but every barrier and ticket below
-    unsigned blocks = 0;   // of four groups, of all segments
+    int buf = 0;           // accumulator of the next group
+    unsigned parity = 0;
+    bool there = false;    // the next group is known to be complete
     while (sg.next(p)) {
       const int tile = sg.tile, q0 = sg.q0, q1 = sg.q1;
       const int n = tile % p.n_tiles * T2_ROWS + r, m0 = tile / p.n_tiles * MT;
+      // 32 and 64 columns: in pairs of columns, two FMAs an instruction (64 x 3584 x 18944 31.9 -> 28.9 us, 16 rows 27.7 ->
+      // 26.2); at 128 columns that loses (610 -> 634 us)
+      constexpr bool PAIRS = MT < 128;
       float acc[HC];
+      unsigned long long acc2[PAIRS ? HC / 2 : 1];
 #pragma unroll
-      for (int i = 0; i < HC; i++) acc[i] = 0.f;
+      for (int i = 0; i < HC; i++) {
+        acc[i] = 0.f;
+        if (PAIRS) acc2[PAIRS ? i / 2 : 0] = 0ull;
+      }
       // the row's group scales, four at a time (K % 128 == 0), fetched a block ahead: an L2 round trip is
       // shorter than the four groups take
       const float4* sc4 = (const float4*)(p.scales + (size_t)(n < p.N ? n : p.N - 1) * (p.K / 32)) + q0 * 2;
       const int nblk = (q1 * 2 < p.K / 128 ? q1 * 2 : p.K / 128) - q0 * 2;
       float4 sc_blk = __ldg(sc4);
-      for (int b = 0; b < nblk && ok; b++, blocks++) {
+      for (int b = 0; b < nblk && ok; b++) {
         const float4 sc_next = b + 1 < nblk ? __ldg(sc4 + b + 1) : sc_blk;
 #pragma unroll
-        for (int buf = 0; buf < T2_NBUF; buf++) {   // four groups a block, one accumulator each
-          const float sc = buf == 0 ? sc_blk.x : (buf == 1 ? sc_blk.y : (buf == 2 ? sc_blk.z : sc_blk.w));
-          if (!mbar_poll_warp(&bars[T2_D_FULL + buf], blocks & 1, p.status, 630)) { ok = false; break; }
+        for (int k = 0; k < 4; k++) {   // four groups a block
+          const float sc = k == 0 ? sc_blk.x : (k == 1 ? sc_blk.y : (k == 2 ? sc_blk.z : sc_blk.w));
+          if (!__all_sync(0xffffffffu, there) && !mbar_wait_warp(&bars[T2_D_FULL + buf], parity, p.status, 630)) {
+            ok = false;
+            break;
+          }
           t2_fence_after();
           const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * MT + c_lo);
-          // 32 columns per read; the accumulator goes back to the issuers as soon as the last
-          // read has landed, before its FMAs.  (Measured and dropped: fma.rn.f32x2 pairs -- the
-          // register pairing costs more than the halved FMA count saves, 200 vs 170 us at M = 512 --
-          // and 16-column reads in flight under the previous 16 columns' FMAs.)
-          constexpr int BATCH = HC < 32 ? HC : 32;
+          // All of the warp's columns in one read: the accumulator goes back to the issuers as soon as it has landed, before
+          // the FMAs, and the look at the next group's barrier passes under them.
+          uint32_t v[HC / 16][16];
 #pragma unroll
-          for (int c0 = 0; c0 < HC; c0 += BATCH) {
-            uint32_t v[BATCH / 16][16];
+          for (int i = 0; i < HC / 16; i++) t2_ld16_issue(taddr + (uint32_t)(16 * i), v[i]);
+          t2_wait_ld();
+          t2_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars[T2_D_EMPTY + buf]);
+          if (++buf == T2_NBUF) { buf = 0; parity ^= 1u; }
+          there = t2_test(&bars[T2_D_FULL + buf], parity);
+          if constexpr (PAIRS) {
+            unsigned long long sc2;
+            asm("mov.b64 %0, {%1, %1};" : "=l"(sc2) : "f"(sc));
 #pragma unroll
-            for (int b = 0; b < BATCH / 16; b++) t2_ld16_issue(taddr + (uint32_t)(c0 + 16 * b), v[b]);
-            t2_wait_ld();
-            if (c0 + BATCH >= HC) {
-              t2_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&bars[T2_D_EMPTY + buf]);
-            }
+            for (int i = 0; i < HC; i += 2) t2_fma2(acc2[i / 2], sc2, v[i / 16][i % 16], v[i / 16][i % 16 + 1]);
+          } else {
 #pragma unroll
-            for (int b = 0; b < BATCH / 16; b++)
-#pragma unroll
-              for (int i = 0; i < 16; i++) acc[c0 + 16 * b + i] = fmaf(sc, __uint_as_float(v[b][i]), acc[c0 + 16 * b + i]);
+            for (int i = 0; i < HC; i++) acc[i] = fmaf(sc, __uint_as_float(v[i / 16][i % 16]), acc[i]);
           }
         }
         sc_blk = sc_next;
       }
+      if constexpr (PAIRS)
+#pragma unroll
+        for (int i = 0; i < HC / 2; i++) asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[2 * i]), "=f"(acc[2 * i + 1]) : "l"(acc2[i]));
       bool mine = true;   // this CTA writes the tile
       if (q1 - q0 < p.box) {
         // a part of the tile: into scratch, and the last of the tile's CTAs sums all parts
@@ -421,7 +479,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
         for (int i = 0; i < HC; i++) __stcg(mp + i * T2_ROWS, acc[i]);
         __threadfence();
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (warp == 6 && lane == 0) {
+        if (warp == 8 && lane == 0) {
           int old;
           asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(p.tickets + first) : "memory");
           *last_part = old == last - first;
@@ -556,7 +614,9 @@ int gemm_q4_tc2_launch(DeviceCtx* c, const float* x, long long ldx, int M, const
 }
 
 int launch_split_rows(const float* x, long long ldx, int M, int K, const Q4Planes& pl, cudaStream_t stream) {
-  LaunchCfg lc(dim3((unsigned)M), dim3(256), 0, stream, pdl_enabled());
+  // few deep rows: more threads a row, since there are fewer rows than SMs (8 x 18944, split and product: 41.8 -> 32.5 us)
+  const int threads = M <= 148 && K >= 4096 ? 1024 : 256;
+  LaunchCfg lc(dim3((unsigned)M), dim3(threads), 0, stream, pdl_enabled());
   TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, split_f16_kernel, x, ldx, K, pl.hi, pl.lo, pl.rowscale));
   return TLB_OK;
 }
