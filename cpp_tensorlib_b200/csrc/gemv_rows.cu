@@ -11,7 +11,9 @@
 //   - a thread owns the same 16-byte chunks of every row: its activations go from memory to its registers, without shared
 //     memory or a barrier, all loads in flight at once;
 //   - the factor of a norm over the whole row multiplies the sums instead of the activations; the norms' weights are
-//     fetched in front of the wait; the sums of several rows go through the warp together.
+//     fetched in front of the wait; the sums of several rows go through the warp together;
+//   - the sums of a norm in parts come from the chunks that the threads hold: a second look at the row waited 1 - 2 us behind
+//     the weights of the next launch (a token of the 8-layer Mamba stack 305 -> 285 us, of the latent stack 386 -> 377).
 // Launches of one shape behind each other, cold weights, us (before: two rows a warp in registers, two blocks an SM):
 //   2048 -> 10304 with norm 11.1 -> 10.1, 2048 -> 11264 11.7 -> 10.8, 4096 -> 2048 6.9 -> 4.9, 5632 -> 2048 7.3 -> 7.0;
 //   the first with the weights in the L2 already: 11.0 -> 7.1.
@@ -34,6 +36,8 @@ constexpr size_t RG_SMEM_SHARED = 112 * 1024, RG_SMEM_MAX = 226 * 1024;
 struct RowPlan {
   int stages, stage_rows, rows_max;   // ring; rows of a stage; most rows of a block
   int wpr;                            // warps on a row
+  int part_chunks;                    // 16-byte chunks' worth of elements of a norm's part
+  unsigned part_magic;                // ceil(2^32 / part_chunks), 0 for one: a chunk's part without a division
   int* status;
 };
 
@@ -77,14 +81,23 @@ __device__ __forceinline__ void rg_parts(const RowGemv& p, float* gs) {
 }
 // N elements of the staged row from e0 on: v holds them as they are in x, w the norm's weights, r and rn the residual and
 // its weights, g the gate; s is the residual's scale
-template <int N>
+// (WHOLE: the segment and its parts are whole pieces of N elements)
+template <int N, bool WHOLE>
 __device__ __forceinline__ void rg_prepare(const RowGemv& p, int e0, float (&v)[N], const float (&w)[N], const float (&r)[N],
-                                           const float (&rn)[N], const float (&g)[N], float s, const float* gs, float& sq) {
+                                           const float (&rn)[N], const float (&g)[N], float s, const float* gs, unsigned magic, float& sq) {
   if (p.res) {
 #pragma unroll
-    for (int k = 0; k < N; k++) {
-      v[k] = fmaf(v[k] * s, rn[k], r[k]);
-      if (p.xout && blockIdx.x == 0 && e0 + k < p.K) p.xout[e0 + k] = v[k];
+    for (int k = 0; k < N; k++) v[k] = fmaf(v[k] * s, rn[k], r[k]);
+    if (p.xout && blockIdx.x == 0) {
+      if (WHOLE) {
+        if (e0 < p.K)
+#pragma unroll
+          for (int k = 0; k < N; k += 4) *(float4*)(p.xout + e0 + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < N; k++)
+          if (e0 + k < p.K) p.xout[e0 + k] = v[k];
+      }
     }
   }
 #pragma unroll
@@ -96,6 +109,13 @@ __device__ __forceinline__ void rg_prepare(const RowGemv& p, int e0, float (&v)[
     return;
   }
   if (e0 + N <= p.n_off || e0 >= p.n_off + p.n_len) return;
+  if constexpr (WHOLE) {
+    const unsigned c = (unsigned)((e0 - p.n_off) / N);
+    const float f = gs[magic ? __umulhi(c, magic) : c];
+#pragma unroll
+    for (int k = 0; k < N; k++) v[k] *= p.gate ? f * w[k] * silu_f(g[k]) : f * w[k];
+    return;
+  }
   const int m = p.n_len / p.n_groups;
   int part = e0 <= p.n_off ? 0 : (e0 - p.n_off) / m;
 #pragma unroll
@@ -220,14 +240,36 @@ __global__ void __launch_bounds__(RG_THREADS + 32, JN < 8 ? 2 : 1) row_gemv_kern
   }
   float* gs = part + pl.wpr * pl.rows_max;
   if (p.nw && !rg_whole(p)) {
-    rg_parts(p, gs);
+    // the parts' sums from the chunks' (a part is whole chunks), a warp a part: no second look at the row, which would
+    // wait behind the next launch's weights
+    float* cs = gs + p.n_groups;
+    const int lo = p.n_off / CE, m = pl.part_chunks;
+#pragma unroll
+    for (int j = 0; j < JN; j++) {
+      const int c = c0 + j * RG_THREADS - lo;
+      if (grp == 0 && c >= 0 && c < m * p.n_groups) {
+        float q = 0.f;
+#pragma unroll
+        for (int e = 0; e < CE; e++) q = fmaf(x[j][e], x[j][e], q);
+        cs[c] = q;
+      }
+    }
+    rg_sync();
+#pragma unroll 1
+    for (int g = warp; g < p.n_groups; g += RG_WARPS) {
+      float q = 0.f;
+#pragma unroll 2
+      for (int c = lane; c < m; c += 32) q += cs[g * m + c];
+      q = warp_sum(q);
+      if (lane == 0) gs[g] = rsqrtf(q / (m * CE) + p.eps) * p.nscale;
+    }
     rg_sync();
   }
 #pragma unroll
   for (int j = 0; j < JN; j++) {
     if (!ONE) { ld_rn(j); ld_res(j); }
     if (!FEW) { ld_nw(j, nw[0]); ld_gate(j, gate[0]); }
-    rg_prepare<CE>(p, (c0 + j * RG_THREADS) * CE, x[j], nw[FEW ? j : 0], res, rn, gate[FEW ? j : 0], s, gs, sq);
+    rg_prepare<CE, true>(p, (c0 + j * RG_THREADS) * CE, x[j], nw[FEW ? j : 0], res, rn, gate[FEW ? j : 0], s, gs, pl.part_magic, sq);
   }
   if (rg_whole(p)) {
     sq = warp_sum(grp == 0 ? sq : 0.f);
@@ -271,8 +313,11 @@ __global__ void __launch_bounds__(RG_THREADS + 32, JN < 8 ? 2 : 1) row_gemv_kern
   rg_sync();
   const float f = rg_whole(p) ? rsqrtf(rg_total(red[1]) / p.K + p.eps) * p.nscale : 1.f;
   auto row_sum = [&](int r) {
-    float a = 0.f;
-    for (int k = 0; k < wpr; k++) a += part[k * pl.rows_max + r];
+    float q[RG_WARPS], a = 0.f;
+#pragma unroll
+    for (int k = 0; k < RG_WARPS; k++) q[k] = k < wpr ? part[k * pl.rows_max + r] : 0.f;
+#pragma unroll
+    for (int k = 0; k < RG_WARPS; k++) a += q[k];
     return a * f;
   };
   for (int r = tid * u; r < rows; r += RG_THREADS * u)
@@ -307,7 +352,7 @@ __global__ void __launch_bounds__(RG_THREADS) row_gemv_long_kernel(const __grid_
     if (p.rn) rg_ld_any<CE>(p.rn, c * CE, p.K, rn);
     if (p.res) rg_ld_any<CE>(p.res, c * CE, p.K, r);
     if (p.gate) rg_ld_any<CE>(p.gate, c * CE - p.n_off, p.n_len, g);
-    rg_prepare<CE>(p, c * CE, v, w, r, rn, g, s, gs, sq);
+    rg_prepare<CE, false>(p, c * CE, v, w, r, rn, g, s, gs, 0u, sq);
 #pragma unroll
     for (int e = 0; e < CE; e++) xs[c * CE + e] = v[e];
   }
@@ -345,17 +390,22 @@ int rg_plan_launch(DeviceCtx* c, const RowGemv& p, cudaStream_t s) {
   constexpr int CE = Vec16<WT>::N;
   const int chunks = (int)(p.ldw / CE), u = p.epi == 2 ? 2 : 1, units = (p.N + u - 1) / u;
   auto aligned = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
-  const bool vec = aligned(p.x) && aligned(p.res) && aligned(p.rn) && aligned(p.nw) && aligned(p.gate) && p.K % CE == 0 &&
-                   (!p.nw || (p.n_off % CE == 0 && p.n_len % CE == 0));
+  const bool vec = aligned(p.x) && aligned(p.res) && aligned(p.rn) && aligned(p.nw) && aligned(p.gate) && aligned(p.xout) &&
+                   p.K % CE == 0 &&
+                   (!p.nw || (p.n_off % CE == 0 && p.n_len % CE == 0 && (p.n_len / p.n_groups) % CE == 0));
   const int groups = p.nw ? p.n_groups : 0;
   const int need = (chunks + RG_THREADS - 1) / RG_THREADS, jn = need <= 4 ? need : (need <= 8 ? 8 : 0);
   const int ctas = units < c->sm_count ? units : c->sm_count;
   RowPlan pl{};
   pl.status = c->status;
   pl.rows_max = (units + ctas - 1) / ctas * u;
+  if (vec && p.nw) {
+    pl.part_chunks = p.n_len / p.n_groups / CE;
+    pl.part_magic = (unsigned)(((1ull << 32) + pl.part_chunks - 1) / pl.part_chunks);   // exact below 2^16 chunks; 1: 0
+  }
   pl.wpr = RG_WARPS;
   while (pl.wpr > 1 && chunks <= pl.wpr / 2 * 32) pl.wpr /= 2;
-  const size_t row = (size_t)p.ldw * sizeof(WT), tail = ((size_t)pl.wpr * pl.rows_max + groups) * sizeof(float) + 16;
+  const size_t row = (size_t)p.ldw * sizeof(WT), tail = ((size_t)pl.wpr * pl.rows_max + groups + (groups ? p.n_len / CE : 0)) * sizeof(float) + 16;
   pl.stage_rows = jn ? rg_rows_of(jn) * (RG_WARPS / pl.wpr) : 1;
   const size_t stage = row * pl.stage_rows;
   const int nst = (pl.rows_max + pl.stage_rows - 1) / pl.stage_rows;
