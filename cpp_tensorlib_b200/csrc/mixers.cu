@@ -18,7 +18,6 @@ namespace tlb {
 namespace {
 
 constexpr int MX_MAXREC = 2;
-constexpr int MX_ROWS = 32;     // state rows per thread of the one-token update
 
 struct DecodeArgs {
   AttnP at;
@@ -28,6 +27,7 @@ struct DecodeArgs {
   const float* proj;
   float* out;
   const unsigned* d_pos;
+  int* status;
 };
 
 // ---- attention, one token ------------------------------------------------------------------
@@ -377,190 +377,226 @@ __device__ void attn_decode_unit16(const AttnP& p, int unit, const float* row, f
 }
 
 // ---- recurrent mixers, one token -----------------------------------------------------------
-// One block a head.  A thread holds up to MX_ROWS rows of one state column, for two column blocks at a
-// time; the first two blocks and the convolutions' history are fetched before the projected row is there.
-__device__ void recur_decode_head(const RecurP& p, int h, const float* row, float* out, int pos, float* sm) {
+// A launch runs this code once, from a cold instruction cache, at some twenty cycles an instruction: what it costs is its
+// length.  A state held in registers, 32 rows a thread with everything unrolled, took 3 - 4 us for the arithmetic of 0.3 and
+// 1.3 us for its stores (timer in the kernel, 64 heads of 128 x 64).  So the state goes to shared memory in front of the
+// wait and the loops over its rows stay loops (2.8 us), and since the block of an SSD head waits 7 us for the projection
+// anyway, it first goes through the code behind the wait once with nothing kept (1.4 us).  The delta rule's code is longer
+// than that wait (its first pass ended 4 us late), so it is gone through once.  A token of the 8-layer Mamba and delta stack:
+// 285 -> 259 us; of the latent-attention and GLA stack 377 -> 373.
+
+// rows of the state for the columns c0.. of a block's threads: V columns a thread, the rows dealt to the row groups
+template <int V> struct Cols { float f[V]; };
+template <int V> __device__ __forceinline__ Cols<V> cols_ld(const float* p);
+template <> __device__ __forceinline__ Cols<1> cols_ld<1>(const float* p) { Cols<1> c; c.f[0] = *p; return c; }
+template <> __device__ __forceinline__ Cols<4> cols_ld<4>(const float* p) {
+  const float4 v = *(const float4*)p;
+  Cols<4> c;
+  c.f[0] = v.x; c.f[1] = v.y; c.f[2] = v.z; c.f[3] = v.w;
+  return c;
+}
+__device__ __forceinline__ void cols_st(float* p, const Cols<1>& c) { *p = c.f[0]; }
+__device__ __forceinline__ void cols_st(float* p, const Cols<4>& c) { *(float4*)p = make_float4(c.f[0], c.f[1], c.f[2], c.f[3]); }
+
+// S <- g S + k u^T and o = q S, u = in v or, for the delta rule, in (v - k (g S)).  src: the state, in shared or global
+// memory (NULL: zero), dst: where the new one goes; red holds MX_THREADS * V floats.  The whole block; barriers inside.
+template <int V>
+__device__ void recur_update(const RecurP& p, const float* src, float* dst, const float* q, const float* k, const float* v,
+                             float* o, float* red, float g, float in, bool delta) {
+  const int tid = threadIdx.x, D = p.D, E = p.E;
+#pragma unroll 1
+  for (int c0 = 0; c0 < E; c0 += MX_THREADS * V) {
+    const int w = E - c0 < MX_THREADS * V ? E - c0 : MX_THREADS * V, ct = w / V, RG = MX_THREADS / ct;
+    const int rg = tid / ct, cl = (tid - rg * ct) * V, c = c0 + cl;
+    const bool on = rg < RG;
+    Cols<V> u, acc;
+#pragma unroll
+    for (int e = 0; e < V; e++) acc.f[e] = u.f[e] = 0.f;
+    if (delta) {
+      if (on && src) {
+#pragma unroll 2
+        for (int r = rg; r < D; r += RG) {
+          const Cols<V> x = cols_ld<V>(src + (size_t)r * E + c);
+#pragma unroll
+          for (int e = 0; e < V; e++) acc.f[e] = fmaf(k[r], x.f[e] * g, acc.f[e]);
+        }
+      }
+      if (on) cols_st(red + rg * w + cl, acc);
+      __syncthreads();
+      // the row groups' sums, in order
+      if (on)
+        for (int i = 0; i < RG; i++) {
+          const Cols<V> x = cols_ld<V>(red + i * w + cl);
+#pragma unroll
+          for (int e = 0; e < V; e++) u.f[e] -= x.f[e];
+        }
+      __syncthreads();
+    }
+    if (on) {
+      const Cols<V> val = cols_ld<V>(v + c);
+#pragma unroll
+      for (int e = 0; e < V; e++) u.f[e] = in * (val.f[e] + u.f[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < V; e++) acc.f[e] = 0.f;
+    if (on) {
+#pragma unroll 2
+      for (int r = rg; r < D; r += RG) {
+        Cols<V> x;
+        if (src) x = cols_ld<V>(src + (size_t)r * E + c);
+        const float kk = k[r], qq = q[r];
+#pragma unroll
+        for (int e = 0; e < V; e++) {
+          x.f[e] = fmaf(kk, u.f[e], src ? x.f[e] * g : 0.f);
+          acc.f[e] = fmaf(qq, x.f[e], acc.f[e]);
+        }
+        cols_st(dst + (size_t)r * E + c, x);
+      }
+    }
+    if (on) cols_st(red + rg * w + cl, acc);
+    __syncthreads();
+    for (int i = tid; i < w; i += MX_THREADS) {
+      float x = 0.f;
+#pragma unroll 4
+      for (int j = 0; j < RG; j++) x += red[j * w + i];
+      o[c0 + i] = x;
+    }
+    __syncthreads();
+  }
+}
+
+// floats of the state that wait in shared memory (0: it is too large, or not whole 16-byte pieces)
+constexpr int MX_STATE_SMEM = 16384;
+__host__ __device__ inline int recur_state_floats(const RecurP& p) {
+  const int n = p.D * p.E;
+  return n <= MX_STATE_SMEM && n % 4 == 0 ? n : 0;
+}
+
+// One block a head.  The state and the convolutions' history are fetched before the projected row is there.  (The row is
+// read past the L1: what the first pass saw of it may be old.)
+__device__ void recur_decode_head(const RecurP& p, int h, const float* row, float* out, int pos, float* sm, int* status) {
+  __shared__ __align__(8) uint64_t bar;
   const int tid = threadIdx.x, D = p.D, E = p.E, rep = p.H / p.G, kg = h / rep, n = 2 * D + E;
-  float* q = sm;               // [D]
+  const int ns = recur_state_floats(p);
+  float* st = sm;              // [ns] state
+  float* q = st + ns;          // [D]
   float* k = q + D;            // [D]
   float* v = k + D;            // [E]
   float* o = v + E;            // [E]
   float* wl = o + E;           // [n] weights of the current token
-  float* red = wl + n;         // [2][MX_THREADS]
-  float* rs = red + 2 * MX_THREADS;  // [33]
+  float* red = wl + n + ((4 - ((ns + 4 * D + 3 * E) & 3)) & 3);   // [4][MX_THREADS], 16-byte aligned
+  float* rs = red + 4 * MX_THREADS;  // [33]
   float* S = p.S + (size_t)h * D * E;
-  const int need = (D + MX_ROWS - 1) / MX_ROWS;
-  const int VB = E < MX_THREADS / need ? E : MX_THREADS / need;
-  const int RS = MX_THREADS / VB;
-  const int grp = tid / VB, col = tid - grp * VB;
-  const size_t stride = (size_t)RS * E;
-  float s[2][MX_ROWS];
-  auto fetch = [&](int c0) {
-#pragma unroll
-    for (int b = 0; b < 2; b++) {
-      const int e = c0 + b * VB + col;
-      const int left = grp < RS && e < E && pos > 0 ? D - grp : 0;   // rows grp, grp + RS, ... below D
-      const float* at = S + (size_t)grp * E + e;
-#pragma unroll
-      for (int i = 0; i < MX_ROWS; i++) {
-        s[b][i] = i * RS < left ? *at : 0.f;
-        at += stride;
-      }
-    }
-  };
-  fetch(0);
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    mbar_fence_init();
+  }
   auto channel = [&](int i) {
     return i < D ? p.cq + kg * D + i : (i < 2 * D ? p.ck + kg * D + i - D : p.cvv + h * E + i - 2 * D);
   };
   const int taps = p.cv.taps;
   const float A_log = p.A_log[h], bias = p.dt_bias[h], skip = p.kind == MIX_SSD ? p.Dskip[h] : 0.f;
   const float nw = p.kind == MIX_DELTA && tid < E ? p.norm[tid] : 0.f;
-  for (int i0 = 0; i0 < n; i0 += 2 * MX_THREADS) {
-    // two channels a thread, four taps at a time: every load of the history before its first use
-    float y[2] = {0.f, 0.f};
-    for (int a0 = 0; a0 + 1 < taps; a0 += 4) {
-      float w[2][4], x[2][4];
-      int at = (pos - (taps - 1 - a0) + taps) % taps;   // ring row of tap a0 (not read in front of the start)
-      if (at < 0) at += taps;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const bool on = a0 + j + 1 < taps && pos - (taps - 1 - a0 - j) >= 0;
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-          const int i = i0 + b * MX_THREADS + tid;
-          const int c = i < n ? channel(i) : 0;
-          w[b][j] = on && i < n ? p.cv.w[(size_t)c * taps + a0 + j] : 0.f;
-          x[b][j] = on && i < n ? p.cv.ring[(size_t)at * p.cv.C + c] : 0.f;
-        }
-        at = at + 1 == taps ? 0 : at + 1;
+  int pass = p.kind == MIX_DELTA;
+  asm volatile("" : "+r"(pass));
+#pragma unroll 1
+  for (; pass < 2; pass++) {
+    const bool real = pass != 0;
+    if (real) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncthreads();   // the first pass has left shared memory
+      if (tid == 0 && ns && pos > 0) {
+        mbar_expect_tx(&bar, ns * 4);
+        bulk_load_1d(st, S, ns * 4, &bar);
       }
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        y[0] = fmaf(w[0][j], x[0][j], y[0]);
-        y[1] = fmaf(w[1][j], x[1][j], y[1]);
-      }
-    }
-#pragma unroll
-    for (int b = 0; b < 2; b++) {
-      const int i = i0 + b * MX_THREADS + tid;
-      if (i < n) {
+#pragma unroll 1
+      for (int i = tid; i < n; i += MX_THREADS) {
+        // four taps at a time: their loads before the first use
         const int c = channel(i);
-        sm[i] = p.cv.b ? y[b] + p.cv.b[c] : y[b];
+        float y = p.cv.b ? p.cv.b[c] : 0.f;
+#pragma unroll 1
+        for (int a0 = 0; a0 + 1 < taps; a0 += 4) {
+          float w[4], x[4];
+          int at = (pos - (taps - 1 - a0) + taps) % taps;   // ring row of tap a0 (not read in front of the start)
+          if (at < 0) at += taps;
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const bool on = a0 + j + 1 < taps && pos - (taps - 1 - a0 - j) >= 0;
+            w[j] = on ? p.cv.w[(size_t)c * taps + a0 + j] : 0.f;
+            x[j] = on ? p.cv.ring[(size_t)at * p.cv.C + c] : 0.f;
+            at = at + 1 == taps ? 0 : at + 1;
+          }
+#pragma unroll
+          for (int j = 0; j < 4; j++) y = fmaf(w[j], x[j], y);
+        }
+        q[i] = y;
         wl[i] = p.cv.w[(size_t)c * taps + taps - 1];
       }
+      pdl_wait();
+      pdl_launch_dependents();
     }
-  }
-  pdl_wait();
-  pdl_launch_dependents();
-  const float* cur = row + p.cv.off;
-  const float gate = tid < E ? row[p.og + h * E + tid] : 0.f;
-  const float raw_in = row[p.ob + h], raw_step = row[p.oa_ + h];
-  for (int i = tid; i < n; i += MX_THREADS) {
-    const int c = channel(i);
-    const float x = cur[c];
-    sm[i] = silu_f(fmaf(wl[i], x, sm[i]));
-    if (taps > 1 && (i >= 2 * D || h == kg * rep)) p.cv.ring[(size_t)(pos % taps) * p.cv.C + c] = x;
-  }
-  const bool delta = p.kind == MIX_DELTA;
-  const float step = softplus_f(raw_step + bias);
-  const float in = delta ? sigmoid_f(raw_in) : step, g = decay_of(expf(A_log) * step);
-  __syncthreads();
-  if (delta) {
-    float sq = 0.f, sk = 0.f;
-    for (int i = tid; i < D; i += MX_THREADS) { sq = fmaf(q[i], q[i], sq); sk = fmaf(k[i], k[i], sk); }
-    sq = block_sum(sq, rs);
-    sk = block_sum(sk, rs);
-    const float fq = rsqrtf(sq + 1e-6f) * rsqrtf((float)D), fk = rsqrtf(sk + 1e-6f);
-    for (int i = tid; i < D; i += MX_THREADS) { q[i] *= fq; k[i] *= fk; }
+    const float *cur = row + p.cv.off, *z = row + p.og + h * E;
+    const float gate = tid < E ? __ldcg(z + tid) : 0.f;
+    const float raw_in = __ldcg(row + (p.ob + h)), raw_step = __ldcg(row + (p.oa_ + h));
+    float xc[2];   // of the first two channels of a thread
+#pragma unroll
+    for (int j = 0; j < 2; j++) xc[j] = tid + j * MX_THREADS < n ? __ldcg(cur + channel(tid + j * MX_THREADS)) : 0.f;
+#pragma unroll 1
+    for (int i = tid; i < n; i += MX_THREADS) {
+      const int c = channel(i);
+      const float x = i < MX_THREADS ? xc[0] : (i < 2 * MX_THREADS ? xc[1] : __ldcg(cur + c));
+      q[i] = silu_f(fmaf(wl[i], x, q[i]));
+      if (real && taps > 1 && (i >= 2 * D || h == kg * rep)) p.cv.ring[(size_t)(pos % taps) * p.cv.C + c] = x;
+    }
+    const bool delta = p.kind == MIX_DELTA;
+    const float step = softplus_f(raw_step + bias);
+    const float in = delta ? sigmoid_f(raw_in) : step, g = decay_of(expf(A_log) * step);
     __syncthreads();
-  }
-  for (int c0 = 0; c0 < E; c0 += 2 * VB) {
-    if (c0) fetch(c0);
-    float u[2], acc[2] = {0.f, 0.f};
     if (delta) {
-      float dot[2] = {0.f, 0.f};
-#pragma unroll
-      for (int i = 0; i < MX_ROWS; i++) {
-        const int r = grp + i * RS;
-        const float kk = r < D ? k[r] : 0.f;
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-          s[b][i] *= g;
-          dot[b] = fmaf(kk, s[b][i], dot[b]);
+      float sq = 0.f, sk = 0.f;
+      for (int i = tid; i < D; i += MX_THREADS) { sq = fmaf(q[i], q[i], sq); sk = fmaf(k[i], k[i], sk); }
+      sq = block_sum(sq, rs);
+      sk = block_sum(sk, rs);
+      const float fq = rsqrtf(sq + 1e-6f) * rsqrtf((float)D), fk = rsqrtf(sk + 1e-6f);
+      for (int i = tid; i < D; i += MX_THREADS) { q[i] *= fq; k[i] *= fk; }
+      __syncthreads();
+    }
+    const float* src = pos > 0 ? (ns ? st : S) : nullptr;
+    bool ok = real || ns;   // (the first pass leaves a state in global memory alone)
+    if (real && ns && pos > 0) ok = mbar_wait_bounded(&bar, 0, status, 810);
+    if (__syncthreads_and(ok)) {
+      // (16-byte pieces need every part of shared memory on 16 bytes)
+      float* dst = ns ? st : S;
+      if ((E & 3) == 0 && (D & 1) == 0) recur_update<4>(p, src, dst, q, k, v, o, red, g, in, delta);
+      else recur_update<1>(p, src, dst, q, k, v, o, red, g, in, delta);
+      if (ns && real) {   // back in one copy, under the read-out below (update ended with a barrier)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (tid == 0) {
+          asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(S), "r"(smem_u32(st)), "r"(ns * 4)
+                       : "memory");
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       }
-      red[tid] = dot[0];
-      red[MX_THREADS + tid] = dot[1];
-      __syncthreads();
-#pragma unroll
-      for (int b = 0; b < 2; b++) {
-        const int e = c0 + b * VB + col;
-        float d = 0.f;
-        for (int w = 0; w < RS; w++) d += red[b * MX_THREADS + w * VB + col];
-        u[b] = grp < RS && e < E ? in * (v[e] - d) : 0.f;
-      }
-      __syncthreads();
+    }
+    if (delta) {
+      float sq = 0.f;
+      for (int e = tid; e < E; e += MX_THREADS) sq = fmaf(o[e], o[e], sq);
+      sq = block_sum(sq, rs);
+      const float r = rsqrtf(sq / E + p.eps) * p.out_scale;
+      for (int e = tid; e < E; e += MX_THREADS)
+        if (real) out[p.oa + h * E + e] = o[e] * r * (e == tid ? nw : p.norm[e]) * silu_f(e == tid ? gate : __ldcg(z + e));
     } else {
-#pragma unroll
-      for (int b = 0; b < 2; b++) {
-        const int e = c0 + b * VB + col;
-        u[b] = grp < RS && e < E ? in * v[e] : 0.f;
-      }
-#pragma unroll
-      for (int i = 0; i < MX_ROWS; i++) { s[0][i] *= g; s[1][i] *= g; }
+      for (int e = tid; e < E; e += MX_THREADS)
+        if (real) out[p.oa + h * E + e] = fmaf(skip, v[e], o[e]) * silu_f(e == tid ? gate : __ldcg(z + e));
     }
-#pragma unroll
-    for (int i = 0; i < MX_ROWS; i++) {
-      const int r = grp + i * RS;
-      if (r < D) {
-        const float kk = k[r], qq = q[r];
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-          s[b][i] = fmaf(kk, u[b], s[b][i]);
-          acc[b] = fmaf(qq, s[b][i], acc[b]);
-        }
-      }
-    }
-    red[tid] = acc[0];
-    red[MX_THREADS + tid] = acc[1];
-#pragma unroll
-    for (int b = 0; b < 2; b++) {
-      const int e = c0 + b * VB + col;
-      const int left = grp < RS && e < E ? D - grp : 0;
-      float* at = S + (size_t)grp * E + e;
-#pragma unroll
-      for (int i = 0; i < MX_ROWS; i++) {
-        if (i * RS < left) *at = s[b][i];
-        at += stride;
-      }
-    }
-    __syncthreads();
-    for (int i = tid; i < 2 * VB; i += MX_THREADS) {
-      const int b = i / VB, c = i - b * VB, e = c0 + i;
-      if (e < E) {
-        float a = 0.f;
-        for (int w = 0; w < RS; w++) a += red[b * MX_THREADS + w * VB + c];
-        o[e] = a;
-      }
-    }
-    __syncthreads();
   }
-  if (delta) {
-    float sq = 0.f;
-    for (int e = tid; e < E; e += MX_THREADS) sq = fmaf(o[e], o[e], sq);
-    sq = block_sum(sq, rs);
-    const float r = rsqrtf(sq / E + p.eps) * p.out_scale;
-    for (int e = tid; e < E; e += MX_THREADS)
-      out[p.oa + h * E + e] = o[e] * r * (e == tid ? nw : p.norm[e]) * silu_f(e == tid ? gate : row[p.og + h * E + e]);
-  } else {
-    for (int e = tid; e < E; e += MX_THREADS)
-      out[p.oa + h * E + e] = fmaf(skip, v[e], o[e]) * silu_f(e == tid ? gate : row[p.og + h * E + e]);
-  }
+  if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // ---- gated linear attention, one token ------------------------------------------------------
-// One block per (head, 32 state columns): warp w holds rows w, w + 8, ... of them.  The state and the
-// decay's weights are fetched before the projected row is there.
+// One block per (head, 32 state columns): warp w holds rows w, w + 8, ... of them.  The state's slice and the
+// decay's weights are fetched before the projected row is there; the loop over the slice stays a loop.
 constexpr int GL_COLS = 32, GL_WARPS = MX_THREADS / 32, GL_PRE = 16;
 __device__ __forceinline__ int gla_slices(const RecurP& p) { return (p.E + GL_COLS - 1) / GL_COLS; }
 __device__ void gla_decode_unit(const RecurP& p, int unit, const float* row, float* out, int pos, float* sm) {
@@ -570,17 +606,14 @@ __device__ void gla_decode_unit(const RecurP& p, int unit, const float* row, flo
   float* k = q + D;            // [D]
   float* al = k + D;           // [D]
   float* red = al + D;         // [GL_WARPS][32]
+  float* st = red + MX_THREADS;   // [D][32]
   float* S = p.S + (size_t)h * D * E + e;
   const bool on = e < E;
-  float s[MX_ROWS], w[GL_PRE];
-  auto fetch = [&](int d0) {
-#pragma unroll
-    for (int i = 0; i < MX_ROWS; i++) {
-      const int d = d0 + warp + i * GL_WARPS;
-      s[i] = on && pos > 0 && d < D ? S[(size_t)d * E] : 0.f;
-    }
-  };
-  fetch(0);
+#pragma unroll 1
+  for (int d = warp; d < D; d += GL_WARPS)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(st + d * GL_COLS + lane)),
+                 "l"(on ? S + (size_t)d * E : p.S), "r"(on && pos > 0 ? 4 : 0) : "memory");
+  float w[GL_PRE];
   const int c0 = h * D + tid;
 #pragma unroll
   for (int r = 0; r < GL_PRE; r++) w[r] = tid < D && r < p.rank ? p.a_up[(size_t)r * HD + c0] : 0.f;
@@ -588,6 +621,7 @@ __device__ void gla_decode_unit(const RecurP& p, int unit, const float* row, flo
   pdl_wait();
   pdl_launch_dependents();
   const float v = on ? row[p.cvv + h * E + e] : 0.f;
+#pragma unroll 1
   for (int d = tid; d < D; d += MX_THREADS) {
     const int c = h * D + d;
     q[d] = row[p.cq + c] * rsqrtf((float)D);
@@ -599,19 +633,14 @@ __device__ void gla_decode_unit(const RecurP& p, int unit, const float* row, flo
     for (int r = GL_PRE; r < p.rank; r++) z = fmaf(row[p.ob + r], p.a_up[(size_t)r * HD + c], z);
     al[d] = decay_of(gla_rate(z, p.tau));
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   float acc = 0.f;
-  for (int d0 = 0; d0 < D; d0 += GL_WARPS * MX_ROWS) {
-    if (d0) fetch(d0);
-#pragma unroll
-    for (int i = 0; i < MX_ROWS; i++) {
-      const int d = d0 + warp + i * GL_WARPS;
-      if (d < D) {
-        s[i] = fmaf(k[d], v, s[i] * al[d]);
-        acc = fmaf(q[d], s[i], acc);
-        if (on) S[(size_t)d * E] = s[i];
-      }
-    }
+#pragma unroll 4
+  for (int d = warp; d < D; d += GL_WARPS) {
+    const float x = fmaf(k[d], v, st[d * GL_COLS + lane] * al[d]);
+    acc = fmaf(q[d], x, acc);
+    if (on) S[(size_t)d * E] = x;
   }
   red[tid] = acc;
   __syncthreads();
@@ -637,7 +666,7 @@ __global__ void __launch_bounds__(MX_THREADS, 2) mixers_decode_kernel(const __gr
     const int n = recur_blocks(a.rec[i]);
     if (b < n) {
       if (a.rec[i].kind == MIX_GLA) gla_decode_unit(a.rec[i], b, a.proj, a.out, pos, sm);
-      else recur_decode_head(a.rec[i], b, a.proj, a.out, pos, sm);
+      else recur_decode_head(a.rec[i], b, a.proj, a.out, pos, sm, a.status);
       return;
     }
     b -= n;
@@ -1030,15 +1059,15 @@ size_t attn_smem(const AttnP& p, int rm) {
   return (size_t)(rm * (2 * p.Dp + p.Ep + MX_TK) + 32 + 40 + 2 * p.Dp + p.Ep + fast) * sizeof(float);
 }
 size_t recur_smem(const RecurP& p) {
-  if (p.kind == MIX_GLA) return (size_t)(3 * p.D + MX_THREADS) * sizeof(float);
-  return (size_t)(4 * p.D + 3 * p.E + 2 * MX_THREADS + 40) * sizeof(float);
+  if (p.kind == MIX_GLA) return (size_t)(3 * p.D + MX_THREADS + p.D * GL_COLS) * sizeof(float);
+  return (size_t)(recur_state_floats(p) + 4 * p.D + 3 * p.E + 4 * MX_THREADS + 44) * sizeof(float);
 }
 int rm_of(int hpb) { return hpb <= 1 ? 1 : (hpb <= 2 ? 2 : (hpb <= 4 ? 4 : 8)); }
 
 template <typename KT, int RM, bool FAST>
 int decode_launch(const DecodeArgs& a, int blocks, size_t smem, cudaStream_t s) {
   static std::atomic<unsigned long long> done{0};
-  const int rc = ensure_dynamic_smem(mixers_decode_kernel<KT, RM, FAST>, 200 * 1024, done);
+  const int rc = ensure_dynamic_smem(mixers_decode_kernel<KT, RM, FAST>, 204 * 1024, done);
   if (rc) return rc;
   LaunchCfg lc(dim3(blocks), dim3(MX_THREADS), smem, s, pdl_enabled());
   TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, mixers_decode_kernel<KT, RM, FAST>, a));
@@ -1101,6 +1130,12 @@ int mixers_decode_launch(const AttnP* attn, const RecurP* rec, int n_rec, const 
     smem = n > smem ? n : smem;
   }
   a.proj = proj; a.out = out; a.d_pos = d_pos;
+  {
+    DeviceCtx* c = nullptr;
+    const int rc = get_ctx(&c);
+    if (rc) return rc;
+    a.status = c->status;
+  }
 #define MX_CASE(m)                                                                     \
   if (rm == m)                                                                         \
     return !kv_bf16 ? decode_launch<float, m, false>(a, blocks, smem, s)                  \

@@ -1,0 +1,33 @@
+"""One token of the recurrent mixers at the sizes where the state's place and the split of its columns change."""
+import numpy as np
+import pytest
+
+import zav_cases as zc
+from oracle import zavilorn as orc
+from test_gpu_zavilorn import close, err, make, ok, run
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,groups,state,vdim,conv,norm_groups", [
+    (4, 2, 16, 16, 4, 8),       # norm parts of 8
+    (2, 1, 128, 128, 4, 1),     # the largest state that waits in shared memory
+    (2, 1, 136, 124, 6, 2),     # above it; more than four taps
+    (3, 1, 15, 21, 2, 3),       # not whole 16-byte pieces; odd parts
+    (2, 2, 12, 21, 3, 2),       # whole pieces, but one column a thread
+    (1, 1, 5, 260, 2, 1),       # more columns than threads, D odd
+    (1, 1, 6, 1032, 2, 3),      # ... four a thread
+])
+def test_token_states(heads, groups, state, vdim, conv, norm_groups, dtype):
+    """Tokens one by one, the state-space and the delta recurrence in turn."""
+    cfg = zc.config([zc.mam(heads, groups, state, vdim, conv, norm_groups), zc.par(right=(heads, groups, state, vdim), conv=conv, ff=0)],
+                    width=72, vocab=151, emb=1.0)
+    w = zc.Weights(cfg, 7)
+    toks = zc.tokens(cfg, 9, 2)
+    want = orc.forward(cfg, w.f64(), toks)
+    m = make(cfg, w, dtype, 16)
+    m.capture()
+    got = run(m, toks, [])
+    assert np.isfinite(got).all() and ok(err(got, want), dtype)
+    close(m)
