@@ -14,14 +14,15 @@
 // accumulators for the whole pass.
 //
 //   delta_solve   (chunk, head): T of every chunk, in two planes
-//   recur_chunk   (32 or 16 value columns, head, segment): a segment's chunks in order
+//   delta_chunk   (32 or 16 value columns, head): the chunks in order
+//   ssd_chunk     (32 value columns, head, segment): a segment's chunks in order
 //   ssd_state     the same grid: what a segment adds to the state, without its outputs
 //
 // The delta rule is one segment.  The state of ssd only decays by a scalar between two places, so a long prompt
 // is cut into segments that run at once: ssd_state first leaves each segment's own state and log decay, and
-// recur_chunk starts from what the segments in front add up to.  One walk over the chunks has four warps an SM
-// and waits on its own latencies; two CTAs an SM and the second, shorter walk take less: 4096 tokens, 64 heads of
-// 128 x 64, 320 us in one walk, 53 + 227 us in eight segments.
+// ssd_chunk starts from what the segments in front add up to.  One walk over the chunks has four warps an SM
+// and waits on its own latencies; three CTAs an SM and the second, shorter walk take less: 4096 tokens, 64 heads of
+// 128 x 64, 53 + 174 us in three segments (320 in one walk; with two CTAs an SM and both buffers doubled 53 + 228 in eight).
 #include "mixers.cuh"
 #include "rows_mma.cuh"
 
@@ -149,8 +150,8 @@ __global__ void __launch_bounds__(RC_THREADS) delta_solve_kernel(const __grid_co
   }
 }
 
-// ---- the chunks of one head and CE value columns -----------------------------------------------
-template <int DP, bool DELTA, int CE>
+// ---- delta rule: the chunks of one head and CE value columns -----------------------------------------------
+template <int DP, int CE>
 struct RcSmem {
   static constexpr int LD = DP + 8;
   static constexpr size_t K = 0;                                            // [2][64][LD]
@@ -158,26 +159,18 @@ struct RcSmem {
   static constexpr size_t X = Q + (size_t)2 * RC_L * LD * 2;                // [2][64][ELD]
   static constexpr size_t S = X + (size_t)2 * RC_L * (CE + 8) * 2;            // [2 planes][DP][ELD]
   static constexpr size_t W = S + (size_t)2 * DP * (CE + 8) * 2;              // [2 planes][64][ELD]
-  static constexpr size_t U = W + (size_t)2 * RC_L * (CE + 8) * 2;            // delta: [2 planes][64][ELD]
-  static constexpr size_t T = U + (DELTA ? (size_t)2 * RC_L * (CE + 8) * 2 : 0);   // delta: [2][2 planes][64][TLD]
-  static constexpr size_t SC = T + (DELTA ? (size_t)4 * RC_L * RC_TLD * 2 : 0);  // [4][64] f32
-  static constexpr size_t TOTAL = SC + 4 * RC_L * 4;
+  static constexpr size_t U = W + (size_t)2 * RC_L * (CE + 8) * 2;            // [2 planes][64][ELD]
+  static constexpr size_t T = U + (size_t)2 * RC_L * (CE + 8) * 2;            // [2][2 planes][64][TLD]
+  static constexpr size_t SC = T + (size_t)4 * RC_L * RC_TLD * 2;             // [3][64] f32
+  static constexpr size_t TOTAL = SC + 3 * RC_L * 4;
 };
 
-// Segments of `chunks` chunks each.  carry [segments][H][D][E]: the state in front of the prompt, then every
-// segment's own but the last; decay [segments][H]: its log decay.  One segment: no carry.
-struct RcSegments {
-  int n, chunks;
-  float *carry, *decay;
-};
-
-template <int DP, bool DELTA, int CE>
-__global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
-    recur_chunk_kernel(const __grid_constant__ RecurP p, const __nv_bfloat16* __restrict__ conv,
+template <int DP, int CE>
+__global__ void __launch_bounds__(RC_THREADS, 1)
+    delta_chunk_kernel(const __grid_constant__ RecurP p, const __nv_bfloat16* __restrict__ conv,
                        const float2* __restrict__ gates, const float2* __restrict__ norms,
-                       const __nv_bfloat16* __restrict__ T, float* __restrict__ o, int rows, int pos0,
-                       const __grid_constant__ RcSegments g) {
-  using SM = RcSmem<DP, DELTA, CE>;
+                       const __nv_bfloat16* __restrict__ T, float* __restrict__ o, int rows, int pos0) {
+  using SM = RcSmem<DP, CE>;
   constexpr int LD = SM::LD, MT = DP / 64, NT = CE / 8;   // state row tiles of 16 per warp, column tiles
   extern __shared__ __align__(16) unsigned char smem[];
   __nv_bfloat16* ksm = (__nv_bfloat16*)(smem + SM::K);
@@ -188,12 +181,11 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
   __nv_bfloat16* usm = (__nv_bfloat16*)(smem + SM::U);
   __nv_bfloat16* tsm = (__nv_bfloat16*)(smem + SM::T);
   float* sb = (float*)(smem + SM::SC);          // b_t
-  float* sg = sb + RC_L;                        // dt_s of ssd
-  float* snk = sg + RC_L;                       // 1 / |k_s|
+  float* snk = sb + RC_L;                       // 1 / |k_s|
   float* snq = snk + RC_L;                      // D^-1/2 / |q_t|
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wr = warp * 16;
   const int h = blockIdx.y, c0 = blockIdx.x * CE, kg = h / (p.H / p.G), D = p.D, E = p.E;
-  const int nch = (rows + RC_L - 1) / RC_L, ch0 = (int)blockIdx.z * g.chunks, ch1 = ch0 + g.chunks < nch ? ch0 + g.chunks : nch;
+  const int nch = (rows + RC_L - 1) / RC_L;
   const int dch = D / 8, ech = (E - c0 < CE ? E - c0 : CE) / 8;
   for (int i = tid; i < (int)(SM::SC / 16); i += RC_THREADS) ((uint4*)smem)[i] = make_uint4(0, 0, 0, 0);
   pdl_wait();
@@ -213,11 +205,9 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
       const bool on = r < n;
       rc_cp16(xsm + (buf * RC_L + r) * (CE + 8) + c * 8, conv + (size_t)(on ? t0 + r : t0) * p.cv.C + p.cvv + h * E + c0 + c * 8, on);
     }
-    if (DELTA) {
-      const __nv_bfloat16* src = T + ((size_t)ch * p.H + h) * 2 * RC_L * RC_L;
-      for (int i = tid; i < 2 * RC_L * 8; i += RC_THREADS)
-        rc_cp16(tsm + ((size_t)buf * 2 * RC_L + (i >> 3)) * RC_TLD + (i & 7) * 8, src + (size_t)i * 8, true);
-    }
+    const __nv_bfloat16* src = T + ((size_t)ch * p.H + h) * 2 * RC_L * RC_L;
+    for (int i = tid; i < 2 * RC_L * 8; i += RC_THREADS)
+      rc_cp16(tsm + ((size_t)buf * 2 * RC_L + (i >> 3)) * RC_TLD + (i & 7) * 8, src + (size_t)i * 8, true);
   };
   // warp 0 carries the next chunk's scalars in registers (tokens lane and lane + 32)
   float2 g0, g1, n0, n1;
@@ -226,10 +216,8 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
     const float2 z = make_float2(0.f, 0.f);
     g0 = t0 < rows ? gates[(size_t)t0 * p.H + h] : z;
     g1 = t1 < rows ? gates[(size_t)t1 * p.H + h] : z;
-    if (DELTA) {
-      n0 = t0 < rows ? norms[(size_t)t0 * p.G + kg] : z;
-      n1 = t1 < rows ? norms[(size_t)t1 * p.G + kg] : z;
-    }
+    n0 = t0 < rows ? norms[(size_t)t0 * p.G + kg] : z;
+    n1 = t1 < rows ? norms[(size_t)t1 * p.G + kg] : z;
   };
   // state: this warp's rows of it, CE columns, as accumulators
   float s[MT][NT][4];
@@ -246,33 +234,13 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
       for (int e = 0; e < 4; e++) {
         int r, c;
         state_at(mt, nt, e, r, c);
-        s[mt][nt][e] = pos0 > 0 && g.n == 1 && r < D && c < E ? S[(size_t)r * E + c] : 0.f;
+        s[mt][nt][e] = pos0 > 0 && r < D && c < E ? S[(size_t)r * E + c] : 0.f;
       }
-  if (!DELTA && g.n > 1) {
-    const size_t HS = (size_t)p.H * D * E;
-    for (int j = pos0 > 0 ? 0 : 1; j <= (int)blockIdx.z; j++) {
-      const float* C = g.carry + j * HS + (size_t)h * D * E;
-      const float f = j > 0 ? expf(g.decay[(j - 1) * p.H + h]) : 0.f;
-#pragma unroll
-      for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-        for (int nt = 0; nt < NT; nt++)
-#pragma unroll
-          for (int e = 0; e < 4; e += 2) {
-            int r, c;
-            state_at(mt, nt, e, r, c);
-            if (r >= D || c >= E) continue;   // E is even
-            const float2 v = __ldcg((const float2*)(C + (size_t)r * E + c));
-            s[mt][nt][e] = fmaf(f, s[mt][nt][e], v.x);
-            s[mt][nt][e + 1] = fmaf(f, s[mt][nt][e + 1], v.y);
-          }
-    }
-  }
-  fetch(ch0, 0);
+  fetch(0, 0);
   rc_commit();
-  if (warp == 0) scalars(ch0);
-  for (int ch = ch0; ch < ch1; ch++) {
-    const int buf = (ch - ch0) & 1, t0 = ch * RC_L, n = rows - t0 < RC_L ? rows - t0 : RC_L;
+  if (warp == 0) scalars(0);
+  for (int ch = 0; ch < nch; ch++) {
+    const int buf = ch & 1, t0 = ch * RC_L, n = rows - t0 < RC_L ? rows - t0 : RC_L;
     // the state in front of the chunk, in two planes, for the products below
 #pragma unroll
     for (int mt = 0; mt < MT; mt++)
@@ -290,13 +258,12 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
       float b0, b1;
       rc_scan(g0.y, g1.y, b0, b1);
       sb[lane] = b0; sb[lane + 32] = b1;
-      sg[lane] = g0.x; sg[lane + 32] = g1.x;
-      if (DELTA) { snk[lane] = n0.y; snk[lane + 32] = n1.y; snq[lane] = n0.x; snq[lane + 32] = n1.x; }
-      if (ch + 1 < ch1) scalars(ch + 1);
+      snk[lane] = n0.y; snk[lane + 32] = n1.y; snq[lane] = n0.x; snq[lane + 32] = n1.x;
+      if (ch + 1 < nch) scalars(ch + 1);
     }
     rc_wait<0>();
     __syncthreads();
-    if (ch + 1 < ch1) {
+    if (ch + 1 < nch) {
       fetch(ch + 1, buf ^ 1);
       rc_commit();
     }
@@ -316,7 +283,7 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
     for (int k = 0; k < DP; k += 16) {
       uint32_t aq[4], ak[4];
       rc_ldm(aq, rc_a(Q, LD, wr, k, lane));
-      if (DELTA) rc_ldm(ak, rc_a(K, LD, wr, k, lane));
+      rc_ldm(ak, rc_a(K, LD, wr, k, lane));
       uint32_t bs[2][CE / 16][4], bk[4][4];   // all of a step's fragments first: one shared-memory latency a step
 #pragma unroll
       for (int pl = 0; pl < 2; pl++)
@@ -331,10 +298,8 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
         for (int j = 0; j < CE / 16; j++) {
           rc_mma(qs[2 * j], aq, bs[pl][j][0], bs[pl][j][1]);
           rc_mma(qs[2 * j + 1], aq, bs[pl][j][2], bs[pl][j][3]);
-          if (DELTA) {
-            rc_mma(kS[2 * j], ak, bs[pl][j][0], bs[pl][j][1]);
-            rc_mma(kS[2 * j + 1], ak, bs[pl][j][2], bs[pl][j][3]);
-          }
+          rc_mma(kS[2 * j], ak, bs[pl][j][0], bs[pl][j][1]);
+          rc_mma(kS[2 * j + 1], ak, bs[pl][j][2], bs[pl][j][3]);
         }
 #pragma unroll
       for (int j = 0; j < 4; j++)
@@ -343,108 +308,89 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
           rc_mma(m[2 * j + 1], aq, bk[j][2], bk[j][3]);
         }
     }
-    // decays (and unit norms, step sizes) of q k^T, then as operand planes
+    // decays and unit norms of q k^T, then as operand planes
     uint32_t mh[4][4], ml[4][4];
-    const float qa = DELTA ? snq[ra] : 1.f, qb = DELTA ? snq[ra + 8] : 1.f;
+    const float qa = snq[ra], qb = snq[ra + 8];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       float w[4];
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         const int c = j * 8 + cb + (e & 1), t = e < 2 ? ra : ra + 8;
-        const float f = c <= t ? expf((e < 2 ? ba : bb) - sb[c]) * (DELTA ? snk[c] * (e < 2 ? qa : qb) : sg[c]) : 0.f;
+        const float f = c <= t ? expf((e < 2 ? ba : bb) - sb[c]) * (snk[c] * (e < 2 ? qa : qb)) : 0.f;
         w[e] = j <= 2 * warp + 1 ? m[j][e] * f : 0.f;
       }
       rc_split(w[0], w[1], mh[j >> 1][(j & 1) * 2], ml[j >> 1][(j & 1) * 2]);
       rc_split(w[2], w[3], mh[j >> 1][(j & 1) * 2 + 1], ml[j >> 1][(j & 1) * 2 + 1]);
     }
-    if (DELTA) {
-      // R = v - exp(b) |k|^-1 (k S), in planes
-      const float fa = expf(ba) * snk[ra], fb = expf(bb) * snk[ra + 8];
+    // R = v - exp(b) |k|^-1 (k S), in planes
+    const float fa = expf(ba) * snk[ra], fb = expf(bb) * snk[ra + 8];
 #pragma unroll
-      for (int j = 0; j < NT; j++)
+    for (int j = 0; j < NT; j++)
 #pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
-          const uint32_t v = *(const uint32_t*)(X + at);
-          const float f = e ? fb : fa;
-          uint32_t hi, lo;
-          rc_split(fmaf(-f, kS[j][2 * e], __uint_as_float(v << 16)),
-                   fmaf(-f, kS[j][2 * e + 1], __uint_as_float(v & 0xffff0000u)), hi, lo);
-          *(uint32_t*)(usm + at) = hi;
-          *(uint32_t*)(usm + RC_L * (CE + 8) + at) = lo;
+      for (int e = 0; e < 2; e++) {
+        const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
+        const uint32_t v = *(const uint32_t*)(X + at);
+        const float f = e ? fb : fa;
+        uint32_t hi, lo;
+        rc_split(fmaf(-f, kS[j][2 * e], __uint_as_float(v << 16)),
+                 fmaf(-f, kS[j][2 * e + 1], __uint_as_float(v & 0xffff0000u)), hi, lo);
+        *(uint32_t*)(usm + at) = hi;
+        *(uint32_t*)(usm + RC_L * (CE + 8) + at) = lo;
+      }
+    __syncthreads();
+    float u[NT][4];
+#pragma unroll
+    for (int i = 0; i < NT; i++) u[i][0] = u[i][1] = u[i][2] = u[i][3] = 0.f;
+    const __nv_bfloat16* Tp = tsm + (size_t)buf * 2 * RC_L * RC_TLD;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (k <= warp) {
+        uint32_t ah[4], al[4];
+        rc_ldm(ah, rc_a(Tp, RC_TLD, wr, k * 16, lane));
+        rc_ldm(al, rc_a(Tp + RC_L * RC_TLD, RC_TLD, wr, k * 16, lane));
+#pragma unroll
+        for (int j = 0; j < CE / 16; j++) {
+          uint32_t bh[4], bl[4];
+          rc_ldmt(bh, rc_bk(usm, (CE + 8), k * 16, j * 16, lane));
+          rc_ldmt(bl, rc_bk(usm + RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
+          rc_mma(u[2 * j], ah, bh[0], bh[1]); rc_mma(u[2 * j + 1], ah, bh[2], bh[3]);
+          rc_mma(u[2 * j], ah, bl[0], bl[1]); rc_mma(u[2 * j + 1], ah, bl[2], bl[3]);
+          rc_mma(u[2 * j], al, bh[0], bh[1]); rc_mma(u[2 * j + 1], al, bh[2], bh[3]);
         }
-      __syncthreads();
-      float u[NT][4];
+      }
+    __syncthreads();   // R is read: its planes become U's
+    const float ga = expf(bL - ba) * snk[ra], gb = expf(bL - bb) * snk[ra + 8];
 #pragma unroll
-      for (int i = 0; i < NT; i++) u[i][0] = u[i][1] = u[i][2] = u[i][3] = 0.f;
-      const __nv_bfloat16* Tp = tsm + (size_t)buf * 2 * RC_L * RC_TLD;
+    for (int j = 0; j < NT; j++)
 #pragma unroll
-      for (int k = 0; k < 4; k++)
-        if (k <= warp) {
-          uint32_t ah[4], al[4];
-          rc_ldm(ah, rc_a(Tp, RC_TLD, wr, k * 16, lane));
-          rc_ldm(al, rc_a(Tp + RC_L * RC_TLD, RC_TLD, wr, k * 16, lane));
-#pragma unroll
-          for (int j = 0; j < CE / 16; j++) {
-            uint32_t bh[4], bl[4];
-            rc_ldmt(bh, rc_bk(usm, (CE + 8), k * 16, j * 16, lane));
-            rc_ldmt(bl, rc_bk(usm + RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
-            rc_mma(u[2 * j], ah, bh[0], bh[1]); rc_mma(u[2 * j + 1], ah, bh[2], bh[3]);
-            rc_mma(u[2 * j], ah, bl[0], bl[1]); rc_mma(u[2 * j + 1], ah, bl[2], bl[3]);
-            rc_mma(u[2 * j], al, bh[0], bh[1]); rc_mma(u[2 * j + 1], al, bh[2], bh[3]);
-          }
-        }
-      __syncthreads();   // R is read: its planes become U's
-      const float ga = expf(bL - ba) * snk[ra], gb = expf(bL - bb) * snk[ra + 8];
-#pragma unroll
-      for (int j = 0; j < NT; j++)
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
-          const float f = e ? gb : ga;
-          uint32_t hi, lo;
-          rc_split(u[j][2 * e], u[j][2 * e + 1], hi, lo);
-          *(uint32_t*)(usm + at) = hi;
-          *(uint32_t*)(usm + RC_L * (CE + 8) + at) = lo;
-          rc_split(u[j][2 * e] * f, u[j][2 * e + 1] * f, hi, lo);
-          *(uint32_t*)(wsm + at) = hi;
-          *(uint32_t*)(wsm + RC_L * (CE + 8) + at) = lo;
-        }
-    } else {
-      const float ga = expf(bL - ba) * sg[ra], gb = expf(bL - bb) * sg[ra + 8];
-#pragma unroll
-      for (int j = 0; j < NT; j++)
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
-          const uint32_t v = *(const uint32_t*)(X + at);
-          const float f = e ? gb : ga;
-          uint32_t hi, lo;
-          rc_split(f * __uint_as_float(v << 16), f * __uint_as_float(v & 0xffff0000u), hi, lo);
-          *(uint32_t*)(wsm + at) = hi;
-          *(uint32_t*)(wsm + RC_L * (CE + 8) + at) = lo;
-        }
-    }
+      for (int e = 0; e < 2; e++) {
+        const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
+        const float f = e ? gb : ga;
+        uint32_t hi, lo;
+        rc_split(u[j][2 * e], u[j][2 * e + 1], hi, lo);
+        *(uint32_t*)(usm + at) = hi;
+        *(uint32_t*)(usm + RC_L * (CE + 8) + at) = lo;
+        rc_split(u[j][2 * e] * f, u[j][2 * e + 1] * f, hi, lo);
+        *(uint32_t*)(wsm + at) = hi;
+        *(uint32_t*)(wsm + RC_L * (CE + 8) + at) = lo;
+      }
     __syncthreads();
     // O = exp(b) (q S) + M U
     const float ea = expf(ba) * qa, eb = expf(bb) * qb;
 #pragma unroll
     for (int j = 0; j < NT; j++) { qs[j][0] *= ea; qs[j][1] *= ea; qs[j][2] *= eb; qs[j][3] *= eb; }
-    const __nv_bfloat16* Up = DELTA ? usm : X;
 #pragma unroll
     for (int k = 0; k < 4; k++)
       if (k <= warp) {
 #pragma unroll
         for (int j = 0; j < CE / 16; j++) {
           uint32_t b[4];
-          rc_ldmt(b, rc_bk(Up, (CE + 8), k * 16, j * 16, lane));
+          rc_ldmt(b, rc_bk(usm, (CE + 8), k * 16, j * 16, lane));
           rc_mma(qs[2 * j], mh[k], b[0], b[1]); rc_mma(qs[2 * j + 1], mh[k], b[2], b[3]);
           rc_mma(qs[2 * j], ml[k], b[0], b[1]); rc_mma(qs[2 * j + 1], ml[k], b[2], b[3]);
-          if (DELTA) {
-            rc_ldmt(b, rc_bk(usm + RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
-            rc_mma(qs[2 * j], mh[k], b[0], b[1]); rc_mma(qs[2 * j + 1], mh[k], b[2], b[3]);
-          }
+          rc_ldmt(b, rc_bk(usm + RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
+          rc_mma(qs[2 * j], mh[k], b[0], b[1]); rc_mma(qs[2 * j + 1], mh[k], b[2], b[3]);
         }
       }
 #pragma unroll
@@ -486,6 +432,268 @@ __global__ void __launch_bounds__(RC_THREADS, DELTA ? 1 : 2)
           }
     }
     __syncthreads();   // the chunk's operands and planes are read: the next one may overwrite them
+  }
+#pragma unroll
+  for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        int r, c;
+        state_at(mt, nt, e, r, c);
+        if (r < D && c < E) S[(size_t)r * E + c] = s[mt][nt][e];
+      }
+}
+
+// ---- ssd: the chunks of one head and 32 value columns ------------------------------------------------
+// The walk waits on its own latencies (mma.sync fragments, barriers, exponentials), so what counts is CTAs an SM: three,
+// with every operand once in shared memory.  The next chunk's rows come as their places fall free: q behind q k^T, k
+// behind the state's update, which is done before the outputs for that, x behind the next chunk's first barrier.
+// Segments of `chunks` chunks each.  carry [segments][H][D][E]: the state in front of the prompt, then every
+// segment's own but the last; decay [segments][H]: its log decay.  One segment: no carry.
+struct RcSegments {
+  int n, chunks;
+  float *carry, *decay;
+};
+
+template <int DP>
+struct ScSmem {
+  static constexpr int LD = DP + 8;
+  static constexpr size_t K = 0;                                            // [64][LD]
+  static constexpr size_t Q = K + (size_t)RC_L * LD * 2;
+  static constexpr size_t X = Q + (size_t)RC_L * LD * 2;                    // [64][ELD]
+  static constexpr size_t S = X + (size_t)RC_L * RC_ELD * 2;                // [2 planes][DP][ELD]
+  static constexpr size_t W = S + (size_t)2 * DP * RC_ELD * 2;              // [2 planes][64][ELD]
+  static constexpr size_t SC = W + (size_t)2 * RC_L * RC_ELD * 2;           // [2][64] f32
+  static constexpr size_t TOTAL = SC + 2 * RC_L * 4;
+};
+
+template <int DP>
+__global__ void __launch_bounds__(RC_THREADS, 3)
+    ssd_chunk_kernel(const __grid_constant__ RecurP p, const __nv_bfloat16* __restrict__ conv,
+                     const float2* __restrict__ gates, float* __restrict__ o, int rows, int pos0,
+                     const __grid_constant__ RcSegments g) {
+  using SM = ScSmem<DP>;
+  constexpr int LD = SM::LD, MT = DP / 64, NT = RC_E / 8;   // state row tiles of 16 per warp, column tiles
+  extern __shared__ __align__(16) unsigned char smem[];
+  __nv_bfloat16* K = (__nv_bfloat16*)(smem + SM::K);
+  __nv_bfloat16* Q = (__nv_bfloat16*)(smem + SM::Q);
+  __nv_bfloat16* X = (__nv_bfloat16*)(smem + SM::X);
+  __nv_bfloat16* ssm = (__nv_bfloat16*)(smem + SM::S);
+  __nv_bfloat16* wsm = (__nv_bfloat16*)(smem + SM::W);
+  float* sb = (float*)(smem + SM::SC);          // b_t
+  float* sg = sb + RC_L;                        // dt_s
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wr = warp * 16;
+  const int h = blockIdx.y, c0 = blockIdx.x * RC_E, kg = h / (p.H / p.G), D = p.D, E = p.E;
+  const int nch = (rows + RC_L - 1) / RC_L, ch0 = (int)blockIdx.z * g.chunks, ch1 = ch0 + g.chunks < nch ? ch0 + g.chunks : nch;
+  const int dch = D / 8, ech = (E - c0 < RC_E ? E - c0 : RC_E) / 8;
+  for (int i = tid; i < (int)(SM::SC / 16); i += RC_THREADS) ((uint4*)smem)[i] = make_uint4(0, 0, 0, 0);
+  pdl_wait();
+  pdl_launch_dependents();
+  __syncthreads();
+  // rows of a chunk, `chunks` pieces of 16 bytes each, from column `at` on (zeros behind the last row)
+  auto fetch = [&](__nv_bfloat16* dst, int ld, int at, int chunks, int ch) {
+    const int t0 = ch * RC_L, n = rows - t0 < RC_L ? rows - t0 : RC_L;
+    for (int i = tid; i < RC_L * chunks; i += RC_THREADS) {
+      const int r = i / chunks, c = i - r * chunks;
+      rc_cp16(dst + r * ld + c * 8, conv + (size_t)(r < n ? t0 + r : t0) * p.cv.C + at + c * 8, r < n);
+    }
+    rc_commit();
+  };
+  // warp 0 carries the next chunk's scalars in registers (tokens lane and lane + 32)
+  float2 g0, g1;
+  auto scalars = [&](int ch) {
+    const int t0 = ch * RC_L + lane, t1 = t0 + 32;
+    const float2 z = make_float2(0.f, 0.f);
+    g0 = t0 < rows ? gates[(size_t)t0 * p.H + h] : z;
+    g1 = t1 < rows ? gates[(size_t)t1 * p.H + h] : z;
+  };
+  fetch(Q, LD, p.cq + kg * D, dch, ch0);
+  fetch(K, LD, p.ck + kg * D, dch, ch0);
+  if (warp == 0) scalars(ch0);
+  // state: this warp's rows of it, 32 columns, as accumulators
+  float s[MT][NT][4];
+  float* S = p.S + (size_t)h * D * E;
+  auto state_at = [&](int mt, int nt, int e, int& r, int& c) {
+    r = (warp * MT + mt) * 16 + (lane >> 2) + (e >> 1) * 8;
+    c = c0 + nt * 8 + (lane & 3) * 2 + (e & 1);
+  };
+#pragma unroll
+  for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        int r, c;
+        state_at(mt, nt, e, r, c);
+        s[mt][nt][e] = pos0 > 0 && g.n == 1 && r < D && c < E ? S[(size_t)r * E + c] : 0.f;
+      }
+  if (g.n > 1) {
+    const size_t HS = (size_t)p.H * D * E;
+    for (int j = pos0 > 0 ? 0 : 1; j <= (int)blockIdx.z; j++) {
+      const float* C = g.carry + j * HS + (size_t)h * D * E;
+      const float f = j > 0 ? expf(g.decay[(j - 1) * p.H + h]) : 0.f;
+#pragma unroll
+      for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) {
+            int r, c;
+            state_at(mt, nt, e, r, c);
+            if (r >= D || c >= E) continue;   // E is even
+            const float2 v = __ldcg((const float2*)(C + (size_t)r * E + c));
+            s[mt][nt][e] = fmaf(f, s[mt][nt][e], v.x);
+            s[mt][nt][e + 1] = fmaf(f, s[mt][nt][e + 1], v.y);
+          }
+    }
+  }
+  for (int ch = ch0; ch < ch1; ch++) {
+    const int t0 = ch * RC_L, n = rows - t0 < RC_L ? rows - t0 : RC_L;
+    // the state in front of the chunk, in two planes, for the products below
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+      for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          uint32_t hi, lo;
+          rc_split(s[mt][nt][2 * e], s[mt][nt][2 * e + 1], hi, lo);
+          const int at = ((warp * MT + mt) * 16 + (lane >> 2) + e * 8) * RC_ELD + nt * 8 + (lane & 3) * 2;
+          *(uint32_t*)(ssm + at) = hi;
+          *(uint32_t*)(ssm + DP * RC_ELD + at) = lo;
+        }
+    if (warp == 0) {
+      float b0, b1;
+      rc_scan(g0.y, g1.y, b0, b1);
+      sb[lane] = b0; sb[lane + 32] = b1;
+      sg[lane] = g0.x; sg[lane + 32] = g1.x;
+      if (ch + 1 < ch1) scalars(ch + 1);
+    }
+    rc_wait<0>();
+    __syncthreads();   // q, k and the state's planes are there; x of the chunk before is read
+    fetch(X, RC_ELD, p.cvv + h * E + c0, ech, ch);
+    const int ra = wr + (lane >> 2), cb = (lane & 3) * 2;     // the thread's rows are ra and ra + 8
+    const float ba = sb[ra], bb = sb[ra + 8], bL = sb[RC_L - 1];
+    const float ga = expf(bL - ba) * sg[ra], gb = expf(bL - bb) * sg[ra + 8];
+    // q S (both planes of S), q k^T for the rows of this warp
+    float qs[NT][4], m[8][4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+#pragma unroll
+      for (int i = 0; i < NT; i++) qs[i][e] = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; i++) m[i][e] = 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < DP; k += 16) {
+      uint32_t aq[4], bs[2][2][4], bk[4][4];   // all of a step's fragments first: one shared-memory latency a step
+      rc_ldm(aq, rc_a(Q, LD, wr, k, lane));
+#pragma unroll
+      for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) rc_ldmt(bs[pl][j], rc_bk(ssm + pl * DP * RC_ELD, RC_ELD, k, j * 16, lane));
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (j <= warp) rc_ldm(bk[j], rc_bn(K, LD, j * 16, k, lane));
+#pragma unroll
+      for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          rc_mma(qs[2 * j], aq, bs[pl][j][0], bs[pl][j][1]);
+          rc_mma(qs[2 * j + 1], aq, bs[pl][j][2], bs[pl][j][3]);
+        }
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (j <= warp) {
+          rc_mma(m[2 * j], aq, bk[j][0], bk[j][1]);
+          rc_mma(m[2 * j + 1], aq, bk[j][2], bk[j][3]);
+        }
+    }
+    // decays and step sizes of q k^T, then as operand planes
+    uint32_t mh[4][4], ml[4][4];
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      if (j <= 2 * warp + 1) {
+        float w[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const int c = j * 8 + cb + (e & 1), t = e < 2 ? ra : ra + 8;
+          w[e] = c <= t ? m[j][e] * (expf((e < 2 ? ba : bb) - sb[c]) * sg[c]) : 0.f;
+        }
+        rc_split(w[0], w[1], mh[j >> 1][(j & 1) * 2], ml[j >> 1][(j & 1) * 2]);
+        rc_split(w[2], w[3], mh[j >> 1][(j & 1) * 2 + 1], ml[j >> 1][(j & 1) * 2 + 1]);
+      }
+    rc_wait<0>();
+    __syncthreads();   // x is there, q is read
+    if (ch + 1 < ch1) fetch(Q, LD, p.cq + kg * D, dch, ch + 1);
+#pragma unroll
+    for (int j = 0; j < NT; j++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int at = (ra + 8 * e) * RC_ELD + j * 8 + cb;
+        const uint32_t v = *(const uint32_t*)(X + at);
+        const float f = e ? gb : ga;
+        uint32_t hi, lo;
+        rc_split(f * __uint_as_float(v << 16), f * __uint_as_float(v & 0xffff0000u), hi, lo);
+        *(uint32_t*)(wsm + at) = hi;
+        *(uint32_t*)(wsm + RC_L * RC_ELD + at) = lo;
+      }
+    __syncthreads();
+    // S = exp(b_L) S + K^T (weighted x)
+    const float eL = expf(bL);
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+      for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) s[mt][nt][e] *= eL;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      uint32_t a[MT][4], b[2][2][4];
+#pragma unroll
+      for (int mt = 0; mt < MT; mt++) rc_ldmt(a[mt], rc_at(K, LD, (warp * MT + mt) * 16, k * 16, lane));
+#pragma unroll
+      for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) rc_ldmt(b[pl][j], rc_bk(wsm + pl * RC_L * RC_ELD, RC_ELD, k * 16, j * 16, lane));
+#pragma unroll
+      for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+          for (int mt = 0; mt < MT; mt++) {
+            rc_mma(s[mt][2 * j], a[mt], b[pl][j][0], b[pl][j][1]);
+            rc_mma(s[mt][2 * j + 1], a[mt], b[pl][j][2], b[pl][j][3]);
+          }
+    }
+    __syncthreads();   // k and the weighted x are read
+    if (ch + 1 < ch1) fetch(K, LD, p.ck + kg * D, dch, ch + 1);
+    // O = exp(b) (q S) + M x
+    const float ea = expf(ba), eb = expf(bb);
+#pragma unroll
+    for (int j = 0; j < NT; j++) { qs[j][0] *= ea; qs[j][1] *= ea; qs[j][2] *= eb; qs[j][3] *= eb; }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (k <= warp) {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          uint32_t b[4];
+          rc_ldmt(b, rc_bk(X, RC_ELD, k * 16, j * 16, lane));
+          rc_mma(qs[2 * j], mh[k], b[0], b[1]); rc_mma(qs[2 * j + 1], mh[k], b[2], b[3]);
+          rc_mma(qs[2 * j], ml[k], b[0], b[1]); rc_mma(qs[2 * j + 1], ml[k], b[2], b[3]);
+        }
+      }
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int t = ra + 8 * e;
+      if (t < n) {
+        float* dst = o + ((size_t)(t0 + t) * p.H + h) * E + c0;
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+          if (j < ech) *(float2*)(dst + j * 8 + cb) = make_float2(qs[j][2 * e], qs[j][2 * e + 1]);
+      }
+    }
   }
   if ((int)blockIdx.z != g.n - 1) return;
 #pragma unroll
@@ -635,70 +843,91 @@ __global__ void __launch_bounds__(RC_THREADS, 3)
 }
 
 // Most segments of a prompt (more rows, no fewer): of four chunks at least, since a segment's start reads the states in
-// front of it, eight at most, and no more than four CTAs for each of the SMs' places, two an SM.
+// front of it, eight at most, and no more than four CTAs for each of two places an SM.
 int rc_most_segments(const RecurP& p, int rows, int sms) {
-  if (p.kind == MIX_DELTA) return 1;
   const int nch = (rows + RC_L - 1) / RC_L, ctas = (p.E + RC_E - 1) / RC_E * p.H;
   int n = nch / 4 < RC_MOST ? nch / 4 : RC_MOST;
   if (n * ctas > 4 * 2 * sms) n = 4 * 2 * sms / ctas;
   return n < 2 ? 1 : n;
 }
+// Up to that many, by what they cost: both kernels run in waves of three CTAs an SM, a wave as long as a segment's chunks
+// and a start of 1.5 chunks; a chunk of ssd_state takes 0.3 of one of ssd_chunk.  4096 tokens, 64 heads of 128 x 64, the
+// 8-layer prompt pass with six such layers, us: 2 segments 6931, 3 6470, 4 6816, 6 6536, 8 6610, 10 6527, 13 6674, 16 6884.
 RcSegments rc_segments(const RecurP& p, int rows, int sms, void* scratch) {
-  const int nch = (rows + RC_L - 1) / RC_L, n = rc_most_segments(p, rows, sms);
+  const int nch = (rows + RC_L - 1) / RC_L, most = rc_most_segments(p, rows, sms), ctas = (p.E + RC_E - 1) / RC_E * p.H;
   RcSegments g{1, nch, nullptr, nullptr};
-  if (n == 1) return g;
-  g.chunks = (nch + n - 1) / n;
-  g.n = (nch + g.chunks - 1) / g.chunks;
+  long long best = 0;
+  for (int want = 1; want <= most; want++) {
+    const int chunks = (nch + want - 1) / want, n = (nch + chunks - 1) / chunks;
+    auto waves = [&](int segments) { return ((long long)segments * ctas + 3 * sms - 1) / (3 * sms); };
+    const long long cost = (10 * waves(n) + 3 * waves(n - 1)) * (2 * chunks + 3);
+    if (want > 1 && cost >= best) continue;
+    best = cost;
+    g.n = n;
+    g.chunks = chunks;
+  }
+  if (g.n == 1) return g;
   g.carry = (float*)scratch;
   g.decay = g.carry + (size_t)g.n * p.H * p.D * p.E;
   return g;
 }
 
-template <int DP, bool DELTA, int CE>
-int rc_walk(const RecurP& p, const void* conv, const float2* gates, const float2* norms, const void* T, float* o, int rows,
-            int pos0, const RcSegments& g, cudaStream_t s) {
-  constexpr int smem = (int)RcSmem<DP, DELTA, CE>::TOTAL;
+template <int DP, int CE>
+int delta_walk(const RecurP& p, const void* conv, const float2* gates, const float2* norms, const void* T, float* o, int rows,
+               int pos0, cudaStream_t s) {
+  constexpr int smem = (int)RcSmem<DP, CE>::TOTAL;
   static std::atomic<unsigned long long> done{0};
-  const int rc = ensure_dynamic_smem(recur_chunk_kernel<DP, DELTA, CE>, smem, done);
+  const int rc = ensure_dynamic_smem(delta_chunk_kernel<DP, CE>, smem, done);
   if (rc) return rc;
-  LaunchCfg lc(dim3((p.E + CE - 1) / CE, p.H, g.n), dim3(RC_THREADS), smem, s, pdl_enabled());
-  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, recur_chunk_kernel<DP, DELTA, CE>, p, (const __nv_bfloat16*)conv, gates, norms,
-                              (const __nv_bfloat16*)T, o, rows, pos0, g));
+  LaunchCfg lc(dim3((p.E + CE - 1) / CE, p.H), dim3(RC_THREADS), smem, s, pdl_enabled());
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, delta_chunk_kernel<DP, CE>, p, (const __nv_bfloat16*)conv, gates, norms,
+                              (const __nv_bfloat16*)T, o, rows, pos0));
   return TLB_OK;
 }
 
-template <int DP, bool DELTA>
-int rc_launch(const RecurP& p, const void* conv, const float2* gates, const float2* norms, void* T, float* o, int rows,
-              int pos0, cudaStream_t s) {
+template <int DP>
+int delta_launch(const RecurP& p, const void* conv, const float2* gates, const float2* norms, void* T, float* o, int rows,
+                 int pos0, cudaStream_t s) {
   DeviceCtx* c = nullptr;
-  {
-    const int rc = get_ctx(&c);
-    if (rc) return rc;
-  }
-  if (DELTA) {
-    constexpr int smem = RC_L * (DP + 8) * 2 + (2 * RC_L * (RC_L + 1) + 3 * 16 * 17) * 4;
-    static std::atomic<unsigned long long> done{0};
-    const int rc = ensure_dynamic_smem(delta_solve_kernel<DP>, smem, done);
-    if (rc) return rc;
-    LaunchCfg lc(dim3((rows + RC_L - 1) / RC_L, p.H), dim3(RC_THREADS), smem, s, pdl_enabled());
-    TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, delta_solve_kernel<DP>, p, (const __nv_bfloat16*)conv, gates, norms,
-                                (__nv_bfloat16*)T, rows));
-  }
-  const RcSegments g = rc_segments(p, rows, c->sm_count, T);
-  if (!DELTA && g.n > 1) {
-    constexpr int smem = (int)SsSmem<DP>::TOTAL;
-    static std::atomic<unsigned long long> done{0};
-    const int rc = ensure_dynamic_smem(ssd_state_kernel<DP>, smem, done);
-    if (rc) return rc;
-    LaunchCfg lc(dim3((p.E + RC_E - 1) / RC_E, p.H, g.n - 1), dim3(RC_THREADS), smem, s, pdl_enabled());
-    TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, ssd_state_kernel<DP>, p, (const __nv_bfloat16*)conv, gates, pos0, g));
-  }
+  int rc = get_ctx(&c);
+  if (rc) return rc;
+  constexpr int smem = RC_L * (DP + 8) * 2 + (2 * RC_L * (RC_L + 1) + 3 * 16 * 17) * 4;
+  static std::atomic<unsigned long long> done{0};
+  rc = ensure_dynamic_smem(delta_solve_kernel<DP>, smem, done);
+  if (rc) return rc;
+  LaunchCfg lc(dim3((rows + RC_L - 1) / RC_L, p.H), dim3(RC_THREADS), smem, s, pdl_enabled());
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, delta_solve_kernel<DP>, p, (const __nv_bfloat16*)conv, gates, norms,
+                              (__nv_bfloat16*)T, rows));
   // few heads: half as many columns a CTA, twice the CTAs, where those still find an SM each (4096 tokens, 16 heads of
   // 128: 392 us on 64 SMs, 318 on 128)
-  if constexpr (DELTA)
-    if (2 * ((p.E + RC_E - 1) / RC_E * p.H) <= c->sm_count)
-      return rc_walk<DP, DELTA, 16>(p, conv, gates, norms, T, o, rows, pos0, g, s);
-  return rc_walk<DP, DELTA, RC_E>(p, conv, gates, norms, T, o, rows, pos0, g, s);
+  if (2 * ((p.E + RC_E - 1) / RC_E * p.H) <= c->sm_count)
+    return delta_walk<DP, 16>(p, conv, gates, norms, T, o, rows, pos0, s);
+  return delta_walk<DP, RC_E>(p, conv, gates, norms, T, o, rows, pos0, s);
+}
+
+template <int DP>
+int ssd_launch(const RecurP& p, const void* conv, const float2* gates, void* scratch, float* o, int rows, int pos0,
+               cudaStream_t s) {
+  DeviceCtx* c = nullptr;
+  int rc = get_ctx(&c);
+  if (rc) return rc;
+  const RcSegments g = rc_segments(p, rows, c->sm_count, scratch);
+  const unsigned cols = (p.E + RC_E - 1) / RC_E;
+  if (g.n > 1) {
+    constexpr int smem = (int)SsSmem<DP>::TOTAL;
+    static std::atomic<unsigned long long> done{0};
+    rc = ensure_dynamic_smem(ssd_state_kernel<DP>, smem, done);
+    if (rc) return rc;
+    LaunchCfg lc(dim3(cols, p.H, g.n - 1), dim3(RC_THREADS), smem, s, pdl_enabled());
+    TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, ssd_state_kernel<DP>, p, (const __nv_bfloat16*)conv, gates, pos0, g));
+  }
+  constexpr int smem = (int)ScSmem<DP>::TOTAL;
+  static std::atomic<unsigned long long> done{0};
+  rc = ensure_dynamic_smem(ssd_chunk_kernel<DP>, smem, done);
+  if (rc) return rc;
+  LaunchCfg lc(dim3(cols, p.H, g.n), dim3(RC_THREADS), smem, s, pdl_enabled());
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, ssd_chunk_kernel<DP>, p, (const __nv_bfloat16*)conv, gates, o, rows, pos0, g));
+  return TLB_OK;
 }
 
 }  // namespace
@@ -716,10 +945,10 @@ size_t recur_chunk_scratch_bytes(const RecurP& p, int rows) {
 int recur_chunk_launch(const RecurP& p, const void* conv, const float2* gates, const float2* norms, void* scratch,
                        float* o, int rows, int pos0, cudaStream_t s) {
   if (p.kind == MIX_DELTA)
-    return p.D <= 64 ? rc_launch<64, true>(p, conv, gates, norms, scratch, o, rows, pos0, s)
-                     : rc_launch<128, true>(p, conv, gates, norms, scratch, o, rows, pos0, s);
-  return p.D <= 64 ? rc_launch<64, false>(p, conv, gates, norms, scratch, o, rows, pos0, s)
-                   : rc_launch<128, false>(p, conv, gates, norms, scratch, o, rows, pos0, s);
+    return p.D <= 64 ? delta_launch<64>(p, conv, gates, norms, scratch, o, rows, pos0, s)
+                     : delta_launch<128>(p, conv, gates, norms, scratch, o, rows, pos0, s);
+  return p.D <= 64 ? ssd_launch<64>(p, conv, gates, scratch, o, rows, pos0, s)
+                   : ssd_launch<128>(p, conv, gates, scratch, o, rows, pos0, s);
 }
 
 }  // namespace tlb
