@@ -22,7 +22,8 @@
 // is cut into segments that run at once: ssd_state first leaves each segment's own state and log decay, and
 // ssd_chunk starts from what the segments in front add up to.  One walk over the chunks has four warps an SM
 // and waits on its own latencies; three CTAs an SM and the second, shorter walk take less: 4096 tokens, 64 heads of
-// 128 x 64, 53 + 174 us in three segments (320 in one walk; with two CTAs an SM and both buffers doubled 53 + 228 in eight).
+// 128 x 64, 44 + 138 us in three segments (53 + 174 with divisions in the copies and branches around the exponentials; two
+// CTAs an SM, every buffer doubled, 53 + 228 in eight; 320 in one walk).
 #include "mixers.cuh"
 #include "rows_mma.cuh"
 
@@ -47,6 +48,24 @@ __device__ __forceinline__ void rc_scan(float x0, float x1, float& b0, float& b1
   b1 = -x1;
 }
 
+// Rows t0 .. of a chunk (n of its 64, zeros behind them): `chunks` of the CPR 16-byte pieces of a row of shared memory, by
+// RC_THREADS threads.  A thread keeps its piece: no division (those of runtime widths were a third of a chunk's time).
+template <int CPR>
+__device__ __forceinline__ void rc_fetch(__nv_bfloat16* dst, int ld, const __nv_bfloat16* src, long long row, int chunks, int n, int tid) {
+  const int c = tid % CPR;
+  if (c >= chunks) return;
+#pragma unroll
+  for (int i = 0; i < RC_L * CPR / RC_THREADS; i++) {
+    const int r = tid / CPR + i * (RC_THREADS / CPR);
+    rc_cp16(dst + r * ld + c * 8, src + (r < n ? r : 0) * row + c * 8, r < n);
+  }
+}
+// x exp(d) f where `on`, else zero, without a branch around the exponential (a hundred cycles an element with one)
+__device__ __forceinline__ float rc_decayed(float x, float d, float f, bool on) {
+  const float y = x * (expf(on ? d : 0.f) * f);
+  return on ? y : 0.f;
+}
+
 // ---- T of one chunk and head -----------------------------------------------------------------
 template <int DP>
 __global__ void __launch_bounds__(RC_THREADS) delta_solve_kernel(const __grid_constant__ RecurP p,
@@ -68,11 +87,8 @@ __global__ void __launch_bounds__(RC_THREADS) delta_solve_kernel(const __grid_co
   pdl_wait();
   pdl_launch_dependents();
   __syncthreads();
-  const int dch = p.D / 8;
-  for (int i = tid; i < n * dch; i += RC_THREADS) {
-    const int r = i / dch, c = i - r * dch;
-    *(uint4*)(ks + r * LD + c * 8) = *(const uint4*)(conv + (size_t)(t0 + r) * p.cv.C + p.ck + kg * p.D + c * 8);
-  }
+  rc_fetch<DP / 8>(ks, LD, conv + (size_t)t0 * p.cv.C + p.ck + kg * p.D, p.cv.C, p.D / 8, n, tid);
+  rc_commit();
   if (warp == 0) {
     const float2 z = make_float2(0.f, 0.f);
     const float2 g0 = lane < n ? gates[(size_t)(t0 + lane) * p.H + h] : z;
@@ -84,6 +100,7 @@ __global__ void __launch_bounds__(RC_THREADS) delta_solve_kernel(const __grid_co
     sn[lane] = lane < n ? norms[(size_t)(t0 + lane) * p.G + kg].y : 0.f;
     sn[lane + 32] = lane + 32 < n ? norms[(size_t)(t0 + lane + 32) * p.G + kg].y : 0.f;
   }
+  rc_wait<0>();
   __syncthreads();
   float s[8][4];
 #pragma unroll
@@ -151,6 +168,16 @@ __global__ void __launch_bounds__(RC_THREADS) delta_solve_kernel(const __grid_co
 }
 
 // ---- delta rule: the chunks of one head and CE value columns -----------------------------------------------
+// One chunk's state is the next one's input, and what costs is that chain: k S, T R and the state's update, with a barrier
+// between each.  Four warps walk it; four others take q S, q k^T and the outputs beside it, and are behind them by what they
+// have to do alone: named barriers tell them that U is there, and the walk that the state's planes are read.  4096 tokens,
+// 16 heads of 128 x 128: four warps for all of it 326 us, eight 282; without branches around the exponentials and waits for
+// the next chunk's scalars 208, without divisions in the copies 200.
+constexpr int RD_THREADS = 2 * RC_THREADS;
+__device__ __forceinline__ void rd_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }   // the four warps of the state
+// U of a chunk is there (2), its state's planes are read (3): four warps arrive and go on, the others wait
+template <int ID> __device__ __forceinline__ void rd_arrive() { asm volatile("bar.arrive %0, 256;" ::"n"(ID) : "memory"); }
+template <int ID> __device__ __forceinline__ void rd_await() { asm volatile("bar.sync %0, 256;" ::"n"(ID) : "memory"); }
 template <int DP, int CE>
 struct RcSmem {
   static constexpr int LD = DP + 8;
@@ -161,12 +188,12 @@ struct RcSmem {
   static constexpr size_t W = S + (size_t)2 * DP * (CE + 8) * 2;              // [2 planes][64][ELD]
   static constexpr size_t U = W + (size_t)2 * RC_L * (CE + 8) * 2;            // [2 planes][64][ELD]
   static constexpr size_t T = U + (size_t)2 * RC_L * (CE + 8) * 2;            // [2][2 planes][64][TLD]
-  static constexpr size_t SC = T + (size_t)4 * RC_L * RC_TLD * 2;             // [3][64] f32
-  static constexpr size_t TOTAL = SC + 3 * RC_L * 4;
+  static constexpr size_t SC = T + (size_t)4 * RC_L * RC_TLD * 2;             // [2][3][64] f32
+  static constexpr size_t TOTAL = SC + 2 * 3 * RC_L * 4;
 };
 
 template <int DP, int CE>
-__global__ void __launch_bounds__(RC_THREADS, 1)
+__global__ void __launch_bounds__(RD_THREADS, 1)
     delta_chunk_kernel(const __grid_constant__ RecurP p, const __nv_bfloat16* __restrict__ conv,
                        const float2* __restrict__ gates, const float2* __restrict__ norms,
                        const __nv_bfloat16* __restrict__ T, float* __restrict__ o, int rows, int pos0) {
@@ -180,44 +207,34 @@ __global__ void __launch_bounds__(RC_THREADS, 1)
   __nv_bfloat16* wsm = (__nv_bfloat16*)(smem + SM::W);
   __nv_bfloat16* usm = (__nv_bfloat16*)(smem + SM::U);
   __nv_bfloat16* tsm = (__nv_bfloat16*)(smem + SM::T);
-  float* sb = (float*)(smem + SM::SC);          // b_t
-  float* snk = sb + RC_L;                       // 1 / |k_s|
-  float* snq = snk + RC_L;                      // D^-1/2 / |q_t|
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wr = warp * 16;
+  const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) & 3, wr = warp * 16;   // rows of the chunk and of the state
+  const bool outs = tid >= RC_THREADS;
   const int h = blockIdx.y, c0 = blockIdx.x * CE, kg = h / (p.H / p.G), D = p.D, E = p.E;
   const int nch = (rows + RC_L - 1) / RC_L;
   const int dch = D / 8, ech = (E - c0 < CE ? E - c0 : CE) / 8;
-  for (int i = tid; i < (int)(SM::SC / 16); i += RC_THREADS) ((uint4*)smem)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = tid; i < (int)(SM::SC / 16); i += RD_THREADS) ((uint4*)smem)[i] = make_uint4(0, 0, 0, 0);
   pdl_wait();
   pdl_launch_dependents();
   __syncthreads();
+  // (the warps of the state fetch and scan: the others have more to do)
   auto fetch = [&](int ch, int buf) {
     const int t0 = ch * RC_L, n = rows - t0 < RC_L ? rows - t0 : RC_L;
-    for (int i = tid; i < RC_L * dch; i += RC_THREADS) {
-      const int r = i / dch, c = i - r * dch;
-      const bool on = r < n;
-      const __nv_bfloat16* row = conv + (size_t)(on ? t0 + r : t0) * p.cv.C + kg * D + c * 8;
-      rc_cp16(ksm + (buf * RC_L + r) * LD + c * 8, row + p.ck, on);
-      rc_cp16(qsm + (buf * RC_L + r) * LD + c * 8, row + p.cq, on);
-    }
-    for (int i = tid; i < RC_L * ech; i += RC_THREADS) {
-      const int r = i / ech, c = i - r * ech;
-      const bool on = r < n;
-      rc_cp16(xsm + (buf * RC_L + r) * (CE + 8) + c * 8, conv + (size_t)(on ? t0 + r : t0) * p.cv.C + p.cvv + h * E + c0 + c * 8, on);
-    }
-    const __nv_bfloat16* src = T + ((size_t)ch * p.H + h) * 2 * RC_L * RC_L;
-    for (int i = tid; i < 2 * RC_L * 8; i += RC_THREADS)
-      rc_cp16(tsm + ((size_t)buf * 2 * RC_L + (i >> 3)) * RC_TLD + (i & 7) * 8, src + (size_t)i * 8, true);
+    const __nv_bfloat16* row = conv + (size_t)t0 * p.cv.C;
+    rc_fetch<DP / 8>(ksm + buf * RC_L * LD, LD, row + p.ck + kg * D, p.cv.C, dch, n, tid);
+    rc_fetch<DP / 8>(qsm + buf * RC_L * LD, LD, row + p.cq + kg * D, p.cv.C, dch, n, tid);
+    rc_fetch<CE / 8>(xsm + buf * RC_L * (CE + 8), CE + 8, row + p.cvv + h * E + c0, p.cv.C, ech, n, tid);
+    rc_fetch<RC_L / 8>(tsm + (size_t)buf * 2 * RC_L * RC_TLD, RC_TLD, T + ((size_t)ch * p.H + h) * 2 * RC_L * RC_L, RC_L, RC_L / 8, RC_L, tid);
+    rc_fetch<RC_L / 8>(tsm + ((size_t)buf * 2 + 1) * RC_L * RC_TLD, RC_TLD, T + (((size_t)ch * p.H + h) * 2 + 1) * RC_L * RC_L, RC_L, RC_L / 8, RC_L, tid);
   };
-  // warp 0 carries the next chunk's scalars in registers (tokens lane and lane + 32)
+  // one of them carries the next chunk's scalars in registers (tokens lane and lane + 32)
   float2 g0, g1, n0, n1;
+  // (the last row's for tokens behind it, zeroed where they are used: nothing waits for a load here)
   auto scalars = [&](int ch) {
-    const int t0 = ch * RC_L + lane, t1 = t0 + 32;
-    const float2 z = make_float2(0.f, 0.f);
-    g0 = t0 < rows ? gates[(size_t)t0 * p.H + h] : z;
-    g1 = t1 < rows ? gates[(size_t)t1 * p.H + h] : z;
-    n0 = t0 < rows ? norms[(size_t)t0 * p.G + kg] : z;
-    n1 = t1 < rows ? norms[(size_t)t1 * p.G + kg] : z;
+    const int t0 = ch * RC_L + lane < rows ? ch * RC_L + lane : rows - 1, t1 = ch * RC_L + lane + 32 < rows ? ch * RC_L + lane + 32 : rows - 1;
+    g0 = gates[(size_t)t0 * p.H + h];
+    g1 = gates[(size_t)t1 * p.H + h];
+    n0 = norms[(size_t)t0 * p.G + kg];
+    n1 = norms[(size_t)t1 * p.G + kg];
   };
   // state: this warp's rows of it, CE columns, as accumulators
   float s[MT][NT][4];
@@ -234,205 +251,250 @@ __global__ void __launch_bounds__(RC_THREADS, 1)
       for (int e = 0; e < 4; e++) {
         int r, c;
         state_at(mt, nt, e, r, c);
-        s[mt][nt][e] = pos0 > 0 && r < D && c < E ? S[(size_t)r * E + c] : 0.f;
+        s[mt][nt][e] = !outs && pos0 > 0 && r < D && c < E ? S[(size_t)r * E + c] : 0.f;
       }
-  fetch(0, 0);
-  rc_commit();
-  if (warp == 0) scalars(0);
+  if (!outs) {
+    fetch(0, 0);
+    rc_commit();
+    if (warp == 0) scalars(0);
+  }
   for (int ch = 0; ch < nch; ch++) {
     const int buf = ch & 1, t0 = ch * RC_L, n = rows - t0 < RC_L ? rows - t0 : RC_L;
-    // the state in front of the chunk, in two planes, for the products below
+    float* sb = (float*)(smem + SM::SC) + buf * 3 * RC_L;   // b_t
+    float* snk = sb + RC_L;                                 // 1 / |k_s|
+    float* snq = snk + RC_L;                                // D^-1/2 / |q_t|
+    if (!outs) {
+      // the state in front of the chunk, in two planes, for the products below
 #pragma unroll
-    for (int mt = 0; mt < MT; mt++)
+      for (int mt = 0; mt < MT; mt++)
 #pragma unroll
-      for (int nt = 0; nt < NT; nt++)
+        for (int nt = 0; nt < NT; nt++)
 #pragma unroll
-        for (int e = 0; e < 2; e++) {
-          uint32_t hi, lo;
-          rc_split(s[mt][nt][2 * e], s[mt][nt][2 * e + 1], hi, lo);
-          const int at = ((warp * MT + mt) * 16 + (lane >> 2) + e * 8) * (CE + 8) + nt * 8 + (lane & 3) * 2;
-          *(uint32_t*)(ssm + at) = hi;
-          *(uint32_t*)(ssm + DP * (CE + 8) + at) = lo;
-        }
-    if (warp == 0) {
+          for (int e = 0; e < 2; e++) {
+            uint32_t hi, lo;
+            rc_split(s[mt][nt][2 * e], s[mt][nt][2 * e + 1], hi, lo);
+            const int at = ((warp * MT + mt) * 16 + (lane >> 2) + e * 8) * (CE + 8) + nt * 8 + (lane & 3) * 2;
+            *(uint32_t*)(ssm + at) = hi;
+            *(uint32_t*)(ssm + DP * (CE + 8) + at) = lo;
+          }
+    }
+    if (warp == 0 && !outs) {
       float b0, b1;
-      rc_scan(g0.y, g1.y, b0, b1);
+      const bool on0 = lane < n, on1 = lane + 32 < n;
+      rc_scan(on0 ? g0.y : 0.f, on1 ? g1.y : 0.f, b0, b1);
       sb[lane] = b0; sb[lane + 32] = b1;
-      snk[lane] = n0.y; snk[lane + 32] = n1.y; snq[lane] = n0.x; snq[lane + 32] = n1.x;
+      snk[lane] = on0 ? n0.y : 0.f; snk[lane + 32] = on1 ? n1.y : 0.f;
+      snq[lane] = on0 ? n0.x : 0.f; snq[lane + 32] = on1 ? n1.x : 0.f;
       if (ch + 1 < nch) scalars(ch + 1);
     }
     rc_wait<0>();
-    __syncthreads();
-    if (ch + 1 < nch) {
-      fetch(ch + 1, buf ^ 1);
-      rc_commit();
-    }
+    __syncthreads();   // the chunk's rows and the state's planes are there
     const __nv_bfloat16 *K = ksm + buf * RC_L * LD, *Q = qsm + buf * RC_L * LD, *X = xsm + buf * RC_L * (CE + 8);
     const int ra = wr + (lane >> 2), cb = (lane & 3) * 2;     // the thread's rows are ra and ra + 8
     const float ba = sb[ra], bb = sb[ra + 8], bL = sb[RC_L - 1];
-    // q S, k S (both planes of S), q k^T for the rows of this warp
-    float qs[NT][4], kS[NT][4], m[8][4];
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-#pragma unroll
-      for (int i = 0; i < NT; i++) qs[i][e] = kS[i][e] = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; i++) m[i][e] = 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < DP; k += 16) {
-      uint32_t aq[4], ak[4];
-      rc_ldm(aq, rc_a(Q, LD, wr, k, lane));
-      rc_ldm(ak, rc_a(K, LD, wr, k, lane));
-      uint32_t bs[2][CE / 16][4], bk[4][4];   // all of a step's fragments first: one shared-memory latency a step
-#pragma unroll
-      for (int pl = 0; pl < 2; pl++)
-#pragma unroll
-        for (int j = 0; j < CE / 16; j++) rc_ldmt(bs[pl][j], rc_bk(ssm + pl * DP * (CE + 8), (CE + 8), k, j * 16, lane));
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (j <= warp) rc_ldm(bk[j], rc_bn(K, LD, j * 16, k, lane));
-#pragma unroll
-      for (int pl = 0; pl < 2; pl++)
-#pragma unroll
-        for (int j = 0; j < CE / 16; j++) {
-          rc_mma(qs[2 * j], aq, bs[pl][j][0], bs[pl][j][1]);
-          rc_mma(qs[2 * j + 1], aq, bs[pl][j][2], bs[pl][j][3]);
-          rc_mma(kS[2 * j], ak, bs[pl][j][0], bs[pl][j][1]);
-          rc_mma(kS[2 * j + 1], ak, bs[pl][j][2], bs[pl][j][3]);
-        }
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (j <= warp) {
-          rc_mma(m[2 * j], aq, bk[j][0], bk[j][1]);
-          rc_mma(m[2 * j + 1], aq, bk[j][2], bk[j][3]);
-        }
-    }
-    // decays and unit norms of q k^T, then as operand planes
-    uint32_t mh[4][4], ml[4][4];
     const float qa = snq[ra], qb = snq[ra + 8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      float w[4];
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const int c = j * 8 + cb + (e & 1), t = e < 2 ? ra : ra + 8;
-        const float f = c <= t ? expf((e < 2 ? ba : bb) - sb[c]) * (snk[c] * (e < 2 ? qa : qb)) : 0.f;
-        w[e] = j <= 2 * warp + 1 ? m[j][e] * f : 0.f;
+    if (!outs) {
+      if (ch + 1 < nch) {
+        fetch(ch + 1, buf ^ 1);
+        rc_commit();
       }
-      rc_split(w[0], w[1], mh[j >> 1][(j & 1) * 2], ml[j >> 1][(j & 1) * 2]);
-      rc_split(w[2], w[3], mh[j >> 1][(j & 1) * 2 + 1], ml[j >> 1][(j & 1) * 2 + 1]);
-    }
-    // R = v - exp(b) |k|^-1 (k S), in planes
-    const float fa = expf(ba) * snk[ra], fb = expf(bb) * snk[ra + 8];
+      // k S (both planes of S)
+      // (a plane or a product of planes has sums of its own: their chains run side by side)
+      float kS[2][NT][4];
 #pragma unroll
-    for (int j = 0; j < NT; j++)
+      for (int i = 0; i < NT; i++)
 #pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
-        const uint32_t v = *(const uint32_t*)(X + at);
-        const float f = e ? fb : fa;
-        uint32_t hi, lo;
-        rc_split(fmaf(-f, kS[j][2 * e], __uint_as_float(v << 16)),
-                 fmaf(-f, kS[j][2 * e + 1], __uint_as_float(v & 0xffff0000u)), hi, lo);
-        *(uint32_t*)(usm + at) = hi;
-        *(uint32_t*)(usm + RC_L * (CE + 8) + at) = lo;
-      }
-    __syncthreads();
-    float u[NT][4];
+        for (int e = 0; e < 4; e++) kS[0][i][e] = kS[1][i][e] = 0.f;
 #pragma unroll
-    for (int i = 0; i < NT; i++) u[i][0] = u[i][1] = u[i][2] = u[i][3] = 0.f;
-    const __nv_bfloat16* Tp = tsm + (size_t)buf * 2 * RC_L * RC_TLD;
+      for (int k = 0; k < DP; k += 16) {
+        uint32_t ak[4], bs[2][CE / 16][4];
+        rc_ldm(ak, rc_a(K, LD, wr, k, lane));
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (k <= warp) {
-        uint32_t ah[4], al[4];
-        rc_ldm(ah, rc_a(Tp, RC_TLD, wr, k * 16, lane));
-        rc_ldm(al, rc_a(Tp + RC_L * RC_TLD, RC_TLD, wr, k * 16, lane));
+        for (int pl = 0; pl < 2; pl++)
 #pragma unroll
-        for (int j = 0; j < CE / 16; j++) {
-          uint32_t bh[4], bl[4];
-          rc_ldmt(bh, rc_bk(usm, (CE + 8), k * 16, j * 16, lane));
-          rc_ldmt(bl, rc_bk(usm + RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
-          rc_mma(u[2 * j], ah, bh[0], bh[1]); rc_mma(u[2 * j + 1], ah, bh[2], bh[3]);
-          rc_mma(u[2 * j], ah, bl[0], bl[1]); rc_mma(u[2 * j + 1], ah, bl[2], bl[3]);
-          rc_mma(u[2 * j], al, bh[0], bh[1]); rc_mma(u[2 * j + 1], al, bh[2], bh[3]);
-        }
-      }
-    __syncthreads();   // R is read: its planes become U's
-    const float ga = expf(bL - ba) * snk[ra], gb = expf(bL - bb) * snk[ra + 8];
+          for (int j = 0; j < CE / 16; j++) rc_ldmt(bs[pl][j], rc_bk(ssm + pl * DP * (CE + 8), (CE + 8), k, j * 16, lane));
 #pragma unroll
-    for (int j = 0; j < NT; j++)
+        for (int pl = 0; pl < 2; pl++)
 #pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
-        const float f = e ? gb : ga;
-        uint32_t hi, lo;
-        rc_split(u[j][2 * e], u[j][2 * e + 1], hi, lo);
-        *(uint32_t*)(usm + at) = hi;
-        *(uint32_t*)(usm + RC_L * (CE + 8) + at) = lo;
-        rc_split(u[j][2 * e] * f, u[j][2 * e + 1] * f, hi, lo);
-        *(uint32_t*)(wsm + at) = hi;
-        *(uint32_t*)(wsm + RC_L * (CE + 8) + at) = lo;
-      }
-    __syncthreads();
-    // O = exp(b) (q S) + M U
-    const float ea = expf(ba) * qa, eb = expf(bb) * qb;
-#pragma unroll
-    for (int j = 0; j < NT; j++) { qs[j][0] *= ea; qs[j][1] *= ea; qs[j][2] *= eb; qs[j][3] *= eb; }
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (k <= warp) {
-#pragma unroll
-        for (int j = 0; j < CE / 16; j++) {
-          uint32_t b[4];
-          rc_ldmt(b, rc_bk(usm, (CE + 8), k * 16, j * 16, lane));
-          rc_mma(qs[2 * j], mh[k], b[0], b[1]); rc_mma(qs[2 * j + 1], mh[k], b[2], b[3]);
-          rc_mma(qs[2 * j], ml[k], b[0], b[1]); rc_mma(qs[2 * j + 1], ml[k], b[2], b[3]);
-          rc_ldmt(b, rc_bk(usm + RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
-          rc_mma(qs[2 * j], mh[k], b[0], b[1]); rc_mma(qs[2 * j + 1], mh[k], b[2], b[3]);
-        }
-      }
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const int t = ra + 8 * e;
-      if (t < n) {
-        float* dst = o + ((size_t)(t0 + t) * p.H + h) * E + c0;
-#pragma unroll
-        for (int j = 0; j < NT; j++)
-          if (j < ech) *(float2*)(dst + j * 8 + cb) = make_float2(qs[j][2 * e], qs[j][2 * e + 1]);
-      }
-    }
-    // S = exp(b_L) S + K^T (weighted U)
-    const float eL = expf(bL);
-#pragma unroll
-    for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-      for (int nt = 0; nt < NT; nt++)
-#pragma unroll
-        for (int e = 0; e < 4; e++) s[mt][nt][e] *= eL;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      uint32_t a[MT][4];
-#pragma unroll
-      for (int mt = 0; mt < MT; mt++) rc_ldmt(a[mt], rc_at(K, LD, (warp * MT + mt) * 16, k * 16, lane));
-      uint32_t b[2][CE / 16][4];
-#pragma unroll
-      for (int pl = 0; pl < 2; pl++)
-#pragma unroll
-        for (int j = 0; j < CE / 16; j++) rc_ldmt(b[pl][j], rc_bk(wsm + pl * RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
-#pragma unroll
-      for (int pl = 0; pl < 2; pl++)
-#pragma unroll
-        for (int j = 0; j < CE / 16; j++)
-#pragma unroll
-          for (int mt = 0; mt < MT; mt++) {
-            rc_mma(s[mt][2 * j], a[mt], b[pl][j][0], b[pl][j][1]);
-            rc_mma(s[mt][2 * j + 1], a[mt], b[pl][j][2], b[pl][j][3]);
+          for (int j = 0; j < CE / 16; j++) {
+            rc_mma(kS[pl][2 * j], ak, bs[pl][j][0], bs[pl][j][1]);
+            rc_mma(kS[pl][2 * j + 1], ak, bs[pl][j][2], bs[pl][j][3]);
           }
+      }
+      // R = v - exp(b) |k|^-1 (k S), in planes
+      const float fa = expf(ba) * snk[ra], fb = expf(bb) * snk[ra + 8];
+#pragma unroll
+      for (int j = 0; j < NT; j++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
+          const uint32_t v = *(const uint32_t*)(X + at);
+          const float f = e ? fb : fa;
+          uint32_t hi, lo;
+          rc_split(fmaf(-f, kS[0][j][2 * e] + kS[1][j][2 * e], __uint_as_float(v << 16)),
+                   fmaf(-f, kS[0][j][2 * e + 1] + kS[1][j][2 * e + 1], __uint_as_float(v & 0xffff0000u)), hi, lo);
+          *(uint32_t*)(usm + at) = hi;
+          *(uint32_t*)(usm + RC_L * (CE + 8) + at) = lo;
+        }
+      rd_sync();
+      float u[NT][4], uc[2][NT][4];
+#pragma unroll
+      for (int i = 0; i < NT; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) u[i][e] = uc[0][i][e] = uc[1][i][e] = 0.f;
+      const __nv_bfloat16* Tp = tsm + (size_t)buf * 2 * RC_L * RC_TLD;
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (k <= warp) {
+          uint32_t ah[4], al[4];
+          rc_ldm(ah, rc_a(Tp, RC_TLD, wr, k * 16, lane));
+          rc_ldm(al, rc_a(Tp + RC_L * RC_TLD, RC_TLD, wr, k * 16, lane));
+#pragma unroll
+          for (int j = 0; j < CE / 16; j++) {
+            uint32_t bh[4], bl[4];
+            rc_ldmt(bh, rc_bk(usm, (CE + 8), k * 16, j * 16, lane));
+            rc_ldmt(bl, rc_bk(usm + RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
+            rc_mma(u[2 * j], ah, bh[0], bh[1]); rc_mma(u[2 * j + 1], ah, bh[2], bh[3]);
+            rc_mma(uc[0][2 * j], ah, bl[0], bl[1]); rc_mma(uc[0][2 * j + 1], ah, bl[2], bl[3]);
+            rc_mma(uc[1][2 * j], al, bh[0], bh[1]); rc_mma(uc[1][2 * j + 1], al, bh[2], bh[3]);
+          }
+        }
+#pragma unroll
+      for (int i = 0; i < NT; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) u[i][e] += uc[0][i][e] + uc[1][i][e];
+      rd_sync();   // R is read: its planes become U's
+      const float ga = expf(bL - ba) * snk[ra], gb = expf(bL - bb) * snk[ra + 8];
+#pragma unroll
+      for (int j = 0; j < NT; j++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const int at = (ra + 8 * e) * (CE + 8) + j * 8 + cb;
+          const float f = e ? gb : ga;
+          uint32_t hi, lo;
+          rc_split(u[j][2 * e], u[j][2 * e + 1], hi, lo);
+          *(uint32_t*)(usm + at) = hi;
+          *(uint32_t*)(usm + RC_L * (CE + 8) + at) = lo;
+          rc_split(u[j][2 * e] * f, u[j][2 * e + 1] * f, hi, lo);
+          *(uint32_t*)(wsm + at) = hi;
+          *(uint32_t*)(wsm + RC_L * (CE + 8) + at) = lo;
+        }
+      rd_arrive<2>();
+      rd_sync();   // the weighted form is there
+      // S = exp(b_L) S + K^T (weighted U)
+      const float eL = expf(bL);
+#pragma unroll
+      for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) s[mt][nt][e] *= eL;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        uint32_t a[MT][4];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++) rc_ldmt(a[mt], rc_at(K, LD, (warp * MT + mt) * 16, k * 16, lane));
+        uint32_t b[2][CE / 16][4];
+#pragma unroll
+        for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+          for (int j = 0; j < CE / 16; j++) rc_ldmt(b[pl][j], rc_bk(wsm + pl * RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
+#pragma unroll
+        for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+          for (int j = 0; j < CE / 16; j++)
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++) {
+              rc_mma(s[mt][2 * j], a[mt], b[pl][j][0], b[pl][j][1]);
+              rc_mma(s[mt][2 * j + 1], a[mt], b[pl][j][2], b[pl][j][3]);
+            }
+      }
+      rd_await<3>();   // before the next chunk's planes
+    } else {
+      float qs[NT][4];
+      uint32_t mh[4][4], ml[4][4];
+      // q S (both planes of S)
+#pragma unroll
+      for (int i = 0; i < NT; i++) qs[i][0] = qs[i][1] = qs[i][2] = qs[i][3] = 0.f;
+#pragma unroll
+      for (int k = 0; k < DP; k += 16) {
+        uint32_t aq[4], bs[2][CE / 16][4];
+        rc_ldm(aq, rc_a(Q, LD, wr, k, lane));
+#pragma unroll
+        for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+          for (int j = 0; j < CE / 16; j++) rc_ldmt(bs[pl][j], rc_bk(ssm + pl * DP * (CE + 8), (CE + 8), k, j * 16, lane));
+#pragma unroll
+        for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+          for (int j = 0; j < CE / 16; j++) {
+            rc_mma(qs[2 * j], aq, bs[pl][j][0], bs[pl][j][1]);
+            rc_mma(qs[2 * j + 1], aq, bs[pl][j][2], bs[pl][j][3]);
+          }
+      }
+      rd_arrive<3>();
+      // q k^T
+      float m[8][4];
+#pragma unroll
+      for (int i = 0; i < 8; i++) m[i][0] = m[i][1] = m[i][2] = m[i][3] = 0.f;
+#pragma unroll
+      for (int k = 0; k < DP; k += 16) {
+        uint32_t aq[4], bk[4][4];   // all of a step's fragments first: one shared-memory latency a step
+        rc_ldm(aq, rc_a(Q, LD, wr, k, lane));
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (j <= warp) rc_ldm(bk[j], rc_bn(K, LD, j * 16, k, lane));
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (j <= warp) {
+            rc_mma(m[2 * j], aq, bk[j][0], bk[j][1]);
+            rc_mma(m[2 * j + 1], aq, bk[j][2], bk[j][3]);
+          }
+      }
+      // decays and unit norms of q k^T, then as operand planes
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+        if (j <= 2 * warp + 1) {
+          const float2 bc = *(const float2*)(sb + j * 8 + cb), kc = *(const float2*)(snk + j * 8 + cb);
+          float w[4];
+#pragma unroll
+          for (int e = 0; e < 4; e++)
+            w[e] = rc_decayed(m[j][e], (e < 2 ? ba : bb) - (e & 1 ? bc.y : bc.x), (e & 1 ? kc.y : kc.x) * (e < 2 ? qa : qb),
+                              j * 8 + cb + (e & 1) <= (e < 2 ? ra : ra + 8));
+          rc_split(w[0], w[1], mh[j >> 1][(j & 1) * 2], ml[j >> 1][(j & 1) * 2]);
+          rc_split(w[2], w[3], mh[j >> 1][(j & 1) * 2 + 1], ml[j >> 1][(j & 1) * 2 + 1]);
+        }
+      rd_await<2>();
+      // O = exp(b) (q S) + M U
+      const float ea = expf(ba) * qa, eb = expf(bb) * qb;
+#pragma unroll
+      for (int j = 0; j < NT; j++) { qs[j][0] *= ea; qs[j][1] *= ea; qs[j][2] *= eb; qs[j][3] *= eb; }
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (k <= warp) {
+#pragma unroll
+          for (int j = 0; j < CE / 16; j++) {
+            uint32_t b[4];
+            rc_ldmt(b, rc_bk(usm, (CE + 8), k * 16, j * 16, lane));
+            rc_mma(qs[2 * j], mh[k], b[0], b[1]); rc_mma(qs[2 * j + 1], mh[k], b[2], b[3]);
+            rc_mma(qs[2 * j], ml[k], b[0], b[1]); rc_mma(qs[2 * j + 1], ml[k], b[2], b[3]);
+            rc_ldmt(b, rc_bk(usm + RC_L * (CE + 8), (CE + 8), k * 16, j * 16, lane));
+            rc_mma(qs[2 * j], mh[k], b[0], b[1]); rc_mma(qs[2 * j + 1], mh[k], b[2], b[3]);
+          }
+        }
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int t = ra + 8 * e;
+        if (t < n) {
+          float* dst = o + ((size_t)(t0 + t) * p.H + h) * E + c0;
+#pragma unroll
+          for (int j = 0; j < NT; j++)
+            if (j < ech) *(float2*)(dst + j * 8 + cb) = make_float2(qs[j][2 * e], qs[j][2 * e + 1]);
+        }
+      }
     }
-    __syncthreads();   // the chunk's operands and planes are read: the next one may overwrite them
   }
+  if (outs) return;
 #pragma unroll
   for (int mt = 0; mt < MT; mt++)
 #pragma unroll
@@ -445,10 +507,6 @@ __global__ void __launch_bounds__(RC_THREADS, 1)
       }
 }
 
-// ---- ssd: the chunks of one head and 32 value columns ------------------------------------------------
-// The walk waits on its own latencies (mma.sync fragments, barriers, exponentials), so what counts is CTAs an SM: three,
-// with every operand once in shared memory.  The next chunk's rows come as their places fall free: q behind q k^T, k
-// behind the state's update, which is done before the outputs for that, x behind the next chunk's first barrier.
 // Segments of `chunks` chunks each.  carry [segments][H][D][E]: the state in front of the prompt, then every
 // segment's own but the last; decay [segments][H]: its log decay.  One segment: no carry.
 struct RcSegments {
@@ -456,6 +514,10 @@ struct RcSegments {
   float *carry, *decay;
 };
 
+// ---- ssd: the chunks of one head and 32 value columns ------------------------------------------------
+// The walk waits on its own latencies (mma.sync fragments, barriers, exponentials), so what counts is CTAs an SM: three,
+// with every operand once in shared memory.  The next chunk's rows come as their places fall free: q behind q k^T, k
+// behind the state's update, which is done before the outputs for that, x behind the next chunk's first barrier.
 template <int DP>
 struct ScSmem {
   static constexpr int LD = DP + 8;
@@ -491,25 +553,26 @@ __global__ void __launch_bounds__(RC_THREADS, 3)
   pdl_wait();
   pdl_launch_dependents();
   __syncthreads();
-  // rows of a chunk, `chunks` pieces of 16 bytes each, from column `at` on (zeros behind the last row)
-  auto fetch = [&](__nv_bfloat16* dst, int ld, int at, int chunks, int ch) {
-    const int t0 = ch * RC_L, n = rows - t0 < RC_L ? rows - t0 : RC_L;
-    for (int i = tid; i < RC_L * chunks; i += RC_THREADS) {
-      const int r = i / chunks, c = i - r * chunks;
-      rc_cp16(dst + r * ld + c * 8, conv + (size_t)(r < n ? t0 + r : t0) * p.cv.C + at + c * 8, r < n);
-    }
+  // rows of a chunk: of k or q from column `at` on, of x
+  auto rows_of = [&](int ch) { return rows - ch * RC_L < RC_L ? rows - ch * RC_L : RC_L; };
+  auto fetch = [&](__nv_bfloat16* dst, int at, int ch) {
+    rc_fetch<DP / 8>(dst, LD, conv + (size_t)ch * RC_L * p.cv.C + at, p.cv.C, dch, rows_of(ch), tid);
+    rc_commit();
+  };
+  auto fetch_x = [&](int ch) {
+    rc_fetch<RC_E / 8>(X, RC_ELD, conv + (size_t)ch * RC_L * p.cv.C + p.cvv + h * E + c0, p.cv.C, ech, rows_of(ch), tid);
     rc_commit();
   };
   // warp 0 carries the next chunk's scalars in registers (tokens lane and lane + 32)
   float2 g0, g1;
+  // (the last row's for tokens behind it, zeroed where they are used: nothing waits for a load here)
   auto scalars = [&](int ch) {
-    const int t0 = ch * RC_L + lane, t1 = t0 + 32;
-    const float2 z = make_float2(0.f, 0.f);
-    g0 = t0 < rows ? gates[(size_t)t0 * p.H + h] : z;
-    g1 = t1 < rows ? gates[(size_t)t1 * p.H + h] : z;
+    const int t0 = ch * RC_L + lane < rows ? ch * RC_L + lane : rows - 1, t1 = ch * RC_L + lane + 32 < rows ? ch * RC_L + lane + 32 : rows - 1;
+    g0 = gates[(size_t)t0 * p.H + h];
+    g1 = gates[(size_t)t1 * p.H + h];
   };
-  fetch(Q, LD, p.cq + kg * D, dch, ch0);
-  fetch(K, LD, p.ck + kg * D, dch, ch0);
+  fetch(Q, p.cq + kg * D, ch0);
+  fetch(K, p.ck + kg * D, ch0);
   if (warp == 0) scalars(ch0);
   // state: this warp's rows of it, 32 columns, as accumulators
   float s[MT][NT][4];
@@ -565,14 +628,15 @@ __global__ void __launch_bounds__(RC_THREADS, 3)
         }
     if (warp == 0) {
       float b0, b1;
-      rc_scan(g0.y, g1.y, b0, b1);
+      const bool on0 = lane < n, on1 = lane + 32 < n;
+      rc_scan(on0 ? g0.y : 0.f, on1 ? g1.y : 0.f, b0, b1);
       sb[lane] = b0; sb[lane + 32] = b1;
-      sg[lane] = g0.x; sg[lane + 32] = g1.x;
+      sg[lane] = on0 ? g0.x : 0.f; sg[lane + 32] = on1 ? g1.x : 0.f;
       if (ch + 1 < ch1) scalars(ch + 1);
     }
     rc_wait<0>();
     __syncthreads();   // q, k and the state's planes are there; x of the chunk before is read
-    fetch(X, RC_ELD, p.cvv + h * E + c0, ech, ch);
+    fetch_x(ch);
     const int ra = wr + (lane >> 2), cb = (lane & 3) * 2;     // the thread's rows are ra and ra + 8
     const float ba = sb[ra], bb = sb[ra + 8], bL = sb[RC_L - 1];
     const float ga = expf(bL - ba) * sg[ra], gb = expf(bL - bb) * sg[ra + 8];
@@ -615,18 +679,18 @@ __global__ void __launch_bounds__(RC_THREADS, 3)
 #pragma unroll
     for (int j = 0; j < 8; j++)
       if (j <= 2 * warp + 1) {
+        const float2 bc = *(const float2*)(sb + j * 8 + cb), gc = *(const float2*)(sg + j * 8 + cb);
         float w[4];
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int c = j * 8 + cb + (e & 1), t = e < 2 ? ra : ra + 8;
-          w[e] = c <= t ? m[j][e] * (expf((e < 2 ? ba : bb) - sb[c]) * sg[c]) : 0.f;
-        }
+        for (int e = 0; e < 4; e++)
+          w[e] = rc_decayed(m[j][e], (e < 2 ? ba : bb) - (e & 1 ? bc.y : bc.x), e & 1 ? gc.y : gc.x,
+                            j * 8 + cb + (e & 1) <= (e < 2 ? ra : ra + 8));
         rc_split(w[0], w[1], mh[j >> 1][(j & 1) * 2], ml[j >> 1][(j & 1) * 2]);
         rc_split(w[2], w[3], mh[j >> 1][(j & 1) * 2 + 1], ml[j >> 1][(j & 1) * 2 + 1]);
       }
     rc_wait<0>();
     __syncthreads();   // x is there, q is read
-    if (ch + 1 < ch1) fetch(Q, LD, p.cq + kg * D, dch, ch + 1);
+    if (ch + 1 < ch1) fetch(Q, p.cq + kg * D, ch + 1);
 #pragma unroll
     for (int j = 0; j < NT; j++)
 #pragma unroll
@@ -668,7 +732,7 @@ __global__ void __launch_bounds__(RC_THREADS, 3)
           }
     }
     __syncthreads();   // k and the weighted x are read
-    if (ch + 1 < ch1) fetch(K, LD, p.ck + kg * D, dch, ch + 1);
+    if (ch + 1 < ch1) fetch(K, p.ck + kg * D, ch + 1);
     // O = exp(b) (q S) + M x
     const float ea = expf(ba), eb = expf(bb);
 #pragma unroll
@@ -741,14 +805,8 @@ __global__ void __launch_bounds__(RC_THREADS, 3)
   __syncthreads();
   auto fetch = [&](int ch, int buf) {
     const __nv_bfloat16* base = conv + (size_t)ch * RC_L * p.cv.C;
-    for (int i = tid; i < RC_L * dch; i += RC_THREADS) {
-      const int r = i / dch, c = i - r * dch;
-      rc_cp16(ksm + (buf * RC_L + r) * LD + c * 8, base + (size_t)r * p.cv.C + p.ck + kg * D + c * 8, true);
-    }
-    for (int i = tid; i < RC_L * ech; i += RC_THREADS) {
-      const int r = i / ech, c = i - r * ech;
-      rc_cp16(xsm + (buf * RC_L + r) * RC_ELD + c * 8, base + (size_t)r * p.cv.C + p.cvv + h * E + c0 + c * 8, true);
-    }
+    rc_fetch<DP / 8>(ksm + buf * RC_L * LD, LD, base + p.ck + kg * D, p.cv.C, dch, RC_L, tid);
+    rc_fetch<RC_E / 8>(xsm + buf * RC_L * RC_ELD, RC_ELD, base + p.cvv + h * E + c0, p.cv.C, ech, RC_L, tid);
   };
   float2 g0, g1;
   auto scalars = [&](int ch) {
@@ -879,7 +937,7 @@ int delta_walk(const RecurP& p, const void* conv, const float2* gates, const flo
   static std::atomic<unsigned long long> done{0};
   const int rc = ensure_dynamic_smem(delta_chunk_kernel<DP, CE>, smem, done);
   if (rc) return rc;
-  LaunchCfg lc(dim3((p.E + CE - 1) / CE, p.H), dim3(RC_THREADS), smem, s, pdl_enabled());
+  LaunchCfg lc(dim3((p.E + CE - 1) / CE, p.H), dim3(RD_THREADS), smem, s, pdl_enabled());
   TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, delta_chunk_kernel<DP, CE>, p, (const __nv_bfloat16*)conv, gates, norms,
                               (const __nv_bfloat16*)T, o, rows, pos0));
   return TLB_OK;
@@ -899,7 +957,7 @@ int delta_launch(const RecurP& p, const void* conv, const float2* gates, const f
   TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, delta_solve_kernel<DP>, p, (const __nv_bfloat16*)conv, gates, norms,
                               (__nv_bfloat16*)T, rows));
   // few heads: half as many columns a CTA, twice the CTAs, where those still find an SM each (4096 tokens, 16 heads of
-  // 128: 392 us on 64 SMs, 318 on 128)
+  // 128, before the outputs had warps of their own: 392 us on 64 SMs, 318 on 128)
   if (2 * ((p.E + RC_E - 1) / RC_E * p.H) <= c->sm_count)
     return delta_walk<DP, 16>(p, conv, gates, norms, T, o, rows, pos0, s);
   return delta_walk<DP, RC_E>(p, conv, gates, norms, T, o, rows, pos0, s);
