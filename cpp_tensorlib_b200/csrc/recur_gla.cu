@@ -54,15 +54,23 @@ __global__ void __launch_bounds__(256) gla_rates_kernel(const __grid_constant__ 
     if (t0 + t < rows) rates[(size_t)(t0 + t) * HD + c] = gla_rate(acc[t], p.tau);
 }
 
+// A column of N rows, zeros from row n on (the last row that there is lies at n - 1, also where that is in front of `at`).
+// Every load is made, of that row where there is no other, and the zeros are put in behind: a branch around each one made
+// each wait for the one before (a third of gla_out's time, and a fifth more for its values).
+template <int N>
+__device__ __forceinline__ void load_column(const float* at, long long stride, int n, bool on, float (&x)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i++) x[i] = at[(i < n ? i : n - 1) * stride];
+#pragma unroll
+  for (int i = 0; i < N; i++) x[i] = on && i < n ? x[i] : 0.f;
+}
 // the rates of one channel for TG of a chunk's tokens, their sum and the sum of all groups
 template <int TG>
-__device__ __forceinline__ float load_rates(const float* rates, size_t stride, int n, bool on, float (&x)[TG]) {
+__device__ __forceinline__ float load_rates(const float* rates, long long stride, int n, bool on, float (&x)[TG]) {
+  load_column<TG>(rates, stride, n, on, x);
   float s = 0.f;
 #pragma unroll
-  for (int i = 0; i < TG; i++) {
-    x[i] = on && i < n ? rates[(size_t)i * stride] : 0.f;
-    s += x[i];
-  }
+  for (int i = 0; i < TG; i++) s += x[i];
   return s;
 }
 __device__ __forceinline__ void put_planes(__nv_bfloat16* at, size_t plane, float v) {
@@ -78,12 +86,29 @@ __device__ __forceinline__ float4 load4(const float* at, int left, bool vec) {
 // 64 rows x W columns of f32 rows as bf16; columns from `cols` on and rows from n on are zero
 template <int W>
 __device__ __forceinline__ void load_values(__nv_bfloat16* vs, const float* src, long long ld, int n, int cols, bool vec) {
-#pragma unroll 4
-  for (int i = threadIdx.x; i < GC_L * W / 4; i += GC_THREADS) {
-    const int t = i / (W / 4), c = (i - t * (W / 4)) * 4;
-    const float4 v = load4(src + (size_t)t * ld + c, t < n ? cols - c : 0, vec);
+  auto put_bf16 = [&](int t, int c, float4 v) {
     const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
     *(uint2*)(vs + t * (W + 8) + c) = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b);
+  };
+  if (vec && cols >= W) {   // whole pieces: all loads first
+    constexpr int N = GC_L * W / 4 / GC_THREADS;
+    const int c = threadIdx.x % (W / 4) * 4, t0 = threadIdx.x / (W / 4);
+    float4 v[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const int t = t0 + i * (GC_THREADS / (W / 4));
+      v[i] = *(const float4*)(src + (t < n ? t : n - 1) * ld + c);
+    }
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const int t = t0 + i * (GC_THREADS / (W / 4));
+      put_bf16(t, c, t < n ? v[i] : make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    return;
+  }
+  for (int i = threadIdx.x; i < GC_L * W / 4; i += GC_THREADS) {
+    const int t = i / (W / 4), c = (i - t * (W / 4)) * 4;
+    put_bf16(t, c, load4(src + (size_t)t * ld + c, t < n ? cols - c : 0, vec));
   }
 }
 
@@ -106,10 +131,9 @@ __global__ void __launch_bounds__(GC_THREADS) gla_state_kernel(const __grid_cons
   pdl_wait();
   pdl_launch_dependents();
   float x[TG], kv[TG];
-  const float* kr = proj + (size_t)(t0 + tg) * ld + p.ck + h * D + d;
-#pragma unroll
-  for (int i = 0; i < TG; i++) kv[i] = d < D && tg + i < n ? kr[(size_t)i * ld] : 0.f;
-  gsum[grp * DP + d] = load_rates<TG>(rates + (size_t)(t0 + tg) * HD + h * D + d, HD, n - tg, d < D, x);
+  const int dc = d < D ? d : 0;
+  load_column<TG>(proj + (size_t)(t0 + tg) * ld + p.ck + h * D + dc, ld, n - tg, d < D, kv);
+  gsum[grp * DP + d] = load_rates<TG>(rates + (size_t)(t0 + tg) * HD + h * D + dc, HD, n - tg, d < D, x);
   load_values<SE>(vs, proj + (size_t)t0 * ld + p.cvv + h * E + e0, ld, n, E - e0, (E & 3) == 0);
   __syncthreads();
   float r = 0.f;
@@ -214,6 +238,7 @@ struct GoSmem {
   static constexpr size_t G = V + (size_t)GC_L * GC_ELD * 2;            // [groups][DP] f32
   static constexpr size_t TOTAL = G + (size_t)GC_THREADS * 4;
 };
+constexpr int GO_BATCH = 8;   // rows of q and k that a thread asks for at once
 template <int DP>
 __global__ void __launch_bounds__(GC_THREADS, DP <= 128 ? 2 : 1)
     gla_out_kernel(const __grid_constant__ RecurP p, const float* __restrict__ proj, long long ld,
@@ -235,10 +260,11 @@ __global__ void __launch_bounds__(GC_THREADS, DP <= 128 ? 2 : 1)
   pdl_wait();
   pdl_launch_dependents();
   const float qscale = rsqrtf((float)D);
-  const float* row = proj + (size_t)(t0 + tg) * ld + h * D + d;
+  const int dc = d < D ? d : 0;
+  const float* row = proj + (size_t)(t0 + tg) * ld + h * D + dc;
   {
     float x[TG];
-    gsum[grp * DP + d] = load_rates<TG>(rates + (size_t)(t0 + tg) * HD + h * D + d, HD, n - tg, d < D, x);
+    gsum[grp * DP + d] = load_rates<TG>(rates + (size_t)(t0 + tg) * HD + h * D + dc, HD, n - tg, d < D, x);
     __syncthreads();
     float b = 0.f, all = 0.f;
 #pragma unroll
@@ -248,13 +274,18 @@ __global__ void __launch_bounds__(GC_THREADS, DP <= 128 ? 2 : 1)
     }
     const bool far = __syncthreads_or(all > GC_MOST);
 #pragma unroll
-    for (int i = 0; i < TG; i++) {
-      const bool on = d < D && tg + i < n;
-      const float qv = on ? row[(size_t)i * ld + p.cq] * qscale : 0.f, kv = on && !far ? row[(size_t)i * ld + p.ck] : 0.f;
-      b += x[i];
-      put_planes(qs + (tg + i) * LD + d, (size_t)GC_L * LD, qv * expf(-b));
-      if (far) bs[(tg + i) * (DP + 1) + d] = b;
-      else put_planes(ks + (tg + i) * LD + d, (size_t)GC_L * LD, kv * expf(b));
+    for (int i0 = 0; i0 < TG; i0 += GO_BATCH) {
+      float qv[GO_BATCH], kv[GO_BATCH];
+      load_column<GO_BATCH>(row + i0 * ld + p.cq, ld, n - tg - i0, d < D, qv);
+      load_column<GO_BATCH>(row + i0 * ld + p.ck, ld, n - tg - i0, d < D, kv);
+#pragma unroll
+      for (int u = 0; u < GO_BATCH; u++) {
+        const int i = i0 + u;
+        b += x[i];
+        put_planes(qs + (tg + i) * LD + d, (size_t)GC_L * LD, qv[u] * qscale * expf(-b));
+        if (far) bs[(tg + i) * (DP + 1) + d] = b;
+        else put_planes(ks + (tg + i) * LD + d, (size_t)GC_L * LD, kv[u] * expf(b));
+      }
     }
     __syncthreads();
     // A for the rows of this warp, then as operand planes
@@ -307,8 +338,26 @@ __global__ void __launch_bounds__(GC_THREADS, DP <= 128 ? 2 : 1)
     for (int e0 = 0; e0 < E; e0 += GC_E) {
       __syncthreads();   // keys, or the columns before, are read
       load_values<GC_E>(vs, proj + (size_t)t0 * ld + p.cvv + h * E + e0, ld, n, E - e0, (E & 3) == 0);
-#pragma unroll 8
-      for (int i = tid; i < DP * GC_E / 2; i += GC_THREADS) {
+      auto put_state = [&](int r, int c, float2 v) {
+        uint32_t hi, lo;
+        rc_split(v.x, v.y, hi, lo);
+        *(uint32_t*)(ss + r * GC_ELD + c) = hi;
+        *(uint32_t*)(ss + (DP + r) * GC_ELD + c) = lo;
+      };
+      const bool whole = D == DP && (E & 1) == 0 && E - e0 >= GC_E;
+      if (whole) {   // all loads of a batch first
+        constexpr int RS = GC_THREADS / (GC_E / 2);
+        const int c = tid % (GC_E / 2) * 2, r0 = tid / (GC_E / 2);
+#pragma unroll
+        for (int i0 = 0; i0 < DP; i0 += 8 * RS) {
+          float2 v[8];
+#pragma unroll
+          for (int u = 0; u < 8; u++) v[u] = *(const float2*)(S + (size_t)(i0 + u * RS + r0) * E + e0 + c);
+#pragma unroll
+          for (int u = 0; u < 8; u++) put_state(i0 + u * RS + r0, c, v[u]);
+        }
+      }
+      for (int i = whole ? DP * GC_E / 2 : tid; i < DP * GC_E / 2; i += GC_THREADS) {
         const int r = i / (GC_E / 2), c = (i - r * (GC_E / 2)) * 2;
         const float* at = S + (size_t)r * E + e0 + c;
         float2 v = make_float2(0.f, 0.f);
@@ -318,10 +367,7 @@ __global__ void __launch_bounds__(GC_THREADS, DP <= 128 ? 2 : 1)
           if (r < D && e0 + c < E) v.x = at[0];
           if (r < D && e0 + c + 1 < E) v.y = at[1];
         }
-        uint32_t hi, lo;
-        rc_split(v.x, v.y, hi, lo);
-        *(uint32_t*)(ss + r * GC_ELD + c) = hi;
-        *(uint32_t*)(ss + (DP + r) * GC_ELD + c) = lo;
+        put_state(r, c, v);
       }
       __syncthreads();
       float y[4][4];
