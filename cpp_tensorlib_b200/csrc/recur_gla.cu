@@ -56,7 +56,8 @@ __global__ void __launch_bounds__(256) gla_rates_kernel(const __grid_constant__ 
 
 // A column of N rows, zeros from row n on (the last row that there is lies at n - 1, also where that is in front of `at`).
 // Every load is made, of that row where there is no other, and the zeros are put in behind: a branch around each one made
-// each wait for the one before (a third of gla_out's time, and a fifth more for its values).
+// each wait for the one before (a third of gla_out's time, and a fifth more for its values).  3001 tokens, 8 heads of
+// 128 x 256: gla_out 99.9 -> 58.8 us, gla_state 41.9 -> 32.7.
 template <int N>
 __device__ __forceinline__ void load_column(const float* at, long long stride, int n, bool on, float (&x)[N]) {
 #pragma unroll
