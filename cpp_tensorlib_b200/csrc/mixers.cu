@@ -465,11 +465,13 @@ __device__ void recur_update(const RecurP& p, const float* src, float* dst, cons
   }
 }
 
-// floats of the state that wait in shared memory (0: it is too large, or not whole 16-byte pieces)
-constexpr int MX_STATE_SMEM = 16384;
+// Floats of a head's block beside its state, and of the state that wait in shared memory (0: it is too large, also together
+// with the others, or not whole 16-byte pieces).
+constexpr size_t MX_SMEM = 204 * 1024, MX_STATE_SMEM = 16384;
+__host__ __device__ inline size_t recur_head_floats(const RecurP& p) { return (size_t)4 * p.D + 3 * p.E + 4 * MX_THREADS + 44; }
 __host__ __device__ inline int recur_state_floats(const RecurP& p) {
-  const int n = p.D * p.E;
-  return n <= MX_STATE_SMEM && n % 4 == 0 ? n : 0;
+  const size_t n = (size_t)p.D * p.E;
+  return n <= MX_STATE_SMEM && n % 4 == 0 && (n + recur_head_floats(p)) * sizeof(float) <= MX_SMEM ? (int)n : 0;
 }
 
 // One block a head.  The state and the convolutions' history are fetched before the projected row is there.  (The row is
@@ -1048,14 +1050,14 @@ size_t attn_smem(const AttnP& p, int rm) {
 }
 size_t recur_smem(const RecurP& p) {
   if (p.kind == MIX_GLA) return (size_t)(3 * p.D + MX_THREADS + p.D * GL_COLS) * sizeof(float);
-  return (size_t)(recur_state_floats(p) + 4 * p.D + 3 * p.E + 4 * MX_THREADS + 44) * sizeof(float);
+  return (recur_state_floats(p) + recur_head_floats(p)) * sizeof(float);
 }
 int rm_of(int hpb) { return hpb <= 1 ? 1 : (hpb <= 2 ? 2 : (hpb <= 4 ? 4 : 8)); }
 
 template <typename KT, int RM, bool FAST>
 int decode_launch(const DecodeArgs& a, int blocks, size_t smem, cudaStream_t s) {
   static std::atomic<unsigned long long> done{0};
-  const int rc = ensure_dynamic_smem(mixers_decode_kernel<KT, RM, FAST>, 204 * 1024, done);
+  const int rc = ensure_dynamic_smem(mixers_decode_kernel<KT, RM, FAST>, MX_SMEM, done);
   if (rc) return rc;
   LaunchCfg lc(dim3(blocks), dim3(MX_THREADS), smem, s, pdl_enabled());
   TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, mixers_decode_kernel<KT, RM, FAST>, a));

@@ -31,3 +31,22 @@ def test_token_states(heads, groups, state, vdim, conv, norm_groups, dtype):
     got = run(m, toks, [])
     assert np.isfinite(got).all() and ok(err(got, want), dtype)
     close(m)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("state,vdim", [
+    (1, 16384),     # a state of 64 KB that does not fit beside its own values
+    (1, 12788),     # the widest of one row that does
+    (1, 12792),     # ... and that does not
+])
+def test_wide_heads(state, vdim, dtype):
+    """Heads on both sides of what waits in shared memory."""
+    cfg = zc.config([zc.mam(1, 1, state, vdim, 2, 1), zc.par(right=(1, 1, state, vdim), conv=2, ff=0)], width=72, vocab=151, emb=1.0)
+    w = zc.Weights(cfg, 7)
+    toks = zc.tokens(cfg, 6, 2)
+    want = orc.forward(cfg, w.f64(), toks)
+    m = make(cfg, w, dtype, 16)
+    m.capture()
+    got = run(m, toks, [])
+    assert np.isfinite(got).all() and ok(err(got, want), dtype)
+    close(m)
