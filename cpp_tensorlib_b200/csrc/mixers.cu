@@ -28,6 +28,7 @@ struct DecodeArgs {
   float* out;
   const unsigned* d_pos;
   int* status;
+  bool first;   // ssd: the first pass of recur_decode_head
 };
 
 // ---- attention, one token ------------------------------------------------------------------
@@ -398,28 +399,49 @@ template <> __device__ __forceinline__ Cols<4> cols_ld<4>(const float* p) {
 __device__ __forceinline__ void cols_st(float* p, const Cols<1>& c) { *p = c.f[0]; }
 __device__ __forceinline__ void cols_st(float* p, const Cols<4>& c) { *(float4*)p = make_float4(c.f[0], c.f[1], c.f[2], c.f[3]); }
 
-// S <- g S + k u^T and o = q S, u = in v or, for the delta rule, in (v - k (g S)).  src: the state, in shared or global
-// memory (NULL: zero), dst: where the new one goes; red holds MX_THREADS * V floats.  The whole block; barriers inside.
-template <int V>
-__device__ void recur_update(const RecurP& p, const float* src, float* dst, const float* q, const float* k, const float* v,
-                             float* o, float* red, float g, float in, bool delta) {
+// S <- g S + k u^T and o = q S, u = in v or, for the delta rule, in (v - k (g S)); zero instead of S where `fresh`.  The
+// state's rows below R lie in shared memory (st), FAR: the others where S is; red holds MX_THREADS * V floats.  The whole
+// block; barriers inside.
+template <int V, bool FAR>
+__device__ void recur_update(const RecurP& p, float* st, int R, float* S, bool fresh, const float* q, const float* k,
+                             const float* v, float* o, float* red, float g, float in, bool delta) {
+  constexpr int B = V == 4 ? 8 : 16;   // rows that a thread asks memory for at once
   const int tid = threadIdx.x, D = p.D, E = p.E;
 #pragma unroll 1
   for (int c0 = 0; c0 < E; c0 += MX_THREADS * V) {
     const int w = E - c0 < MX_THREADS * V ? E - c0 : MX_THREADS * V, ct = w / V, RG = MX_THREADS / ct;
     const int rg = tid / ct, cl = (tid - rg * ct) * V, c = c0 + cl;
     const bool on = rg < RG;
+    // B rows from r0 on, in steps of RG (the first one again for those behind the last)
+    auto far_rows = [&](int r0, Cols<V> (&x)[B]) {
+#pragma unroll
+      for (int i = 0; i < B; i++) x[i] = cols_ld<V>(S + (size_t)(r0 + i * RG < D ? r0 + i * RG : r0) * E + c);
+    };
     Cols<V> u, acc;
 #pragma unroll
     for (int e = 0; e < V; e++) acc.f[e] = u.f[e] = 0.f;
     if (delta) {
-      if (on && src) {
+      if (on && !fresh) {
 #pragma unroll 2
-        for (int r = rg; r < D; r += RG) {
-          const Cols<V> x = cols_ld<V>(src + (size_t)r * E + c);
+        for (int r = rg; r < R; r += RG) {
+          const Cols<V> x = cols_ld<V>(st + (size_t)r * E + c);
 #pragma unroll
           for (int e = 0; e < V; e++) acc.f[e] = fmaf(k[r], x.f[e] * g, acc.f[e]);
         }
+        if (FAR)
+#pragma unroll 1
+          for (int r0 = R + rg; r0 < D; r0 += RG * B) {
+            Cols<V> x[B];
+            far_rows(r0, x);
+#pragma unroll
+            for (int i = 0; i < B; i++) {
+              // (no branch: one around each row would make its load wait for the row before)
+              const bool there = r0 + i * RG < D;
+              const float kk = there ? k[r0 + i * RG] : 0.f;
+#pragma unroll
+              for (int e = 0; e < V; e++) acc.f[e] = fmaf(kk, there ? x[i].f[e] * g : 0.f, acc.f[e]);
+            }
+          }
       }
       if (on) cols_st(red + rg * w + cl, acc);
       __syncthreads();
@@ -439,19 +461,31 @@ __device__ void recur_update(const RecurP& p, const float* src, float* dst, cons
     }
 #pragma unroll
     for (int e = 0; e < V; e++) acc.f[e] = 0.f;
+    auto update = [&](float* at, int r, Cols<V> x) {
+      const float kk = k[r], qq = q[r];
+#pragma unroll
+      for (int e = 0; e < V; e++) {
+        x.f[e] = fmaf(kk, u.f[e], fresh ? 0.f : x.f[e] * g);
+        acc.f[e] = fmaf(qq, x.f[e], acc.f[e]);
+      }
+      cols_st(at + (size_t)r * E + c, x);
+    };
     if (on) {
 #pragma unroll 2
-      for (int r = rg; r < D; r += RG) {
+      for (int r = rg; r < R; r += RG) {
         Cols<V> x;
-        if (src) x = cols_ld<V>(src + (size_t)r * E + c);
-        const float kk = k[r], qq = q[r];
-#pragma unroll
-        for (int e = 0; e < V; e++) {
-          x.f[e] = fmaf(kk, u.f[e], src ? x.f[e] * g : 0.f);
-          acc.f[e] = fmaf(qq, x.f[e], acc.f[e]);
-        }
-        cols_st(dst + (size_t)r * E + c, x);
+        if (!fresh) x = cols_ld<V>(st + (size_t)r * E + c);
+        update(st, r, x);
       }
+      if (FAR)
+#pragma unroll 1
+        for (int r0 = R + rg; r0 < D; r0 += RG * B) {
+          Cols<V> x[B];
+          if (!fresh) far_rows(r0, x);
+#pragma unroll
+          for (int i = 0; i < B; i++)
+            if (r0 + i * RG < D) update(S, r0 + i * RG, x[i]);
+        }
     }
     if (on) cols_st(red + rg * w + cl, acc);
     __syncthreads();
@@ -465,21 +499,30 @@ __device__ void recur_update(const RecurP& p, const float* src, float* dst, cons
   }
 }
 
-// Floats of a head's block beside its state, and of the state that wait in shared memory (0: it is too large, also together
-// with the others, or not whole 16-byte pieces).
-constexpr size_t MX_SMEM = 204 * 1024, MX_STATE_SMEM = 16384;
+// Floats of a head's block beside its state, and the rows of the state that wait in shared memory: all of a state of up to
+// 64 KB, else as many as that holds; whole 16-byte pieces; and no more than leaves room for two blocks an SM.  The others
+// come from memory behind the wait, B rows of a thread in flight.  Six layers a token, us, with everything in registers /
+// all of such a state from memory, a row or two in flight / this: delta 64 heads of 128 x 256 324 / 421 / 298, 16 of
+// 256 x 256 278 / 273 / 236, 16 of 128 x 512 301 / 341 / 291, 16 of 128 x 255 210 / 320 / 211; SSD 64 heads of 128 x 256
+// 293 / 274 / 242, 16 of 1024 x 256 669 / 930 / 421, 16 of 136 x 124 178 / 139 / 130.
 __host__ __device__ inline size_t recur_head_floats(const RecurP& p) { return (size_t)4 * p.D + 3 * p.E + 4 * MX_THREADS + 44; }
-__host__ __device__ inline int recur_state_floats(const RecurP& p) {
-  const size_t n = (size_t)p.D * p.E;
-  return n <= MX_STATE_SMEM && n % 4 == 0 && (n + recur_head_floats(p)) * sizeof(float) <= MX_SMEM ? (int)n : 0;
+__host__ __device__ inline int recur_near_rows(const RecurP& p) {
+  constexpr size_t STATE = 16384, BLOCK = 112 * 1024 / sizeof(float);
+  const size_t n = (size_t)p.D * p.E, rest = recur_head_floats(p);
+  if (n % 4 || rest >= BLOCK) return 0;
+  const size_t room = BLOCK - rest < STATE ? BLOCK - rest : STATE;
+  return n <= room ? p.D : (int)(room / p.E) & ~3;
 }
 
 // One block a head.  The state and the convolutions' history are fetched before the projected row is there.  (The row is
 // read past the L1: what the first pass saw of it may be old.)
-__device__ void recur_decode_head(const RecurP& p, int h, const float* row, float* out, int pos, float* sm, int* status) {
+// first: the code behind the wait is gone through once in front of it, with nothing kept.
+template <bool FAR>
+__device__ void recur_decode_head(const RecurP& p, int h, const float* row, float* out, int pos, float* sm, int* status,
+                                  bool first) {
   __shared__ __align__(8) uint64_t bar;
   const int tid = threadIdx.x, D = p.D, E = p.E, rep = p.H / p.G, kg = h / rep, n = 2 * D + E;
-  const int ns = recur_state_floats(p);
+  const int R = FAR ? recur_near_rows(p) : D, ns = R * E;
   float* st = sm;              // [ns] state
   float* q = st + ns;          // [D]
   float* k = q + D;            // [D]
@@ -499,7 +542,7 @@ __device__ void recur_decode_head(const RecurP& p, int h, const float* row, floa
   const int taps = p.cv.taps;
   const float A_log = p.A_log[h], bias = p.dt_bias[h], skip = p.kind == MIX_SSD ? p.Dskip[h] : 0.f;
   const float nw = p.kind == MIX_DELTA && tid < E ? p.norm[tid] : 0.f;
-  int pass = p.kind == MIX_DELTA;
+  int pass = FAR || !first;
   asm volatile("" : "+r"(pass));
 #pragma unroll 1
   for (; pass < 2; pass++) {
@@ -507,7 +550,7 @@ __device__ void recur_decode_head(const RecurP& p, int h, const float* row, floa
     if (real) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncthreads();   // the first pass has left shared memory
-      if (tid == 0 && ns && pos > 0) {
+      if (tid == 0 && ns > 0 && pos > 0) {
         mbar_expect_tx(&bar, ns * 4);
         bulk_load_1d(st, S, ns * 4, &bar);
       }
@@ -563,15 +606,13 @@ __device__ void recur_decode_head(const RecurP& p, int h, const float* row, floa
       for (int i = tid; i < D; i += MX_THREADS) { q[i] *= fq; k[i] *= fk; }
       __syncthreads();
     }
-    const float* src = pos > 0 ? (ns ? st : S) : nullptr;
-    bool ok = real || ns;   // (the first pass leaves a state in global memory alone)
-    if (real && ns && pos > 0) ok = mbar_wait_bounded(&bar, 0, status, 810);
+    bool ok = true;
+    if (real && ns > 0 && pos > 0) ok = mbar_wait_bounded(&bar, 0, status, 810);
     if (__syncthreads_and(ok)) {
       // (16-byte pieces need every part of shared memory on 16 bytes)
-      float* dst = ns ? st : S;
-      if ((E & 3) == 0 && (D & 1) == 0) recur_update<4>(p, src, dst, q, k, v, o, red, g, in, delta);
-      else recur_update<1>(p, src, dst, q, k, v, o, red, g, in, delta);
-      if (ns && real) {   // back in one copy, under the read-out below (update ended with a barrier)
+      if ((E & 3) == 0 && (D & 1) == 0) recur_update<4, FAR>(p, st, R, S, pos == 0, q, k, v, o, red, g, in, delta);
+      else recur_update<1, FAR>(p, st, R, S, pos == 0, q, k, v, o, red, g, in, delta);
+      if (ns > 0 && real) {   // back in one copy, under the read-out below (update ended with a barrier)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (tid == 0) {
@@ -658,7 +699,9 @@ __host__ __device__ inline int recur_blocks(const RecurP& p) {
   return p.kind == MIX_GLA ? p.H * ((p.E + GL_COLS - 1) / GL_COLS) : p.H;
 }
 
-template <typename KT, int RM, bool FAST>
+// FAR: a recurrent mixer has rows of its state in memory.  An instantiation of its own: in one for all, a token whose states
+// fit took 261 us instead of 253 (registers).
+template <typename KT, int RM, bool FAST, bool FAR>
 __global__ void __launch_bounds__(MX_THREADS, 2) mixers_decode_kernel(const __grid_constant__ DecodeArgs a) {
   extern __shared__ __align__(16) float sm[];
   const int pos = (int)*a.d_pos;
@@ -668,7 +711,7 @@ __global__ void __launch_bounds__(MX_THREADS, 2) mixers_decode_kernel(const __gr
     const int n = recur_blocks(a.rec[i]);
     if (b < n) {
       if (a.rec[i].kind == MIX_GLA) gla_decode_unit(a.rec[i], b, a.proj, a.out, pos, sm);
-      else recur_decode_head(a.rec[i], b, a.proj, a.out, pos, sm, a.status);
+      else recur_decode_head<FAR>(a.rec[i], b, a.proj, a.out, pos, sm, a.status, a.first && a.rec[i].kind == MIX_SSD);
       return;
     }
     b -= n;
@@ -1050,18 +1093,22 @@ size_t attn_smem(const AttnP& p, int rm) {
 }
 size_t recur_smem(const RecurP& p) {
   if (p.kind == MIX_GLA) return (size_t)(3 * p.D + MX_THREADS + p.D * GL_COLS) * sizeof(float);
-  return (recur_state_floats(p) + recur_head_floats(p)) * sizeof(float);
+  return ((size_t)recur_near_rows(p) * p.E + recur_head_floats(p)) * sizeof(float);
 }
 int rm_of(int hpb) { return hpb <= 1 ? 1 : (hpb <= 2 ? 2 : (hpb <= 4 ? 4 : 8)); }
 
-template <typename KT, int RM, bool FAST>
+template <typename KT, int RM, bool FAST, bool FAR>
 int decode_launch(const DecodeArgs& a, int blocks, size_t smem, cudaStream_t s) {
   static std::atomic<unsigned long long> done{0};
-  const int rc = ensure_dynamic_smem(mixers_decode_kernel<KT, RM, FAST>, MX_SMEM, done);
+  const int rc = ensure_dynamic_smem(mixers_decode_kernel<KT, RM, FAST, FAR>, 204 * 1024, done);
   if (rc) return rc;
   LaunchCfg lc(dim3(blocks), dim3(MX_THREADS), smem, s, pdl_enabled());
-  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, mixers_decode_kernel<KT, RM, FAST>, a));
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, mixers_decode_kernel<KT, RM, FAST, FAR>, a));
   return TLB_OK;
+}
+template <typename KT, int RM, bool FAST>
+int decode_far(const DecodeArgs& a, int blocks, size_t smem, bool far, cudaStream_t s) {
+  return far ? decode_launch<KT, RM, FAST, true>(a, blocks, smem, s) : decode_launch<KT, RM, FAST, false>(a, blocks, smem, s);
 }
 template <typename KT, int RM>
 int attn_rows_t(const AttnP& p, const void* q, const float* proj, long long ld, void* act, long long lda, int rows,
@@ -1101,9 +1148,10 @@ int scan_d(const RecurP& p, const float* conv, long long ld, const void* gates, 
 int mixers_decode_launch(const AttnP* attn, const RecurP* rec, int n_rec, const float* proj, float* out,
                          const unsigned* d_pos, bool kv_bf16, cudaStream_t s) {
   DecodeArgs a{};
+  a.first = true;
   int rm = 1;
   size_t smem = 0;
-  bool fast = true;
+  bool fast = true, far = false;
   if (attn) {
     a.at = *attn;
     fast = attn->Dp <= 128 && attn->Ep <= 128;
@@ -1118,6 +1166,7 @@ int mixers_decode_launch(const AttnP* attn, const RecurP* rec, int n_rec, const 
     blocks += recur_blocks(rec[i]);
     const size_t n = recur_smem(rec[i]);
     smem = n > smem ? n : smem;
+    far = far || (rec[i].kind != MIX_GLA && recur_near_rows(rec[i]) < rec[i].D);
   }
   a.proj = proj; a.out = out; a.d_pos = d_pos;
   {
@@ -1128,9 +1177,9 @@ int mixers_decode_launch(const AttnP* attn, const RecurP* rec, int n_rec, const 
   }
 #define MX_CASE(m)                                                                     \
   if (rm == m)                                                                         \
-    return !kv_bf16 ? decode_launch<float, m, false>(a, blocks, smem, s)                  \
-           : fast   ? decode_launch<__nv_bfloat16, m, true>(a, blocks, smem, s)           \
-                    : decode_launch<__nv_bfloat16, m, false>(a, blocks, smem, s);
+    return !kv_bf16 ? decode_far<float, m, false>(a, blocks, smem, far, s)                \
+           : fast   ? decode_far<__nv_bfloat16, m, true>(a, blocks, smem, far, s)         \
+                    : decode_far<__nv_bfloat16, m, false>(a, blocks, smem, far, s);
   MX_CASE(1) MX_CASE(2) MX_CASE(4) MX_CASE(8)
 #undef MX_CASE
   return set_error(TLB_ERR_STATE, "mixers: no head-block width");

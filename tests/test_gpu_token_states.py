@@ -38,6 +38,12 @@ def test_token_states(heads, groups, state, vdim, conv, norm_groups, dtype):
     (1, 16384),     # a state of 64 KB that does not fit beside its own values
     (1, 12788),     # the widest of one row that does
     (1, 12792),     # ... and that does not
+    (1, 6900),      # the widest of one row that leaves room for two blocks an SM
+    (1, 6904),      # ... and that does not
+    (128, 256),     # half of the rows in shared memory
+    (96, 255),      # 64 of 96 rows, one column a thread
+    (63, 65),       # not whole 16-byte pieces
+    (1024, 20),     # the most rows
 ])
 def test_wide_heads(state, vdim, dtype):
     """Heads on both sides of what waits in shared memory."""
