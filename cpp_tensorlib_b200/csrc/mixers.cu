@@ -381,10 +381,15 @@ __device__ void attn_decode_unit16(const AttnP& p, int unit, const float* row, f
 // A launch runs this code once, from a cold instruction cache, at some twenty cycles an instruction: what it costs is its
 // length.  A state held in registers, 32 rows a thread with everything unrolled, took 3 - 4 us for the arithmetic of 0.3 and
 // 1.3 us for its stores (timer in the kernel, 64 heads of 128 x 64).  So the state goes to shared memory in front of the
-// wait and the loops over its rows stay loops (2.8 us), and since the block of an SSD head waits 7 us for the projection
-// anyway, it first goes through the code behind the wait once with nothing kept (1.4 us).  The delta rule's code is longer
-// than that wait (its first pass ended 4 us late), so it is gone through once.  A token of the 8-layer Mamba and delta stack:
-// 285 -> 259 us; of the latent-attention and GLA stack 377 -> 373.
+// wait and the loops over its rows stay loops (2.8 us), and where the block of an SSD head waits long enough for the
+// projection anyway (MX_FIRST_BYTES), it first goes through the code behind the wait once with nothing kept (1.4 us).  The
+// delta rule's code is longer than the wait of a 2048-wide projection (its first pass ended 4 us late), so it is gone
+// through once.  A token of the 8-layer Mamba and delta stack: 285 -> 259 us; of the latent-attention and GLA stack
+// 377 -> 373.
+// The projection's matrix from which on the first pass ends inside the wait: below that the launch comes late by it.  A token
+// of the 8-layer stack (six SSD layers), us with / without: 1.6 MB 169 / 151, 4.2 MB 172 / 151, 8 MB 182 / 171, 12.6 MB
+// 183 / 173, 15.8 MB (f32) 187 / 175, 18.5 MB 212 / 218, 25 MB 218 / 225, in f32 200 / 199, 42 MB 251 / 262, 89 MB 428 / 440.
+constexpr size_t MX_FIRST_BYTES = (size_t)16 << 20;
 
 // rows of the state for the columns c0.. of a block's threads: V columns a thread, the rows dealt to the row groups
 template <int V> struct Cols { float f[V]; };
@@ -1146,9 +1151,9 @@ int scan_d(const RecurP& p, const float* conv, long long ld, const void* gates, 
 }  // namespace
 
 int mixers_decode_launch(const AttnP* attn, const RecurP* rec, int n_rec, const float* proj, float* out,
-                         const unsigned* d_pos, bool kv_bf16, cudaStream_t s) {
+                         const unsigned* d_pos, bool kv_bf16, size_t in_bytes, cudaStream_t s) {
   DecodeArgs a{};
-  a.first = true;
+  a.first = in_bytes >= MX_FIRST_BYTES;
   int rm = 1;
   size_t smem = 0;
   bool fast = true, far = false;

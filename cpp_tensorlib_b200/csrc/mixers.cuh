@@ -326,8 +326,9 @@ __device__ __forceinline__ float gla_rate(float z, float tau) { return softplus_
 #endif  // __CUDACC__
 
 // launchers (mixers.cu, rows.cu)
+// in_bytes: of the matrix that the launch in front, which makes proj, streams
 int mixers_decode_launch(const AttnP* attn, const RecurP* rec, int n_rec, const float* proj, float* out,
-                         const unsigned* d_pos, bool kv_bf16, cudaStream_t s);
+                         const unsigned* d_pos, bool kv_bf16, size_t in_bytes, cudaStream_t s);
 int attn_rows_prep_launch(const AttnP& p, const float* proj, long long ld, int rows, int pos0, void* q, bool bf16,
                           cudaStream_t s);
 int attn_rows_launch(const AttnP& p, const void* q, const float* proj, long long ld, void* act, long long lda, int rows,

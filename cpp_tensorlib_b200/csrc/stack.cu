@@ -169,7 +169,8 @@ int StackDecoder::forward(cudaStream_t s) {
     if (!post_norm) normed(g, L.norm1, 0, hidden, 1, 1.f);
     RUN(gemv(g));
     if (L.has_attn || L.n_rec)
-      RUN(mixers_decode_launch(L.has_attn ? &L.at : nullptr, L.rec, L.n_rec, proj, act, d_pos, bf16, s));
+      RUN(mixers_decode_launch(L.has_attn ? &L.at : nullptr, L.rec, L.n_rec, proj, act, d_pos, bf16,
+                               (size_t)L.in.N * L.in.ld * es(), s));
     if (L.has_latent) {
       g = product1(L.uq, proj + L.la.oq, qv, 0);
       normed(g, L.la.qn, 0, L.la.Q, 1, 1.f);

@@ -56,3 +56,17 @@ def test_wide_heads(state, vdim, dtype):
     got = run(m, toks, [])
     assert np.isfinite(got).all() and ok(err(got, want), dtype)
     close(m)
+
+
+@pytest.mark.parametrize("width,dtype", [(896, "float32"), (912, "float32"), (1800, "bfloat16"), (1816, "bfloat16")])
+def test_first_pass(width, dtype):
+    """Projections of 4640 rows on both sides of 16 MiB, where the code in front of the wait changes."""
+    cfg = zc.config([zc.mam(32, 4, 64, 64, 4, 2)] * 2, width=width, vocab=151, emb=1.0)
+    w = zc.Weights(cfg, 7)
+    toks = zc.tokens(cfg, 9, 2)
+    want = orc.forward(cfg, w.f64(), toks)
+    m = make(cfg, w, dtype, 16)
+    m.capture()
+    got = run(m, toks, [])
+    assert np.isfinite(got).all() and ok(err(got, want), dtype)
+    close(m)
