@@ -7,7 +7,8 @@
 // it costs is the chain from the end of the launch in front to the first weight used.  So
 //   - a block takes at most half an SM (112 KB, 96 registers x 288 threads): the next launch's block fits beside it and has
 //     its ring of weights full when this launch ends.  One block an SM, a contiguous range of rows each, so that a stage
-//     of the ring (8 rows of 2048, 4 of 4096, ...) is one bulk copy;
+//     of the ring (8 rows of 2048, 4 of 4096, ...) is one bulk copy.  (Rows of 16 - 32 KB, up to
+//     eight chunks a thread, take the registers of a whole SM: the next launch's ring starts when a block ends);
 //   - a thread owns the same 16-byte chunks of every row: its activations go from memory to its registers, without shared
 //     memory or a barrier, all loads in flight at once;
 //   - the factor of a norm over the whole row multiplies the sums instead of the activations; the norms' weights are
@@ -52,52 +53,23 @@ __device__ __forceinline__ void rg_ld(const float* base, int i, int n, float (&o
     o[k] = on ? v.x : 0.f; o[k + 1] = on ? v.y : 0.f; o[k + 2] = on ? v.z : 0.f; o[k + 3] = on ? v.w : 0.f;
   }
 }
-// the same for any n and alignment
-template <int N>
-__device__ __forceinline__ void rg_ld_any(const float* base, int i, int n, float (&o)[N]) {
-#pragma unroll
-  for (int k = 0; k < N; k++) o[k] = i + k >= 0 && i + k < n ? __ldcg(base + i + k) : 0.f;
-}
 
-// What the elements of the row are multiplied with needs sums over it: of the whole row the factor is taken out of
-// the product (rg_scale), of a segment in parts a warp sums each part here.  gs [n_groups], ends with a barrier.
+// A norm over the whole row: its factor multiplies the row sums instead of the elements.  (Of a segment, in parts or not,
+// the elements are multiplied with their part's factor, gs.)
 __device__ __forceinline__ bool rg_whole(const RowGemv& p) { return p.nw && p.n_groups == 1 && p.n_len == p.K; }
-__device__ __forceinline__ void rg_parts(const RowGemv& p, float* gs) {
-  const int m = p.n_len / p.n_groups, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll 1
-  for (int g = warp; g < p.n_groups; g += RG_WARPS) {
-    float q = 0.f;
-#pragma unroll 1
-    for (int i0 = 0; i0 < m; i0 += 512) {
-      float v[16];
-#pragma unroll
-      for (int k = 0; k < 16; k++) v[k] = i0 + lane + 32 * k < m ? __ldcg(p.x + p.n_off + g * m + i0 + lane + 32 * k) : 0.f;
-#pragma unroll
-      for (int k = 0; k < 16; k++) q = fmaf(v[k], v[k], q);
-    }
-    q = warp_sum(q);
-    if (lane == 0) gs[g] = rsqrtf(q / m + p.eps) * p.nscale;
-  }
-}
 // N elements of the staged row from e0 on: v holds them as they are in x, w the norm's weights, r and rn the residual and
 // its weights, g the gate; s is the residual's scale
-// (WHOLE: the segment and its parts are whole pieces of N elements)
-template <int N, bool WHOLE>
+// (the row, the segment and its parts are whole pieces of N elements)
+template <int N>
 __device__ __forceinline__ void rg_prepare(const RowGemv& p, int e0, float (&v)[N], const float (&w)[N], const float (&r)[N],
                                            const float (&rn)[N], const float (&g)[N], float s, const float* gs, unsigned magic, float& sq) {
   if (p.res) {
 #pragma unroll
     for (int k = 0; k < N; k++) v[k] = fmaf(v[k] * s, rn[k], r[k]);
     if (p.xout && blockIdx.x == 0) {
-      if (WHOLE) {
-        if (e0 < p.K)
+      if (e0 < p.K)
 #pragma unroll
-          for (int k = 0; k < N; k += 4) *(float4*)(p.xout + e0 + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
-      } else {
-#pragma unroll
-        for (int k = 0; k < N; k++)
-          if (e0 + k < p.K) p.xout[e0 + k] = v[k];
-      }
+        for (int k = 0; k < N; k += 4) *(float4*)(p.xout + e0 + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
     }
   }
 #pragma unroll
@@ -109,22 +81,10 @@ __device__ __forceinline__ void rg_prepare(const RowGemv& p, int e0, float (&v)[
     return;
   }
   if (e0 + N <= p.n_off || e0 >= p.n_off + p.n_len) return;
-  if constexpr (WHOLE) {
-    const unsigned c = (unsigned)((e0 - p.n_off) / N);
-    const float f = gs[magic ? __umulhi(c, magic) : c];
+  const unsigned c = (unsigned)((e0 - p.n_off) / N);
+  const float f = gs[magic ? __umulhi(c, magic) : c];
 #pragma unroll
-    for (int k = 0; k < N; k++) v[k] *= p.gate ? f * w[k] * silu_f(g[k]) : f * w[k];
-    return;
-  }
-  const int m = p.n_len / p.n_groups;
-  int part = e0 <= p.n_off ? 0 : (e0 - p.n_off) / m;
-#pragma unroll
-  for (int k = 0; k < N; k++) {
-    const int e = e0 + k - p.n_off;
-    if (e < 0 || e >= p.n_len) continue;
-    if (e >= (part + 1) * m) part++;
-    v[k] *= p.gate ? gs[part] * w[k] * silu_f(g[k]) : gs[part] * w[k];
-  }
+  for (int k = 0; k < N; k++) v[k] *= p.gate ? f * w[k] * silu_f(g[k]) : f * w[k];
 }
 // R sums over a warp: afterwards lane l holds the sum of v[rg_sum_of<R>(l)] in v[0]
 template <int R>
@@ -269,7 +229,7 @@ __global__ void __launch_bounds__(RG_THREADS + 32, JN < 8 ? 2 : 1) row_gemv_kern
   for (int j = 0; j < JN; j++) {
     if (!ONE) { ld_rn(j); ld_res(j); }
     if (!FEW) { ld_nw(j, nw[0]); ld_gate(j, gate[0]); }
-    rg_prepare<CE, true>(p, (c0 + j * RG_THREADS) * CE, x[j], nw[FEW ? j : 0], res, rn, gate[FEW ? j : 0], s, gs, pl.part_magic, sq);
+    rg_prepare<CE>(p, (c0 + j * RG_THREADS) * CE, x[j], nw[FEW ? j : 0], res, rn, gate[FEW ? j : 0], s, gs, pl.part_magic, sq);
   }
   if (rg_whole(p)) {
     sq = warp_sum(grp == 0 ? sq : 0.f);
@@ -324,56 +284,235 @@ __global__ void __launch_bounds__(RG_THREADS + 32, JN < 8 ? 2 : 1) row_gemv_kern
     rg_emit(p, r0 + r, row_sum(r), u == 2 ? row_sum(r + 1) : 0.f, p.epi != 1 || r == tid ? y0 : p.y[r0 + r]);
 }
 
-// Rows too long for the registers of a block, and rows of odd widths or places: the staged row in shared memory, weights straight from memory, a block
-// for a row (or pair) at a time.
-template <typename WT>
-__global__ void __launch_bounds__(RG_THREADS) row_gemv_long_kernel(const __grid_constant__ RowGemv p) {
-  constexpr int CE = Vec16<WT>::N;
-  extern __shared__ __align__(128) unsigned char smem[];
+// ---- rows too long for the registers of a block, and rows of odd widths or places ------------
+// The staged row in shared memory, weights straight from memory: a stream of ks adjacent warps owns one row, or two adjacent
+// rows (gate and up interleaved), each warp its own part of K; ks is picked on the host so that the streams of all SMs come
+// out even.  Every warp keeps eight 16-byte loads in flight plus the next eight, and the first eight are issued in front of
+// the wait.
+// What lies where, us a token of models with such products, streams / ring: rows of 16384 in bf16 (`down` of four layers of
+// 4096 x 16384) 460 / 436, of 14336 371 / 362, of 10240 282 / 275; f32 rows of 8192 281 / 285, of 4928 188 / 188.  Longer rows
+// do not fit the ring's registers: 20000 in bf16 325 (a block for a row at a time, three barriers a row, 393), 16384 in f32
+// 769 (951).
+constexpr size_t RS_SMEM_MAX = 225 * 1024;
+
+__device__ __forceinline__ uint4 rs_ld(const void* p, uint64_t pol) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(pol));
+  return v;
+}
+
+// x into xs [ldw], zero behind K; returns this thread's share of its sum of squares.  Kept short: a
+// launch runs this code once, from a cold instruction cache.
+__device__ __forceinline__ float rs_stage(const RowGemv& p, float* xs) {
+  float sq = 0.f;
+  const int k4 = ((uintptr_t)p.x & 15) ? 0 : p.K / 4;   // rows of an odd width go one by one
+  for (int i0 = threadIdx.x; i0 < k4; i0 += 4 * RG_THREADS) {
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (i0 + u * RG_THREADS < k4) v[u] = ((const float4*)p.x)[i0 + u * RG_THREADS];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (i0 + u * RG_THREADS < k4) {
+        ((float4*)xs)[i0 + u * RG_THREADS] = v[u];
+        sq = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, fmaf(v[u].w, v[u].w, sq))));
+      }
+  }
+#pragma unroll 1
+  for (int i = 4 * k4 + threadIdx.x; i < p.ldw; i += RG_THREADS) {
+    const float x = i < p.K ? p.x[i] : 0.f;
+    xs[i] = x;
+    sq = fmaf(x, x, sq);
+  }
+  return sq;
+}
+
+// the preceding sublayer's output, normed, added to the residual: every block computes the row, block 0
+// leaves it for the launches behind.  Returns the thread's share of the new row's sum of squares.
+__device__ __forceinline__ float rs_residual(const RowGemv& p, float* xs, float sq, float* red) {
+  const float s = rsqrtf(block_sum(sq, red) / p.K + p.eps);
+  sq = 0.f;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < p.K; i += RG_THREADS) {
+    const float v = fmaf(xs[i] * s, p.rn[i], p.res[i]);
+    xs[i] = v;
+    if (p.xout && blockIdx.x == 0) p.xout[i] = v;
+    sq = fmaf(v, v, sq);
+  }
+  return sq;
+}
+
+// the norm in place: the whole row by the block, a segment in parts a warp each
+__device__ __forceinline__ void rs_norm(const RowGemv& p, float* xs, float sq, float* red) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (p.n_groups == 1 && p.n_len == p.K) {
+    const float s = rsqrtf(block_sum(sq, red) / p.K + p.eps) * p.nscale;
+#pragma unroll 4
+    for (int i = tid; i < p.K; i += RG_THREADS) xs[i] *= p.gate ? s * p.nw[i] * silu_f(p.gate[i]) : s * p.nw[i];
+    return;
+  }
+  __syncthreads();
+  const int m = p.n_len / p.n_groups;
+#pragma unroll 1
+  for (int g = tid >> 5; g < p.n_groups; g += RG_WARPS) {
+    float* seg = xs + p.n_off + g * m;
+    float q = 0.f;
+#pragma unroll 4
+    for (int i = lane; i < m; i += 32) q = fmaf(seg[i], seg[i], q);
+    const float s = rsqrtf(warp_sum(q) / m + p.eps) * p.nscale;
+#pragma unroll 4
+    for (int i = lane; i < m; i += 32)
+      seg[i] *= p.gate ? s * p.nw[g * m + i] * silu_f(p.gate[g * m + i]) : s * p.nw[g * m + i];
+  }
+}
+
+template <int R>
+__device__ __forceinline__ void rs_emit(const RowGemv& p, int rg, const float (&a)[R]) {
+  if (p.epi == 2) {
+    if (R == 2) rg_emit(p, 2 * rg, a[0], a[R - 1], 0.f);
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const int n = rg * R + r;
+    if (n < p.N) rg_emit(p, n, a[r], 0.f, p.epi == 1 ? p.y[n] : 0.f);
+  }
+}
+
+template <typename WT, int R>
+__global__ void __launch_bounds__(RG_THREADS, 2) row_gemv_stream_kernel(const __grid_constant__ RowGemv p, int ks) {
+  constexpr int CE = Vec16<WT>::N, U = 8 / R;
+  extern __shared__ __align__(16) float xs[];   // [ldw], then the streams' partial sums
   __shared__ float red[33];
-  float* xs = (float*)smem;
-  float* gs = xs + p.ldw;
-  const int tid = threadIdx.x, chunks = (int)(p.ldw / CE), u = p.epi == 2 ? 2 : 1, units = (p.N + u - 1) / u;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int groups = (p.N + R - 1) / R, ns = RG_WARPS / ks, stream = warp / ks, sub = warp - stream * ks;
+  const int stride = gridDim.x * ns, chunks = (int)(p.ldw / CE), per = (chunks + ks - 1) / ks;
+  const int c_lo = sub * per, c_hi = c_lo + per < chunks ? c_lo + per : chunks;
+  float* part = xs + p.ldw;                     // [local group][stream][R][ks]
+  const WT* W = (const WT*)p.W;
+  const uint64_t pol = l2_evict_first_policy();
+  int rg = blockIdx.x * ns + stream, cb = c_lo, loc = 0;
+  uint4 cur[R][U], nxt[R][U];
+  auto fetch = [&](uint4 (&w)[R][U], int g, int b) {
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const WT* row = W + (size_t)(g * R + r < p.N ? g * R + r : p.N - 1) * p.ldw;
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int c = b + lane + 32 * u;
+        w[r][u] = c < c_hi ? rs_ld(row + (size_t)c * CE, pol) : make_uint4(0, 0, 0, 0);
+      }
+    }
+  };
+  if (rg < groups) fetch(cur, rg, cb);
+  if (p.nw)   // the norm's weights into the L2
+    for (int i = tid * 32; i < p.n_len; i += RG_THREADS * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.nw + i));
+  if (p.rn)
+    for (int i = tid * 32; i < p.K; i += RG_THREADS * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.rn + i));
   pdl_wait();
   pdl_launch_dependents();
-  float s = 0.f, sq = 0.f;
-  if (p.res) {
-    for (int i = tid; i < p.K; i += RG_THREADS) { const float v = p.x[i]; sq = fmaf(v, v, sq); }
-    s = rsqrtf(block_sum(sq, red) / p.K + p.eps);
-    sq = 0.f;
-  }
-  if (p.nw && !rg_whole(p)) rg_parts(p, gs);
+  float sq = rs_stage(p, xs);
+  if (p.res) sq = rs_residual(p, xs, sq, red);
+  if (p.nw) rs_norm(p, xs, sq, red);
   __syncthreads();
-  for (int c = tid; c < chunks; c += RG_THREADS) {
-    float v[CE];
-    float w[CE], r[CE], rn[CE], g[CE];
-    rg_ld_any<CE>(p.x, c * CE, p.K, v);
-    if (p.nw) rg_ld_any<CE>(p.nw, c * CE - p.n_off, p.n_len, w);
-    if (p.rn) rg_ld_any<CE>(p.rn, c * CE, p.K, rn);
-    if (p.res) rg_ld_any<CE>(p.res, c * CE, p.K, r);
-    if (p.gate) rg_ld_any<CE>(p.gate, c * CE - p.n_off, p.n_len, g);
-    rg_prepare<CE, false>(p, c * CE, v, w, r, rn, g, s, gs, 0u, sq);
+  float acc[R][2];
 #pragma unroll
-    for (int e = 0; e < CE; e++) xs[c * CE + e] = v[e];
-  }
-  sq = block_sum(sq, red);
-  const float f = rg_whole(p) ? rsqrtf(sq / p.K + p.eps) * p.nscale : 1.f;
-  for (int b = blockIdx.x; b < units; b += gridDim.x) {
-    float a[2] = {0.f, 0.f};
-    for (int r = 0; r < u; r++) {
-      const uint4* w = (const uint4*)((const WT*)p.W + (size_t)(b * u + r) * p.ldw);
-      float acc = 0.f;
-#pragma unroll 4
-      for (int c = tid; c < chunks; c += RG_THREADS) {
-        float wv[CE];
-        widen16(__ldcs(w + c), wv, (const WT*)nullptr);
+  for (int r = 0; r < R; r++) acc[r][0] = acc[r][1] = 0.f;
+  while (rg < groups) {
+    int ng = rg, nb = cb + 32 * U;
+    if (nb >= c_hi) { ng += stride; nb = c_lo; }
+    if (ng < groups) fetch(nxt, ng, nb);
 #pragma unroll
-        for (int e = 0; e < CE; e++) acc = fmaf(wv[e], xs[c * CE + e], acc);
+    for (int u = 0; u < U; u++) {
+      const int c = cb + lane + 32 * u;
+      if (c < c_hi) {
+        float x[CE];
+#pragma unroll
+        for (int e = 0; e < CE; e += 4) {
+          const float4 v = *(const float4*)(xs + (size_t)c * CE + e);
+          x[e] = v.x; x[e + 1] = v.y; x[e + 2] = v.z; x[e + 3] = v.w;
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          float w[CE];
+          widen16(cur[r][u], w, (const WT*)nullptr);
+#pragma unroll
+          for (int e = 0; e < CE; e++) acc[r][e & 1] = fmaf(w[e], x[e], acc[r][e & 1]);
+        }
       }
-      a[r] = block_sum(acc, red) * f;
     }
-    if (tid == 0) rg_emit(p, b * u, a[0], a[1], p.epi == 1 ? p.y[b] : 0.f);
+    if (ng != rg) {
+      float a[R];
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        a[r] = warp_sum(acc[r][0] + acc[r][1]);
+        acc[r][0] = acc[r][1] = 0.f;
+      }
+      if (lane == 0) {
+        if (ks == 1) {
+          rs_emit<R>(p, rg, a);
+        } else {
+#pragma unroll
+          for (int r = 0; r < R; r++) part[((loc * ns + stream) * R + r) * ks + sub] = a[r];
+        }
+      }
+      loc++;
+    }
+    rg = ng;
+    cb = nb;
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+      for (int u = 0; u < U; u++) cur[r][u] = nxt[r][u];
   }
+  if (ks == 1) return;
+  __syncthreads();
+  for (int i = tid;; i += RG_THREADS) {
+    const int l = i / ns, g = (blockIdx.x * ns + i - l * ns) + l * stride;
+    if (l * stride + (int)blockIdx.x * ns >= groups) break;
+    if (g >= groups) continue;
+    float a[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      a[r] = 0.f;
+      for (int k = 0; k < ks; k++) a[r] += part[(i * R + r) * ks + k];
+    }
+    rs_emit<R>(p, g, a);
+  }
+}
+
+template <typename WT, int R>
+int rs_launch(DeviceCtx* c, const RowGemv& p, cudaStream_t s) {
+  static std::atomic<unsigned long long> done{0};
+  const int rc = ensure_dynamic_smem(row_gemv_stream_kernel<WT, R>, RS_SMEM_MAX, done);
+  if (rc) return rc;
+  const int groups = (p.N + R - 1) / R, chunks = (int)(p.ldw / Vec16<WT>::N), full = 2 * c->sm_count;
+  // warps a stream (single rows): the fewest that come within 3 % of the most even division
+  int ks = 1;
+  double best = 1e30;
+  for (int k = 1; k <= RG_WARPS; k *= 2) {
+    if (k > 1 && chunks / k < 32 * 4) break;
+    const int ns = RG_WARPS / k;
+    const double cost = (double)((groups + full * ns - 1) / (full * ns)) / k;
+    if (cost < best * 0.97) { best = cost; ks = k; }
+    if (R == 2) break;   // two rows a warp: the extra sums cost more than the unevenness
+  }
+  auto blocks = [&] {
+    const int ns = RG_WARPS / ks, need = (groups + ns - 1) / ns;
+    return need < full ? need : full;
+  };
+  auto bytes = [&] {   // the row and, of streams of several warps, their partial sums
+    const int ns = RG_WARPS / ks, all = blocks() * ns, local = (groups + all - 1) / all;
+    return ((size_t)p.ldw + (ks > 1 ? (size_t)local * ns * R * ks : 0)) * sizeof(float);
+  };
+  if (bytes() > RS_SMEM_MAX) ks = 1;
+  const int ctas = blocks();
+  const size_t smem = bytes();
+  if (smem > RS_SMEM_MAX) return set_error(TLB_ERR_UNSUPPORTED, "row_gemv: the activation row does not fit the shared-memory stage");
+  LaunchCfg lc(dim3(ctas), dim3(RG_THREADS), smem, s, pdl_enabled());
+  TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, row_gemv_stream_kernel<WT, R>, p, ks));
+  return TLB_OK;
 }
 
 template <typename WT, int JN>
@@ -413,14 +552,9 @@ int rg_plan_launch(DeviceCtx* c, const RowGemv& p, cudaStream_t s) {
   while (pl.stages > 2 && pl.stages * stage + tail > RG_SMEM_SHARED) pl.stages--;
   const size_t smem = pl.stages * stage + tail;
   if (!jn || !vec || smem > RG_SMEM_MAX) {
-    const size_t bytes = ((size_t)p.ldw + groups) * sizeof(float);
-    if (bytes > 225 * 1024) return set_error(TLB_ERR_UNSUPPORTED, "row_gemv: the activation row does not fit the shared-memory stage");
-    static std::atomic<unsigned long long> done{0};
-    const int rc = ensure_dynamic_smem(row_gemv_long_kernel<WT>, 225 * 1024, done);
-    if (rc) return rc;
-    LaunchCfg lc(dim3(ctas), dim3(RG_THREADS), bytes, s, pdl_enabled());
-    TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, row_gemv_long_kernel<WT>, p));
-    return TLB_OK;
+    // two rows a stream where the rows come in pairs, or where there are enough of them to fill the SMs
+    const bool two = p.epi == 2 || p.N >= 2 * 2 * c->sm_count * RG_WARPS;
+    return two ? rs_launch<WT, 2>(c, p, s) : rs_launch<WT, 1>(c, p, s);
   }
   if (jn == 1) return rg_launch<WT, 1>(p, pl, ctas, smem, s);
   if (jn == 2) return rg_launch<WT, 2>(p, pl, ctas, smem, s);
