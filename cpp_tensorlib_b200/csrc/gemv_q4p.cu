@@ -596,7 +596,9 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
     }
     return p.alpha * (1.0f / sqrtf(tot / (float)p.K + p.eps));
   };
-  auto emit = [&](int n, float v, float alpha_n) {
+  float alpha_n = 0.f;
+  bool scaled = false;
+  auto emit = [&](int n, float v) {
     v = v * alpha_n + p.beta;
     if (PUSH) {
       for (int r = 0; r < p.comm.size; r++) st_packet_sys(&p.comm.stage[r][ar_off + n], v, ar_seq + 1u);
@@ -605,7 +607,7 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
     }
   };
   // pair index pi of a pair-packed matrix, a = its first row's sum, b = its second's
-  auto emit_pair = [&](int pi, float a, float b, float alpha_n, bool here) {
+  auto emit_pair = [&](int pi, float a, float b, bool here) {
     a = a * alpha_n + p.beta;
     b = b * alpha_n + p.beta;
     if (EPI == 1) {
@@ -691,14 +693,17 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
     const unsigned t0 = (unsigned)rt * SL, t1 = t0 + SL;
     const bool complete = (u0 <= t0) && (u1 >= t1);
     const int r0 = rt * 16;
-    const float alpha_n = scale_of();
+    if (!scaled) {   // once a warp, not for every row tile of its range
+      alpha_n = scale_of();
+      scaled = true;
+    }
     if (complete) {
       if (t == 0) {
         if (EPI) {
-          emit_pair(rt * 8 + g, v0, v1, alpha_n, false);
+          emit_pair(rt * 8 + g, v0, v1, false);
         } else {
-          if (r0 + g < p.N) emit(r0 + g, v0, alpha_n);
-          if (r0 + g + 8 < p.N) emit(r0 + g + 8, v1, alpha_n);
+          if (r0 + g < p.N) emit(r0 + g, v0);
+          if (r0 + g + 8 < p.N) emit(r0 + g + 8, v1);
         }
       }
       return;
@@ -733,11 +738,11 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
 #pragma unroll
         for (int k = 0; k < 16; k++) s += pv[k];
       }
-      if (!EPI && r0 + lane < p.N) emit(r0 + lane, s, alpha_n);
+      if (!EPI && r0 + lane < p.N) emit(r0 + lane, s);
     }
     if (EPI) {
       const float s2 = __shfl_down_sync(0xffffffffu, s, 8);   // row lane + 8 of the tile
-      if (lane < 8) emit_pair(rt * 8 + lane, s, s2, alpha_n, false);
+      if (lane < 8) emit_pair(rt * 8 + lane, s, s2, false);
     }
     if (lane == 0) p.counters[rt] = 0;  // leave the counter clean for the next launch
   };
@@ -825,7 +830,7 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
   if (own) {
     __syncthreads();
     const int ntl = n_loc / ks;   // row tiles of this block
-    const float alpha_n = scale_of();
+    alpha_n = scale_of();
     // one thread per output row: fold the row's unit results in slab order
     if (EPI) {
       // one thread per pair: rows (lr, lr + 8) of a tile (whole rows only: KB == 1)
@@ -844,7 +849,7 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
 #pragma unroll
           for (int k = 0; k < 4; k++) { sa += qa[k]; sb += qb[k]; }
         }
-        emit_pair((tile_b + tl) * 8 + lr, sa, sb, alpha_n, ep_here && idx == tid);
+        emit_pair((tile_b + tl) * 8 + lr, sa, sb, ep_here && idx == tid);
       }
       return;
     }
@@ -862,7 +867,7 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
       }
       const int n = (tile_b + tl) * 16 + row;
       if (KB == 1) {
-        if (n < p.N) emit(n, sum, alpha_n);
+        if (n < p.N) emit(n, sum);
       } else {
         __stcg(p.partials + ((size_t)kb * p.RT + tile_b + tl) * 16 + row, sum);
       }
@@ -888,7 +893,7 @@ __device__ __forceinline__ void gemv_q4p_body(const GemvPParams& p, const GvCurs
 #pragma unroll
         for (int k = 0; k < 8; k++) sum += pv[k];
       }
-      if ((int)off < p.N) emit((int)off, sum, alpha_n);
+      if ((int)off < p.N) emit((int)off, sum);
     }
     if (tid == 0) p.counters[rb] = 0;  // clean for the next launch
     return;
