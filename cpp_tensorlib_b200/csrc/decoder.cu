@@ -506,7 +506,7 @@ int Decoder::prefill_pass(const int* d_ids, int rows, int pos, cudaStream_t s) {
     PF(launch_qkv_rows(qkv, L.bq, L.bk, L.bv, L.Kc, L.Vc, rows, NQ, NKV, D, pos, max_ctx, rope_base, kv_bf16, s));
     PF(launch_attn_prefill_rows(c, qkv, QKV, L.Kc, L.Vc, at, NQ, NKV, rows, max_ctx, D, scale, pos, kv_bf16, s));
     if (planes(L.wo)) {
-      PF(launch_split_rows(at, NQ * D, rows, NQ * D, q4_planes_at(pf_planes, rows, NQ * D), s));
+      PF(launch_split_rows(at, NQ * D, rows, NQ * D, q4_planes_at(pf_planes, rows, NQ * D), c->sm_count, s));
       PF(gemm_planes(L.wo, md));
     } else {
       PF(gemm(L.wo, at, md, rows));

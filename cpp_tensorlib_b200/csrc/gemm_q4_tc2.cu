@@ -518,8 +518,10 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
 // X -> two fp16 planes of x * 2^-e_m (hi, lo) + the row's 2^e_m.  One block per row.  Inside every
 // group of 8 k the planes are stored in the order 0,4,1,5,2,6,3,7 -- the order in which the
 // converters' nibble extraction lays out the weights.
-__global__ void split_f16_kernel(const float* __restrict__ x, long long ldx, int K, __half* __restrict__ x1,
-                                 __half* __restrict__ x2, float* __restrict__ rowscale) {
+constexpr int SPLIT_MOST = 1024;   // threads a row
+__global__ void __launch_bounds__(SPLIT_MOST)
+    split_f16_kernel(const float* __restrict__ x, long long ldx, int K, __half* __restrict__ x1, __half* __restrict__ x2,
+                     float* __restrict__ rowscale) {
   __shared__ float sm[32];
   pdl_wait();
   pdl_launch_dependents();
@@ -609,13 +611,13 @@ int gemm_q4_tc2_launch(DeviceCtx* c, const float* x, long long ldx, int M, const
                        float* y, long long ldy, int N, int K, float alpha, float beta, void* scratch,
                        void* work, cudaStream_t stream) {
   const Q4Planes pl = q4_planes_at(scratch, M, K);
-  const int rc = launch_split_rows(x, ldx, M, K, pl, stream);
+  const int rc = launch_split_rows(x, ldx, M, K, pl, c->sm_count, stream);
   return rc ? rc : gemm_q4_planes_launch(c, pl, M, qw, scales, y, ldy, N, K, alpha, beta, work, stream);
 }
 
-int launch_split_rows(const float* x, long long ldx, int M, int K, const Q4Planes& pl, cudaStream_t stream) {
+int launch_split_rows(const float* x, long long ldx, int M, int K, const Q4Planes& pl, int sms, cudaStream_t stream) {
   // few deep rows: more threads a row, since there are fewer rows than SMs (8 x 18944, split and product: 41.8 -> 32.5 us)
-  const int threads = M <= 148 && K >= 4096 ? 1024 : 256;
+  const int threads = M <= sms && K >= 4096 ? SPLIT_MOST : 256;
   LaunchCfg lc(dim3((unsigned)M), dim3(threads), 0, stream, pdl_enabled());
   TLB_CUDA(cudaLaunchKernelEx(&lc.cfg, split_f16_kernel, x, ldx, K, pl.hi, pl.lo, pl.rowscale));
   return TLB_OK;

@@ -32,8 +32,8 @@ bool gemm_q4_planes_eligible(const void* qw, const void* scales, int N, int K, i
 bool gemm_q4_planes_possible(const void* qw, const void* scales, int N, int K, int M);
 int gemm_q4_planes_launch(DeviceCtx* c, const Q4Planes& x, int M, const void* qw, const float* scales, float* y,
                           long long ldy, int N, int K, float alpha, float beta, void* work, cudaStream_t stream);
-// x f32 rows -> planes
-int launch_split_rows(const float* x, long long ldx, int M, int K, const Q4Planes& pl, cudaStream_t stream);
+// x f32 rows -> planes, on a device of `sms` SMs
+int launch_split_rows(const float* x, long long ldx, int M, int K, const Q4Planes& pl, int sms, cudaStream_t stream);
 
 #ifdef __CUDACC__
 
