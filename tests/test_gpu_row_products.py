@@ -25,3 +25,22 @@ def test_row_products(width, ff, dtype):
     got = run(m, toks, [])
     assert np.isfinite(got).all() and ok(err(got, want), dtype)
     close(m)
+
+
+def test_longest_row():
+    """The longest row that a block holds, without room for the partial sums of split rows, and one beyond."""
+    from cpp_tensorlib_b200 import TlbError
+    for ff in (57600, 57608):
+        cfg = zc.config([zc.mam(6, 2, 16, 24, 4, 3, ff=ff)], width=64, vocab=151, emb=1.0)
+        w = zc.Weights(cfg, 5)
+        toks = zc.tokens(cfg, 3, 2)
+        m = make(cfg, w, "bfloat16", 16)
+        if ff > 57600:
+            with pytest.raises(TlbError, match="does not fit"):
+                run(m, toks, [])
+            m.close()
+            continue
+        want = orc.forward(cfg, w.f64(), toks)
+        got = run(m, toks, [])
+        assert np.isfinite(got).all() and ok(err(got, want), "bfloat16")
+        close(m)
