@@ -32,6 +32,8 @@ namespace tlb {
 namespace {
 
 constexpr int RC_MOST = 8;   // segments
+// CTAs of both ssd kernels that an SM holds, and the most of them an SM that segments may come to: under three rounds
+constexpr int RC_PLACES = 3, RC_CTAS_MOST = 8;
 constexpr int RC_L = 64, RC_E = 32, RC_THREADS = 128;
 constexpr int RC_TLD = RC_L + 8, RC_ELD = RC_E + 8;
 
@@ -531,7 +533,7 @@ struct ScSmem {
 };
 
 template <int DP>
-__global__ void __launch_bounds__(RC_THREADS, 3)
+__global__ void __launch_bounds__(RC_THREADS, RC_PLACES)
     ssd_chunk_kernel(const __grid_constant__ RecurP p, const __nv_bfloat16* __restrict__ conv,
                      const float2* __restrict__ gates, float* __restrict__ o, int rows, int pos0,
                      const __grid_constant__ RcSegments g) {
@@ -784,7 +786,7 @@ struct SsSmem {
 };
 
 template <int DP>
-__global__ void __launch_bounds__(RC_THREADS, 3)
+__global__ void __launch_bounds__(RC_THREADS, RC_PLACES)
     ssd_state_kernel(const __grid_constant__ RecurP p, const __nv_bfloat16* __restrict__ conv,
                      const float2* __restrict__ gates, int pos0, const __grid_constant__ RcSegments g) {
   using SM = SsSmem<DP>;
@@ -901,23 +903,24 @@ __global__ void __launch_bounds__(RC_THREADS, 3)
 }
 
 // Most segments of a prompt (more rows, no fewer): of four chunks at least, since a segment's start reads the states in
-// front of it, eight at most, and no more than four CTAs for each of two places an SM.
+// front of it, RC_MOST, and RC_CTAS_MOST CTAs an SM.
 int rc_most_segments(const RecurP& p, int rows, int sms) {
   const int nch = (rows + RC_L - 1) / RC_L, ctas = (p.E + RC_E - 1) / RC_E * p.H;
   int n = nch / 4 < RC_MOST ? nch / 4 : RC_MOST;
-  if (n * ctas > 4 * 2 * sms) n = 4 * 2 * sms / ctas;
+  if (n * ctas > RC_CTAS_MOST * sms) n = RC_CTAS_MOST * sms / ctas;
   return n < 2 ? 1 : n;
 }
-// Up to that many, by what they cost: both kernels run in waves of three CTAs an SM, a wave as long as a segment's chunks
-// and a start of 1.5 chunks; a chunk of ssd_state takes 0.3 of one of ssd_chunk.  4096 tokens, 64 heads of 128 x 64, the
-// 8-layer prompt pass with six such layers, us: 2 segments 6931, 3 6470, 4 6816, 6 6536, 8 6610, 10 6527, 13 6674, 16 6884.
+// Up to that many, by what they cost: both kernels run in waves of RC_PLACES CTAs an SM, a wave as long as a segment's
+// chunks and a start of 1.5 chunks; a chunk of ssd_state takes 0.3 of one of ssd_chunk.  4096 tokens, 64 heads of 128 x 64,
+// the 8-layer prompt pass with six such layers, us, the number set by hand: 2 segments 6931, 3 (the rule's) 6470, 4 6816,
+// 6 6536, 8 6610, and beyond RC_MOST, which such a number does not repay in scratch, 10 6527, 13 6674, 16 6884.
 RcSegments rc_segments(const RecurP& p, int rows, int sms, void* scratch) {
   const int nch = (rows + RC_L - 1) / RC_L, most = rc_most_segments(p, rows, sms), ctas = (p.E + RC_E - 1) / RC_E * p.H;
   RcSegments g{1, nch, nullptr, nullptr};
   long long best = 0;
   for (int want = 1; want <= most; want++) {
     const int chunks = (nch + want - 1) / want, n = (nch + chunks - 1) / chunks;
-    auto waves = [&](int segments) { return ((long long)segments * ctas + 3 * sms - 1) / (3 * sms); };
+    auto waves = [&](int segments) { return ((long long)segments * ctas + RC_PLACES * sms - 1) / (RC_PLACES * sms); };
     const long long cost = (10 * waves(n) + 3 * waves(n - 1)) * (2 * chunks + 3);
     if (want > 1 && cost >= best) continue;
     best = cost;
