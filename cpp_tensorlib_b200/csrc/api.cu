@@ -324,7 +324,9 @@ static int skinny_rows(const void* qw, const void* scales, int N, int K, int mos
 }
 // Up to 8 rows that would take three or more launches of the skinny kernel, each streaming all weights, are one
 // product on planes instead: 8 x 18944 x 3584 144 -> 32 us, 3 x 18944 x 3584 54 -> 32, 5 x 11008 x 4096 48 -> 25.  One
-// launch costs less than the planes (8 x 3584 x 18944: 24 us, 26 for up to 32 rows on planes).  By the shape
+// launch costs less than the planes (8 x 3584 x 18944: 24 us, 26 for up to 32 rows on planes).  Two launches cost more (8 rows:
+// 4864 x 896 18.5 us, 14.5 on planes; 4864 x 4096 25.6, 16.9; 4864 x 18944 45.0, 31.0; 4 rows: 8192 x 896 17.7, 14.5; 2 rows:
+// 18944 x 3584 35.2, 32.3) and stay skinny for its scale of every 256 k: see below.  By the shape
 // alone, with scratch that is made with the context and never moves: such a call allocates nothing, gives the same bits
 // under capture, and a graph of it stays valid.  (Rows deeper than that scratch holds, 131000 at 8 rows, stay skinny.)
 // The planes have one power of two a row where the skinny kernel has one for every 256 k: an element 2^15 or more

@@ -11,7 +11,7 @@
 // (K = 16 each) instead of 12 kind::tf32 MMAs at half the rate: a sixth of the tensor time of
 // the formulation that folds the f32 scale into the weight operand (gemm_q4_tc.cu), which is
 // tensor bound at a third of the tf32 peak.  Each group's product lands in one of four TMEM
-// accumulators used in rotation; accumulate warps read it back with tcgen05.ld, multiply by
+// accumulators (three at 128 columns) used in rotation; accumulate warps read it back with tcgen05.ld, multiply by
 // the row's f32 group scale and add into registers -- the same order of operations as the
 // reference's dequantise-then-multiply in f32 (include/array.h:666-684, 1980-1984).
 //

@@ -9,7 +9,8 @@
 //  * Work unit = 16 weight rows x 256 k (2 KB of nibbles + 512 B of scales).
 //    Units are numbered row-tile-major and dealt out in equal contiguous ranges
 //    to every warp of a persistent grid, so the load balance does not depend on
-//    the matrix shape.  Each warp owns a private ring of TMA stages
+//    the matrix shape; of small matrices a block owns whole row tiles instead
+//    (p.own).  Each warp owns a private ring of TMA stages
 //    (cp.async.bulk.tensor, 128-byte swizzle) with one mbarrier per stage: no
 //    block-wide barrier sits in the streaming loop and ~100 KB per SM stay in
 //    flight.
@@ -563,7 +564,7 @@ int make_q4_tensor_maps(const void* qw, const void* scales, int N, int K, CUtens
 }
 
 // Kernel shape for a problem: 8 warps x 4 stages when two CTAs fit on an SM,
-// else 16 warps x 3 stages.
+// else 16 warps x 3 stages, or x 2 for five to eight rows that leave no room for three.
 static void gemv_pick(int M, int K, int* warps, int* stages) {
   if (const char* e = getenv("TLB_GEMV_CFG")) {  // diagnostics: "16x3" / "16x4"
     if (!strcmp(e, "16x3")) { *warps = 16; *stages = 3; return; }
