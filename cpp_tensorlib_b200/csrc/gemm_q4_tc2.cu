@@ -27,7 +27,7 @@
 // owns weight row r; the k order inside every group of 8 is the one the nibble extraction produces -- 0,4,1,5,2,6,3,7 -- and
 // the X planes are stored in the same order, so no byte permute is needed), warps 8-15 accumulate + epilogue (two per TMEM
 // lane quarter, each half of the MT columns).  The converters leave the weights in TMEM, a lane a row: the A operand of the
-// MMAs comes from there.  The feeding warpgroups give registers to the accumulating ones.  All waits are bounded; a timeout
+// MMAs comes from there.  At 128 columns the feeding warpgroups give registers to the accumulating ones.  All waits are bounded; a timeout
 // sets the status word, the kernel still frees its TMEM and returns, and no warp is split by it.  No cluster launch, no
 // multicast.
 //
@@ -55,8 +55,11 @@ constexpr int T2_ROWS = 128;     // weight rows per CTA (UMMA M)
 constexpr int T2_KS = 64;        // k per stage = two groups = one 128-byte swizzle row of fp16
 constexpr int T2_RAW_BYTES = T2_ROWS * 128;   // one box: 128 rows x 128 bytes = 256 k per row
 constexpr int T2_SUB = 4;                     // 64-k stages per packed box
-// registers a thread of the two warpgroups that feed the tensor pipe, and of the two that accumulate: 256 (72 + 184) =
-// what 512 threads of 128 are launched with
+// Registers a thread of the two warpgroups that feed the tensor pipe, and of the two that accumulate: 256 (72 + 184) =
+// what 512 threads of 128 are launched with.  At 128 columns alone: up to 64 the accumulators fit 108 registers a thread, and
+// what that leaves of an SM's takes the first blocks of the next launch (the split of its rows).  Products on all SMs, one
+// behind the other, us with the exchange / without: 64 x 3584 x 3584 19.3 / 17.5, 16 rows 16.2 / 14.5, 64 x 3584 x 4608
+// 20.0 / 18.2; where the split takes 1024 threads a row, or SMs are idle anyway, nothing (64 x 18944 x 3584 38.0 / 38.2).
 constexpr int T2_REGS_FEED = 72, T2_REGS_ACC = 184;
 
 struct T2Params {
@@ -278,7 +281,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
   pdl_launch_dependents();
 
   if (warp < 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(T2_REGS_FEED));
+    if constexpr (MT == 128) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(T2_REGS_FEED));
   if (warp == 3) {
     // ---------------- TMA producer: packed weights, 128 rows x 256 k per box ----------------
     if (lane == 0) {
@@ -402,7 +405,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
   }
   } else {
     // ---------------- accumulate (sc * group product) + epilogue ----------------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(T2_REGS_ACC));
+    if constexpr (MT == 128) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(T2_REGS_ACC));
     const int quarter = warp & 3, half = (warp - 8) >> 2;
     const int r = quarter * 32 + lane;
     const int c_lo = half * HC;
