@@ -640,8 +640,8 @@ int gemv_q4_launch(DeviceCtx* c, const CUtensorMap& tmW, const CUtensorMap& tmS,
   if (ctas > need) ctas = need;
   if (ctas * warps > c->gemv_max_workers) ctas = c->gemv_max_workers / warps;
   // Block-owned row tiles where that leaves a warp at most two units and a tile has several to add: the partials and the
-  // ticket in global memory cost about a microsecond (in a graph, 1 x 896 x 4864: 5.66 -> 4.67 us, 1 x 896 x 896: 4.79 ->
-  // 3.69, 1 x 3584 x 4608: 8.36 -> 6.84, 8 x 896 x 4864: 8.20 -> 6.69; a tile of one unit, 1 x 128 x 16, would lose:
+  // ticket in global memory cost about a microsecond (in a graph, 1 x 896 x 4864: 5.69 -> 4.40 us, 1 x 896 x 896: 4.86 ->
+  // 3.58, 1 x 3584 x 4608: 8.36 -> 6.60, 8 x 896 x 4864: 8.15 -> 6.32; a tile of one unit, 1 x 128 x 16, would lose:
   // 3.04 -> 3.78, there is nothing to add).
   p.own = 0;
   if (max_ctas <= 0 && !p.push && p.SL > 1) {
